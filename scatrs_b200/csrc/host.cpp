@@ -146,10 +146,13 @@ struct DevBuf {
   size_t cap = 0;
   void* get(size_t bytes) {
     if (bytes > cap) {
+      // Regrown with room to spare (half, at most 64 MiB), so that calls of slightly varying
+      // sizes settle instead of freeing and allocating (0.1 to 1 ms each) again and again.
+      size_t want = std::max<size_t>(bytes, 1 << 16);
+      if (cap > 0) want = std::max(want, bytes + std::min<size_t>(bytes / 2, 64u << 20));
       if (p) cudaFree(p);
       p = nullptr;
       cap = 0;
-      size_t want = std::max<size_t>(bytes, 256);
       if (g_fail_allocation.load() > 0 && g_fail_allocation.fetch_sub(1) == 1)
         throw Failure{SCATRS_CUDA, std::string("cudaMalloc(&p, want): ") +
                                        cudaGetErrorString(cudaErrorMemoryAllocation)};
@@ -176,16 +179,27 @@ struct UserTables {
   std::vector<double> rows;  // each table row's cosine (a cosine, or a pair c, -c)
   int64_t n_orders = 0;
   int h = 0, h_pad = 0, ld = 0;
-  DevBuf ge, go, map;
+  DevBuf ge, go, map, rows_d;
 };
 
+// The tables of one Greek order (-1: none): the phase levels the requested cosines allow (see
+// chunk_band; none where the limit is 0), then the projector bands. The bands' G_E and G_O rows
+// are host-made (ge_d, go_d), the levels' made on the device (lge_d, lgo_d).
 struct BandTables {
   int order = -1;
-  int n_bands = 0;
-  int nq_max = 0;
-  std::vector<BandDesc> desc;
+  int n_levels = 0;
+  int n_bands = 0;                // projector bands
+  std::vector<BandDesc> desc;     // the levels, then the bands
+  std::vector<BandDesc> bands;
   std::vector<double> ge, go, d;  // host copies, appended band by band
-  DevBuf ge_d, go_d, d_d, desc_d;
+  std::vector<int> half0;         // each level's first half node
+  std::vector<double> mu;         // the cosines me_d and mo_d interpolate onto
+  DevBuf ge_d, go_d, lge_d, lgo_d, d_d, desc_d, half0_d, x0_d, node_d, me_d, mo_d;
+  int merge_max() const { return n_levels > 0 ? desc[n_levels - 1].upper : 0; }
+  void release() {
+    for (DevBuf* b : {&ge_d, &go_d, &lge_d, &lgo_d, &d_d, &desc_d, &half0_d, &x0_d, &node_d, &me_d, &mo_d})
+      b->release();
+  }
 };
 
 struct Context {
@@ -194,10 +208,10 @@ struct Context {
   int unit_bps = 1;
   std::mutex mtx;
   UserTables user;
-  std::map<int, BandTables> bands;  // by Greek order
+  std::map<std::pair<int, int>, BandTables> bands;  // by Greek order and level limit
   std::map<int64_t, std::pair<std::vector<double>, std::vector<double>>> rules;
   DevBuf radius, weight, wtheta, wthdiff, wdiff, unit_norm, wl, m, fractions, chunk_n, chunk_n_slab, chunk_row, chunk_acc, plan_units,
-      unit_acc, unit_slots, slots, items, proj_items, slot_index, slot_greek, X, uz, ux,
+      unit_acc, unit_slots, slots, items, proj_items, slot_index, slot_greek, slot_phase, X, uz, ux,
       chunk_sums, err, acc, counter, values, phase, greek;
   // Pass 1 of the adaptive ensemble.
   DevBuf p1_radius, p1_wl, p1_wlu, p1_scratch, p1_uz, p1_ux, p1_q, p1_n, p1_status;
@@ -214,7 +228,7 @@ struct Context {
     std::vector<double> mu;
     int64_t user_orders = 0;
     int order = -2;
-    int n_bands = 0;
+    int n_bands = 0, n_levels = 0;
     std::vector<I8Table> user, band;
     DevBuf dig, scale, user_d, band_d;
   } i8;
@@ -364,32 +378,106 @@ void ensure_user(Context& c, const double* mu, int64_t n_mu, int64_t n_orders, c
   if (!map.empty())
     SB_CUDA(cudaMemcpyAsync(u.map.get(map.size() * sizeof(int2)), map.data(),
                             map.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
+  if (!cosines.empty())
+    SB_CUDA(cudaMemcpyAsync(u.rows_d.get(cosines.size() * 8), cosines.data(), cosines.size() * 8,
+                            cudaMemcpyHostToDevice, s));
   SB_CUDA(cudaStreamSynchronize(s));
 }
 
-// Bands 0..last_band for Greek order L (engine.rs:2034-2072).
-BandTables& ensure_bands(Context& c, int L, int last_band, cudaStream_t s) {
-  BandTables& bt = c.bands[L];
+// The level limit of the fixed grid for h_u requested rows and Greek order L: a level of t tiles
+// is used while it runs fewer tiles than the requested rows and its largest chunk's projector
+// band. A unit's interpolation from the level costs about h_u / 1024 of the tiles it replaces per
+// chunk (2 h_u h multiply-adds per element against 8 x 32 x 32 per tile row and order), counted
+// twice as it runs at a lower rate. The levels' interpolation matrices stay below 1 GiB. Returns
+// the tiles of the last level, 0 for none.
+int level_limit(int h_u, int L) {
+  const int t_user = (h_u + 31) / 32;
+  int last = 0, n = 0;
+  double bytes = 0.0;
+  for (int t = 1; h_u > 0 && n < kMaxLevels; t = next_level_tiles(t), ++n) {
+    const int64_t upper = 32 * (int64_t)t - 1;
+    int64_t direct = t_user;
+    if (L >= 0) {
+      const int64_t u = bucket(upper), n_q = u + (std::min<int64_t>(L, 2 * u) + 2) / 2;
+      direct += ((n_q + 1) / 2 + 31) / 32;
+    }
+    bytes += 2.0 * 8.0 * 32.0 * t * round_up(h_u, 32);
+    if (!(t + h_u / 512.0 < (double)direct) || bytes > 1073741824.0) break;
+    last = t;
+  }
+  return last;
+}
+
+// The projection matrices (2l+1)/2 w_k d_l(mu_k) of d00, d22, d2-2 and d02 at a rule's nodes.
+void append_projection(const std::pair<std::vector<double>, std::vector<double>>& r, int64_t n_q,
+                       int64_t len, std::vector<double>& d) {
+  const size_t off = d.size();
+  const int64_t ld = round_up(len, 32);
+  d.resize(off + 4 * (size_t)n_q * ld, 0.0);
+  std::vector<double> buf(len);
+  const int mn[4][2] = {{0, 0}, {2, 2}, {2, -2}, {0, 2}};
+  for (int f = 0; f < 4; ++f)
+    for (int64_t k = 0; k < n_q; ++k) {
+      wigner_d(mn[f][0], mn[f][1], r.first[k], buf.data(), len);
+      double* dst = &d[off + ((size_t)f * n_q + k) * ld];
+      for (int64_t l = 0; l < len; ++l) dst[l] = (double)(2 * l + 1) * 0.5 * r.second[k] * buf[l];
+    }
+}
+
+// The tables for chunks of up to n_max terms and Greek order L (engine.rs:2034-2072): phase
+// levels up to `limit` tiles (0: none), projector bands for the chunks beyond them.
+BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream_t s) {
+  constexpr size_t kMaxLevelSets = 8;  // (Greek order, limit) pairs with levels kept
+  if (limit > 0 && !c.bands.count({L, limit})) {
+    size_t sets = 0;
+    for (auto& kv : c.bands) sets += kv.first.second > 0;
+    if (sets >= kMaxLevelSets)
+      for (auto it = c.bands.begin(); it != c.bands.end();) {
+        if (it->first.second > 0) {
+          it->second.release();
+          it = c.bands.erase(it);
+        } else {
+          ++it;
+        }
+      }
+  }
+  BandTables& bt = c.bands[{L, limit}];
   bt.order = L;
-  if (bt.n_bands > last_band) return bt;
-  for (int b = bt.n_bands; b <= last_band; ++b) {
+  int need_levels = 0;
+  int64_t reach = 0;
+  for (int t = 1; t <= limit && reach < n_max; t = next_level_tiles(t), ++need_levels)
+    reach = 32 * (int64_t)t - 1;
+  int need_bands = L >= 0 && n_max > reach ? band_index(n_max) + 1 : 0;
+  if (bt.n_levels >= need_levels && bt.n_bands >= need_bands) return bt;
+  // Built for half as many terms again (levels), a quarter (bands), so that slightly larger
+  // inputs find them ready.
+  if (need_bands > 0) need_bands += 1;
+  for (int64_t at = reach; reach < limit * 32 - 1 && reach < at + at / 2; ++need_levels) {
+    int t = 1;
+    for (int l = 0; l < need_levels; ++l) t = next_level_tiles(t);
+    reach = 32 * (int64_t)t - 1;
+  }
+  const int n_levels = std::max(bt.n_levels, need_levels);
+  const int64_t merge_max = limit > 0 ? 32 * (int64_t)limit - 1 : 0;
+  for (int b = bt.n_bands; b < need_bands; ++b) {
     int64_t upper = band_upper(b);
     int64_t order = std::min<int64_t>(L, 2 * upper);
     int64_t n_q = upper + (order + 2) / 2;
-    const auto& r = rule(c, n_q);
-    BandDesc d;
+    BandDesc d{};
     d.upper = (int)upper;
     d.order = (int)order;
-    d.n_q = (int)n_q;
-    int64_t lo = n_q / 2;
-    d.h = (int)(n_q - lo);
-    d.h_pad = (int)round_up(d.h, 32);
-    d.ld = (int)round_up(upper, 16);
-    d.g_off = (int64_t)bt.ge.size();
-    d.d_off = (int64_t)bt.d.size();
-    bt.ge.resize(bt.ge.size() + (size_t)d.h_pad * d.ld, 0.0);
-    bt.go.resize(bt.go.size() + (size_t)d.h_pad * d.ld, 0.0);
-    {
+    if (upper > merge_max) {  // the others' chunks are on a level
+      const auto& r = rule(c, n_q);
+      d.n_q = (int)n_q;
+      int64_t lo = n_q / 2;
+      d.h = (int)(n_q - lo);
+      d.h_pad = (int)round_up(d.h, 32);
+      d.d_ld = (int)round_up(order + 1, 32);
+      d.ld = (int)round_up(upper, 16);
+      d.g_off = (int64_t)bt.ge.size();
+      d.d_off = (int64_t)bt.d.size();
+      bt.ge.resize(bt.ge.size() + (size_t)d.h_pad * d.ld, 0.0);
+      bt.go.resize(bt.go.size() + (size_t)d.h_pad * d.ld, 0.0);
       // Order-major, as the requested cosines' tables.
       std::vector<double> re(upper), ro(upper);
       for (int i = 0; i < d.h; ++i) {
@@ -399,31 +487,98 @@ BandTables& ensure_bands(Context& c, int L, int last_band, cudaStream_t s) {
           bt.go[d.g_off + (size_t)k * d.h_pad + i] = ro[k];
         }
       }
+      append_projection(r, n_q, order + 1, bt.d);
     }
-    int64_t len = order + 1;
-    bt.d.resize(bt.d.size() + 4 * (size_t)n_q * len);
-    std::vector<double> buf(len);
-    const int mn[4][2] = {{0, 0}, {2, 2}, {2, -2}, {0, 2}};
-    for (int f = 0; f < 4; ++f)
-      for (int64_t k = 0; k < n_q; ++k) {
-        wigner_d(mn[f][0], mn[f][1], r.first[k], buf.data(), len);
-        double* dst = &bt.d[d.d_off + ((size_t)f * n_q + k) * len];
-        for (int64_t l = 0; l < len; ++l) dst[l] = (double)(2 * l + 1) * 0.5 * r.second[k] * buf[l];
-      }
-    bt.desc.push_back(d);
-    bt.nq_max = std::max(bt.nq_max, d.n_q);
+    bt.bands.push_back(d);
   }
-  bt.n_bands = last_band + 1;
-  SB_CUDA(cudaMemcpyAsync(bt.ge_d.get(bt.ge.size() * 8), bt.ge.data(), bt.ge.size() * 8,
-                          cudaMemcpyHostToDevice, s));
-  SB_CUDA(cudaMemcpyAsync(bt.go_d.get(bt.go.size() * 8), bt.go.data(), bt.go.size() * 8,
-                          cudaMemcpyHostToDevice, s));
-  SB_CUDA(cudaMemcpyAsync(bt.d_d.get(bt.d.size() * 8), bt.d.data(), bt.d.size() * 8,
-                          cudaMemcpyHostToDevice, s));
-  SB_CUDA(cudaMemcpyAsync(bt.desc_d.get(bt.desc.size() * sizeof(BandDesc)), bt.desc.data(),
-                          bt.desc.size() * sizeof(BandDesc), cudaMemcpyHostToDevice, s));
+  // The levels, kept from the last build while none are added.
+  std::vector<BandDesc> levels(bt.desc.begin(), bt.desc.begin() + bt.n_levels);
+  int64_t g = 0;
+  std::vector<int> half0;
+  std::vector<double> x0;
+  int n_half = 0, t = 1;
+  for (int l = 0; l < n_levels; ++l, t = next_level_tiles(t)) {
+    BandDesc d = l < (int)levels.size() ? levels[l] : BandDesc{};
+    d.upper = 32 * t - 1;
+    d.order = L >= 0 ? (int)std::min<int64_t>(L, 2 * (int64_t)d.upper) : -1;
+    d.n_q = 64 * t - 1;
+    d.h = d.h_pad = 32 * t;
+    d.ld = 32 * t;
+    d.d_ld = (int)round_up(d.order + 1, 32);
+    d.g_off = g;
+    g += (int64_t)d.h_pad * d.ld;
+    const auto& r = rule(c, d.n_q);
+    if (l >= (int)levels.size()) {
+      d.d_off = (int64_t)bt.d.size();
+      if (L >= 0) append_projection(r, d.n_q, d.order + 1, bt.d);
+      levels.push_back(d);
+    } else {
+      levels[l] = d;
+    }
+    half0.push_back(n_half);
+    n_half += d.h;
+    x0.push_back(0.0);
+    for (int i = 1; i < d.h; ++i) x0.push_back(r.first[d.n_q / 2 + i]);
+  }
+  bt.half0 = half0;
+  bt.desc = levels;
+  bt.desc.insert(bt.desc.end(), bt.bands.begin(), bt.bands.end());
+  auto upload = [&](DevBuf& to, const void* from, size_t bytes) {
+    void* p = to.get(std::max<size_t>(bytes, 16));
+    if (bytes > 0) SB_CUDA(cudaMemcpyAsync(p, from, bytes, cudaMemcpyHostToDevice, s));
+  };
+  upload(bt.ge_d, bt.ge.data(), bt.ge.size() * 8);
+  upload(bt.go_d, bt.go.data(), bt.go.size() * 8);
+  upload(bt.d_d, bt.d.data(), bt.d.size() * 8);
+  upload(bt.desc_d, bt.desc.data(), bt.desc.size() * sizeof(BandDesc));
+  if (n_levels > bt.n_levels) {
+    upload(bt.half0_d, half0.data(), half0.size() * sizeof(int));
+    upload(bt.x0_d, x0.data(), x0.size() * 8);
+    double* node = bt.node_d.as<double>(3 * (size_t)n_half);
+    LevelTableArgs la{};
+    la.n_levels = n_levels;
+    la.n_half = n_half;
+    la.bands = bt.desc_d.as<BandDesc>(0);
+    la.half0 = bt.half0_d.as<int>(0);
+    la.x0 = bt.x0_d.as<double>(0);
+    la.x_hi = node;
+    la.x_lo = node + n_half;
+    la.bary = node + 2 * (size_t)n_half;
+    la.ge = bt.lge_d.as<double>((size_t)g);
+    la.go = bt.lgo_d.as<double>((size_t)g);
+    launch_level_tables(la, s);
+    SB_CUDA(cudaGetLastError());
+    g_launches++;
+    bt.mu.clear();  // the interpolation matrices follow the levels
+  }
+  bt.n_levels = n_levels;
+  bt.n_bands = (int)bt.bands.size();
   SB_CUDA(cudaStreamSynchronize(s));
   return bt;
+}
+
+// The levels' interpolation matrices onto the context's requested rows.
+void ensure_interp(Context& c, BandTables& bt, cudaStream_t s) {
+  if (bt.n_levels == 0 || bt.mu == c.user.mu) return;
+  const BandDesc& last = bt.desc[bt.n_levels - 1];
+  const size_t n_half = (size_t)bt.half0.back() + last.h;
+  double* node = bt.node_d.as<double>(0);
+  LevelMatrixArgs la{};
+  la.n_levels = bt.n_levels;
+  la.h_u = c.user.h;
+  la.h_pad = c.user.h_pad;
+  la.bands = bt.desc_d.as<BandDesc>(0);
+  la.half0 = bt.half0_d.as<int>(0);
+  la.x_hi = node;
+  la.x_lo = node + n_half;
+  la.bary = node + 2 * n_half;
+  la.rows = c.user.rows_d.as<double>(0);
+  la.me = bt.me_d.as<double>(n_half * c.user.h_pad);
+  la.mo = bt.mo_d.as<double>(n_half * c.user.h_pad);
+  launch_level_matrices(la, s);
+  SB_CUDA(cudaGetLastError());
+  g_launches++;
+  bt.mu = c.user.mu;
 }
 
 // The digits of one table of the mixed form (kernels.h): pairs [0, h) whose E and O rows over
@@ -486,16 +641,16 @@ I8Table i8_table(int h, int64_t n_orders, int n_kb, Row row, std::vector<unsigne
 
 // The mixed form's digit tables for the requested cosines (versions v = 0, 1, ... covering
 // orders < 64 2^v up to n_max, each row scaled over its version's orders, so that a chunk's
-// rows keep their bits relative to the orders it uses) and for bands 0 .. n_bands - 1 of Greek
-// order L (L < 0: none); cached per context until the cosines, the order or the reach change.
+// rows keep their bits relative to the orders it uses) and for the levels and bands of `bt`
+// (null: none); cached per context until the cosines, the order or the reach change.
 void ensure_i8(Context& c, int64_t n_max, const BandTables* bt, cudaStream_t s) {
   Context::I8Tables& T = c.i8;
   const int L = bt ? bt->order : -1;
-  const int nb = bt ? bt->n_bands : 0;
+  const int nb = bt ? (int)bt->desc.size() : 0, n_levels = bt ? bt->n_levels : 0;
   int n_ver = 1;
   while (((int64_t)kI8KB << (n_ver - 1)) < std::min<int64_t>(n_max, kI8MaxTerms)) ++n_ver;
   if (T.mu == c.user.mu && T.user_orders >= ((int64_t)kI8KB << (n_ver - 1)) && T.order == L &&
-      T.n_bands >= nb)
+      T.n_bands == nb && T.n_levels == n_levels)
     return;
   std::vector<unsigned char> dig;
   std::vector<double> scale;
@@ -511,15 +666,28 @@ void ensure_i8(Context& c, int64_t n_max, const BandTables* bt, cudaStream_t s) 
         [&](int pair, int64_t n, double* e, double* o) { pi_tau_row(cosines[pair], n, e, o); },
         dig, scale));
   }
+  std::vector<double> le, lo;  // the levels' rows, made on the device
+  if (n_levels > 0) {
+    const BandDesc& last = bt->desc[n_levels - 1];
+    const size_t n = (size_t)last.g_off + (size_t)last.h_pad * last.ld;
+    le.resize(n);
+    lo.resize(n);
+    SB_CUDA(cudaMemcpyAsync(le.data(), bt->lge_d.p, n * 8, cudaMemcpyDeviceToHost, s));
+    SB_CUDA(cudaMemcpyAsync(lo.data(), bt->lgo_d.p, n * 8, cudaMemcpyDeviceToHost, s));
+    SB_CUDA(cudaStreamSynchronize(s));
+  }
   for (int b = 0; b < nb; ++b) {
     const BandDesc& d = bt->desc[b];
     const int n_kb = (d.upper + kI8KB - 1) / kI8KB;
+    const bool level = b < n_levels;
+    const double* ge = (level ? le : bt->ge).data() + d.g_off;
+    const double* go = (level ? lo : bt->go).data() + d.g_off;
     T.band.push_back(i8_table(
         d.h, d.upper, n_kb,
         [&](int pair, int64_t n, double* e, double* o) {
           for (int64_t k = 0; k < n; ++k) {
-            e[k] = bt->ge[d.g_off + (size_t)k * d.h_pad + pair];
-            o[k] = bt->go[d.g_off + (size_t)k * d.h_pad + pair];
+            e[k] = ge[(size_t)k * d.h_pad + pair];
+            o[k] = go[(size_t)k * d.h_pad + pair];
           }
         },
         dig, scale));
@@ -538,6 +706,7 @@ void ensure_i8(Context& c, int64_t n_max, const BandTables* bt, cudaStream_t s) 
   T.user_orders = (int64_t)kI8KB << (n_ver - 1);
   T.order = L;
   T.n_bands = nb;
+  T.n_levels = n_levels;
 }
 
 // A distribution's density at r: its closed form, or a tabulated one's interpolation.
@@ -765,8 +934,13 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   // Tables.
   const int L = opt->greek_order;
   ensure_user(c, mu, n_mu, n_max, s);
+  // Phase levels: the fixed grid's sums are linear over the chunks (adaptive calls take each
+  // panel's error in absolute value at the requested cosines).
+  const int limit = ad.on ? 0 : level_limit(c.user.h, L);
   BandTables* bt = nullptr;
-  if (L >= 0) bt = &ensure_bands(c, L, band_index(n_max), s);
+  if (L >= 0 || limit > 0) bt = &ensure_bands(c, L, limit, n_max, s);
+  const int n_levels = bt ? bt->n_levels : 0, merge_max = bt ? bt->merge_max() : 0;
+  if (bt) ensure_interp(c, *bt, s);
   // The mixed form: values of the fixed grid only.
   const int i8_above = (call && !ad.on && !dv.on) ? call->i8_above : 0;
   auto on_i8 = [&](int nc) { return i8_above > 0 && nc > i8_above && nc <= kI8MaxTerms; };
@@ -778,20 +952,17 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     call->i8_err = i8_err;
   }
   // 3. Slabs. Each unit's work: its chunks' rows times the table rows they meet.
-  const int nb = bt ? bt->n_bands : 0;
+  const int nb = bt ? (int)bt->desc.size() : 0;
   std::vector<int> band_of_n(n_max + 1, -1), band_tiles(nb), band_nq(nb);
   if (bt) {
-    int b = 0;
-    for (int n = 1; n <= n_max; ++n) {
-      while (bt->desc[b].upper < n) ++b;
-      band_of_n[n] = b;
-    }
+    for (int n = 1; n <= n_max; ++n) band_of_n[n] = chunk_band(n, merge_max, n_levels, L);
     for (int k = 0; k < nb; ++k) {
       band_tiles[k] = (bt->desc[k].h + 31) / 32;
       band_nq[k] = bt->desc[k].n_q;
     }
   }
   const int t_user = (c.user.h + 31) / 32;
+  const int tile_slots = ad.on ? 32 : kSlotGroup;  // slots per projection item
   const int64_t acc_head = 4 * n_mu * n_blk;
   std::vector<int64_t> urows(n_units), uacc(n_units), ui8(n_units, 0), ui8n(n_units, 0);
   std::vector<int> uslots(n_units), utiles(n_units);
@@ -802,7 +973,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     const int* cu = cn + u * cpu;
     int64_t rows = 0, acc = acc_head;
     double cost = 0.0;
-    int prev = -1, slots = 0, max_tiles = 1;
+    int prev = -1, run = 0, slots = 0, max_tiles = 1;
     for (int k = 0; k < cpu; ++k) {
       const int nc = cu[k];
       rows += (int64_t)rows_per_term * nc;
@@ -810,18 +981,22 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
         ui8[u] += 2 * (int64_t)((nc + kI8KB - 1) / kI8KB) * kI8HalfBytes;
         ui8n[u] += 1;
       }
-      int tiles = t_user;
-      if (bt && nc > 0) {
+      int tiles = nc <= merge_max ? 0 : t_user;
+      if (bt && nc > 0 && band_of_n[nc] >= 0) {
         const int b = band_of_n[nc];
         tiles += band_tiles[b];
         if (b != prev) {
           acc += 4 * (int64_t)band_nq[b] * n_blk;
           slots += n_blk;
           prev = b;
+          run = k / kRunChunks;
+        } else if (b < n_levels && k / kRunChunks != run) {
+          acc += 4 * (int64_t)band_nq[b] * n_blk;
+          run = k / kRunChunks;
         }
       }
       cost += (double)tiles * ((double)nc + 24.0) * rows_per_term * (dv.on ? 1.5 : 1.0);
-      max_tiles = std::max(max_tiles, tiles);
+      max_tiles = std::max(max_tiles, nc <= merge_max ? tiles + k / kRunChunks : tiles);
     }
     urows[u] = rows;
     uacc[u] = acc;
@@ -874,7 +1049,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   struct Slab {
     int64_t u0 = 0, nu = 0;      // units (flat list, slab-major)
     int64_t sl0 = 0, n_slots = 0;
-    int64_t pi0 = 0, pi_cap = 0;  // projection items: nb + n_slots / 32 at most
+    int64_t pi0 = 0, pi_cap = 0;  // projection items: 2 nb + n_slots / tile_slots at most
     int64_t it0 = 0, n_items = 0;
     int64_t acc_len = 0;
     int64_t n_proj = 0;
@@ -900,7 +1075,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       S.nu = count[sl];
       S.sl0 = sl0;
       S.pi0 = pi0;
-      S.pi_cap = 2 * nb + S.n_slots / 32 + 1;
+      S.pi_cap = 2 * nb + S.n_slots / tile_slots + 1;
       S.it0 = it0;
       u0 += S.nu;
       sl0 += S.n_slots;
@@ -956,6 +1131,10 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   double* acc = c.acc.as<double>((size_t)acc_max);
   double* slot_greek =
       L >= 0 ? c.slot_greek.as<double>((size_t)slots_max * 6 * (L + 1)) : nullptr;
+  double* slot_phase =
+      n_levels > 0 ? c.slot_phase.as<double>((size_t)slots_max * 4 * n_mu) : nullptr;
+  // The row tiles of a slot's projections at most (slot_project_kernel).
+  const int slot_tiles = (n_levels > 0 ? t_user : 0) + (L >= 0 ? 2 * (L / 32 + 1) : 0);
   int* counter = c.counter.as<int>(64);
   int64_t* chunk_xoff_d = nullptr;
   int* chunk_xidx_d = nullptr;
@@ -1026,6 +1205,8 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     ua.bands = bt->desc_d.as<BandDesc>(0);
     ua.band_ge = bt->ge_d.as<double>(0);
     ua.band_go = bt->go_d.as<double>(0);
+    ua.level_ge = bt->lge_d.as<double>(0);
+    ua.level_go = bt->lgo_d.as<double>(0);
   }
   ua.acc = acc;
   ua.work_counter = counter;
@@ -1036,13 +1217,12 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   ua.wdiff = ka.wdiff;
   ua.wthdiff = ka.wthdiff;
   ua.i8_above = i8_above;
+  ua.n_levels = n_levels;
+  ua.merge_max = merge_max;
   ProjArgs pj{};
-  pj.cpu = cpu;
   pj.greek_order = L;
   pj.acc = acc;
-  pj.chunk_sums = chunk_sums;
   pj.slot_greek = slot_greek;
-  pj.raw = dv.on && !ad.on ? 1 : 0;
   if (ad.on) pj.unit_norm = c.unit_norm.as<double>(0);
   if (ad.on && dv.on) {
     pj.ad_blocks = 3 + dv.n_theta;
@@ -1061,6 +1241,8 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   fa.greek_order = L;
   if (bt) fa.bands = ua.bands;
   fa.slot_greek = slot_greek;
+  fa.slot_phase = slot_phase;
+  fa.n_levels = n_levels;
   fa.acc = acc;
   fa.n_units_total = n_units;
   fa.values = values;
@@ -1122,7 +1304,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       P_uacc[lu] = accpos;
       int64_t band_acc = accpos + acc_head;
       int2 us = make_int2((int)nslot, 0);
-      int prev = -1;
+      int prev = -1, first_run = 0;
       for (int k = 0; k < cpu; ++k) {
         const int64_t ci = lu * cpu + k;
         const int nc = cn[(int64_t)u * cpu + k];
@@ -1140,7 +1322,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
         }
         row += (int64_t)rows_per_term * nc;
         P_cacc[ci] = -1;
-        if (bt && nc > 0) {
+        if (bt && nc > 0 && band_of_n[nc] >= 0) {
           const int b = band_of_n[nc];
           if (b != prev) {
             // One slot per block of sums, their tables 4 n_q doubles apart.
@@ -1151,13 +1333,28 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
               // Adaptive: the value slots, then the error slots; pad is the block.
               P_slots[nslot].kind = ad.on ? (2 * blk >= n_blk ? 1 : 0) : 0;
               P_slots[nslot].pad = ad.on ? blk % (n_blk / 2) : 0;
+              P_slots[nslot].order = bt->desc[b].order;
+              P_slots[nslot].reps = 1;
               band_acc += 4 * (int64_t)band_nq[b];
               ++nslot;
             }
             us.y += n_blk;
             prev = b;
+            first_run = k / kRunChunks;
           }
           P_cacc[ci] = P_slots[nslot - n_blk].off;
+          if (b < n_levels) {
+            // A level's slot: a copy of its sums per run of chunks; it reaches the orders of
+            // its chunks' projector bands.
+            const int r = k / kRunChunks - first_run;
+            const int order = L >= 0 ? (int)std::min<int64_t>(bt->desc[b].order, 2 * bucket(nc)) : -1;
+            for (int blk = 0; blk < n_blk; ++blk) {
+              P_slots[nslot - n_blk + blk].reps = r + 1;
+              P_slots[nslot - n_blk + blk].order = order;
+            }
+            P_cacc[ci] += r * 4 * (int64_t)band_nq[b] * n_blk;
+            band_acc = std::max(band_acc, P_cacc[ci] + 4 * (int64_t)band_nq[b] * n_blk);
+          }
         }
       }
       P_uslots[lu] = us;
@@ -1176,7 +1373,8 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       P_items[k].n_groups = ugroups[P_units[lu]];
       P_items[k].pad = 0;
     }
-    // Projection tiles: the slab's slots grouped by band (largest bands first), 32 at a time.
+    // Projection tiles: the slab's slots grouped by band (largest bands first), tile_slots at a
+    // time.
     S.n_proj = 0;
     if (bt && S.n_slots > 0) {
       // Slots grouped by (band, kind): a tile's slots share the band's matrices and the kind
@@ -1195,12 +1393,12 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       for (int g = 0; g < ng; ++g) cursor[g] = start[g];
       for (int64_t k = 0; k < S.n_slots; ++k) P_sidx[cursor[key(P_slots[k])]++] = (int)k;
       for (int g = ng - 1; g >= 0; --g)
-        for (int64_t k0 = 0; k0 < per_band[g + 1]; k0 += 32) {
+        for (int64_t k0 = 0; k0 < per_band[g + 1]; k0 += tile_slots) {
           ProjItem& pi = P_proj[S.n_proj++];
           pi.band = g / nk;
           pi.kind = g % nk;
           pi.pad = 0;
-          pi.count = (int)std::min<int64_t>(32, per_band[g + 1] - k0);
+          pi.count = (int)std::min<int64_t>(tile_slots, per_band[g + 1] - k0);
           pi.first = start[g] + k0;
         }
     }
@@ -1305,13 +1503,41 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       ia.n_user_tabs = (int)c.i8.user.size();
       ia.band_tabs = c.i8.band_d.as<I8Table>(0);
       ia.levels = call->i8_levels;
+      ia.n_levels = n_levels;
+      ia.merge_max = merge_max;
       ia.err = i8_err;
       const int grid8 = (int)std::min<int64_t>(c.sms, S.n_items);
       cudaError_t le = cudaSuccess;
       timed_launch(K_UNITS_I8, s, [&] { le = launch_units_i8(ia, grid8, s); });
       SB_CUDA(le);
     }
-    if (bt && S.n_proj > 0) {
+    if (bt && S.n_proj > 0 && !ad.on) {
+      SlotArgs sa{};
+      sa.items = proj_d + S.pi0;
+      sa.n_items = (int)S.n_proj;
+      sa.slot_index = slot_index_d + S.sl0;
+      sa.slots = slots_d + S.sl0;
+      sa.bands = ua.bands;
+      sa.n_levels = n_levels;
+      sa.n_blk = n_blk;
+      sa.acc = acc;
+      sa.n_mu = (int)n_mu;
+      sa.h_u = c.user.h;
+      sa.h_pad = c.user.h_pad;
+      if (n_levels > 0) {
+        sa.half0 = bt->half0_d.as<int>(0);
+        sa.me = bt->me_d.as<double>(0);
+        sa.mo = bt->mo_d.as<double>(0);
+      }
+      sa.user_map = ua.user_map;
+      sa.slot_phase = slot_phase;
+      sa.greek_order = L;
+      sa.band_d = bt->d_d.as<double>(0);
+      sa.slot_greek = slot_greek;
+      cudaError_t le = cudaSuccess;
+      timed_launch(K_PROJ, s, [&] { le = launch_slot_project(sa, slot_tiles, s); });
+      SB_CUDA(le);
+    } else if (bt && S.n_proj > 0) {
       pj.items = proj_d + S.pi0;
       pj.n_items = (int)S.n_proj;
       pj.slot_index = slot_index_d + S.sl0;
@@ -1324,7 +1550,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     fa.n_units = (int)S.nu;
     fa.unit_acc = ua.unit_acc;
     fa.unit_slots = unit_slots_d + S.u0;
-    fa.slots = slots_d + S.sl0;
+    fa.slots = S.n_slots > 0 ? slots_d + S.sl0 : nullptr;
     timed_launch(K_FINAL, s, [&] { launch_final(fa, s); });
     SB_CUDA(cudaGetLastError());
     if (call && call->h_values && !ad.on && !dv.on) {
@@ -6496,18 +6722,16 @@ void scatrs_release(void) {
     Context& c = *g_ctx[dev];
     for (DevBuf* b : {&c.radius, &c.weight, &c.wtheta, &c.wthdiff, &c.wdiff, &c.unit_norm, &c.wl, &c.m, &c.fractions, &c.chunk_n, &c.chunk_n_slab,
                       &c.chunk_row, &c.chunk_acc, &c.plan_units, &c.unit_acc, &c.unit_slots,
-                      &c.slots, &c.items, &c.proj_items, &c.slot_index, &c.slot_greek,
+                      &c.slots, &c.items, &c.proj_items, &c.slot_index, &c.slot_greek, &c.slot_phase,
                       &c.X, &c.uz, &c.ux, &c.chunk_sums, &c.err, &c.acc,
                       &c.counter, &c.values, &c.phase, &c.greek, &c.user.ge, &c.user.go,
-                      &c.user.map, &c.tc_a_hi, &c.tc_a_lo, &c.tc_prod, &c.tc_err, &c.xdig,
+                      &c.user.map, &c.user.rows_d, &c.tc_a_hi, &c.tc_a_lo, &c.tc_prod, &c.tc_err, &c.xdig,
                       &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.i8_err,
                       &c.i8.dig, &c.i8.scale, &c.i8.user_d, &c.i8.band_d})
       b->release();
     for (auto& kv : c.projectors)
       for (DevBuf* b : {&kv.second.d, &kv.second.d_hi, &kv.second.d_lo}) b->release();
-    for (auto& kv : c.bands)
-      for (DevBuf* b : {&kv.second.ge_d, &kv.second.go_d, &kv.second.d_d, &kv.second.desc_d})
-        b->release();
+    for (auto& kv : c.bands) kv.second.release();
     if (c.pinned_chunk_n) cudaFreeHost(c.pinned_chunk_n);
     for (int h = 0; h < 2; ++h)
       if (c.staged[h]) {

@@ -84,8 +84,67 @@ struct BandDesc {
   int h_pad;
   int ld;
   int64_t g_off;  // into band_ge / band_go
-  int64_t d_off;  // into band_d: 4 matrices of n_q x (order + 1)
+  int64_t d_off;  // into band_d: 4 matrices of n_q x d_ld (order + 1 used)
+  int d_ld;       // a multiple of 32
 };
+
+// The tables a chunk's angle sums run on. The fixed grid's band list starts with n_levels phase
+// levels (phase_levels.cu), level l holding the chunks with at most 32 level_tiles - 1 orders
+// (tiles 1, 2, .. 8, then growing by an eighth); merge_max is the last one's reach (0: none).
+// Chunks on a level run its rows only; the others the requested cosines' and, with Greek
+// coefficients, their projector band's (buckets 1, 2, 3, 4, 5, 7, ..., each the ceiling of 1.25
+// times the last, engine.rs:951-957), listed after the levels.
+constexpr int kMaxLevels = 48;
+// The chunks of a unit on a level add into one copy of its sums per run of this many chunks, so
+// that a unit of few row tiles still splits into work items (each copy has one owner); whatever
+// reads the sums adds the copies in order.
+constexpr int kRunChunks = 2;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int next_level_tiles(int t) { return t + (t < 8 ? 1 : t / 8); }
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int chunk_band(int nc, int merge_max, int n_levels, int greek_order) {
+  if (nc <= merge_max) {
+    int l = 0;
+    for (int t = 1; 32 * t - 1 < nc; t = next_level_tiles(t)) ++l;
+    return l;
+  }
+  if (greek_order < 0) return -1;
+  int idx = n_levels;
+  for (int u = 1; u < nc; u = (5 * u + 3) >> 2) ++idx;
+  return idx;
+}
+
+// The level tables: half nodes (>= 0) of every level, level l's from half0[l], their double
+// values x0 in; out the nodes in double-double, the barycentric weights and the G_E, G_O rows.
+struct LevelTableArgs {
+  int n_levels, n_half;
+  const BandDesc* bands;
+  const int* half0;
+  const double* x0;
+  double* x_hi;
+  double* x_lo;
+  double* bary;
+  double* ge;
+  double* go;
+};
+// The interpolation onto the requested rows: per half node h_pad even and h_pad odd weights.
+struct LevelMatrixArgs {
+  int n_levels, h_u, h_pad;
+  const BandDesc* bands;
+  const int* half0;
+  const double* x_hi;
+  const double* x_lo;
+  const double* bary;
+  const double* rows;  // the requested rows' cosines
+  double* me;
+  double* mo;
+};
+void launch_level_tables(const LevelTableArgs& a, cudaStream_t s);
+void launch_level_matrices(const LevelMatrixArgs& a, cudaStream_t s);
 
 // A share of one unit's angle GEMMs: row tiles t (over the requested cosines' tiles, then the
 // chunk's band tiles) with t % n_groups == group, for every chunk of the unit.
@@ -105,6 +164,8 @@ struct BandSlot {
   int64_t off;
   int kind;
   int pad;
+  int order;  // the last Greek order its chunks reach
+  int reps;   // a level's slot: copies of the sums, one per run of chunks (kRunChunks)
 };
 
 // A tile of up to 32 band slots of one band, projected together (they share the band's
@@ -117,7 +178,33 @@ struct ProjItem {
   int pad;
 };
 
-// K-d over one slab: each band slot's averaged tables projected onto its Greek coefficients,
+// K-d of the fixed grid over one slab: each slot's raw sums onto its Greek coefficients
+// (slot_greek + slot * 6 (L + 1)) and, on a level, onto the requested cosines (slot_phase + slot *
+// 4 n_mu), in tiles of up to kSlotGroup slots of one table.
+constexpr int kSlotGroup = 16;
+struct SlotArgs {
+  const ProjItem* items;
+  int n_items;
+  const int* slot_index;
+  const BandSlot* slots;
+  const BandDesc* bands;
+  int n_levels, n_blk;
+  const double* acc;
+  // The requested cosines.
+  int n_mu, h_u, h_pad;
+  const int* half0;
+  const double* me;
+  const double* mo;
+  const int2* user_map;
+  double* slot_phase;
+  // The Greek coefficients.
+  int greek_order;
+  const double* band_d;
+  double* slot_greek;
+};
+cudaError_t launch_slot_project(const SlotArgs& a, int max_tiles, cudaStream_t s);
+
+// K-d of the adaptive calls over one slab: each band slot's averaged tables projected onto its Greek coefficients,
 // 6 (L + 1) doubles per slot at slot_greek + slot * 6 (L + 1).
 struct ProjArgs {
   const ProjItem* items;
@@ -127,11 +214,8 @@ struct ProjArgs {
   const BandDesc* bands;
   const double* band_d;
   const double* acc;
-  const double* chunk_sums;  // for each unit's Z
-  int cpu;
   int greek_order;
   double* slot_greek;
-  int raw;  // project the raw sums (derivatives: averaged after the projection)
   // Adaptive: per unit (z, ez, truncation, ...; see FinalArgs): values averaged as s / z, error
   // sums as (e + |s/z| ez) / z + truncation |s/z| (engine.rs:1782-1800), then bounded with |d|.
   const double* unit_norm;
@@ -205,6 +289,7 @@ struct UnitI8Args {
   int n_user_tabs;
   const I8Table* band_tabs;
   int levels;     // product levels kept: 5 (15 products) or 6 (19)
+  int n_levels, merge_max;  // the phase levels (chunk_band)
   unsigned* err;  // set when a bounded wait gave up
 };
 
@@ -261,6 +346,8 @@ struct UnitArgs {
   const BandDesc* bands;
   const double* band_ge;
   const double* band_go;
+  const double* level_ge;
+  const double* level_go;
   double* acc;
   int* work_counter;
   int per_unit;
@@ -276,6 +363,7 @@ struct UnitArgs {
   // The mixed form (i8_above > 0): chunks with i8_above < nc <= kI8MaxTerms are left to
   // unit_i8_kernel.
   int i8_above;
+  int n_levels, merge_max;  // the phase levels (chunk_band)
 };
 
 // K-d and the outputs over one slab: averages, band projections, assembly.
@@ -288,6 +376,8 @@ struct FinalArgs {
   const int2* unit_slots;    // per unit: first band slot and count
   const BandSlot* slots;
   const double* slot_greek;  // each slot's projected coefficients
+  const double* slot_phase;  // and a level slot's elements at the requested cosines
+  int n_levels;
   int n_mu, greek_order;
   const BandDesc* bands;
   double* acc;

@@ -215,38 +215,32 @@ __device__ __forceinline__ void recombine(const uint32_t (&q)[LEV][16], double* 
   }
 }
 
-__device__ __forceinline__ int band_of(int n) {
-  int u = 1, idx = 0;
-  while (u < n) {
-    u = (int)ceil((double)u * 1.25);
-    ++idx;
-  }
-  return idx;
-}
-
-// One job: chunk ci (nc terms, band b) of item unit ul, M tile `tile` (user tiles first), half.
+// One job: chunk ci (nc terms, band b) of item unit ul, M tile `tile` (the t_user tiles of the
+// requested cosines first, none for a chunk on a phase level), half.
 struct Job {
   int ul;
   int64_t ci;
   int c;  // chunk within the unit
-  int nc, b, tile, half;
+  int nc, b, t_user, tile, half;
 };
 
 // Calls f(job) for every job of this CTA, in the order every role sees them.
 template <class F>
 __device__ __forceinline__ void for_each_job(const UnitI8Args& a, F&& f) {
-  const int t_user = (a.h_u + kI8Pairs - 1) / kI8Pairs;
   for (int item = blockIdx.x; item < a.n_items; item += gridDim.x) {
     const WorkItem it = a.items[item];
     for (int c = 0; c < a.cpu; ++c) {
       const int64_t ci = (int64_t)it.unit * a.cpu + c;
       if (a.chunk_xoff[ci] < 0) continue;
       const int nc = a.chunk_n[ci];
-      const int b = a.greek_order >= 0 ? band_of(nc) : -1;
+      const int b = chunk_band(nc, a.merge_max, a.n_levels, a.greek_order);
+      const int t_user = nc <= a.merge_max ? 0 : (a.h_u + kI8Pairs - 1) / kI8Pairs;
       const int t_band = b >= 0 ? (a.bands[b].h + kI8Pairs - 1) / kI8Pairs : 0;
-      for (int tile = it.group; tile < t_user + t_band; tile += it.n_groups)
+      const int shift = nc <= a.merge_max ? (c / kRunChunks) % it.n_groups : 0;
+      const int tile0 = it.group >= shift ? it.group - shift : it.group - shift + it.n_groups;
+      for (int tile = tile0; tile < t_user + t_band; tile += it.n_groups)
         for (int half = 0; half < 2; ++half)
-          if (!f(Job{it.unit, ci, c, nc, b, tile, half})) return;
+          if (!f(Job{it.unit, ci, c, nc, b, t_user, tile, half})) return;
     }
   }
 }
@@ -254,14 +248,13 @@ __device__ __forceinline__ void for_each_job(const UnitI8Args& a, F&& f) {
 // The table of a job: its digits (tile's K block 0) and its rows' scales.
 __device__ __forceinline__ const I8Table& job_table(const UnitI8Args& a, const Job& j,
                                                     int& tile_local) {
-  const int t_user = (a.h_u + kI8Pairs - 1) / kI8Pairs;
-  if (j.tile < t_user) {
+  if (j.tile < j.t_user) {
     tile_local = j.tile;
     int v = 0;
     while ((kI8KB << v) < j.nc) ++v;  // the version covering the chunk's orders
     return a.user_tabs[v < a.n_user_tabs ? v : a.n_user_tabs - 1];
   }
-  tile_local = j.tile - t_user;
+  tile_local = j.tile - j.t_user;
   return a.band_tabs[j.b];
 }
 
@@ -393,7 +386,6 @@ __global__ void __launch_bounds__(kThreads, 1) unit_i8_kernel(UnitI8Args a) {
     const int side = r & 1;            // 0: E row, elements at +mu; 1: O row, at -mu
     const int p = r >> 1;              // the angle pair within the tile
     const int e_thread = t - 64;       // 0 .. 255
-    const int t_user = (a.h_u + kI8Pairs - 1) / kI8Pairs;
     int job = 0, q = -1;
     int64_t cur = -1;
     double out[4] = {0.0, 0.0, 0.0, 0.0};
@@ -441,7 +433,7 @@ __global__ void __launch_bounds__(kThreads, 1) unit_i8_kernel(UnitI8Args a) {
       warp_arrive(&sm.tmem_empty);
 #pragma unroll
       for (int g = 2 - kHeld; g < 2; ++g) recombine<LEV>(sums[g - (2 - kHeld)], v + 16 * g);
-      const bool user = j.tile < t_user;
+      const bool user = j.tile < j.t_user;
       const double* cs = sm.side[q & 1];
       const double* nf = sm.side[q & 1] + 128;
       const double sg = side ? -1.0 : 1.0;
@@ -488,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, 1) unit_i8_kernel(UnitI8Args a) {
             base = a.acc + a.unit_acc[j.ul];
           } else {
             const BandDesc B = a.bands[j.b];
-            const int row = (j.tile - t_user) * kI8Pairs + p;
+            const int row = (j.tile - j.t_user) * kI8Pairs + p;
             if (row < B.h) {
               const int qn = B.n_q, jn = qn / 2 + row, mirror = qn - 1 - jn;
               if (side == 0 || mirror != jn) jo = side ? mirror : jn;

@@ -50,17 +50,6 @@ __device__ __forceinline__ void element_derivs4(double s1r, double s1i, double s
   e[3] = (d2i * s1r - d2r * s1i) + (s2i * d1r - s2r * d1i);
 }
 
-// The band of a chunk with n terms: the index of bucket(n) in 1, 2, 3, 4, 5, 7, ... (each the
-// ceiling of 1.25 times the last; engine.rs:951-957).
-__device__ __forceinline__ int band_of(int n) {
-  int u = 1, idx = 0;
-  while (u < n) {
-    u = (int)ceil((double)u * 1.25);
-    ++idx;
-  }
-  return idx;
-}
-
 struct Smem {
   double a[2][2][KB][TRP];  // [stage][G_E, G_O][order][row] (rows 32 .. 35 unused)
   double xs[2][KB][XP];    // [stage][order][4 columns x 32 nodes] (128 .. 131 unused)
@@ -453,7 +442,6 @@ __device__ __forceinline__ void unit_body(const UnitArgs& a) {
   const int t = threadIdx.x, rg = t >> 4, ng = t & 15;
   // This thread's share of a reduced tile: side (+mu, -mu), row, two elements.
   const int side = ng >> 3, rr = (ng >> 1) & 3, e0 = 2 * (ng & 1);
-  const int t_user = (a.h_u + TR - 1) / TR;
   // Blocks of sums: the values, then (with derivatives) each distribution parameter, Re m and
   // Im m; halves: a chunk's coefficient rows are one 32-node tile, or two of 16 nodes with
   // their derivative columns.
@@ -476,9 +464,13 @@ __device__ __forceinline__ void unit_body(const UnitArgs& a) {
       const int nc = a.chunk_n[ci];
       if (nc == 0) continue;
       if (a.i8_above > 0 && nc > a.i8_above && nc <= kI8MaxTerms) continue;  // the int8 path's
-      const int b = a.greek_order >= 0 ? band_of(nc) : -1;
+      const int b = chunk_band(nc, a.merge_max, a.n_levels, a.greek_order);
+      const int t_user = nc <= a.merge_max ? 0 : (a.h_u + TR - 1) / TR;
       const int t_band = b >= 0 ? (a.bands[b].h + TR - 1) / TR : 0;
-      if (it.group >= t_user + t_band) continue;
+      // This item's first tile; a level's tiles move on by one item per run of chunks.
+      const int shift = nc <= a.merge_max ? (c / kRunChunks) % it.n_groups : 0;
+      const int tile0 = it.group >= shift ? it.group - shift : it.group - shift + it.n_groups;
+      if (tile0 >= t_user + t_band) continue;
       if (t < 32) {
         const int j = c * 32 + t;
         double w = 0.0, cu = 0.0, ar = 0.0, sc = 0.0, wd = 0.0;
@@ -526,21 +518,21 @@ __device__ __forceinline__ void unit_body(const UnitArgs& a) {
         auto source = [&](int tl) {
           const bool u = tl < t_user;
           const BandDesc Bd = u ? BandDesc{} : a.bands[b];
-          return TileSrc{u ? a.ge_u : a.band_ge + Bd.g_off, u ? a.go_u : a.band_go + Bd.g_off,
+          const bool lv = b < a.n_levels;
+          return TileSrc{u ? a.ge_u : (lv ? a.level_ge : a.band_ge) + Bd.g_off,
+                         u ? a.go_u : (lv ? a.level_go : a.band_go) + Bd.g_off,
                          u ? a.h_u_pad : Bd.h_pad, (u ? tl : tl - t_user) * TR};
         };
         int st0 = 0;  // the stage buffer of the next MMA tile's first stage (kMode 0)
         if constexpr (kMode == 0) {
-          const TileSrc s0 = source(it.group);
+          const TileSrc s0 = source(tile0);
           load_stage_z(sm, 0, s0.ge, s0.go, s0.ldr, s0.r0, 0, nc, xc);
         }
-        for (int tile = it.group; tile < t_user + t_band; tile += it.n_groups) {
+        for (int tile = tile0; tile < t_user + t_band; tile += it.n_groups) {
           const bool user = tile < t_user;
           const BandDesc B = user ? BandDesc{} : a.bands[b];
           const int r0 = (user ? tile : tile - t_user) * TR;
-          const double* ge = user ? a.ge_u : a.band_ge + B.g_off;
-          const double* go = user ? a.go_u : a.band_go + B.g_off;
-          const int ldr = user ? a.h_u_pad : B.h_pad;
+          const TileSrc src = source(tile);
           // The output index of this thread's sums, or -1.
           const int row = r0 + o_row;
           int j = -1;
@@ -559,7 +551,7 @@ __device__ __forceinline__ void unit_body(const UnitArgs& a) {
             double cE[16][2], cO[16][2];
             const int tn = tile + it.n_groups;
             const TileSrc nx = source(tn < t_user + t_band ? tn : tile);
-            gemm_tile_mma(sm, TileSrc{ge, go, ldr, r0}, nc, xc, cE, cO, st0,
+            gemm_tile_mma(sm, src, nc, xc, cE, cO, st0,
                           tn < t_user + t_band ? &nx : nullptr);
             if (user)
               chunk_elements_mma<true>(sm, cE, cO, v);
@@ -571,7 +563,7 @@ __device__ __forceinline__ void unit_body(const UnitArgs& a) {
             }
           } else {
             double accE[4][8], accO[4][8];
-            gemm_tile(sm, ge, go, ldr, r0, nc, xc, accE, accO);
+            gemm_tile(sm, src.ge, src.go, src.ldr, r0, nc, xc, accE, accO);
             for (int blk = 0; blk < n_blk; ++blk) {
               if (user) {
                 if (kDeriv)
@@ -643,7 +635,6 @@ constexpr int PL = 72;   // orders per pass: 8 warps x 9
 struct ProjSmem {
   double fs[4][PQ][33];  // F11, F12, F33, F34 per node and slot (padded against conflicts)
   double ds[4][PQ][PL];  // d00, d22, d2-2, d02 (scaled) per node and order
-  double rz[32];         // 1/Z per slot
   double z[32], ez[32], tr[32];  // adaptive: Z, its error, the truncation term
   double dz[32], edz[32];        // adaptive derivatives: the slot's Z_p and its error
   int blk[32];                   // adaptive derivatives: the slot's block
@@ -691,32 +682,22 @@ __global__ void __launch_bounds__(PT) proj_kernel(ProjArgs a) {
     const int q = B.n_q, len = B.order + 1;
     const bool bounds = it.kind == 1;
     if (t < 32) {
-      double rz = 0.0;
       int64_t off = -1;
       if (t < it.count) {
         const BandSlot bs = a.slots[a.slot_index[it.first + t]];
-        if (a.unit_norm) {
-          const int stride = a.ad_blocks > 0 ? kNormStrideD : 8;
-          const double* un = a.unit_norm + stride * (int64_t)a.units[bs.unit];
-          sm.z[t] = un[0];
-          sm.ez[t] = un[1];
-          sm.tr[t] = un[2];
-          if (a.ad_blocks > 0) {
-            const int b = bs.pad, p = b - 1;
-            sm.blk[t] = b;
-            sm.dz[t] = (b >= 1 && b <= a.n_theta) ? un[8 + p] : 0.0;
-            sm.edz[t] = (b >= 1 && b <= a.n_theta) ? un[11 + p] : 0.0;
-          }
-        } else if (a.raw) {
-          rz = 1.0;
-        } else {
-          double z = 0.0;
-          for (int c = 0; c < a.cpu; ++c) z += a.chunk_sums[((int64_t)bs.unit * a.cpu + c) * 8];
-          rz = 1.0 / z;
+        const int stride = a.ad_blocks > 0 ? kNormStrideD : 8;
+        const double* un = a.unit_norm + stride * (int64_t)a.units[bs.unit];
+        sm.z[t] = un[0];
+        sm.ez[t] = un[1];
+        sm.tr[t] = un[2];
+        if (a.ad_blocks > 0) {
+          const int b = bs.pad, p = b - 1;
+          sm.blk[t] = b;
+          sm.dz[t] = (b >= 1 && b <= a.n_theta) ? un[8 + p] : 0.0;
+          sm.edz[t] = (b >= 1 && b <= a.n_theta) ? un[11 + p] : 0.0;
         }
         off = bs.off;
       }
-      sm.rz[t] = rz;
       sm.offs[t] = off;
     }
     __syncthreads();
@@ -739,8 +720,6 @@ __global__ void __launch_bounds__(PT) proj_kernel(ProjArgs a) {
             const int64_t o = off + (int64_t)e * q + k0 + kk;
             if (a.ad_blocks > 0) {
               v = ad_table(a, sm, s, o, q, bounds);
-            } else if (!a.unit_norm) {
-              v = a.acc[o] * sm.rz[s];
             } else if (!bounds) {
               v = a.acc[o] / sm.z[s];
             } else {
@@ -754,7 +733,7 @@ __global__ void __launch_bounds__(PT) proj_kernel(ProjArgs a) {
         for (int idx = t; idx < 4 * PQ * PL; idx += PT) {
           const int l = idx % PL, kk = (idx / PL) % PQ, m = idx / (PL * PQ);
           double v = 0.0;
-          if (kk < kn && l0 + l < len) v = D[((int64_t)m * q + k0 + kk) * len + l0 + l];
+          if (kk < kn && l0 + l < len) v = D[((int64_t)m * q + k0 + kk) * B.d_ld + l0 + l];
           sm.ds[m][kk][l] = bounds ? fabs(v) : v;
         }
         __syncthreads();
@@ -840,12 +819,18 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a) {
 #pragma unroll
       for (int k = 0; k < 11; ++k) a.values[k * nu + unit] = out[k];
     }
+    const int2 sl = a.slots ? a.unit_slots[ul] : make_int2(0, 0);
     if (a.phase) {
+      int n_lev = 0;  // the unit's level slots, which come first
+      while (n_lev < sl.y && a.slots[sl.x + n_lev].band < a.n_levels) ++n_lev;
       for (int j = t; j < a.n_mu; j += NT) {
         double f[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          f[e] = acc_user[e * a.n_mu + j] / z;
+          double v = acc_user[e * a.n_mu + j];
+          for (int k = 0; k < n_lev; ++k)
+            v += a.slot_phase[((int64_t)(sl.x + k) * 4 + e) * a.n_mu + j];
+          f[e] = v / z;
           if (a.normalized) f[e] = f[e] / sca;
         }
         const double o6[6] = {f[0], f[1], f[0], f[2], f[3], f[2]};
@@ -854,16 +839,15 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a) {
       }
     }
     if (glen > 0 && a.greek) {
-      const int2 sl = a.unit_slots[ul];
       auto sum = [&](int idx) {
         const int e = idx / glen, l = idx % glen;
         double g = 0.0;
         for (int k = 0; k < sl.y; ++k) {
           const BandSlot bs = a.slots[sl.x + k];
-          if (l <= a.bands[bs.band].order)
+          if (l <= bs.order)
             g += a.slot_greek[(int64_t)(sl.x + k) * 6 * glen + (int64_t)e * glen + l];
         }
-        return g;
+        return g / z;
       };
       if (t == 0) a0s = sum(0);
       __syncthreads();
@@ -957,12 +941,21 @@ __global__ void __launch_bounds__(NT) final_deriv_kernel(FinalArgs a) {
       avg(&S[0][2], 8, v);
       for (int p = 0; p <= P; ++p) sca[p] = v[p];
     }
+    // The unit's slots are B consecutive entries (one per block) per table, the levels first.
+    const int2 sl = a.slots ? a.unit_slots[ul] : make_int2(0, 0);
     if (a.phase) {
+      int n_lev = 0;
+      while (n_lev < sl.y && a.slots[sl.x + n_lev].band < a.n_levels) ++n_lev;
       const int64_t blk = 4 * (int64_t)a.n_mu;
       for (int j = t; j < a.n_mu; j += NT) {
         double f[4][6];
         for (int e = 0; e < 4; ++e) {
-          avg(acc_user + e * a.n_mu + j, (int)blk, f[e]);
+          double raw[6];
+          for (int b = 0; b < B; ++b) raw[b] = acc_user[b * blk + (int64_t)e * a.n_mu + j];
+          for (int k = 0; k < n_lev; k += B)
+            for (int b = 0; b < B; ++b)
+              raw[b] += a.slot_phase[((int64_t)(sl.x + k + b) * 4 + e) * a.n_mu + j];
+          avg(raw, 1, f[e]);
           if (a.normalized) {
             double o[6];
             ldiv(f[e], sca, o);
@@ -978,14 +971,12 @@ __global__ void __launch_bounds__(NT) final_deriv_kernel(FinalArgs a) {
       }
     }
     if (glen > 0 && a.greek) {
-      // The unit's slots are B consecutive entries (one per block) per band, bands ascending.
-      const int2 sl = a.unit_slots[ul];
       auto sum = [&](int b, int idx) {
         const int e = idx / glen, l = idx % glen;
         double g = 0.0;
         for (int k = b; k < sl.y; k += B) {
           const BandSlot bs = a.slots[sl.x + k];
-          if (l <= a.bands[bs.band].order)
+          if (l <= bs.order)
             g += a.slot_greek[(int64_t)(sl.x + k) * 6 * glen + (int64_t)e * glen + l];
         }
         return g;
@@ -1084,7 +1075,7 @@ __global__ void __launch_bounds__(NT) final_adaptive_kernel(FinalArgs a) {
         double gv = 0.0, ge = 0.0;
         for (int k = 0; k + 1 < sl.y; k += 2) {
           const BandSlot bs = a.slots[sl.x + k];
-          if (l <= a.bands[bs.band].order) {
+          if (l <= bs.order) {
             gv += a.slot_greek[(int64_t)(sl.x + k) * 6 * glen + (int64_t)e * glen + l];
             ge += a.slot_greek[(int64_t)(sl.x + k + 1) * 6 * glen + (int64_t)e * glen + l];
           }
@@ -1183,7 +1174,7 @@ __global__ void __launch_bounds__(NT) final_adaptive_d_kernel(FinalArgs a) {
         double gv = 0.0, ge = 0.0;
         for (int k = 0; k + 2 * B <= sl.y; k += 2 * B) {
           const BandSlot bs = a.slots[sl.x + k];
-          if (l <= a.bands[bs.band].order) {
+          if (l <= bs.order) {
             gv += a.slot_greek[(int64_t)(sl.x + k + b) * 6 * glen + (int64_t)e * glen + l];
             ge += a.slot_greek[(int64_t)(sl.x + k + B + b) * 6 * glen + (int64_t)e * glen + l];
           }
