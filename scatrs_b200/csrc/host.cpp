@@ -234,7 +234,7 @@ struct Context {
   } i8;
   DevBuf xdig, xside, colmax, chunk_xoff, chunk_xidx, i8_list, i8_err;
   // Spheroid T-matrices.
-  DevBuf tm_geoms, tm_jobs, tm_rules, tm_node, tm_rad, tm_ang, tm_ser, tm_J, tm_work, tm_piv, tm_T,
+  DevBuf tm_geoms, tm_jobs, tm_rules, tm_node, tm_rad, tm_ang, tm_ser, tm_J, tm_work, tm_list, tm_T,
       tm_sums, tm_err;
   DevBuf ro_sph, ro_rank, ro_w, ro_part, ro_f, ro_greek, ro_mu, ro_proj;
   DevBuf p1_fr, p1_ml;  // layered parts of an adaptive call
@@ -2882,7 +2882,7 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
     std::vector<TmJob> jobs;
     std::map<int64_t, int64_t> rule_at;
     std::vector<double> rules;
-    int64_t nodes = 0, rad = 0, ang_nodes = 0, ang = 0, pairs = 0, J = 0, W = 0, P = 0, T = 0;
+    int64_t nodes = 0, rad = 0, ang_nodes = 0, ang = 0, pairs = 0, J = 0, W = 0, T = 0;
     int64_t ser = 0, ser_threads = 0, forms_threads = 0;
     double bytes = 0.0;
     size_t j1 = j0;
@@ -2891,8 +2891,8 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       check_tm_spec(t);
       const bool new_geom = j1 == j0 || t.m == 0 || !same_geom(specs[j1 - 1], t);
       const int K = t.N - std::max(t.m, 1) + 1, n2 = 2 * K, nq = 2 * t.n_theta;
-      double b = 8.0 * ((double)nq * (t.N + 1) * 6 + 32.0 * K * K + 14.0 * n2 * n2 +
-                        (t_out || ro ? 2.0 * n2 * n2 : 0.0)) + 4.0 * n2;
+      double b = 8.0 * ((double)nq * (t.N + 1) * 6 + 32.0 * K * K + 28.0 * K * K +
+                        (t_out || ro ? 2.0 * n2 * n2 : 0.0)) + 4.0;
       if (new_geom)
         b += 8.0 * ((double)nq * 16 + (double)nq * (t.N + 1) * 20 +
                     (double)t.n_theta * (t.N + 1) * tm_series_slot(t.N));
@@ -2944,14 +2944,12 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       jb.pair0 = pairs;
       jb.J0 = J;
       jb.W0 = W;
-      jb.piv0 = P;
       jb.T0 = T;
       ang_nodes += nq;
       ang += (int64_t)nq * (t.N + 1) * 6;
       pairs += (int64_t)K * K;
       J += 8 * (int64_t)K * K;
-      W += 14 * (int64_t)n2 * n2;
-      P += n2;
+      W += 28 * (int64_t)K * K;
       T += (int64_t)n2 * n2;
       jobs.push_back(jb);
     }
@@ -2974,9 +2972,26 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
     a.form = tm_form_override();
     a.J = c.tm_J.as<double>(4 * (size_t)J);
     a.work = c.tm_work.as<double>((size_t)W);
-    a.piv = c.tm_piv.as<int>((size_t)P);
     a.T = t_out || ro ? c.tm_T.as<double>(2 * (size_t)T) : nullptr;
-    a.sums = c.tm_sums.as<double>(3 * jobs.size());
+    a.sums = c.tm_sums.as<double>(6 * jobs.size());
+    // The solves by size, largest first, in groups of one shared-memory size.
+    std::vector<int> by_k(jobs.size());
+    for (size_t k = 0; k < jobs.size(); ++k) by_k[k] = (int)k;
+    std::stable_sort(by_k.begin(), by_k.end(),
+                     [&](int x, int y) { return jobs[x].K > jobs[y].K; });
+    std::vector<TmSolveGroup> solves;
+    for (size_t k = 0; k < jobs.size(); ++k) {
+      const int K = jobs[by_k[k]].K;
+      const int bin = K > 112 ? 4 : K > 80 ? 3 : K > 56 ? 2 : K > 36 ? 1 : 0;
+      const int prev = k == 0 ? -1 : jobs[by_k[k - 1]].K;
+      const int prev_bin = prev > 112 ? 4 : prev > 80 ? 3 : prev > 56 ? 2 : prev > 36 ? 1 : 0;
+      if (k == 0 || bin != prev_bin) solves.push_back(TmSolveGroup{(int)k, 0, K});
+      solves.back().n++;
+    }
+    int* list_d = c.tm_list.as<int>(jobs.size());
+    a.solve_list = list_d;
+    SB_CUDA(cudaMemcpyAsync(list_d, by_k.data(), by_k.size() * sizeof(int),
+                            cudaMemcpyHostToDevice, s));
     a.err = c.tm_err.as<unsigned>(1);
     a.max_sweeps = 4;
     SB_CUDA(cudaMemcpyAsync((void*)a.geoms, geoms.data(), geoms.size() * sizeof(TmGeom),
@@ -2992,7 +3007,10 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
     }
     timed_launch(K_TM_TABLES, s, [&] { launch_tm_tables(a, s); });
     timed_launch(K_TM_SURFACE, s, [&] { launch_tm_surface(a, s); });
-    timed_launch(K_TM_SOLVE, s, [&] { launch_tm_solve(a, s); });
+    cudaError_t le = cudaSuccess;
+    timed_launch(K_TM_SOLVE, s,
+                 [&] { le = launch_tm_solve(a, solves.data(), (int)solves.size(), s); });
+    SB_CUDA(le);
     SB_CUDA(cudaGetLastError());
     std::vector<double> greek_all;
     std::vector<RoSph> sph;
@@ -3061,7 +3079,8 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       SB_CUDA(cudaMemcpyAsync(greek_all.data(), r.greek, (size_t)g * 8, cudaMemcpyDeviceToHost, s));
     }
     unsigned flag = 0;
-    SB_CUDA(cudaMemcpyAsync(sums.data() + 3 * j0, a.sums, 3 * jobs.size() * 8,
+    std::vector<double> class_sums(6 * jobs.size());
+    SB_CUDA(cudaMemcpyAsync(class_sums.data(), a.sums, class_sums.size() * 8,
                             cudaMemcpyDeviceToHost, s));
     SB_CUDA(cudaMemcpyAsync(&flag, a.err, sizeof flag, cudaMemcpyDeviceToHost, s));
     std::vector<double> all;
@@ -3074,6 +3093,13 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       throw Failure{SCATRS_INVALID_INPUT,
                     "a spheroid's radial series needs more than 4000 terms (size too large)"};
     if (flag) throw Failure{SCATRS_INVALID_INPUT, "a spheroid's Q matrix is singular"};
+    for (size_t k = 0; k < jobs.size(); ++k) {
+      const double* cs = &class_sums[6 * k];
+      double* o = &sums[3 * (j0 + k)];
+      o[0] = cs[0] + cs[3];
+      o[1] = cs[1] + cs[4];
+      o[2] = std::max(cs[2], cs[5]);
+    }
     for (const RoSph& e : sph)
       greek_out->emplace_back(greek_all.begin() + e.g0, greek_all.begin() + e.g0 + 6 * (e.L + 1));
     if (t_out)
@@ -3250,6 +3276,8 @@ void spheroid_solve(Context& c, int64_t n, const double* x, const double* aspect
     r.nth = st[i].nth;
     r.q_ext = 2.0 * pi * ext[i] / area;
     r.q_sca = 2.0 * pi * sca[i] / area;
+    // A lossless spheroid scatters what it extinguishes; the two sums round differently.
+    if (m[2 * i + 1] == 0.0) r.q_sca = std::min(r.q_sca, r.q_ext);
     r.q_abs = r.q_ext - r.q_sca;
     if (greek) {
       r.greek = std::move(greeks[i]);
@@ -3305,6 +3333,7 @@ void spheroid_fixed_outputs(Context& c, const std::vector<SphEval>& ev, int orde
     o.assign(5 + (order >= 0 ? 6 * len : 0), 0.0);
     o[0] = 2.0 * pi * ext[i] / area;
     o[1] = 2.0 * pi * sca[i] / area;
+    if (ev[i].m_im == 0.0) o[1] = std::min(o[1], o[0]);  // as spheroid_solve
     o[2] = o[0] - o[1];
     o[3] = 4.0 * pi * f11 / area;
     o[4] = a0 > 0.0 ? (have > 1 ? gr[1] : 0.0) / (3.0 * a0) : 0.0;

@@ -513,8 +513,7 @@ struct TmJob {
   int64_t ang0;       // angular table [node][order 0..N][6]
   int64_t pair0;      // first (i, k) pair
   int64_t J0;         // surface integrals: 8 K^2 complex double-doubles (4 doubles each)
-  int64_t W0;         // workspace: 14 (2K)^2 doubles
-  int64_t piv0;       // pivots: 2K ints
+  int64_t W0;         // workspace: 28 K^2 doubles
   int64_t T0;         // T: (2K)^2 complex doubles (2 each), if kept
 };
 struct TmArgs {
@@ -529,19 +528,27 @@ struct TmArgs {
   double* ang;
   double* J;
   double* work;
-  int* piv;
   double* T;      // or null
-  double* sums;   // per job: -Re tr T, sum |T|^2, the refinement's last relative correction
+  double* sums;   // per job and parity class: -Re tr T, sum |T|^2, the refinement's last
+                  // relative correction
+  const int* solve_list;  // the jobs in solve order
   unsigned* err;  // 1: a singular Q, 2: a series longer than its cap
   int max_sweeps;
   double* ser;    // series and forms tables (tm_series_kernel, tm_forms_kernel)
   int64_t n_ser_total, n_forms_total;
   int form;       // -1: each element's cleanest form; 0: plain; 1, 2: that form where it applies
 };
-void launch_tmatrix(const TmArgs& a, cudaStream_t s);
 void launch_tm_tables(const TmArgs& a, cudaStream_t s);
 void launch_tm_surface(const TmArgs& a, cudaStream_t s);
-void launch_tm_solve(const TmArgs& a, cudaStream_t s);
+// Modes solved in one launch: n of solve_list from `first`, none with more than max_k unknowns.
+struct TmSolveGroup {
+  int first, n, max_k;
+};
+// Where a solve of K unknowns keeps its matrices: 0 factors and right-hand sides in shared
+// memory, 1 the factors, 2 neither.
+inline int tm_solve_where(int K) { return K <= 80 ? 0 : (K <= 112 ? 1 : 2); }
+cudaError_t launch_tm_solve(const TmArgs& a, const TmSolveGroup* groups, int n_groups,
+                            cudaStream_t s);
 
 // The orientation average of a spheroid's phase matrix from its T-matrix (random.cu): one
 // entry per spheroid, whose modes 0..N are the consecutive jobs from job0 of a TmArgs batch.

@@ -14,7 +14,7 @@
 //                      J[a][b]_{ik} = sum_nodes w r^2 2 pi n . (A_i x B_k) of the regular
 //                      and inner vector spherical wave functions, and the y-part of the outgoing
 //                      ones in the cleanest of three exact forms per element of Q;
-//   tm_solve_kernel    one block per mode: Q^T and -P^T from J, an FP64 LU factorization of Q^T
+//   tm_solve_kernel    one block per (mode, parity class): Q^T and -P^T from J, an FP64 LU of Q^T
 //                      with partial pivoting, the solve, and residual sweeps X += LU^{-1}
 //                      (-P^T - Q^T X) with the residual in double-double; then the mode's
 //                      -Re tr T and sum |T|^2.
@@ -678,236 +678,318 @@ struct Cd {  // complex double
   double re, im;
 };
 __device__ __forceinline__ Cd cmul(Cd a, Cd b) {
-  return Cd{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
+  return Cd{fma(a.re, b.re, -(a.im * b.im)), fma(a.re, b.im, a.im * b.re)};
 }
-__device__ __forceinline__ Cd csub(Cd a, Cd b) { return Cd{a.re - b.re, a.im - b.im}; }
-__device__ __forceinline__ Cd cdiv(Cd a, Cd b) {
+// a - b c.
+__device__ __forceinline__ Cd cfms(Cd a, Cd b, Cd c) {
+  return Cd{fma(b.im, c.im, fma(-b.re, c.re, a.re)), fma(-b.im, c.re, fma(-b.re, c.im, a.im))};
+}
+__device__ __forceinline__ Cd crecip(Cd b) {
   const double s = fmax(fabs(b.re), fabs(b.im));
   const Cd bs{b.re / s, b.im / s};
-  const double d = bs.re * bs.re + bs.im * bs.im;
-  const Cd as{a.re / s, a.im / s};
-  return Cd{(as.re * bs.re + as.im * bs.im) / d, (as.im * bs.re - as.re * bs.im) / d};
+  const double d = (bs.re * bs.re + bs.im * bs.im) * s;
+  return Cd{bs.re / d, -(bs.im / d)};
 }
 
-// Block-wide max of v (blockDim.x = 256) through red; every thread gets the result.
-__device__ double block_max(double v, double* red) {
-  const int t = threadIdx.x;
-  red[t] = v;
-  __syncthreads();
-  for (int off = 128; off > 0; off >>= 1) {
-    if (t < off) red[t] = fmax(red[t], red[t + off]);
-    __syncthreads();
-  }
-  const double r = red[0];
-  __syncthreads();
-  return r;
+constexpr int kSolveThreads = 256, kSolveWarps = kSolveThreads / 32;
+
+__device__ __forceinline__ double warp_max(double v) {
+  for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
+  return v;
+}
+__device__ __forceinline__ double warp_sum(double v) {
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
 }
 
-// Applies the LU factors (row swaps piv in order, unit L, U) to column c of X (row-major n2 x n2
-// complex doubles), one column per thread.
-__device__ void lu_apply(const Cd* A, const int* piv, Cd* X, int n2, int c) {
-  for (int k = 0; k < n2; ++k) {
-    const int p = piv[k];
-    if (p != k) {
-      const Cd x = X[(int64_t)k * n2 + c];
-      X[(int64_t)k * n2 + c] = X[(int64_t)p * n2 + c];
-      X[(int64_t)p * n2 + c] = x;
+// Y := U^-1 L^-1 Y (rows already permuted) on this warp's columns: 4 columns at a time, 8 lanes
+// over the rows, right-looking, so that a step is one multiply-subtract per row and no warp waits
+// for another.
+__device__ __forceinline__ void solve_columns(const Cd* A, const Cd* dinv, Cd* Y, int K, int warp,
+                                              int lane) {
+  const int rl = lane >> 2, cl = lane & 3;
+  for (int c0 = 4 * warp; c0 < K; c0 += 4 * kSolveWarps) {
+    const int c = c0 + cl;
+    const bool on = c < K;
+    for (int k = 0; k + 1 < K; ++k) {
+      if (on) {
+        const Cd y = Y[(int64_t)k * K + c];
+        for (int r = k + 1 + rl; r < K; r += 8) {
+          const int64_t at = (int64_t)r * K + c;
+          Y[at] = cfms(Y[at], A[(int64_t)r * K + k], y);
+        }
+      }
+      __syncwarp();
     }
-  }
-  for (int i = 1; i < n2; ++i) {
-    Cd v = X[(int64_t)i * n2 + c];
-    for (int j = 0; j < i; ++j) v = csub(v, cmul(A[(int64_t)i * n2 + j], X[(int64_t)j * n2 + c]));
-    X[(int64_t)i * n2 + c] = v;
-  }
-  for (int i = n2 - 1; i >= 0; --i) {
-    Cd v = X[(int64_t)i * n2 + c];
-    for (int j = i + 1; j < n2; ++j)
-      v = csub(v, cmul(A[(int64_t)i * n2 + j], X[(int64_t)j * n2 + c]));
-    X[(int64_t)i * n2 + c] = cdiv(v, A[(int64_t)i * n2 + i]);
+    for (int k = K - 1; k >= 0; --k) {
+      Cd y{0.0, 0.0};
+      if (on) {
+        y = cmul(Y[(int64_t)k * K + c], dinv[k]);
+        for (int r = rl; r < k; r += 8) {
+          const int64_t at = (int64_t)r * K + c;
+          Y[at] = cfms(Y[at], A[(int64_t)r * K + k], y);
+        }
+      }
+      __syncwarp();
+      if (on && rl == 0) Y[(int64_t)k * K + c] = y;
+    }
+    __syncwarp();
   }
 }
 
 }  // namespace
 
-// One mode per block of 256 threads. Workspace (doubles): Q^T and -P^T as complex double-double
-// (4 (2K)^2 each), the LU factors, X and the residual as complex doubles (2 (2K)^2 each).
-__global__ void __launch_bounds__(256) tm_solve_kernel(TmArgs a) {
-  __shared__ double red_v[256];
-  __shared__ int red_i[256];
-  __shared__ double sums[2][256];
-  const TmJob jb = a.jobs[blockIdx.x];
+// One block per (mode, parity class). Q and P couple (element 0 or 1, order i) only with (element,
+// order) of the same parity of element + order (the surface integrals of the others are exactly
+// zero: the spheroid's mirror symmetry), so the 2K x 2K system is two of K unknowns: a quarter of
+// the operations and half the storage of the whole. Workspace per class (doubles): Q^T and -P^T as
+// complex double-double (4 K^2 each), X (2 K^2), and A and Y (2 K^2 each) where they do not fit
+// shared memory. kWhere: 0 the factors A and the right-hand sides Y in shared memory, 1 the
+// factors, 2 neither.
+//
+// Bound by the latency of a step's dependent reads: a factorization step is a pivot search that
+// every warp does by itself (no exchange), one barrier, the rank-1 update, one barrier; the
+// triangular solves need no block barrier (solve_columns). Against the undivided system in global
+// memory with a column per thread (ten barriers a step): 366 -> 109 ms per pass of
+// 288 spheroids to x = 21.
+template <int kWhere>
+__global__ void __launch_bounds__(kSolveThreads) tm_solve_kernel(TmArgs a, const int* list) {
+  extern __shared__ __align__(16) unsigned char solve_raw[];
+  __shared__ double red[3][kSolveWarps];
+  const int job = list[blockIdx.x >> 1], p = blockIdx.x & 1;
+  const TmJob jb = a.jobs[job];
   const TmGeom g = a.geoms[jb.geom];
-  const int t = threadIdx.x;
-  const int K = jb.K, n2 = 2 * K;
-  const int64_t KK = (int64_t)K * K, NN = (int64_t)n2 * n2;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int K = jb.K;
+  const int64_t KK = (int64_t)K * K;
   const double* J = a.J + 4 * jb.J0;
-  double* Qd = a.work + jb.W0;  // Q^T, dd complex
-  double* Bd = Qd + 4 * NN;     // -P^T, dd complex
-  Cd* A = reinterpret_cast<Cd*>(Bd + 4 * NN);
-  Cd* X = A + NN;
-  Cd* R = X + NN;
-  int* piv = a.piv + jb.piv0;
+  double* Qd = a.work + jb.W0 + p * 14 * KK;  // Q^T, dd complex
+  double* Bd = Qd + 4 * KK;                   // -P^T, dd complex
+  Cd* X = reinterpret_cast<Cd*>(Bd + 4 * KK);
+  // Shared: the class's inverse pivots, a column of L, the row order; then A and Y.
+  Cd* dinv = reinterpret_cast<Cd*>(solve_raw);
+  Cd* lcol = dinv + K;
+  int* perm = reinterpret_cast<int*>(lcol + K);   // factored row -> row
+  int* place = perm + K;                          // row -> factored row
+  Cd* sh = reinterpret_cast<Cd*>(place + K + (K & 1) * 2);
+  Cd* A = kWhere < 2 ? sh : X + KK;
+  Cd* Y = kWhere < 1 ? sh + KK : X + 2 * KK;
+  // Unknown u of the class: element 0's orders of parity p, then element 1's of the other.
+  const int n_a = (K + 1 - p) / 2;
+  auto element = [&](int u) { return u >= n_a; };
+  auto order = [&](int u) { return u < n_a ? 2 * u + p : 2 * (u - n_a) + 1 - p; };
   const cdd s = mkc(g.s_re, g.s_im);
   const cdd mis = -ddm::times_i(s), mi = mkc(0.0, -1.0);
-  auto Jv = [&](int o, int p, int b, int64_t e) { return ldc(J + 4 * (((o * 2 + p) * 2 + b) * KK + e)); };
+  auto Jv = [&](int o, int q, int b, int64_t e) { return ldc(J + 4 * (((o * 2 + q) * 2 + b) * KK + e)); };
   // RgQ11 = -i s J12 - i J21, RgQ12 = -i s J11 - i J22, RgQ21 = -i s J22 - i J11,
   // RgQ22 = -i s J21 - i J12 (ebcm.py:189-195) of the regular J, and Q = RgQ + its y-part
   // (tm_surface_kernel); element (row, col) of Q goes to (col, row).
-  for (int64_t idx = t; idx < NN; idx += blockDim.x) {
-    const int row = (int)(idx / n2), col = (int)(idx % n2);
-    const int bi = row >= K, bk = col >= K;
-    const int64_t e = (int64_t)(row - bi * K) * K + (col - bk * K);
-    cdd q[2];
-    if (!bi && !bk) q[0] = mis * Jv(0, 0, 1, e) + mi * Jv(0, 1, 0, e);
-    else if (!bi && bk) q[0] = mis * Jv(0, 0, 0, e) + mi * Jv(0, 1, 1, e);
-    else if (bi && !bk) q[0] = mis * Jv(0, 1, 1, e) + mi * Jv(0, 0, 0, e);
-    else q[0] = mis * Jv(0, 1, 0, e) + mi * Jv(0, 0, 1, e);
-    q[1] = q[0] + Jv(1, bi, bk, e);
-    const int64_t tr = (int64_t)col * n2 + row;
-    stc(Qd + 4 * tr, q[1]);
-    stc(Bd + 4 * tr, -q[0]);
-    A[tr] = Cd{q[1].re.hi + q[1].re.lo, q[1].im.hi + q[1].im.lo};
-    X[tr] = Cd{-(q[0].re.hi + q[0].re.lo), -(q[0].im.hi + q[0].im.lo)};
+  for (int64_t idx = t; idx < KK; idx += kSolveThreads) {
+    const int row = (int)(idx / K), col = (int)(idx % K);
+    const int bi = element(row), bk = element(col);
+    const int64_t e = (int64_t)order(row) * K + order(col);
+    cdd q0;
+    if (!bi && !bk) q0 = mis * Jv(0, 0, 1, e) + mi * Jv(0, 1, 0, e);
+    else if (!bi && bk) q0 = mis * Jv(0, 0, 0, e) + mi * Jv(0, 1, 1, e);
+    else if (bi && !bk) q0 = mis * Jv(0, 1, 1, e) + mi * Jv(0, 0, 0, e);
+    else q0 = mis * Jv(0, 1, 0, e) + mi * Jv(0, 0, 1, e);
+    const cdd q1 = q0 + Jv(1, bi, bk, e);
+    const int64_t tr = (int64_t)col * K + row;
+    stc(Qd + 4 * tr, q1);
+    stc(Bd + 4 * tr, -q0);
+    A[tr] = Cd{q1.re.hi + q1.re.lo, q1.im.hi + q1.im.lo};
   }
   __syncthreads();
   // Each equation scaled by the power of two that brings its largest coefficient to [1, 2):
   // the unscaled radial functions give the rows magnitudes over hundreds of decades, and
   // partial pivoting is only as good as the rows' balance. Exact, and the solution is unchanged.
-  for (int r = t; r < n2; r += blockDim.x) {
+  for (int r = warp; r < K; r += kSolveWarps) {
     double mx = 0.0;
-    for (int c = 0; c < n2; ++c) {
-      const Cd v = A[(int64_t)r * n2 + c];
+    for (int c = lane; c < K; c += 32) {
+      const Cd v = A[(int64_t)r * K + c];
       mx = fmax(mx, fmax(fabs(v.re), fabs(v.im)));
     }
+    mx = warp_max(mx);
+    if (lane == 0) perm[r] = r;
     if (!(mx > 0.0) || !isfinite(mx)) continue;
     const int e = -ilogb(mx);
-    for (int c = 0; c < n2; ++c) {
-      const int64_t idx = (int64_t)r * n2 + c;
+    for (int c = lane; c < K; c += 32) {
+      const int64_t idx = (int64_t)r * K + c;
       A[idx] = Cd{ldexp(A[idx].re, e), ldexp(A[idx].im, e)};
-      X[idx] = Cd{ldexp(X[idx].re, e), ldexp(X[idx].im, e)};
-      for (int p = 0; p < 4; ++p) {
-        Qd[4 * idx + p] = ldexp(Qd[4 * idx + p], e);
-        Bd[4 * idx + p] = ldexp(Bd[4 * idx + p], e);
+      for (int q = 0; q < 4; ++q) {
+        Qd[4 * idx + q] = ldexp(Qd[4 * idx + q], e);
+        Bd[4 * idx + q] = ldexp(Bd[4 * idx + q], e);
       }
     }
   }
   __syncthreads();
   // LU of A with partial pivoting (the largest modulus, the first row on ties).
-  for (int kk = 0; kk < n2; ++kk) {
+  for (int kk = 0; kk < K; ++kk) {
     double best = -1.0;
-    int bi = kk;
-    for (int r = kk + t; r < n2; r += blockDim.x) {
-      const Cd v = A[(int64_t)r * n2 + kk];
-      const double mag = hypot(v.re, v.im);
+    int at = kk;
+    for (int r = kk + lane; r < K; r += 32) {
+      const Cd v = A[(int64_t)r * K + kk];
+      const double mag = v.re * v.re + v.im * v.im;
       if (mag > best) {
         best = mag;
-        bi = r;
+        at = r;
       }
     }
-    red_v[t] = best;
-    red_i[t] = bi;
-    __syncthreads();
-    for (int off = 128; off > 0; off >>= 1) {
-      if (t < off) {
-        const double ov = red_v[t + off];
-        const int oi = red_i[t + off];
-        if (ov > red_v[t] || (ov == red_v[t] && oi < red_i[t])) {
-          red_v[t] = ov;
-          red_i[t] = oi;
-        }
+    for (int off = 16; off > 0; off >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, off);
+      const int oa = __shfl_xor_sync(0xffffffffu, at, off);
+      if (ob > best || (ob == best && oa < at)) {
+        best = ob;
+        at = oa;
       }
-      __syncthreads();
     }
-    const int p = red_i[0];
-    const bool singular = !(red_v[0] > 0.0);
-    __syncthreads();
-    if (singular) {
+    if (!(best > 0.0)) {  // the same in every warp
       if (t == 0) atomicExch(a.err, 1u);
       return;
     }
-    if (t == 0) piv[kk] = p;
-    if (p != kk)
-      for (int c = t; c < n2; c += blockDim.x) {
-        const Cd x = A[(int64_t)kk * n2 + c];
-        A[(int64_t)kk * n2 + c] = A[(int64_t)p * n2 + c];
-        A[(int64_t)p * n2 + c] = x;
+    const Cd inv = crecip(A[(int64_t)at * K + kk]);
+    // Column kk itself is rewritten after the barrier, so that a warp still searching reads it
+    // whole.
+    for (int r = kk + 1 + t; r < K; r += kSolveThreads)
+      lcol[r] = cmul(A[(int64_t)(r == at ? kk : r) * K + kk], inv);
+    const Cd pivot = A[(int64_t)at * K + kk];
+    if (at != kk)
+      for (int c = t; c < K; c += kSolveThreads)
+        if (c != kk) {
+          const Cd x = A[(int64_t)kk * K + c];
+          A[(int64_t)kk * K + c] = A[(int64_t)at * K + c];
+          A[(int64_t)at * K + c] = x;
+        }
+    __syncthreads();
+    if (t == 0) {
+      dinv[kk] = inv;
+      A[(int64_t)kk * K + kk] = pivot;
+      const int x = perm[kk];
+      perm[kk] = perm[at];
+      perm[at] = x;
+    }
+    for (int c = kk + lane; c < K; c += 32) {
+      const Cd u = A[(int64_t)kk * K + c];
+      for (int r = kk + 1 + warp; r < K; r += kSolveWarps) {
+        const int64_t idx = (int64_t)r * K + c;
+        A[idx] = c == kk ? lcol[r] : cfms(A[idx], lcol[r], u);
       }
-    __syncthreads();
-    const Cd pv = A[(int64_t)kk * n2 + kk];
-    for (int r = kk + 1 + t; r < n2; r += blockDim.x)
-      A[(int64_t)r * n2 + kk] = cdiv(A[(int64_t)r * n2 + kk], pv);
-    __syncthreads();
-    const int w = n2 - kk - 1;
-    for (int idx = t; idx < w * w; idx += blockDim.x) {
-      const int r = kk + 1 + idx / w, c = kk + 1 + idx % w;
-      A[(int64_t)r * n2 + c] =
-          csub(A[(int64_t)r * n2 + c], cmul(A[(int64_t)r * n2 + kk], A[(int64_t)kk * n2 + c]));
     }
     __syncthreads();
   }
-  for (int c = t; c < n2; c += blockDim.x) lu_apply(A, piv, X, n2, c);
+  for (int r = t; r < K; r += kSolveThreads) place[perm[r]] = r;
   __syncthreads();
-  // Residual sweeps: R = -P^T - Q^T X with the products and sums in double-double.
+  for (int64_t idx = t; idx < KK; idx += kSolveThreads) {
+    const int r = (int)(idx / K), c = (int)(idx % K);
+    const double* b = Bd + 4 * idx;
+    Y[(int64_t)place[r] * K + c] = Cd{b[0] + b[1], b[2] + b[3]};
+  }
+  __syncthreads();
+  solve_columns(A, dinv, Y, K, warp, lane);
+  __syncthreads();
+  for (int64_t idx = t; idx < KK; idx += kSolveThreads) X[idx] = Y[idx];
+  __syncthreads();
+  // Residual sweeps: R = -P^T - Q^T X, every product exact and the sums compensated (about
+  // 2^-106 of |Q^T| |X|, as mixed-precision refinement needs), four rows at a time per thread.
   double rel = 0.0;
   for (int sweep = 0; sweep < a.max_sweeps; ++sweep) {
-    double xm = 0.0, rm = 0.0;
-    for (int64_t idx = t; idx < NN; idx += blockDim.x) {
-      const int i = (int)(idx / n2), c = (int)(idx % n2);
-      cdd acc = ldc(Bd + 4 * idx);
-      const double* qrow = Qd + 4 * (int64_t)i * n2;
-      for (int j = 0; j < n2; ++j) {
-        const cdd qv = ldc(qrow + 4 * j);
-        const Cd x = X[(int64_t)j * n2 + c];
-        // The residual's accuracy is measured against its terms (2^-106 of |Q^T| |X|), as
-        // mixed-precision refinement needs.
-        acc = ddm::sub_terms(acc, cdd{ddm::add_terms(qv.re * x.re, -(qv.im * x.im)),
-                                      ddm::add_terms(qv.re * x.im, qv.im * x.re)});
+    for (int i0 = 4 * warp; i0 < K; i0 += 4 * kSolveWarps)
+      for (int c = lane; c < K; c += 32) {
+        double sr[4], si[4], er[4], ei[4];  // the sums and their errors
+        const double* q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = min(i0 + i, K - 1);
+          const double* b = Bd + 4 * ((int64_t)row * K + c);
+          sr[i] = b[0];
+          er[i] = b[1];
+          si[i] = b[2];
+          ei[i] = b[3];
+          q[i] = Qd + 4 * (int64_t)row * K;
+        }
+        for (int j = 0; j < K; ++j) {
+          const Cd x = X[(int64_t)j * K + c];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const double2 re = *reinterpret_cast<const double2*>(q[i] + 4 * j);
+            const double2 im = *reinterpret_cast<const double2*>(q[i] + 4 * j + 2);
+            auto sub = [](double& sum, double& err, double hi, double lo, double v) {
+              const double h = hi * v;
+              const dd w = ddm::two_sum(sum, -h);
+              sum = w.hi;
+              err += w.lo - fma(lo, v, fma(hi, v, -h));
+            };
+            sub(sr[i], er[i], re.x, re.y, x.re);
+            sub(sr[i], er[i], im.x, im.y, -x.im);
+            sub(si[i], ei[i], re.x, re.y, x.im);
+            sub(si[i], ei[i], im.x, im.y, x.re);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i0 + i < K)
+            Y[(int64_t)place[i0 + i] * K + c] = Cd{sr[i] + er[i], si[i] + ei[i]};
       }
-      const Cd rv{acc.re.hi + acc.re.lo, acc.im.hi + acc.im.lo};
-      R[idx] = rv;
-      const Cd xv = X[idx];
-      xm = fmax(xm, fmax(fabs(xv.re), fabs(xv.im)));
-    }
     __syncthreads();
-    for (int c = t; c < n2; c += blockDim.x) lu_apply(A, piv, R, n2, c);
+    solve_columns(A, dinv, Y, K, warp, lane);
     __syncthreads();
-    for (int64_t idx = t; idx < NN; idx += blockDim.x) {
-      const Cd d = R[idx];
+    double xm = 0.0, rm = 0.0;
+    for (int64_t idx = t; idx < KK; idx += kSolveThreads) {
+      const Cd x = X[idx], d = Y[idx];
+      xm = fmax(xm, fmax(fabs(x.re), fabs(x.im)));
       rm = fmax(rm, fmax(fabs(d.re), fabs(d.im)));
-      X[idx] = Cd{X[idx].re + d.re, X[idx].im + d.im};
+      X[idx] = Cd{x.re + d.re, x.im + d.im};
     }
-    xm = block_max(xm, red_v);
-    rm = block_max(rm, red_v);
+    xm = warp_max(xm);
+    rm = warp_max(rm);
+    if (lane == 0) {
+      red[0][warp] = xm;
+      red[1][warp] = rm;
+    }
+    __syncthreads();
+    for (int w = 0; w < kSolveWarps; ++w) {
+      xm = fmax(xm, red[0][w]);
+      rm = fmax(rm, red[1][w]);
+    }
+    __syncthreads();
     rel = xm > 0.0 ? rm / xm : 0.0;
     if (!(rel > 0x1p-54)) break;
   }
-  // T[i][k] = X[k][i].
+  // T[i][k] = X[k][i], zero between the classes.
   double ext = 0.0, sca = 0.0;
   double* T = a.T ? a.T + 2 * jb.T0 : nullptr;
-  for (int64_t idx = t; idx < NN; idx += blockDim.x) {
-    const int i = (int)(idx / n2), k = (int)(idx % n2);
-    const Cd v = X[(int64_t)k * n2 + i];
+  for (int64_t idx = t; idx < 2 * KK; idx += kSolveThreads) {
+    const int u = (int)(idx / (2 * K)), col = (int)(idx % (2 * K));
+    const int bk = col >= K, ko = col - bk * K;
+    Cd v{0.0, 0.0};
+    if (((ko + bk) & 1) == p) {
+      const int w = bk ? n_a + ko / 2 : ko / 2;
+      v = X[(int64_t)w * K + u];
+      if (w == u) ext -= v.re;
+      sca += v.re * v.re + v.im * v.im;
+    }
     if (T) {
-      T[2 * idx] = v.re;
-      T[2 * idx + 1] = v.im;
+      const int64_t row = order(u) + (element(u) ? K : 0);
+      T[2 * (row * 2 * K + col)] = v.re;
+      T[2 * (row * 2 * K + col) + 1] = v.im;
     }
-    if (i == k) ext -= v.re;
-    sca += v.re * v.re + v.im * v.im;
   }
-  sums[0][t] = ext;
-  sums[1][t] = sca;
+  ext = warp_sum(ext);
+  sca = warp_sum(sca);
+  if (lane == 0) {
+    red[0][warp] = ext;
+    red[1][warp] = sca;
+  }
   __syncthreads();
-  for (int off = 128; off > 0; off >>= 1) {
-    if (t < off) {
-      sums[0][t] += sums[0][t + off];
-      sums[1][t] += sums[1][t + off];
-    }
-    __syncthreads();
-  }
   if (t == 0) {
-    a.sums[3 * blockIdx.x] = sums[0][0];
-    a.sums[3 * blockIdx.x + 1] = sums[1][0];
-    a.sums[3 * blockIdx.x + 2] = rel;
+    for (int w = 1; w < kSolveWarps; ++w) {
+      ext += red[0][w];
+      sca += red[1][w];
+    }
+    double* o = a.sums + 3 * (2 * (int64_t)job + p);
+    o[0] = ext;
+    o[1] = sca;
+    o[2] = rel;
   }
 }
 
@@ -924,14 +1006,22 @@ void launch_tm_surface(const TmArgs& a, cudaStream_t s) {
   if (a.n_jobs <= 0) return;
   tm_surface_kernel<<<(unsigned)((a.n_pair_total + 127) / 128), 128, 0, s>>>(a);
 }
-void launch_tm_solve(const TmArgs& a, cudaStream_t s) {
-  if (a.n_jobs <= 0) return;
-  tm_solve_kernel<<<a.n_jobs, 256, 0, s>>>(a);
+// The solves in groups of similar K, each with the shared memory its largest needs: both matrices
+// up to 80 unknowns, the factors up to 112, neither beyond.
+cudaError_t launch_tm_solve(const TmArgs& a, const TmSolveGroup* groups, int n_groups,
+                            cudaStream_t s) {
+  for (int k = 0; k < n_groups; ++k) {
+    const TmSolveGroup& g = groups[k];
+    if (g.n == 0) continue;
+    const int where = tm_solve_where(g.max_k);
+    const size_t head = (size_t)g.max_k * (2 * sizeof(Cd) + 2 * sizeof(int)) + 16;
+    const size_t bytes = head + (size_t)(2 - where) * g.max_k * g.max_k * sizeof(Cd);
+    auto f = where == 0 ? tm_solve_kernel<0> : where == 1 ? tm_solve_kernel<1> : tm_solve_kernel<2>;
+    const cudaError_t e =
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    f<<<2 * g.n, kSolveThreads, bytes, s>>>(a, a.solve_list + g.first);
+  }
+  return cudaGetLastError();
 }
-void launch_tmatrix(const TmArgs& a, cudaStream_t s) {
-  launch_tm_tables(a, s);
-  launch_tm_surface(a, s);
-  launch_tm_solve(a, s);
-}
-
 }  // namespace sb
