@@ -236,7 +236,8 @@ struct Context {
   // Spheroid T-matrices.
   DevBuf tm_geoms, tm_jobs, tm_rules, tm_node, tm_rad, tm_ang, tm_ser, tm_J, tm_work, tm_list, tm_T,
       tm_sums, tm_err;
-  DevBuf ro_sph, ro_rank, ro_w, ro_part, ro_f, ro_greek, ro_mu, ro_proj;
+  DevBuf ro_sph, ro_rank, ro_w, ro_part, ro_f, ro_greek, ro_mu, ro_proj, ro_cgr, ro_cgw;
+  RoCg ro_cg{0};  // the reach of ro_cgr and ro_cgw
   DevBuf p1_fr, p1_ml;  // layered parts of an adaptive call
   DevBuf p1_ml_aug;     // their indices with a vacuum shell (a single radius's radius)
   std::map<int64_t, std::vector<double>> dd_rules;  // n -> per node x (hi, lo), w (hi, lo)
@@ -3034,18 +3035,14 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
         e.f0 = f;
         e.g0 = g;
         e.mu0 = (int64_t)mus.size();
-        e.t_rank = r.n_rank;
-        e.t_w = r.n_w;
         e.t_phi = r.n_phi;
         e.t_f = r.n_f;
         e.t_g = r.n_g;
         rank += 2 * 4 * n1 * n1 * S;
-        w += 2 * Q * 4 * S * n1;
+        w += 2 * Q * 4 * S * e.N;
         part += 2 * Q * 16 * e.nq;
         f += 6 * e.nq;
         g += 6 * (e.L + 1);
-        r.n_rank += (int64_t)e.N * e.N;
-        r.n_w += Q * 2 * e.N;
         r.n_phi += Q * ((e.nq + 31) / 32);  // blocks: a tile of 32 cosines per q
         r.max_n = std::max(r.max_n, e.N);
         r.n_f += e.nq;
@@ -3057,6 +3054,17 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       }
       r.sph = c.ro_sph.as<RoSph>(sph.size());
       r.n_sph = (int)sph.size();
+      // The coefficient tables, for the largest order met so far (they depend on nothing else).
+      if (c.ro_cg.n < r.max_n) {
+        c.ro_cg.n = std::min(kRoMaxN, (r.max_n + 7) / 8 * 8);
+        launch_cg(c.ro_cg, c.ro_cgr.as<double>((size_t)c.ro_cg.r_size()),
+                  c.ro_cgw.as<double>((size_t)c.ro_cg.w_size()), s);
+        SB_CUDA(cudaGetLastError());
+        g_launches++;
+      }
+      r.cg = c.ro_cg;
+      r.cg_r = c.ro_cgr.as<double>(0);
+      r.cg_w = c.ro_cgw.as<double>(0);
       r.jobs = a.jobs;
       r.T = a.T;
       r.rank = c.ro_rank.as<double>((size_t)rank);
@@ -3073,8 +3081,8 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       SB_CUDA(cudaMemcpyAsync(mu_d, mus.data(), mus.size() * 8, cudaMemcpyHostToDevice, s));
       SB_CUDA(cudaMemcpyAsync((void*)proj_d, projs.data(), projs.size() * sizeof(double*),
                               cudaMemcpyHostToDevice, s));
-      timed_launch(K_RANDOM, s, [&] { launch_random(r, s); });
-      SB_CUDA(cudaGetLastError());
+      timed_launch(K_RANDOM, s, [&] { le = launch_random(r, s); });
+      SB_CUDA(le);
       greek_all.resize((size_t)g);
       SB_CUDA(cudaMemcpyAsync(greek_all.data(), r.greek, (size_t)g * 8, cudaMemcpyDeviceToHost, s));
     }
@@ -6756,7 +6764,7 @@ void scatrs_release(void) {
                       &c.counter, &c.values, &c.phase, &c.greek, &c.user.ge, &c.user.go,
                       &c.user.map, &c.user.rows_d, &c.tc_a_hi, &c.tc_a_lo, &c.tc_prod, &c.tc_err, &c.xdig,
                       &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.i8_err,
-                      &c.i8.dig, &c.i8.scale, &c.i8.user_d, &c.i8.band_d})
+                      &c.i8.dig, &c.i8.scale, &c.i8.user_d, &c.i8.band_d, &c.ro_cgr, &c.ro_cgw})
       b->release();
     for (auto& kv : c.projectors)
       for (DevBuf* b : {&kv.second.d, &kv.second.d_hi, &kv.second.d_lo}) b->release();

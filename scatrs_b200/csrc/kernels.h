@@ -556,26 +556,57 @@ cudaError_t launch_tm_solve(const TmArgs& a, const TmSolveGroup* groups, int n_g
 struct RoSph {
   int N, nq, L, job0;
   int64_t rank0;  // [4][N+1][N+1][2N+1] complex
-  int64_t w0;     // [2N+3][2][2][2N+1][N+1] complex
+  int64_t w0;     // [2N+3][2][2][N][2N+1] complex
   int64_t part0;  // [2N+3][16][nq] complex
   int64_t f0;     // [6][nq]
   int64_t g0;     // [6][L+1]
   int64_t mu0;    // nq Gauss nodes
-  int64_t t_rank, t_w, t_phi, t_f, t_g;  // first thread of each kernel (ro_phi: first block)
+  int64_t t_phi, t_f, t_g;  // first thread of each kernel (ro_phi: first block)
 };
+// The Clebsch-Gordan tables up to order n (ro_cg_kernel): where a vector starts.
+struct RoCg {
+  int n;
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  // C^{s 0}_{k u; kp -u}, k <= kp, 0 <= u <= k: 2k + 1 places, s from kp - k. The vectors of the
+  // smaller k come first: sum over j < k of (n - j + 1) (j + 1) (2j + 1), from j = 1.
+  inline int64_t r_row(int64_t k, int64_t kp, int64_t u) const {
+    const int64_t j = k - 1;  // the sum's last term
+    const int64_t s1 = j * (j + 1) / 2, s2 = j * (j + 1) * (2 * j + 1) / 6, s3 = s1 * s1;
+    // (n + 1 - j)(2 j^2 + 3 j + 1) = -2 j^3 + (2 n - 1) j^2 + (3 n + 2) j + (n + 1)
+    const int64_t before = -2 * s3 + (2 * (int64_t)n - 1) * s2 + (3 * (int64_t)n + 2) * s1 +
+                           ((int64_t)n + 1) * j;
+    return before + ((kp - k) * (k + 1) + u) * (2 * k + 1);
+  }
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  // C^{s, m - 1}_{k m; kp -1}, |m| <= k, kp = 1..n: 2k + 1 places, s from |k - kp|.
+  inline int64_t w_row(int64_t k, int64_t m, int64_t kp) const {
+    const int64_t before = (k * (4 * k * k - 1) / 3 - 1) * n;  // sum of (2j + 1)^2 n, 1 <= j < k
+    return before + ((m + k) * n + kp - 1) * (2 * k + 1);
+  }
+  int64_t r_size() const { return r_row(n + 1, n + 1, 0); }
+  int64_t w_size() const { return w_row(n + 1, -(int64_t)(n + 1), 1); }
+};
+void launch_cg(const RoCg& cg, double* r, double* w, cudaStream_t s);
 struct RoArgs {
   const RoSph* sph;
   int n_sph;
-  int64_t n_rank, n_w, n_phi, n_f, n_g;  // threads of each kernel (ro_phi: blocks)
+  int64_t n_phi, n_f, n_g;  // threads of each kernel (ro_phi: blocks)
   int max_n;                              // the batch's largest N
   const TmJob* jobs;
   const double* T;  // the batch's T-matrices (complex doubles at each job's T0)
   double *rank, *w, *part, *f, *greek;
   const double* mu;
+  RoCg cg;  // the coefficient tables (cg.n at least max_n)
+  const double* cg_r;
+  const double* cg_w;
   const double* const* proj;  // per spheroid: [4][nq][L+1] of (2l+1)/2 w_k d_l(mu_k)
 };
 constexpr int kRoMaxN = 120;  // the largest truncation the orientation average takes
-void launch_random(const RoArgs& a, cudaStream_t s);
+cudaError_t launch_random(const RoArgs& a, cudaStream_t s);
 
 void launch_greek_fp64(const double* phase, int64_t n_units, int n_q, int len, const double* d,
                        double* greek, cudaStream_t s);
