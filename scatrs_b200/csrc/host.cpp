@@ -2895,7 +2895,7 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       double b = 8.0 * ((double)nq * (t.N + 1) * 6 + 32.0 * K * K + 28.0 * K * K +
                         (t_out || ro ? 2.0 * n2 * n2 : 0.0)) + 4.0;
       if (new_geom)
-        b += 8.0 * ((double)nq * 16 + (double)nq * (t.N + 1) * 20 +
+        b += 8.0 * ((double)nq * 28 + (double)nq * (t.N + 1) * 20 +
                     (double)t.n_theta * (t.N + 1) * tm_series_slot(t.N));
       if (ro && new_geom) {
         if (t.m != 0 || t.N > kRoMaxN)
@@ -2964,7 +2964,7 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
     a.jobs = c.tm_jobs.as<TmJob>(jobs.size());
     double* rl = c.tm_rules.as<double>(rules.size());
     a.rule = rl;
-    a.node = c.tm_node.as<double>(16 * (size_t)nodes);
+    a.node = c.tm_node.as<double>(28 * (size_t)nodes);
     a.rad = c.tm_rad.as<double>((size_t)rad);
     a.ang = c.tm_ang.as<double>((size_t)ang);
     a.ser = c.tm_ser.as<double>((size_t)ser);

@@ -523,7 +523,8 @@ struct TmArgs {
   int n_jobs;
   int64_t n_node_total, n_ang_total, n_pair_total;
   const double* rule;  // per rule node: x (hi, lo), w (hi, lo)
-  double* node;        // [node][16]: r, 1/r, nu_theta, weight factor (dd), s r (cdd), cos, sin (dd)
+  double* node;        // [node][28]: r, 1/r, (4 unused), s r (cdd), cos, sin (dd), then the surface
+                       // integrals' constants (tm_geom_kernel)
   double* rad;
   double* ang;
   double* J;

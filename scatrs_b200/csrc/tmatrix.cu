@@ -48,7 +48,7 @@ using ddm::mkdd;
 
 namespace {
 
-constexpr int kNodeD = 16;  // doubles per node
+constexpr int kNodeD = 28;  // doubles per node
 constexpr int kRadD = 20;   // doubles per (node, order): j, j', y, y' (dd), w, w', w/(s r) (cdd)
 constexpr int kAngD = 6;    // doubles per (node, order): d, pi, tau (dd)
 constexpr double kPiHi = 3.141592653589793, kPiLo = 1.2246467991473532e-16;
@@ -98,13 +98,20 @@ __global__ void __launch_bounds__(128) tm_geom_kernel(TmArgs a) {
   double* ns = a.node + t * kNodeD;
   st(ns + 0, r);
   st(ns + 2, ir);
-  st(ns + 4, -(dr * ir));
-  st(ns + 6, wq * (r * r) * dd{2.0 * kPiHi, 2.0 * kPiLo});
   const cdd s = mkc(g.s_re, g.s_im);
   const cdd sr = s * r;
   stc(ns + 8, sr);
   st(ns + 12, ct);
   st(ns + 14, stt);
+  // The surface integrals' node constants: 2 w r^2 2 pi, that over r^2, nu, nu / r^2, r^2, r^4.
+  const dd nu = -(dr * ir), ir2 = ir * ir, fac = (wq * (r * r) * dd{2.0 * kPiHi, 2.0 * kPiLo}) * 2.0;
+  const dd r2 = r * r;
+  st(ns + 16, fac);
+  st(ns + 18, fac * ir2);
+  st(ns + 20, nu);
+  st(ns + 22, nu * ir2);
+  st(ns + 24, r2);
+  st(ns + 26, r2 * r2);
   double* f = a.rad + g.rad0 + (int64_t)q * (N + 1) * kRadD;
   // j_n(r): ratios rho_n = j_n / j_{n-1} = r / (2n + 1 - r rho_{n+1}) downward from far above
   // N (kept in the j slots), then values upward from j_0 = sin r / r, j_{-1} = cos r / r;
@@ -237,6 +244,7 @@ struct YTab {  // the y-table of one (node, kind)
     const double* q = p + (int64_t)l * 5 * n1 + n;
     return dd{q[0], q[n1]};
   }
+  __device__ double hi(int l, int n) const { return p[(int64_t)l * 5 * n1 + n]; }
   __device__ dd sum(int l, int n) const {
     const double* q = p + ((int64_t)l * 5 + 2) * n1 + n;
     return dd{q[0], q[n1]};
@@ -256,6 +264,13 @@ __device__ __forceinline__ double* forms_slot(const double* ser0, int n_theta, i
   const int64_t n1 = N + 1;
   return const_cast<double*>(ser0) + (int64_t)n_theta * n1 * (j_slot_size(G) + 15 * (int64_t)(G + 1)) +
          (((int64_t)h * n1 + k) * 4 + ts) * 10 * n1;
+}
+
+// 1 / y in double-double from one division and its exact remainder, so that a series' terms cost a
+// product each instead of a double-double division.
+__device__ __forceinline__ dd recip(double y) {
+  const double q = 1.0 / y;
+  return ddm::fast_two_sum(q, q * fma(-q, y, 1.0));
 }
 
 // The number of terms of a series with term ratios x^2 / den(l), l >= 1, until the terms at
@@ -295,12 +310,9 @@ __global__ void __launch_bounds__(128) tm_series_kernel(TmArgs a) {
   const int h = (int)(local / N), n = 1 + (int)(local % N);
   const int64_t JS = j_slot_size(G), n1 = N + 1;
   double* p = a.ser + g.ser0 + ((int64_t)h * n1 + n) * JS;
-  for (int64_t j = 0; j < JS; ++j) p[j] = 0.0;
   double* yb[3];
-  for (int c = 0; c < 3; ++c) {
+  for (int c = 0; c < 3; ++c)
     yb[c] = const_cast<double*>(y_table(a.ser + g.ser0, g.n_theta, N, G, h, c)) + n;
-    for (int64_t j = 0; j < 5 * (int64_t)(G + 1); ++j) yb[c][j * n1] = 0.0;
-  }
   const double* ns = a.node + (g.node0 + g.n_theta + h) * kNodeD;
   const dd r = ld(ns), ir = ld(ns + 2);
   const cdd sr = ldc(ns + 8);
@@ -320,9 +332,13 @@ __global__ void __launch_bounds__(128) tm_series_kernel(TmArgs a) {
     const dd r2 = r * r, ir2 = ir * ir;
     dd v = -ir;
     for (int i = 1; i <= n; ++i) v = (v * (double)(2 * i - 1)) * ir;
-    for (int l = 1; l < Ly; ++l) v = -(v * r2) / (2.0 * l * (2.0 * l - 2.0 * n - 1.0));
+    for (int l = 1; l < Ly; ++l) v = -(v * r2) * recip(2.0 * l * (2.0 * l - 2.0 * n - 1.0));
     dd sum[3] = {mkdd(0.0), mkdd(0.0), mkdd(0.0)};
     double mag[3] = {0.0, 0.0, 0.0};
+    // The sums past a series shorter than the table (the forms read none further).
+    if (Ly <= G)
+      for (int c = 0; c < 3; ++c)
+        for (int f = 0; f < 5; ++f) yb[c][((int64_t)Ly * 5 + f) * n1] = 0.0;
     for (int l = Ly - 1; l >= 0; --l) {
       const dd over = v * ir;
       const dd term[3] = {v, over * (double)(2 * l - n), over};
@@ -348,16 +364,13 @@ __global__ void __launch_bounds__(128) tm_series_kernel(TmArgs a) {
     const cdd sr2 = sr * sr, isr = ddm::inv(sr), isr2 = isr * isr;
     cdd v = mkc(1.0);
     for (int i = 1; i <= n; ++i) {
-      v = v * sr;
-      v = cdd{v.re / (double)(2 * i + 1), v.im / (double)(2 * i + 1)};
+      v = (v * sr) * recip((double)(2 * i + 1));
     }
     cdd sum[3] = {mkc(0.0), mkc(0.0), mkc(0.0)};
     double mag[3] = {0.0, 0.0, 0.0};
     for (int i = 0; i < Lj; ++i) {
       if (i > 0) {
-        const double den = 2.0 * i * (2.0 * i + 2.0 * n + 1.0);
-        v = -(v * sr2);
-        v = cdd{v.re / den, v.im / den};
+        v = -(v * sr2) * recip(2.0 * i * (2.0 * i + 2.0 * n + 1.0));
       }
       if (i < G) {
         const cdd over = v * isr;
@@ -373,6 +386,10 @@ __global__ void __launch_bounds__(128) tm_series_kernel(TmArgs a) {
     for (int c = 0; c < 3; ++c) {
       sum[c] = mkc(0.0);
       mag[c] = 0.0;
+      if (Lj <= G) {
+        stc(jb[c] + 5 * G + 4 * Lj, sum[c]);
+        jb[c][9 * G + 4 + Lj] = 0.0;
+      }
     }
     for (int i = Lj - 1; i >= 0; --i) {
       const cdd over = v * isr;
@@ -393,50 +410,65 @@ __global__ void __launch_bounds__(128) tm_series_kernel(TmArgs a) {
 namespace {
 
 // R+ of one radial product R_t = r^e Y_t(r) J_t(s r) of the y-part at one node: R minus the
-// terms of its Laurent series in r of power <= cut, by the series of its higher powers or as
-// R minus the lower ones, whichever adds less in magnitude (regular.rs:255-311). yk, jk: the
-// kinds of the y_n and j_k factors (0 f, 1 [z f]'/z, 2 f/z); full = R_t at the node, xe = r^e.
-__device__ __forceinline__ void reg_form(const YTab& yt, int Ly, const JSlot& sk, int Lj, int yk,
-                                         int jk, int e, int n, int k, int cut, dd xe, cdd full,
-                                         cdd* out, double* out_abs) {
+// terms of its Laurent series in r of power <= 0 (out[0]) and, with `below`, of power < 0 (out[1]),
+// by the series of its higher powers or as R minus the lower ones, whichever adds less in magnitude
+// (regular.rs:255-311). yk, jk: the kinds of the y_n and j_k factors (0 f, 1 [z f]'/z, 2 f/z);
+// full = R_t at the node, xe = r^e. The magnitudes decide first, in FP64; only the chosen sum runs
+// in double-double. The powers of a product are all even, so the two cuts differ by one term of
+// each l's series (and by the last l).
+__device__ __forceinline__ void reg_forms(const YTab& yt, int Ly, const JSlot& sk, int Lj, int yk,
+                                          int jk, int e, int n, int k, bool below, dd xe, cdd full,
+                                          cdd out[2], double out_abs[2]) {
   const double* jb = sk.jk(jk);
   const int G = sk.G;
   const int base0 = (-n - 1 - (yk > 0)) + (k - (jk > 0)) + e;
-  int l_end = cut >= base0 ? (cut - base0) / 2 + 1 : 0;
-  l_end = min(min(l_end, Ly), G - 1);
-  cdd neg = mkc(0.0), pos = mkc(0.0);
-  double neg_abs = 0.0, pos_abs = 0.0;
-  for (int l = 0; l < l_end; ++l) {
-    const int i_max = (cut - base0 - 2 * l) / 2;
-    const dd yv = yt.term(l, n) * xe;
-    const double ya = fabs(yv.hi);
-    const int ii = max(min(min(i_max, Lj - 1), G - 1), 0);
-    neg = ddm::add_terms(neg, ldc(jb + 4 * ii) * yv);
-    neg_abs += jb[4 * G + ii] * ya;
-    const int from = min(min(i_max + 1, Lj), G);
-    pos = ddm::add_terms(pos, ldc(jb + 5 * G + 4 * from) * yv);
-    pos_abs += jb[9 * G + 4 + from] * ya;
+  // Terms l < l_end[c] reach power <= 0 (c = 0) or <= -2 (c = 1); i <= i0 - l - c.
+  const int i0 = base0 <= 0 ? -base0 / 2 : -1;
+  int l_end[2];
+  l_end[0] = min(min(i0 + 1, Ly), G - 1);
+  l_end[1] = min(min(max(i0, 0), Ly), G - 1);
+  double neg_abs[2] = {0.0, 0.0}, pos_abs[2] = {0.0, 0.0};
+  for (int l = 0; l < l_end[0]; ++l) {
+    const double ya = fabs(yt.hi(l, n) * xe.hi);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (c == 1 && (!below || l >= l_end[1])) continue;
+      const int i_max = i0 - l - c;
+      neg_abs[c] += jb[4 * G + max(min(min(i_max, Lj - 1), G - 1), 0)] * ya;
+      pos_abs[c] += jb[9 * G + 4 + min(min(i_max + 1, Lj), G)] * ya;
+    }
   }
-  const dd ysum = yt.sum(l_end, n) * xe;
-  pos = ddm::add_terms(pos, ldc(jb + 5 * G) * ysum);
-  pos_abs += jb[9 * G + 4] * yt.mag(l_end, n) * fabs(xe.hi);
-  const double sub_abs = fabs(full.re.hi) + fabs(full.im.hi) + neg_abs;
-  if (pos_abs <= sub_abs) {
-    *out = pos;
-    *out_abs = pos_abs;
-  } else {
-    *out = ddm::sub_terms(full, neg);
-    *out_abs = sub_abs;
+  bool take_pos[2];
+  cdd sum[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    if (c == 1 && !below) continue;
+    pos_abs[c] += jb[9 * G + 4] * yt.mag(l_end[c], n) * fabs(xe.hi);
+    const double sub_abs = fabs(full.re.hi) + fabs(full.im.hi) + neg_abs[c];
+    take_pos[c] = pos_abs[c] <= sub_abs;
+    out_abs[c] = take_pos[c] ? pos_abs[c] : sub_abs;
+    sum[c] = mkc(0.0);
+  }
+  for (int l = 0; l < l_end[0]; ++l) {
+    const dd yv = yt.term(l, n) * xe;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (c == 1 && (!below || l >= l_end[1])) continue;
+      const int i_max = i0 - l - c;
+      const double* j = take_pos[c] ? jb + 5 * G + 4 * min(min(i_max + 1, Lj), G)
+                                    : jb + 4 * max(min(min(i_max, Lj - 1), G - 1), 0);
+      sum[c] = ddm::add_terms(sum[c], ldc(j) * yv);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    if (c == 1 && !below) continue;
+    out[c] = take_pos[c]
+                 ? ddm::add_terms(sum[c], ldc(jb + 5 * G) * (yt.sum(l_end[c], n) * xe))
+                 : ddm::sub_terms(full, sum[c]);
   }
 }
 
-// One term c R_t of a y-part integrand (c = alpha or i alpha, im) in the three forms: plain,
-// minus the powers < 0 (|n - k| >= 3) and minus the powers <= 0 (n != k), each with the sum of
-// the magnitudes it adds (kernel.rs:418-442).
-struct Forms3 {
-  cdd v0, v1, v2;
-  double a0, a1, a2;
-};
 // The series' view at one node for a row order n and a column order k.
 struct SerView {
   YTab yt[3];  // y-table of the node per kind
@@ -453,30 +485,6 @@ __device__ __forceinline__ void product_kind(bool even, int ts, int* yk, int* jk
   *yk = v[0];
   *jk = v[1];
   *e = v[2];
-}
-
-// One term c R_t of a y-part integrand (c = alpha or i alpha, im) in the three forms: plain,
-// minus the powers < 0 (|n - k| >= 3) and minus the powers <= 0 (n != k), each with the sum of
-// the magnitudes it adds (kernel.rs:418-442); the regularized forms from the forms table
-// (fs: the pair's slot at the node, row n at offset 0).
-__device__ __forceinline__ void add_type(Forms3& f, const double* fs, int n1, int n, int k,
-                                         cdd full, dd alpha, bool im, dd W) {
-  const dd cw = alpha * W;
-  const double ca = fabs(cw.hi);
-  auto scaled = [&](cdd v) {
-    const cdd x = v * cw;
-    return im ? ddm::times_i(x) : x;
-  };
-  f.v0 = ddm::add_terms(f.v0, scaled(full));
-  f.a0 += ca * (fabs(full.re.hi) + fabs(full.im.hi));
-  if (n == k) return;
-  auto field = [&](int j) { return fs[(int64_t)j * n1]; };
-  f.v2 = ddm::add_terms(f.v2, scaled(cdd{dd{field(0), field(1)}, dd{field(2), field(3)}}));
-  f.a2 += ca * field(4);
-  if (abs(n - k) >= 3) {
-    f.v1 = ddm::add_terms(f.v1, scaled(cdd{dd{field(5), field(6)}, dd{field(7), field(8)}}));
-    f.a1 += ca * field(9);
-  }
 }
 
 }  // namespace
@@ -522,21 +530,19 @@ __global__ void __launch_bounds__(128) tm_forms_kernel(TmArgs a) {
     const dd xe = e == 2 ? r2 : r4;
     const cdd full = jv * (yv * xe);
     double* fs = forms_slot(ser, nh, N, G, h, k, ts) + n;
-    cdd v;
-    double va;
-    reg_form(sv.yt[yk], sv.Ly, sv.sk, sv.Lj, yk, jk, e, n, k, 0, xe, full, &v, &va);
-    fs[0] = v.re.hi;
-    fs[n1] = v.re.lo;
-    fs[2 * n1] = v.im.hi;
-    fs[3 * n1] = v.im.lo;
-    fs[4 * n1] = va;
-    if (abs(n - k) >= 3) {
-      reg_form(sv.yt[yk], sv.Ly, sv.sk, sv.Lj, yk, jk, e, n, k, -1, xe, full, &v, &va);
-      fs[5 * n1] = v.re.hi;
-      fs[6 * n1] = v.re.lo;
-      fs[7 * n1] = v.im.hi;
-      fs[8 * n1] = v.im.lo;
-      fs[9 * n1] = va;
+    const bool below = abs(n - k) >= 3;
+    cdd v[2];
+    double va[2];
+    reg_forms(sv.yt[yk], sv.Ly, sv.sk, sv.Lj, yk, jk, e, n, k, below, xe, full, v, va);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (c == 1 && !below) continue;
+      double* f = fs + (int64_t)5 * c * n1;
+      f[0] = v[c].re.hi;
+      f[n1] = v[c].re.lo;
+      f[2 * n1] = v[c].im.hi;
+      f[3 * n1] = v[c].im.lo;
+      f[4 * n1] = va[c];
     }
   }
 }
@@ -560,117 +566,229 @@ __global__ void __launch_bounds__(128) tm_forms_kernel(TmArgs a) {
 // powers of r whose terms <= 0 integrate, over the element's four types together, to zero when
 // i != k, and those < 0 when |i - k| >= 3 (the spheroid's 1/r^2 is a polynomial in cos theta);
 // removing them removes the catastrophic cancellation of the plain integrals. The form whose
-// magnitude sum is the smallest is kept.
-__global__ void __launch_bounds__(128) tm_surface_kernel(TmArgs a) {
+// magnitude sum is the smallest is kept: the magnitudes are summed first, in FP64, and only the
+// chosen form runs in double-double.
+//
+// One form instead of three (and no state for the others) halves the
+// operations and leaves the reads of the forms table (3 TB/s) as its bound: 196 -> 128 ms per pass
+// of 288 spheroids to x = 21 (3 blocks per SM without spills: the same).
+namespace {
+
+// One (mode, i, k): its rows of the tables and the half surface's sums.
+struct SurfacePair {
+  const double* node;  // the first half node's record
+  const double* ri;    // radial records of orders i and k at it, and their stride
+  const double* rk;
+  const double* ai;  // angular records
+  const double* ak;
+  const double* fs;  // forms of (k, row i)
+  int64_t rad_stride, ang_stride, form_stride;
+  int n1, nh, i, k;
+  double cki, ckk;
+  bool even;
+};
+
+// The magnitude sums of the two integrals in the three forms (plain, without the powers < 0,
+// without those <= 0), with the double-double sums' weights rounded to FP64 (kernel.rs:418-442).
+__device__ __forceinline__ void surface_magnitudes(const SurfacePair& P, double m0[3],
+                                                   double m1[3]) {
+  m0[0] = m0[1] = m0[2] = m1[0] = m1[1] = m1[2] = 0.0;
+  const bool below = abs(P.i - P.k) >= 3;
+  for (int h = 0; h < P.nh; ++h) {
+    const double* ns = P.node + h * kNodeD;
+    const double* ri = P.ri + h * P.rad_stride;
+    const double* rk = P.rk + h * P.rad_stride;
+    const double* ai = P.ai + h * P.ang_stride;
+    const double* ak = P.ak + h * P.ang_stride;
+    const double* fs = P.fs + h * P.form_stride;
+    const double W = ns[18], nup = ns[22], r2 = ns[24], r4 = ns[26], ir = ns[2];
+    const double yr = fabs(ri[4]), ydr = fabs(ri[6]), yo = yr * ir;
+    const double w = fabs(rk[8]) + fabs(rk[10]), wd = fabs(rk[12]) + fabs(rk[14]),
+                 u = fabs(rk[16]) + fabs(rk[18]);
+    double c[4], full[4];  // |weight| and |plain product| of the four terms
+    if (P.even) {
+      const double A2 = fabs(fma(ai[2], ak[2], ai[4] * ak[4]) * W);
+      c[0] = c[3] = A2;
+      c[1] = fabs(ai[4] * ak[0] * nup * P.ckk * W);
+      c[2] = fabs(ai[0] * ak[4] * nup * P.cki * W);
+      full[0] = wd * yr * r2;
+      full[1] = u * yr * r4;
+      full[2] = w * yo * r4;
+      full[3] = w * ydr * r2;
+    } else {
+      const double A1 = fabs(fma(ai[2], ak[4], ai[4] * ak[2]) * W);
+      c[0] = c[1] = A1;
+      c[2] = fabs(ai[2] * ak[0] * nup * P.ckk * W);
+      c[3] = fabs(ai[0] * ak[2] * nup * P.cki * W);
+      full[0] = w * yr * r2;
+      full[1] = wd * ydr * r2;
+      full[2] = u * ydr * r4;
+      full[3] = wd * yo * r4;
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const double f2 = fs[(int64_t)(10 * t + 4) * P.n1];
+      const double f1 = below ? fs[(int64_t)(10 * t + 9) * P.n1] : 0.0;
+      // Terms 0 and 1 (even) or 0 (odd) are the first integral's.
+      double* m = (P.even ? t < 2 : t < 1) ? m0 : m1;
+      m[0] = fma(c[t], full[t], m[0]);
+      m[1] = fma(c[t], f1, m[1]);
+      m[2] = fma(c[t], f2, m[2]);
+    }
+  }
+}
+
+// The two integrals of the y-part in one form (0 plain, 1, 2) and, with kRegular, the regular
+// ones.
+template <bool kRegular>
+__device__ __forceinline__ void surface_sums(const SurfacePair& P, int form, cdd& Y0, cdd& Y1,
+                                             cdd& R0, cdd& R1) {
+  Y0 = Y1 = mkc(0.0);
+  if (kRegular) R0 = R1 = mkc(0.0);
+  const int n1 = P.n1;
+  for (int h = 0; h < P.nh; ++h) {
+    const double* ns = P.node + h * kNodeD;
+    const double* ri = P.ri + h * P.rad_stride;
+    const double* rk = P.rk + h * P.rad_stride;
+    const double* ai = P.ai + h * P.ang_stride;
+    const double* ak = P.ak + h * P.ang_stride;
+    const double* fs = P.fs + h * P.form_stride + (form == 1 ? (int64_t)5 * n1 : 0);
+    const dd ir = ld(ns + 2), W = ld(ns + 18), nup = ld(ns + 22);
+    const dd di = ld(ai), pii = ld(ai + 2), ti = ld(ai + 4);
+    const dd dk = ld(ak), pik = ld(ak + 2), tk = ld(ak + 4);
+    // One term: the form's value at the node times alpha W, times i where im.
+    auto add = [&](cdd& sum, int t, dd alpha, bool im, cdd plain) {
+      cdd v = plain;
+      if (form != 0) {
+        const double* f = fs + (int64_t)10 * t * n1;
+        v = cdd{dd{f[0], f[n1]}, dd{f[2 * n1], f[3 * n1]}};
+      }
+      const cdd x = v * (alpha * W);
+      sum = ddm::add_terms(sum, im ? ddm::times_i(x) : x);
+    };
+    auto product = [&](int at, dd y, dd xe) {  // the plain product; unused in the other forms
+      return form == 0 ? ldc(rk + at) * (y * xe) : mkc(0.0);
+    };
+    dd yr{}, ydr{}, yo{}, r2{}, r4{};
+    if (form == 0) {
+      yr = ld(ri + 4);
+      ydr = ld(ri + 6);
+      yo = yr * ir;
+      r2 = ld(ns + 24);
+      r4 = ld(ns + 26);
+    }
+    if (P.even) {
+      const dd A2 = ddm::add_terms(pii * pik, ti * tk), A3 = ti * dk, A4 = di * tk;
+      if (kRegular) {
+        // MN = j w' A2 - nu k(k+1) j u A3, NM = nu i(i+1) (j/r) w A4 - j' w A2.
+        const cdd w = ldc(rk + 8), wd = ldc(rk + 12), u = ldc(rk + 16);
+        const dd jr = ld(ri), jdr = ld(ri + 2), nu = ld(ns + 20), fac = ld(ns + 16);
+        const cdd mn = ddm::sub_terms(wd * (jr * A2), u * ((jr * A3) * (nu * P.ckk)));
+        const cdd nm = ddm::sub_terms(w * (((jr * ir) * A4) * (nu * P.cki)), w * (jdr * A2));
+        R0 = ddm::add_terms(R0, mn * fac);
+        R1 = ddm::add_terms(R1, nm * fac);
+      }
+      // MN = i A2 R_1 - i k(k+1) A3 nu' R_4, NM = i i(i+1) A4 nu' R_6 - i A2 R_2.
+      add(Y0, 0, A2, true, product(12, yr, r2));
+      add(Y0, 1, -((A3 * nup) * P.ckk), true, product(16, yr, r4));
+      add(Y1, 2, (A4 * nup) * P.cki, true, product(8, yo, r4));
+      add(Y1, 3, -A2, true, product(8, ydr, r2));
+    } else {
+      const dd A1 = ddm::add_terms(pii * tk, ti * pik), A5 = pii * dk, A6 = di * pik;
+      if (kRegular) {
+        // MM = i j w A1, NN = i [j' w' A1 - nu (k(k+1) j' u A5 + i(i+1) (j/r) w' A6)].
+        const cdd w = ldc(rk + 8), wd = ldc(rk + 12), u = ldc(rk + 16);
+        const dd jr = ld(ri), jdr = ld(ri + 2), nu = ld(ns + 20), fac = ld(ns + 16);
+        const cdd mm = ddm::times_i(w * (jr * A1));
+        const cdd nn = ddm::times_i(ddm::sub_terms(
+            wd * (jdr * A1), ddm::add_terms(u * ((jdr * A5) * P.ckk),
+                                            wd * (((jr * ir) * A6) * P.cki)) * nu));
+        R0 = ddm::add_terms(R0, mm * fac);
+        R1 = ddm::add_terms(R1, nn * fac);
+      }
+      // MM = -A1 R_0, NN = -A1 R_3 + k(k+1) A5 nu' R_5 + i(i+1) A6 nu' R_7.
+      add(Y0, 0, -A1, false, product(8, yr, r2));
+      add(Y1, 1, -A1, false, product(12, ydr, r2));
+      add(Y1, 2, (A5 * nup) * P.ckk, false, product(16, ydr, r4));
+      add(Y1, 3, (A6 * nup) * P.cki, false, product(12, yo, r4));
+    }
+  }
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(128, 4) tm_surface_kernel(TmArgs a) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n_pair_total) return;
   const int ji = owner(a.n_jobs, t, [&](int i) { return a.jobs[i].pair0; });
   const TmJob jb = a.jobs[ji];
   const TmGeom g = a.geoms[jb.geom];
   const int N = g.N, m = jb.m, n0 = m > 1 ? m : 1, K = jb.K;
-  // Rows fastest: a warp's threads share the column order k, so its j-slot, and read the
-  // y-table's consecutive orders.
+  // Rows fastest: a warp's threads share the column order k and read the forms table's
+  // consecutive orders.
   const int pr = (int)(t - jb.pair0), i = n0 + pr % K, k = n0 + pr / K;
-  const bool even = ((i + k) & 1) == 0;
-  const int G = N / 2 + 2;
-  const double* ser = a.ser + g.ser0;
-  cdd R0 = mkc(0.0), R1 = mkc(0.0);  // regular: MN, NM (even) or MM, NN (odd)
-  Forms3 Y0, Y1;                     // y-part: the same two
-  Y0.v0 = Y0.v1 = Y0.v2 = Y1.v0 = Y1.v1 = Y1.v2 = mkc(0.0);
-  Y0.a0 = Y0.a1 = Y0.a2 = Y1.a0 = Y1.a1 = Y1.a2 = 0.0;
-
-  const double cki = (double)i * (i + 1), ckk = (double)k * (k + 1);
-  const int nh = g.n_theta;
-  for (int h = 0; h < nh; ++h) {
-    const int q = nh + h;
-    const double* ns = a.node + (g.node0 + q) * kNodeD;
-    const dd ir = ld(ns + 2), nu = ld(ns + 4), fac = ld(ns + 6) * 2.0;
-    const dd r = ld(ns), r2 = r * r, r4 = r2 * r2, ir2 = ir * ir;
-    const dd W = fac * ir2, nup = nu * ir2;
-    const double* ri = a.rad + g.rad0 + ((int64_t)q * (N + 1) + i) * kRadD;
-    const double* rk = a.rad + g.rad0 + ((int64_t)q * (N + 1) + k) * kRadD;
-    const double* ai = a.ang + jb.ang0 + ((int64_t)q * (N + 1) + i) * kAngD;
-    const double* ak = a.ang + jb.ang0 + ((int64_t)q * (N + 1) + k) * kAngD;
-    const dd di = ld(ai), pii = ld(ai + 2), ti = ld(ai + 4);
-    const dd dk = ld(ak), pik = ld(ak + 2), tk = ld(ak + 4);
-    const cdd w = ldc(rk + 8), wd = ldc(rk + 12), u = ldc(rk + 16);
-    const dd jr = ld(ri), jdr = ld(ri + 2), yr = ld(ri + 4), ydr = ld(ri + 6);
-    const dd yo = yr * ir;  // y / r
-    const int n1 = N + 1;
-    const double* fs = forms_slot(ser, nh, N, G, h, k, 0) + i;  // product slot ts at ts 10 n1
-    if (even) {
-      const dd A2 = ddm::add_terms(pii * pik, ti * tk), A3 = ti * dk, A4 = di * tk;
-      // Regular: MN = j w' A2 - nu k(k+1) j u A3, NM = nu i(i+1) (j/r) w A4 - j' w A2.
-      const cdd mn = ddm::sub_terms(wd * (jr * A2), u * ((jr * A3) * (nu * ckk)));
-      const cdd nm = ddm::sub_terms(w * (((jr * ir) * A4) * (nu * cki)), w * (jdr * A2));
-      R0 = ddm::add_terms(R0, mn * fac);
-      R1 = ddm::add_terms(R1, nm * fac);
-      // y-part: MN = i A2 R_1 - i k(k+1) A3 nu' R_4, NM = i i(i+1) A4 nu' R_6 - i A2 R_2.
-      add_type(Y0, fs, n1, i, k, wd * (yr * r2), A2, true, W);
-      add_type(Y0, fs + 10 * n1, n1, i, k, u * (yr * r4), -((A3 * nup) * ckk), true, W);
-      add_type(Y1, fs + 20 * n1, n1, i, k, w * (yo * r4), (A4 * nup) * cki, true, W);
-      add_type(Y1, fs + 30 * n1, n1, i, k, w * (ydr * r2), -A2, true, W);
-    } else {
-      const dd A1 = ddm::add_terms(pii * tk, ti * pik), A5 = pii * dk, A6 = di * pik;
-      // Regular: MM = i j w A1, NN = i [j' w' A1 - nu (k(k+1) j' u A5 + i(i+1) (j/r) w' A6)].
-      const cdd mm = ddm::times_i(w * (jr * A1));
-      const cdd nn = ddm::times_i(ddm::sub_terms(
-          wd * (jdr * A1),
-          ddm::add_terms(u * ((jdr * A5) * ckk), wd * (((jr * ir) * A6) * cki)) * nu));
-      R0 = ddm::add_terms(R0, mm * fac);
-      R1 = ddm::add_terms(R1, nn * fac);
-      // y-part: MM = -A1 R_0, NN = -A1 R_3 + k(k+1) A5 nu' R_5 + i(i+1) A6 nu' R_7.
-      add_type(Y0, fs, n1, i, k, w * (yr * r2), -A1, false, W);
-      add_type(Y1, fs + 10 * n1, n1, i, k, wd * (ydr * r2), -A1, false, W);
-      add_type(Y1, fs + 20 * n1, n1, i, k, u * (ydr * r4), (A5 * nup) * ckk, false, W);
-      add_type(Y1, fs + 30 * n1, n1, i, k, wd * (yo * r4), (A6 * nup) * cki, false, W);
+  const int G = N / 2 + 2, nh = g.n_theta;
+  SurfacePair P;
+  P.node = a.node + (g.node0 + nh) * kNodeD;
+  P.rad_stride = (int64_t)(N + 1) * kRadD;
+  P.ri = a.rad + g.rad0 + nh * P.rad_stride + i * kRadD;
+  P.rk = a.rad + g.rad0 + nh * P.rad_stride + k * kRadD;
+  P.ang_stride = (int64_t)(N + 1) * kAngD;
+  P.ai = a.ang + jb.ang0 + nh * P.ang_stride + i * kAngD;
+  P.ak = a.ang + jb.ang0 + nh * P.ang_stride + k * kAngD;
+  P.fs = forms_slot(a.ser + g.ser0, nh, N, G, 0, k, 0) + i;
+  P.form_stride = (int64_t)(N + 1) * 40 * (N + 1);
+  P.n1 = N + 1;
+  P.nh = nh;
+  P.i = i;
+  P.k = k;
+  P.cki = (double)i * (i + 1);
+  P.ckk = (double)k * (k + 1);
+  P.even = ((i + k) & 1) == 0;
+  // The forms of the two elements of Q this (i, k) feeds: the cleanest, or the one asked for.
+  const double sa = fabs(g.s_re) + fabs(g.s_im);
+  int best[2] = {0, 0};
+  if (a.form >= 0) {
+    if (a.form == 2 && i != k) best[0] = best[1] = 2;
+    if (a.form == 1 && abs(i - k) >= 3) best[0] = best[1] = 1;
+  } else if (i != k) {
+    double m0[3], m1[3];
+    surface_magnitudes(P, m0, m1);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const double* first = e ? m1 : m0;
+      const double* second = e ? m0 : m1;
+      const double of2 = sa * first[2] + second[2];
+      double mb = kPlainBias * (sa * first[0] + second[0]);
+      if (of2 < mb) {
+        best[e] = 2;
+        mb = of2;
+      }
+      if (abs(i - k) >= 3 && sa * first[1] + second[1] < mb) best[e] = 1;
     }
   }
   // g_i g_k = sqrt((2i+1)(2k+1) / (16 pi^2 i(i+1) k(k+1))).
   const dd pi2 = dd{kPiHi, kPiLo} * dd{kPiHi, kPiLo};
   const dd gg = ddm::dd_sqrt((mkdd((double)(2 * i + 1) * (2 * k + 1)) / (pi2 * 16.0)) /
-                             (cki * ckk));
-  // The two elements of Q this (i, k) feeds, with s on the first of their pair:
-  // even: (0, 0) = -i s MN - i NM, (1, 1) = -i s NM - i MN; odd: (0, 1) = -i s MM - i NN,
-  // (1, 0) = -i s NN - i MM.
+                             (P.cki * P.ckk));
+  // With s on the first of their pair: even: (0, 0) = -i s MN - i NM, (1, 1) = -i s NM - i MN;
+  // odd: (0, 1) = -i s MM - i NN, (1, 0) = -i s NN - i MM.
   const cdd s = mkc(g.s_re, g.s_im), mis = -ddm::times_i(s);
-  const double sa = fabs(g.s_re) + fabs(g.s_im);
-  auto element = [&](const Forms3& first, const Forms3& second) {
-    int best = 0;
-    if (a.form >= 0) {
-      if (a.form == 2 && i != k) best = 2;
-      if (a.form == 1 && abs(i - k) >= 3) best = 1;
-    } else if (i != k) {
-      const double m2 = sa * first.a2 + second.a2;
-      double mb = kPlainBias * (sa * first.a0 + second.a0);
-      if (m2 < mb) {
-        best = 2;
-        mb = m2;
-      }
-      if (abs(i - k) >= 3 && sa * first.a1 + second.a1 < mb) best = 1;
-    }
-    const cdd fv = best == 0 ? first.v0 : (best == 1 ? first.v1 : first.v2);
-    const cdd sv = best == 0 ? second.v0 : (best == 1 ? second.v1 : second.v2);
-    return ddm::add_terms(mis * fv, ddm::times_i(sv) * -1.0) * gg;
+  auto element = [&](cdd first, cdd second) {
+    return ddm::add_terms(mis * first, ddm::times_i(second) * -1.0) * gg;
   };
-  cdd out[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) out[c] = mkc(0.0);
-  if (even) {
-    out[1] = R0 * gg;
-    out[2] = R1 * gg;
-    out[4 + 0] = element(Y0, Y1);
-    out[4 + 3] = element(Y1, Y0);
-  } else {
-    out[0] = R0 * gg;
-    out[3] = R1 * gg;
-    out[4 + 1] = element(Y0, Y1);
-    out[4 + 2] = element(Y1, Y0);
-  }
   double* o = a.J + 4 * jb.J0;
   const int64_t KK = (int64_t)K * K, e = (int64_t)(i - n0) * K + (k - n0);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) stc(o + 4 * (c * KK + e), out[c]);
+  // The places J[0..3] of the regular integrals and J[4..7] of the elements; the others are zero
+  // (and not read: the solve takes the two parity classes apart).
+  const int c0 = P.even ? 1 : 0, c1 = P.even ? 2 : 3, e0 = P.even ? 4 : 5, e1 = P.even ? 7 : 6;
+  cdd Y0, Y1, R0, R1;
+  surface_sums<true>(P, best[0], Y0, Y1, R0, R1);
+  stc(o + 4 * (c0 * KK + e), R0 * gg);
+  stc(o + 4 * (c1 * KK + e), R1 * gg);
+  stc(o + 4 * (e0 * KK + e), element(Y0, Y1));
+  if (best[1] != best[0]) surface_sums<false>(P, best[1], Y0, Y1, R0, R1);
+  stc(o + 4 * (e1 * KK + e), element(Y1, Y0));
 }
 namespace {
 
