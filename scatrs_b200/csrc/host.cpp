@@ -179,25 +179,25 @@ struct UserTables {
   std::vector<double> rows;  // each table row's cosine (a cosine, or a pair c, -c)
   int64_t n_orders = 0;
   int h = 0, h_pad = 0, ld = 0;
-  DevBuf ge, go, map, rows_d;
+  DevBuf g, map, rows_d;
 };
 
 // The tables of one Greek order (-1: none): the phase levels the requested cosines allow (see
 // chunk_band; none where the limit is 0), then the projector bands. The bands' G_E and G_O rows
-// are host-made (ge_d, go_d), the levels' made on the device (lge_d, lgo_d).
+// are host-made (g_d), the levels' made on the device (lg_d).
 struct BandTables {
   int order = -1;
   int n_levels = 0;
   int n_bands = 0;                // projector bands
   std::vector<BandDesc> desc;     // the levels, then the bands
   std::vector<BandDesc> bands;
-  std::vector<double> ge, go, d;  // host copies, appended band by band
+  std::vector<double> g, d;       // host copies, appended band by band
   std::vector<int> half0;         // each level's first half node
   std::vector<double> mu;         // the cosines me_d and mo_d interpolate onto
-  DevBuf ge_d, go_d, lge_d, lgo_d, d_d, desc_d, half0_d, x0_d, node_d, me_d, mo_d;
+  DevBuf g_d, lg_d, d_d, desc_d, half0_d, x0_d, node_d, me_d, mo_d;
   int merge_max() const { return n_levels > 0 ? desc[n_levels - 1].upper : 0; }
   void release() {
-    for (DevBuf* b : {&ge_d, &go_d, &lge_d, &lgo_d, &d_d, &desc_d, &half0_d, &x0_d, &node_d, &me_d, &mo_d})
+    for (DevBuf* b : {&g_d, &lg_d, &d_d, &desc_d, &half0_d, &x0_d, &node_d, &me_d, &mo_d})
       b->release();
   }
 };
@@ -205,7 +205,7 @@ struct BandTables {
 struct Context {
   int device = -1;
   int sms = 0;
-  int unit_bps = 1;
+  int unit_bps[4] = {1, 1, 1, 1};  // resident unit-kernel CTAs per SM
   std::mutex mtx;
   UserTables user;
   std::map<std::pair<int, int>, BandTables> bands;  // by Greek order and level limit
@@ -232,7 +232,7 @@ struct Context {
     std::vector<I8Table> user, band;
     DevBuf dig, scale, user_d, band_d;
   } i8;
-  DevBuf xdig, xside, colmax, chunk_xoff, chunk_xidx, i8_list, i8_err;
+  DevBuf xdig, xside, colmax, chunk_xoff, chunk_xidx, i8_list, side;
   // Spheroid T-matrices.
   DevBuf tm_geoms, tm_jobs, tm_rules, tm_node, tm_rad, tm_ang, tm_ser, tm_J, tm_work, tm_list, tm_T,
       tm_sums, tm_err;
@@ -300,7 +300,7 @@ Context& context() {
     cudaDeviceProp prop;
     SB_CUDA(cudaGetDeviceProperties(&prop, dev));
     c->sms = prop.multiProcessorCount;
-    c->unit_bps = unit_kernel_blocks_per_sm();
+    for (int mode = 0; mode < 4; ++mode) c->unit_bps[mode] = unit_kernel_blocks_per_sm(mode);
     g_ctx[dev] = std::move(c);
   }
   return *g_ctx[dev];
@@ -361,20 +361,16 @@ void ensure_user(Context& c, const double* mu, int64_t n_mu, int64_t n_orders, c
   u.rows = cosines;
   u.h_pad = (int)round_up(std::max(u.h, 1), 32);
   u.ld = (int)u.n_orders;
-  // Order-major (transposed) tables: element (row, order k) at k * h_pad + row, so that one
-  // order of a 32-row tile is 256 contiguous bytes.
-  std::vector<double> ge((size_t)u.h_pad * u.ld, 0.0), go((size_t)u.h_pad * u.ld, 0.0);
+  std::vector<double> tab(2 * (size_t)u.h_pad * u.ld, 0.0);
   std::vector<double> re(u.ld), ro(u.ld);
   for (int r = 0; r < u.h; ++r) {
     pi_tau_row(cosines[r], u.n_orders, re.data(), ro.data());
     for (int k = 0; k < u.ld; ++k) {
-      ge[(size_t)k * u.h_pad + r] = re[k];
-      go[(size_t)k * u.h_pad + r] = ro[k];
+      tab[table_at(r, k, u.ld)] = re[k];
+      tab[table_at(r, k, u.ld) + 32] = ro[k];
     }
   }
-  SB_CUDA(cudaMemcpyAsync(u.ge.get(ge.size() * 8), ge.data(), ge.size() * 8,
-                          cudaMemcpyHostToDevice, s));
-  SB_CUDA(cudaMemcpyAsync(u.go.get(go.size() * 8), go.data(), go.size() * 8,
+  SB_CUDA(cudaMemcpyAsync(u.g.get(tab.size() * 8), tab.data(), tab.size() * 8,
                           cudaMemcpyHostToDevice, s));
   if (!map.empty())
     SB_CUDA(cudaMemcpyAsync(u.map.get(map.size() * sizeof(int2)), map.data(),
@@ -475,17 +471,15 @@ BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream
       d.h_pad = (int)round_up(d.h, 32);
       d.d_ld = (int)round_up(order + 1, 32);
       d.ld = (int)round_up(upper, 16);
-      d.g_off = (int64_t)bt.ge.size();
+      d.g_off = (int64_t)bt.g.size();
       d.d_off = (int64_t)bt.d.size();
-      bt.ge.resize(bt.ge.size() + (size_t)d.h_pad * d.ld, 0.0);
-      bt.go.resize(bt.go.size() + (size_t)d.h_pad * d.ld, 0.0);
-      // Order-major, as the requested cosines' tables.
+      bt.g.resize(bt.g.size() + 2 * (size_t)d.h_pad * d.ld, 0.0);
       std::vector<double> re(upper), ro(upper);
       for (int i = 0; i < d.h; ++i) {
         pi_tau_row(r.first[lo + i], upper, re.data(), ro.data());
         for (int64_t k = 0; k < upper; ++k) {
-          bt.ge[d.g_off + (size_t)k * d.h_pad + i] = re[k];
-          bt.go[d.g_off + (size_t)k * d.h_pad + i] = ro[k];
+          bt.g[d.g_off + table_at(i, k, d.ld)] = re[k];
+          bt.g[d.g_off + table_at(i, k, d.ld) + 32] = ro[k];
         }
       }
       append_projection(r, n_q, order + 1, bt.d);
@@ -507,7 +501,7 @@ BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream
     d.ld = 32 * t;
     d.d_ld = (int)round_up(d.order + 1, 32);
     d.g_off = g;
-    g += (int64_t)d.h_pad * d.ld;
+    g += 2 * (int64_t)d.h_pad * d.ld;
     const auto& r = rule(c, d.n_q);
     if (l >= (int)levels.size()) {
       d.d_off = (int64_t)bt.d.size();
@@ -528,8 +522,7 @@ BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream
     void* p = to.get(std::max<size_t>(bytes, 16));
     if (bytes > 0) SB_CUDA(cudaMemcpyAsync(p, from, bytes, cudaMemcpyHostToDevice, s));
   };
-  upload(bt.ge_d, bt.ge.data(), bt.ge.size() * 8);
-  upload(bt.go_d, bt.go.data(), bt.go.size() * 8);
+  upload(bt.g_d, bt.g.data(), bt.g.size() * 8);
   upload(bt.d_d, bt.d.data(), bt.d.size() * 8);
   upload(bt.desc_d, bt.desc.data(), bt.desc.size() * sizeof(BandDesc));
   if (n_levels > bt.n_levels) {
@@ -545,8 +538,7 @@ BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream
     la.x_hi = node;
     la.x_lo = node + n_half;
     la.bary = node + 2 * (size_t)n_half;
-    la.ge = bt.lge_d.as<double>((size_t)g);
-    la.go = bt.lgo_d.as<double>((size_t)g);
+    la.g = bt.lg_d.as<double>((size_t)g);
     launch_level_tables(la, s);
     SB_CUDA(cudaGetLastError());
     g_launches++;
@@ -667,28 +659,23 @@ void ensure_i8(Context& c, int64_t n_max, const BandTables* bt, cudaStream_t s) 
         [&](int pair, int64_t n, double* e, double* o) { pi_tau_row(cosines[pair], n, e, o); },
         dig, scale));
   }
-  std::vector<double> le, lo;  // the levels' rows, made on the device
+  std::vector<double> lg;  // the levels' rows, made on the device
   if (n_levels > 0) {
     const BandDesc& last = bt->desc[n_levels - 1];
-    const size_t n = (size_t)last.g_off + (size_t)last.h_pad * last.ld;
-    le.resize(n);
-    lo.resize(n);
-    SB_CUDA(cudaMemcpyAsync(le.data(), bt->lge_d.p, n * 8, cudaMemcpyDeviceToHost, s));
-    SB_CUDA(cudaMemcpyAsync(lo.data(), bt->lgo_d.p, n * 8, cudaMemcpyDeviceToHost, s));
+    lg.resize((size_t)last.g_off + 2 * (size_t)last.h_pad * last.ld);
+    SB_CUDA(cudaMemcpyAsync(lg.data(), bt->lg_d.p, lg.size() * 8, cudaMemcpyDeviceToHost, s));
     SB_CUDA(cudaStreamSynchronize(s));
   }
   for (int b = 0; b < nb; ++b) {
     const BandDesc& d = bt->desc[b];
     const int n_kb = (d.upper + kI8KB - 1) / kI8KB;
-    const bool level = b < n_levels;
-    const double* ge = (level ? le : bt->ge).data() + d.g_off;
-    const double* go = (level ? lo : bt->go).data() + d.g_off;
+    const double* tab = (b < n_levels ? lg : bt->g).data() + d.g_off;
     T.band.push_back(i8_table(
         d.h, d.upper, n_kb,
         [&](int pair, int64_t n, double* e, double* o) {
           for (int64_t k = 0; k < n; ++k) {
-            e[k] = ge[(size_t)k * d.h_pad + pair];
-            o[k] = go[(size_t)k * d.h_pad + pair];
+            e[k] = tab[table_at(pair, k, d.ld)];
+            o[k] = tab[table_at(pair, k, d.ld) + 32];
           }
         },
         dig, scale));
@@ -760,7 +747,6 @@ struct FixedCall {
   // kI8MaxTerms run their angle GEMMs on int8 digits (unit_i8_kernel); 0 for plain FP64.
   int i8_above = 0;
   int i8_levels = 5;           // product levels kept (5 or 6)
-  unsigned* i8_err = nullptr;  // the int8 kernel's timeout flag, checked with the errors
 };
 
 // The device pipeline; wl_dev and m_dev are device arrays, outputs device arrays.
@@ -903,8 +889,11 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   // of a chunk (two 16-node halves with derivatives).
   // Adaptive calls add the error sums of every block (a second set of n_blk / 2).
   const int n_blk = (dv.on ? 3 + dv.n_theta : 1) * (ad.on ? 2 : 1);
-  const int rows_per_term = dv.on ? 2 : 1;  unsigned long long* err = c.err.as<unsigned long long>(2);
-  SB_CUDA(cudaMemsetAsync(err, 0xff, 2 * sizeof(unsigned long long), s));
+  const int rows_per_term = dv.on ? 2 : 1;
+  // Error words: invalid nodes, undefined ratios, a bounded wait that gave up.
+  unsigned long long* err = c.err.as<unsigned long long>(3);
+  SB_CUDA(cudaMemsetAsync(err, 0xff, 3 * sizeof(unsigned long long), s));
+  unsigned* wait_err = reinterpret_cast<unsigned*>(err + 2);
   // 2. Plan: every chunk's largest number of terms.
   PlanArgs pa{};
   pa.radius = c.radius.as<double>(0);
@@ -945,13 +934,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   // The mixed form: values of the fixed grid only.
   const int i8_above = (call && !ad.on && !dv.on) ? call->i8_above : 0;
   auto on_i8 = [&](int nc) { return i8_above > 0 && nc > i8_above && nc <= kI8MaxTerms; };
-  unsigned* i8_err = nullptr;
-  if (i8_above > 0) {
-    ensure_i8(c, n_max, bt, s);
-    i8_err = c.i8_err.as<unsigned>(1);
-    SB_CUDA(cudaMemsetAsync(i8_err, 0, sizeof(unsigned), s));
-    call->i8_err = i8_err;
-  }
+  if (i8_above > 0) ensure_i8(c, n_max, bt, s);
   // 3. Slabs. Each unit's work: its chunks' rows times the table rows they meet.
   const int nb = bt ? (int)bt->desc.size() : 0;
   std::vector<int> band_of_n(n_max + 1, -1), band_tiles(nb), band_nq(nb);
@@ -977,7 +960,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     int prev = -1, run = 0, slots = 0, max_tiles = 1;
     for (int k = 0; k < cpu; ++k) {
       const int nc = cu[k];
-      rows += (int64_t)rows_per_term * nc;
+      rows += (int64_t)rows_per_term * round_up(nc, 4);
       if (on_i8(nc)) {
         ui8[u] += 2 * (int64_t)((nc + kI8KB - 1) / kI8KB) * kI8HalfBytes;
         ui8n[u] += 1;
@@ -1040,7 +1023,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     n_slabs = (int64_t)slab_lo.size();
   }
   // A large unit's row tiles split into work items of about item_target work each.
-  const int grid_max = c.sms * c.unit_bps;
+  const int grid_max = c.sms * c.unit_bps[(dv.on ? 1 : 0) + (ad.on ? 2 : 0)];
   const double item_target =
       std::max(1.0, total_cost / (double)n_slabs / ((double)g_split.load() * grid_max));
   std::vector<int> ugroups(n_units);
@@ -1169,6 +1152,11 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     ka.m_layers = reinterpret_cast<const double2*>(layers.m_dev);
   }
   ka.X = X;
+  // Weights per node: values, each parameter's, and the same with the error weights.
+  const int side_stride = 32 * (dv.on ? 1 + dv.n_theta : 1) * (ad.on ? 2 : 1) + 4;
+  double* side = c.side.as<double>((size_t)kMaxSlabChunks * side_stride);
+  ka.side = side;
+  ka.side_stride = side_stride;
   ka.colmax = colmax;  // the mixed form's digit scales; null otherwise
   ka.uz = uz;
   ka.ux = ux;
@@ -1187,36 +1175,28 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     if (dv.on) ka.wthdiff = c.wthdiff.as<double>(0);
   }
   UnitArgs ua{};
-  ua.radius = ka.radius;
-  ua.weight = ka.weight;
-  ua.wl = wl_dev;
-  ua.n_dist = (int)n_dist;
   ua.n_wl = (int)n_wl;
-  ua.n_nodes = (int)n_nodes;
   ua.cpu = cpu;
+  ua.side = side;
+  ua.side_stride = side_stride;
+  ua.wait_err = wait_err;
   ua.X = X;
   ua.n_mu = (int)n_mu;
   ua.h_u = c.user.h;
-  ua.h_u_pad = c.user.h_pad;
-  ua.ge_u = c.user.ge.as<double>(0);
-  ua.go_u = c.user.go.as<double>(0);
+  ua.ld_u = c.user.ld;
+  ua.g_u = c.user.g.as<double>(0);
   ua.user_map = c.user.map.as<int2>(0);
   ua.greek_order = L;
   if (bt) {
     ua.bands = bt->desc_d.as<BandDesc>(0);
-    ua.band_ge = bt->ge_d.as<double>(0);
-    ua.band_go = bt->go_d.as<double>(0);
-    ua.level_ge = bt->lge_d.as<double>(0);
-    ua.level_go = bt->lgo_d.as<double>(0);
+    ua.band_g = bt->g_d.as<double>(0);
+    ua.level_g = bt->lg_d.as<double>(0);
   }
   ua.acc = acc;
   ua.work_counter = counter;
   ua.deriv = ka.deriv;
   ua.n_theta = ka.n_theta;
-  ua.wtheta = ka.wtheta;
-  ua.per_unit = ka.per_unit;
-  ua.wdiff = ka.wdiff;
-  ua.wthdiff = ka.wthdiff;
+  ua.adaptive = ad.on ? 1 : 0;
   ua.i8_above = i8_above;
   ua.n_levels = n_levels;
   ua.merge_max = merge_max;
@@ -1321,7 +1301,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
             xoff += 2 * (int64_t)((nc + kI8KB - 1) / kI8KB) * kI8HalfBytes;
           }
         }
-        row += (int64_t)rows_per_term * nc;
+        row += (int64_t)rows_per_term * round_up(nc, 4);
         P_cacc[ci] = -1;
         if (bt && nc > 0 && band_of_n[nc] >= 0) {
           const int b = band_of_n[nc];
@@ -1442,7 +1422,6 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     SB_CUDA(cudaGetLastError());
     SB_CUDA(cudaMemsetAsync(acc, 0, (size_t)S.acc_len * 8, s));
     SB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), s));
-    ua.units = ka.units;
     ua.n_items = (int)S.n_items;
     ua.items = items_d + S.it0;
     ua.chunk_n = ka.chunk_n;
@@ -1465,24 +1444,24 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       xa.chunk_xidx = chunk_xidx_d + ch0;
       xa.xdig = xdig;
       xa.xside = xside;
-      xa.radius = ua.radius;
-      xa.weight = ua.weight;
+      xa.radius = ka.radius;
+      xa.weight = ka.weight;
       xa.wl = wl_dev;
-      xa.units = ua.units;
+      xa.units = ka.units;
       xa.n_wl = (int)n_wl;
       xa.n_nodes = (int)n_nodes;
       xa.cpu = cpu;
       timed_launch(K_X_SPLIT, s, [&] { launch_x_split(xa, s); });
       SB_CUDA(cudaGetLastError());
       UnitI8Args ia{};
-      ia.radius = ua.radius;
-      ia.weight = ua.weight;
+      ia.radius = ka.radius;
+      ia.weight = ka.weight;
       ia.wl = wl_dev;
       ia.n_dist = (int)n_dist;
       ia.n_wl = (int)n_wl;
       ia.n_nodes = (int)n_nodes;
       ia.cpu = cpu;
-      ia.units = ua.units;
+      ia.units = ka.units;
       ia.n_items = ua.n_items;
       ia.items = ua.items;
       ia.chunk_n = ua.chunk_n;
@@ -1506,7 +1485,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       ia.levels = call->i8_levels;
       ia.n_levels = n_levels;
       ia.merge_max = merge_max;
-      ia.err = i8_err;
+      ia.err = wait_err;
       const int grid8 = (int)std::min<int64_t>(c.sms, S.n_items);
       cudaError_t le = cudaSuccess;
       timed_launch(K_UNITS_I8, s, [&] { le = launch_units_i8(ia, grid8, s); });
@@ -1583,19 +1562,14 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
 
 // Reads the error words of the last call (synchronizes the stream).
 void check_device_errors(Context& c, cudaStream_t s, const FixedCall* call) {
-  unsigned long long h[2];
-  SB_CUDA(cudaMemcpyAsync(h, c.err.as<unsigned long long>(2), sizeof h, cudaMemcpyDeviceToHost, s));
+  unsigned long long h[3];
+  SB_CUDA(cudaMemcpyAsync(h, c.err.as<unsigned long long>(3), sizeof h, cudaMemcpyDeviceToHost, s));
   SB_CUDA(cudaStreamSynchronize(s));
   // A forced node error (test hook) merges as a kernel's atomicMin would: the first in order.
   h[0] = std::min(h[0], g_forced_node_error.exchange(~0ull));
-  if (call && call->i8_err) {
-    unsigned f = 0;
-    SB_CUDA(cudaMemcpy(&f, call->i8_err, sizeof f, cudaMemcpyDeviceToHost));
-    if (f)
-      throw Failure{SCATRS_CUDA,
-                    "the int8 angle GEMMs gave up waiting on the tensor cores or the copies "
-                    "(bounded wait)"};
-  }
+  if (h[2] != ~0ull)
+    throw Failure{SCATRS_CUDA,
+                  "the angle GEMMs gave up waiting on the tensor cores or the copies (bounded wait)"};
   if (h[0] != ~0ull) {
     int status = (int)(h[0] & 3);
     unsigned long long key = h[0] >> 2;
@@ -2546,7 +2520,7 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
   mx.phase_err = p_d ? p_d + pl : nullptr;
   mx.greek = g_d;
   mx.greek_err = g_d ? g_d + gl : nullptr;
-  mx.err = c.err.as<unsigned long long>(2);
+  mx.err = c.err.as<unsigned long long>(3);
   timed_launch(K_FINAL, s, [&] { launch_mix(mx, s); });
   SB_CUDA(cudaGetLastError());
   call.radius = std::move(radius);
@@ -6761,9 +6735,9 @@ void scatrs_release(void) {
                       &c.chunk_row, &c.chunk_acc, &c.plan_units, &c.unit_acc, &c.unit_slots,
                       &c.slots, &c.items, &c.proj_items, &c.slot_index, &c.slot_greek, &c.slot_phase,
                       &c.X, &c.uz, &c.ux, &c.chunk_sums, &c.err, &c.acc,
-                      &c.counter, &c.values, &c.phase, &c.greek, &c.user.ge, &c.user.go,
+                      &c.counter, &c.values, &c.phase, &c.greek, &c.user.g,
                       &c.user.map, &c.user.rows_d, &c.tc_a_hi, &c.tc_a_lo, &c.tc_prod, &c.tc_err, &c.xdig,
-                      &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.i8_err,
+                      &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.side,
                       &c.i8.dig, &c.i8.scale, &c.i8.user_d, &c.i8.band_d, &c.ro_cgr, &c.ro_cgw})
       b->release();
     for (auto& kv : c.projectors)

@@ -34,6 +34,8 @@ struct MieFixedArgs {
   const int* chunk_n;       // slab-local: each chunk's largest number of terms
   const int64_t* chunk_row; // slab-local: first coefficient row of each chunk
   double* X;                // coefficient rows, 128 doubles each
+  double* side;             // per chunk side_stride doubles (UnitArgs::side)
+  int side_stride;
   double* colmax;           // or null; per chunk, each of its 128 columns' largest |X|
   double2* uz;              // scratch rows of u_k(mx), 32 lanes each
   double* ux;               // scratch rows of u_k(x)
@@ -73,9 +75,22 @@ struct MieNodesArgs {
   int allow_unvalidated;
 };
 
+// The angle GEMMs' operands are stored as the FP64 MMA reads them from shared memory, so that a stage
+// of 8 orders is one bulk copy per operand. Tables: 32-row tiles one after another, a tile ld orders
+// of 64 doubles, the rows of G_E then those of G_O, row r of order index k at r ^ 4 (k & 3).
+// Coefficients: rows of 32 nodes x 4, node j of order index k at j ^ (k & 3). The exclusive-ors
+// spread an MMA operand's 4 orders over the banks.
+constexpr int kTableRow = 64;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int64_t table_at(int64_t row, int64_t k, int64_t ld) {
+  return ((row >> 5) * ld + k) * kTableRow + ((row & 31) ^ (4 * (k & 3)));
+}
+
 // One projector band (engine.rs:2034-2072): orders up to `order` on n_q Gauss nodes, the
-// pi/tau tables G_E, G_O of its h = ceil(n_q/2) non-negative nodes (order-major: ld orders of
-// h_pad rows) and the projection matrices (2l+1)/2 w_k d_l(mu_k) of d00, d22, d2-2, d02.
+// pi/tau tables G_E, G_O of its h = ceil(n_q/2) non-negative nodes (ld orders of h_pad rows, h_pad a
+// multiple of 32; see table_at) and the projection matrices (2l+1)/2 w_k d_l(mu_k) of d00, d22, d2-2, d02.
 struct BandDesc {
   int upper;
   int order;
@@ -83,7 +98,7 @@ struct BandDesc {
   int h;
   int h_pad;
   int ld;
-  int64_t g_off;  // into band_ge / band_go
+  int64_t g_off;  // into band_g (or level_g)
   int64_t d_off;  // into band_d: 4 matrices of n_q x d_ld (order + 1 used)
   int d_ld;       // a multiple of 32
 };
@@ -128,8 +143,7 @@ struct LevelTableArgs {
   double* x_hi;
   double* x_lo;
   double* bary;
-  double* ge;
-  double* go;
+  double* g;
 };
 // The interpolation onto the requested rows: per half node h_pad even and h_pad odd weights.
 struct LevelMatrixArgs {
@@ -324,46 +338,40 @@ constexpr int kNormStrideD = 32;
 
 // K-b and K-c over one slab: the work items write the per-unit accumulators (zeroed before).
 struct UnitArgs {
-  const double* radius;
-  const double* weight;
-  const double* wl;
-  int n_dist, n_wl, n_nodes, cpu;
-  const int* units;
+  int n_wl, cpu;
   int n_items;
   const WorkItem* items;
   const int* chunk_n;
-  const int64_t* chunk_row;
+  const int64_t* chunk_row;  // first coefficient row of each chunk: rows4 = nc rounded up to 4
+                             // rows (zero above nc), twice with derivatives
   const int64_t* chunk_acc;  // offset of each chunk's band accumulator, or -1
   const int64_t* unit_acc;   // offset of each unit's cosine accumulator (4 n_mu doubles)
   const double* X;
-  // Phase matrix at the requested cosines: tables G_E, G_O of h_u rows (order-major: ld_u
-  // orders of h_u_pad rows) and each row's output cosines (plus side, minus side or -1).
-  int n_mu, h_u, h_u_pad;
-  const double* ge_u;
-  const double* go_u;
+  // K-a's record of each chunk: per node the factor w 4 pi r^2 / x^2 of its elements with w the
+  // values' weight, then each parameter's (derivatives), then (adaptive) the same with the error
+  // weights, 32 doubles each; then the largest number of terms of each 8 nodes.
+  const double* side;
+  int side_stride;
+  // Phase matrix at the requested cosines: the table of h_u rows (ld_u orders; see table_at) and
+  // each row's output cosines (plus side, minus side or -1).
+  int n_mu, h_u, ld_u;
+  const double* g_u;
   const int2* user_map;
   int greek_order;
   const BandDesc* bands;
-  const double* band_ge;
-  const double* band_go;
-  const double* level_ge;
-  const double* level_go;
+  const double* band_g;
+  const double* level_g;
   double* acc;
   int* work_counter;
-  int per_unit;
-  const double* wdiff;  // adaptive: the error weights (see MieFixedArgs)
-  // Derivatives (deriv != 0): n_theta distribution parameters, their node weights in wtheta
-  // ([n_dist][n_nodes][3]).
-  int deriv;
+  // With derivatives (n_theta distribution parameters) the accumulators hold each block's sums;
+  // adaptive calls add each block's error sums.
+  int deriv, adaptive;
   int n_theta;
-  const double* wtheta;
-  // Adaptive panels with derivatives (deriv and wdiff): the parameters' error weights; the
-  // accumulators hold each block's sums, then each block's error sums (2 (3 + n_theta) blocks).
-  const double* wthdiff;
   // The mixed form (i8_above > 0): chunks with i8_above < nc <= kI8MaxTerms are left to
   // unit_i8_kernel.
   int i8_above;
   int n_levels, merge_max;  // the phase levels (chunk_band)
+  unsigned* wait_err;  // set when a bounded wait gave up
 };
 
 // K-d and the outputs over one slab: averages, band projections, assembly.
@@ -458,7 +466,7 @@ void launch_pass1_layered_deriv(const Pass1Args& a, cudaStream_t s);
 void launch_plan_chunks(const PlanArgs& a, cudaStream_t s);
 void launch_mie_fixed(const MieFixedArgs& a, cudaStream_t s);
 void launch_mie_nodes(const MieNodesArgs& a, cudaStream_t s);
-int unit_kernel_blocks_per_sm();
+int unit_kernel_blocks_per_sm(int mode);  // 0 values, 1 derivatives, 2 adaptive, 3 both
 void launch_units(const UnitArgs& a, int grid, cudaStream_t s);
 void launch_proj(const ProjArgs& a, cudaStream_t s);
 void launch_final(const FinalArgs& a, cudaStream_t s);

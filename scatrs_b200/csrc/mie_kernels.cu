@@ -1,7 +1,8 @@
 // K-a: the Mie recurrences of every size node, one thread per node, one warp per chunk of 32
 // consecutive nodes of a (distribution, wavelength) unit. Compiled with -fmad=false (see
 // mie_device.cuh). The coefficients leave in the layout the angle GEMM reads: for each chunk a
-// row per order n (n = 1..N_c, N_c the chunk's largest number of terms) of 128 doubles,
+// row per order n (n = 1..N_c, N_c the chunk's largest number of terms, then zero rows to a multiple
+// of 4) of 128 doubles,
 // 4 per lane: u.re, u.im, v.re, v.im with (u, v) = (a_n, b_n) for odd n and (b_n, a_n) for even
 // n (scatrs/src/ensemble/fast.rs:95-137), zero above the node's own N.
 #include "kernels.h"
@@ -46,6 +47,20 @@ __global__ void plan_chunks_kernel(PlanArgs a) {
   if (lane == 0) a.chunk_n[warp] = nn;
 }
 
+// A chunk's side record (UnitArgs::side), from lane j's node: the factor sc = 4 pi r^2 / x^2 of its
+// elements times the values' and the parameters' weights wb[0..P], then times the error weights wbd
+// where there are any, and the largest number of terms n of each 8 nodes.
+__device__ __forceinline__ void put_side(const MieFixedArgs& a, int chunk, int lane, double sc,
+                                         const double* wb, const double* wbd, int P, int64_t n) {
+  double* o = a.side + (int64_t)chunk * a.side_stride;
+  for (int b = 0; b <= P; ++b) o[32 * b + lane] = wb[b] * sc;
+  if (wbd)
+    for (int b = 0; b <= P; ++b) o[32 * (1 + P + b) + lane] = wbd[b] * sc;
+  int top = (int)n;
+  for (int off = 1; off < 8; off <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, off));
+  if ((lane & 7) == 0) o[a.side_stride - 4 + (lane >> 3)] = (double)top;
+}
+
 template <bool kLayered, bool kAdaptive>
 __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
   int wslot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -58,7 +73,8 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
   int j = c * 32 + lane;
   int nc = a.chunk_n[chunk];
   int64_t row0 = a.chunk_row[chunk];
-  double* X = a.X + row0 * 128 + lane * 4;
+  // This lane's place in the coefficient row of order index k (kernels.h).
+  auto Xk = [&](int64_t k) { return a.X + (row0 + k) * 128 + ((lane ^ (int)(k & 3)) << 2); };
   // Scratch: 2L - 1 complex ratio arrays (one for a sphere) of nc + 2 rows, and u_k(x).
   const int n_arr = kLayered ? 2 * a.n_layers - 1 : 1;
   Scratch s;
@@ -68,6 +84,7 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
   double q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   double qe[kAdaptive ? 8 : 1] = {};  // adaptive: weighted by w_K - w_G
   double cm[4] = {0.0, 0.0, 0.0, 0.0};  // the largest |X| of this lane's four columns
+  double sc = 0.0, wv = 0.0, wd = 0.0;
   int64_t n = 0;
   const int64_t node = (a.per_unit ? unit : d) * a.n_nodes + j;
   if (j < a.n_nodes && a.radius[node] > 0.0) {
@@ -78,7 +95,7 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
     auto emit = [&](int64_t k, cplx an, cplx bn) {
       const bool odd = (k & 1) != 0;
       const cplx u = odd ? an : bn, v = odd ? bn : an;
-      *reinterpret_cast<double4*>(X + (k - 1) * 128) = make_double4(u.re, u.im, v.re, v.im);
+      *reinterpret_cast<double4*>(Xk(k - 1)) = make_double4(u.re, u.im, v.re, v.im);
       cm[0] = fmax(cm[0], fabs(u.re));
       cm[1] = fmax(cm[1], fabs(u.im));
       cm[2] = fmax(cm[2], fabs(v.re));
@@ -133,15 +150,19 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
       const double qv[8] = {1.0,           area * e.q_ext, area * e.q_sca, area * e.q_sca * e.g,
                             area * e.q_abs, area * e.q_back, r * r,         r * r * r};
       for (int k = 0; k < 8; ++k) q[k] = w * qv[k];
+      sc = 4.0 / (x * x) * (kPi * r * r);
+      wv = w;
       if constexpr (kAdaptive) {
-        const double wd = a.wdiff[node];
+        wd = a.wdiff[node];
         for (int k = 0; k < 8; ++k) qe[k] = wd * qv[k];
       }
     }
   }
-  // Orders above the node's own N are zero up to the chunk's.
-  for (int64_t k = n + 1; k <= nc; ++k)
-    *reinterpret_cast<double4*>(X + (k - 1) * 128) = make_double4(0.0, 0.0, 0.0, 0.0);
+  put_side(a, chunk, lane, sc, &wv, kAdaptive ? &wd : nullptr, 0, n);
+  // Orders above the node's own N are zero up to the chunk's, rounded up to the GEMM's 4.
+  const int nc4 = (nc + 3) & ~3;
+  for (int64_t k = n + 1; k <= nc4; ++k)
+    *reinterpret_cast<double4*>(Xk(k - 1)) = make_double4(0.0, 0.0, 0.0, 0.0);
   if (a.colmax != nullptr)
     *reinterpret_cast<double4*>(a.colmax + (int64_t)chunk * 128 + lane * 4) =
         make_double4(cm[0], cm[1], cm[2], cm[3]);
@@ -180,7 +201,11 @@ __device__ __forceinline__ void mie_chunk_deriv(const MieFixedArgs& a) {
   int j = c * 32 + lane;
   int nc = a.chunk_n[chunk];
   int64_t row0 = a.chunk_row[chunk];
-  double* X = a.X + (row0 + (int64_t)(lane >> 4) * nc) * 128 + (lane & 15) * 4;
+  const int nc4 = (nc + 3) & ~3;  // rows of a half, rounded up to the GEMM's 4
+  auto Xk = [&](int64_t k) {
+    return a.X + (row0 + (int64_t)(lane >> 4) * nc4 + k) * 128 +
+           (((lane & 15) ^ (int)(k & 3)) << 2);
+  };
   Scratch s;
   s.uz = a.uz + (row0 + 2 * (int64_t)chunk) * 32 + lane;
   s.ux = a.ux + (row0 + 2 * (int64_t)chunk) * 32 + lane;
@@ -192,6 +217,7 @@ __device__ __forceinline__ void mie_chunk_deriv(const MieFixedArgs& a) {
   double qv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   double qd[2][8] = {{0, 0, 0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0, 0, 0}};
   double wb[4] = {0, 0, 0, 0}, wbd[4] = {0, 0, 0, 0};  // values, then each parameter
+  double sc = 0.0;
   const bool adaptive = a.wdiff != nullptr;
   int64_t n = 0;
   const int64_t node = (a.per_unit ? unit : d) * a.n_nodes + j;
@@ -214,8 +240,9 @@ __device__ __forceinline__ void mie_chunk_deriv(const MieFixedArgs& a) {
         const bool odd = (k & 1) != 0;
         const cplx u = odd ? an : bn, v = odd ? bn : an;
         const cplx du = odd ? dan : dbn, dv = odd ? dbn : dan;
-        *reinterpret_cast<double4*>(X + (k - 1) * 128) = make_double4(u.re, u.im, v.re, v.im);
-        *reinterpret_cast<double4*>(X + (k - 1) * 128 + 64) =
+        double* x = Xk(k - 1);
+        *reinterpret_cast<double4*>(x) = make_double4(u.re, u.im, v.re, v.im);
+        *reinterpret_cast<double4*>(x + 64) =
             make_double4(du.re, du.im, dv.re, dv.im);
         ds.add(k, an, bn, dan, dbn);
       };
@@ -244,6 +271,7 @@ __device__ __forceinline__ void mie_chunk_deriv(const MieFixedArgs& a) {
                               0.0};
         for (int k = 0; k < 8; ++k) qd[p][k] = q1[k];
       }
+      sc = 4.0 / (x * x) * (kPi * r * r);
       wb[0] = a.weight[node];
       for (int p = 0; p < P; ++p) wb[1 + p] = a.wtheta[node * 3 + p];
       if (adaptive) {
@@ -252,9 +280,11 @@ __device__ __forceinline__ void mie_chunk_deriv(const MieFixedArgs& a) {
       }
     }
   }
-  for (int64_t k = n + 1; k <= nc; ++k) {
-    *reinterpret_cast<double4*>(X + (k - 1) * 128) = make_double4(0.0, 0.0, 0.0, 0.0);
-    *reinterpret_cast<double4*>(X + (k - 1) * 128 + 64) = make_double4(0.0, 0.0, 0.0, 0.0);
+  put_side(a, chunk, lane, sc, wb, adaptive ? wbd : nullptr, P, n);
+  for (int64_t k = n + 1; k <= nc4; ++k) {
+    double* x = Xk(k - 1);
+    *reinterpret_cast<double4*>(x) = make_double4(0.0, 0.0, 0.0, 0.0);
+    *reinterpret_cast<double4*>(x + 64) = make_double4(0.0, 0.0, 0.0, 0.0);
   }
   // Per block: the values and each parameter weight the node's quantities, Re m and Im m
   // weight its derivatives with the values' weight. The chunk's sums in a fixed tree order;
@@ -314,7 +344,11 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
   int j = c * 32 + lane;
   int nc = a.chunk_n[chunk];
   int64_t row0 = a.chunk_row[chunk];
-  double* X = a.X + (row0 + (int64_t)(lane >> 4) * nc) * 128 + (lane & 15) * 4;
+  const int nc4 = (nc + 3) & ~3;  // rows of a half, rounded up to the GEMM's 4
+  auto Xk = [&](int64_t k) {
+    return a.X + (row0 + (int64_t)(lane >> 4) * nc4 + k) * 128 +
+           (((lane & 15) ^ (int)(k & 3)) << 2);
+  };
   const int L = a.n_layers, n_arr = 2 * L - 1;
   Scratch s;
   s.uz = a.uz + (row0 + 2 * (int64_t)chunk) * (2 * n_arr) * 32 + lane;
@@ -327,6 +361,7 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
   double qv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   double qd[2][8] = {{0, 0, 0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0, 0, 0}};
   double wb[4] = {0, 0, 0, 0}, wbd[4] = {0, 0, 0, 0};
+  double sc = 0.0;
   const bool adaptive = a.wdiff != nullptr;
   int64_t n = 0;
   const int64_t node = (a.per_unit ? unit : d) * a.n_nodes + j;
@@ -367,8 +402,9 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
         const bool odd = (k & 1) != 0;
         const cplx u = odd ? an : bn, v = odd ? bn : an;
         const cplx du = odd ? dan : dbn, dv = odd ? dbn : dan;
-        *reinterpret_cast<double4*>(X + (k - 1) * 128) = make_double4(u.re, u.im, v.re, v.im);
-        *reinterpret_cast<double4*>(X + (k - 1) * 128 + 64) =
+        double* x = Xk(k - 1);
+        *reinterpret_cast<double4*>(x) = make_double4(u.re, u.im, v.re, v.im);
+        *reinterpret_cast<double4*>(x + 64) =
             make_double4(du.re, du.im, dv.re, dv.im);
         ds.add(k, an, bn, dan, dbn);
       };
@@ -398,6 +434,7 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
                               0.0};
         for (int k = 0; k < 8; ++k) qd[p][k] = q1[k];
       }
+      sc = 4.0 / (x * x) * (kPi * r * r);
       wb[0] = a.weight[node];
       for (int p = 0; p < P; ++p) wb[1 + p] = a.wtheta[node * 3 + p];
       if (adaptive) {
@@ -406,9 +443,11 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
       }
     }
   }
-  for (int64_t k = n + 1; k <= nc; ++k) {
-    *reinterpret_cast<double4*>(X + (k - 1) * 128) = make_double4(0.0, 0.0, 0.0, 0.0);
-    *reinterpret_cast<double4*>(X + (k - 1) * 128 + 64) = make_double4(0.0, 0.0, 0.0, 0.0);
+  put_side(a, chunk, lane, sc, wb, adaptive ? wbd : nullptr, P, n);
+  for (int64_t k = n + 1; k <= nc4; ++k) {
+    double* x = Xk(k - 1);
+    *reinterpret_cast<double4*>(x) = make_double4(0.0, 0.0, 0.0, 0.0);
+    *reinterpret_cast<double4*>(x + 64) = make_double4(0.0, 0.0, 0.0, 0.0);
   }
   // The chunk's sums per block (values and each parameter on the values' quantities, the
   // direction's blocks on the derivatives with the values' weight) in a fixed tree order;

@@ -25,7 +25,7 @@ using ddm::dd;
 using ddm::mkdd;
 
 // One thread per (level, half node): the node in double-double, its barycentric weight, and its
-// rows of the G_E, G_O tables (order-major, h_pad = h rows).
+// rows of the G_E, G_O tables.
 __global__ void __launch_bounds__(128) level_table_kernel(LevelTableArgs a) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n_half) return;
@@ -54,8 +54,7 @@ __global__ void __launch_bounds__(128) level_table_kernel(LevelTableArgs a) {
   a.x_lo[t] = x.lo;
   a.bary[t] = 1.0 / dpn;
   // pi_n, tau_n by their three-term recurrence, scaled by (2n + 1) / (n (n + 1)).
-  double* ge = a.ge + B.g_off + i;
-  double* go = a.go + B.g_off + i;
+  double* tab = a.g + B.g_off;
   dd pi_prev = mkdd(0.0), pi = mkdd(1.0);
   for (int k = 1; k <= B.upper; ++k) {
     const double kf = (double)k, k1 = kf + 1.0;
@@ -64,12 +63,16 @@ __global__ void __launch_bounds__(128) level_table_kernel(LevelTableArgs a) {
     const dd wp = (pi * (double)(2 * k + 1)) / (kf * k1);
     const dd wt = (tau * (double)(2 * k + 1)) / (kf * k1);
     const double vp = wp.hi, vt = wt.hi;
-    ge[(int64_t)(k - 1) * B.h_pad] = (k & 1) ? vp : vt;
-    go[(int64_t)(k - 1) * B.h_pad] = (k & 1) ? vt : vp;
+    double* o = tab + table_at(i, k - 1, B.ld);
+    o[0] = (k & 1) ? vp : vt;
+    o[32] = (k & 1) ? vt : vp;
     const dd next = (mp * (double)(2 * k + 1) - pi_prev * k1) / kf;
     pi_prev = pi;
     pi = next;
   }
+  // The row past the last order, which a rounded-up contraction meets with zero coefficients.
+  double* o = tab + table_at(i, B.upper, B.ld);
+  o[0] = o[32] = 0.0;
 }
 
 // One thread per (level, requested row): the row's interpolation weights onto the level's half

@@ -28,6 +28,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "mbar.cuh"
 
 namespace sb {
 
@@ -40,7 +41,6 @@ constexpr int kASlice = 128 * kI8KB;                                // 8 KiB
 constexpr int kBSlice = 64 * kI8KB;                                 // 4 KiB
 constexpr int kStageBytes = kI8Levels * (kASlice + kBSlice);        // 60 KiB
 constexpr uint32_t kTmemCols = 512;
-constexpr long long kSpinCycles = 4000000000LL;  // about 2 s at the B200's clocks
 
 struct I8Smem {
   alignas(16) double side[2][kI8Side];  // two chunks' side records (column scales, node factors)
@@ -52,75 +52,6 @@ struct I8Smem {
   int stop;  // the epilogue warps' common decision to stop
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned long long* b, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(b)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(b)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(b)) : "memory");
-}
-// One arrival for the calling warp, after all its lanes got here.
-__device__ __forceinline__ void warp_arrive(unsigned long long* b) {
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) mbar_arrive(b);
-}
-// A bounded wait on phase `parity`: false if it gave up (then *err and sm.abort are set) or if
-// another role gave up first.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, uint32_t parity, I8Smem& sm,
-                                          unsigned* err) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_u32(b)), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (*(volatile int*)&sm.abort) return false;
-    if (clock64() - t0 > kSpinCycles) {
-      atomicExch(err, 1u);
-      *(volatile int*)&sm.abort = 1;
-      return false;
-    }
-  }
-}
-// A bounded wait that ignores the abort flag: the drains of copies and MMAs in flight.
-__device__ __forceinline__ void mbar_wait_drain(unsigned long long* b, uint32_t parity,
-                                                unsigned* err) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_u32(b)), "r"(parity)
-        : "memory");
-    if (done) return;
-    if (clock64() - t0 > kSpinCycles) {
-      atomicExch(err, 1u);
-      return;
-    }
-  }
-}
-// Bulk copy of `bytes` (a multiple of 16) from global to shared memory, completing on `bar`.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes,
-                                          unsigned long long* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-          smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
 // A K-major operand in shared memory with the 64-byte swizzle: rows of 64 bytes, groups of 8
 // rows 512 bytes apart (the canonical layout of the tcgen05 shared-memory descriptor).
 __device__ __forceinline__ uint64_t sdesc64(uint32_t addr) {
@@ -549,7 +480,7 @@ __global__ void __launch_bounds__(128) x_split_kernel(XSplitArgs a) {
 #pragma unroll
       for (int b = 0; b < 32; ++b) {
         const int k = kb * kI8KB + q2 * 32 + b;
-        xv[b] = (k < nc && m > 0.0) ? X[(int64_t)k * 128 + c] : 0.0;
+        xv[b] = (k < nc && m > 0.0) ? X[(int64_t)k * 128 + (c ^ (4 * (k & 3)))] : 0.0;
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {

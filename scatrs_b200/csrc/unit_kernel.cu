@@ -1,6 +1,5 @@
-// K-b, K-c and K-d for the fixed-grid ensemble: one persistent CTA works through whole
-// (distribution, wavelength) units, each in a fixed order, so the sums are deterministic and
-// need no atomics.
+// K-b, K-c and K-d: persistent CTAs work through shares of (distribution, wavelength) units, each in a
+// fixed order, so the sums are deterministic.
 //
 // Per unit, per chunk of 32 nodes (ascending radius):
 //   * K-b: S1, S2 of the chunk's 32 spheres at the table cosines as real FP64 GEMMs,
@@ -8,118 +7,56 @@
 //     pi/tau tables of the requested cosines and of the chunk's projector band;
 //   * K-c: the phase-matrix elements at mu and at -mu (fast.rs:151-204), scaled per sphere and
 //     weighted by w_j u(r_j) r_j, summed over the chunk into the unit's accumulators;
-//   * K-d: when the band changes, the band's averaged tables projected onto the Greek
-//     coefficients with (2l+1)/2 w_k d_l(mu_k) (fast.rs:238-253, engine.rs:2310-2355).
+//   * K-d: the tables projected onto the Greek coefficients with (2l+1)/2 w_k d_l(mu_k)
+//     (fast.rs:238-253, engine.rs:2310-2355): here for adaptive calls, on the fixed grid in
+//     slot_project_kernel (phase_levels.cu).
 // Then the averages and the outputs of engine.rs:2396-2497.
 #include "kernels.h"
+#include "mbar.cuh"
 
 namespace sb {
 
 namespace {
 
 constexpr double kPi = 3.14159265358979323846264338327950288;
-constexpr int KB = 8;     // orders per GEMM stage
+constexpr int KB = 8;     // orders per stage
 constexpr int TR = 32;    // table rows per tile
-constexpr int NT = 128;   // threads: 8 row groups of 4 rows x 16 node groups of 2 nodes
-// The stage rows' strides in shared memory: 4 doubles past 32 and 128, so that the FP64 MMA's
-// operand loads (lane = 4 g + q reads order k4 + q, row or column g) of a half-warp fall in 16
-// distinct 8-byte banks.
-constexpr int TRP = TR + 4;
-constexpr int XP = 128 + 4;
+constexpr int NT = 128;   // threads: 4 warps of 8 rows x 128 columns
+constexpr int NS = 4;     // stages in flight (5: the same)
+constexpr int RING = 8;   // job records: more than the stages, so none is overwritten in use
 
-__device__ __forceinline__ void elements4(double s1r, double s1i, double s2r, double s2i,
-                                          double e[4]) {
-  // (|S1|^2+|S2|^2)/2, (|S2|^2-|S1|^2)/2, Re(S2 S1*), Im(S2 S1*) (scatrs/src/mie/phase.rs:54-59)
-  double n1 = s1r * s1r + s1i * s1i, n2 = s2r * s2r + s2i * s2i;
-  e[0] = 0.5 * (n1 + n2);
-  e[1] = 0.5 * (n2 - n1);
-  e[2] = s2r * s1r + s2i * s1i;
-  e[3] = s2i * s1r - s2r * s1i;
-}
-
-// element_derivatives (scatrs/src/mie/phase.rs:62-73): the elements' derivatives for amplitude
-// derivatives (D1, D2).
-__device__ __forceinline__ void element_derivs4(double s1r, double s1i, double s2r, double s2i,
-                                                double d1r, double d1i, double d2r, double d2i,
-                                                double e[4]) {
-  const double r1 = s1r * d1r + s1i * d1i;
-  const double r2 = s2r * d2r + s2i * d2i;
-  e[0] = r1 + r2;
-  e[1] = r2 - r1;
-  e[2] = (d2r * s1r + d2i * s1i) + (s2r * d1r + s2i * d1i);
-  e[3] = (d2i * s1r - d2r * s1i) + (s2i * d1r - s2r * d1i);
-}
-
-struct Smem {
-  double a[2][2][KB][TRP];  // [stage][G_E, G_O][order][row] (rows 32 .. 35 unused)
-  double xs[2][KB][XP];    // [stage][order][4 columns x 32 nodes] (128 .. 131 unused)
-  double w[32], cu[32], area[32], sc[32];
-  double wth[3][32];  // the distribution parameters' weights (derivatives only)
-  double wd[32], wthd[3][32];  // adaptive derivatives: the error weights (w_K - w_G) ...
-  int nn[32];  // each node's number of terms plus one (an upper bound of K-a's), 0 for padding
-  double S[8];
-  int slot;
+// One tile of one chunk (or half chunk, with derivatives) as every warp sees it.
+struct Job {
+  int end;    // no more work
+  int rows4;  // orders, rounded up to the MMA's 4
+  int r0, h;  // the tile's first table row; the table's rows
+  int user;   // the requested cosines' table (outputs by user_map), else a band's or level's
+  int len;    // outputs per element: n_mu or n_q
+  int half;
+  int64_t out;  // the sums' offset in acc
 };
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::); }
-
-// One stage: orders k0 .. k0+KB-1 (those below nc) of the 32 table rows and of the chunk's
-// coefficient rows, copied asynchronously into stage buffer st. The tables are stored
-// transposed (order-major, ldr doubles per order) so that each order's 32 rows are contiguous.
-__device__ __forceinline__ void load_stage(Smem& sm, int st, const double* __restrict__ ge,
-                                           const double* __restrict__ go, int ldr, int r0,
-                                           int k0, int nc, const double* __restrict__ xc) {
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int i = t; i < KB * 16; i += NT) {
-    const int kk = i >> 4, c = i & 15;
-    if (k0 + kk < nc) {
-      const int64_t off = (int64_t)(k0 + kk) * ldr + r0 + 2 * c;
-      cp_async16(&sm.a[st][0][kk][2 * c], ge + off);
-      cp_async16(&sm.a[st][1][kk][2 * c], go + off);
-    }
-  }
-#pragma unroll
-  for (int i = t; i < KB * 64; i += NT) {
-    const int kk = i >> 6, c = i & 63;
-    if (k0 + kk < nc) cp_async16(&sm.xs[st][kk][2 * c], xc + (int64_t)(k0 + kk) * 128 + 2 * c);
-  }
-  cp_commit();
-}
-
-// As load_stage, with the rows at or above nc zero-filled (cp.async with a zero source size), so
-// that whole 4-order steps of the FP64 MMA can run past the chunk's last order.
-__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool valid) {
-  unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n));
-}
-__device__ __forceinline__ void load_stage_z(Smem& sm, int st, const double* __restrict__ ge,
-                                             const double* __restrict__ go, int ldr, int r0,
-                                             int k0, int nc, const double* __restrict__ xc) {
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int i = t; i < KB * 16; i += NT) {
-    const int kk = i >> 4, c = i & 15;
-    const bool valid = k0 + kk < nc;
-    const int64_t off = valid ? (int64_t)(k0 + kk) * ldr + r0 + 2 * c : 0;
-    cp_async16_zfill(&sm.a[st][0][kk][2 * c], ge + off, valid);
-    cp_async16_zfill(&sm.a[st][1][kk][2 * c], go + off, valid);
-  }
-#pragma unroll
-  for (int i = t; i < KB * 64; i += NT) {
-    const int kk = i >> 6, c = i & 63;
-    const bool valid = k0 + kk < nc;
-    cp_async16_zfill(&sm.xs[st][kk][2 * c], xc + (valid ? (int64_t)(k0 + kk) * 128 + 2 * c : 0),
-                     valid);
-  }
-  cp_commit();
-}
+// kNw: weights per node (UnitArgs::side): values; then the parameters'; then the error weights.
+template <int kNw>
+struct UnitSmem {
+  double a[NS][KB][kTableRow];  // [stage][order][G_E rows, G_O rows] (table_at)
+  double xs[NS][KB][128];       // [stage][order][32 nodes x 4 columns]
+  double side[RING][32 * kNw + 4];
+  Job job[RING];
+  unsigned long long full[NS], empty[NS];
+  int abort;
+  // The producer (warp 0): the item's next chunks with work for it, and its place among them.
+  struct {
+    int first_tile, tiles, t_user, rows4, h, n_q, ld;
+    int64_t row, acc, ci;
+    const double* g;
+  } chunk[32];
+  struct {
+    int unit, group, n_groups, chunk0, n_chunks, c, tile, half, rows4, k0, next_item;
+    int64_t user_acc;
+    const double *g, *x, *side;
+  } p;
+};
 
 // D (8x8) += A (8x4, row) B (4x8, col) in FP64 on the tensor cores (PTX mma.sync m8n8k4):
 // lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2 (l%4) + {0, 1}].
@@ -129,500 +66,429 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// A row tile's table source: G_E, G_O (order-major, ldr doubles per order) from row r0.
-struct TileSrc {
-  const double* ge;
-  const double* go;
-  int ldr, r0;
+__device__ __forceinline__ double swap_add(double v, int lane_bit) {
+  return v + __shfl_xor_sync(0xffffffffu, v, lane_bit);
+}
+
+// The producer's next work item (its counter is taken one item ahead, so that only the item's chunks
+// are waited for), then the records of its next 32 chunks: one lane per chunk, the chunks with rows
+// for this item kept in order. Returns false when no item is left.
+template <class Smem>
+__device__ __forceinline__ bool next_chunks(const UnitArgs& a, Smem& sm) {
+  auto& p = sm.p;
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    int c0 = p.chunk0 + 32;
+    __syncwarp();
+    if (c0 >= a.cpu) {
+      const int slot = p.next_item;
+      if (slot >= a.n_items) return false;
+      const WorkItem it = a.items[slot];
+      __syncwarp();
+      if (lane == 0) {
+        p.next_item = atomicAdd(a.work_counter, 1);
+        p.unit = it.unit;
+        p.group = it.group;
+        p.n_groups = it.n_groups;
+        p.user_acc = a.unit_acc[it.unit];
+      }
+      c0 = 0;
+      __syncwarp();
+    }
+    const int c = c0 + lane;
+    bool on = c < a.cpu;
+    const int64_t ci = (int64_t)p.unit * a.cpu + (on ? c : 0);
+    const int nc = on ? a.chunk_n[ci] : 0;
+    const int64_t row = a.chunk_row[ci], band_acc = a.chunk_acc[ci];
+    // The int8 path's chunks are not this kernel's.
+    on = on && nc > 0 && !(a.i8_above > 0 && nc > a.i8_above && nc <= kI8MaxTerms);
+    int t_user = 0, tiles = 0, tile0 = 0;
+    BandDesc B{};
+    const double* g = nullptr;
+    if (on) {
+      const int b = chunk_band(nc, a.merge_max, a.n_levels, a.greek_order);
+      t_user = nc <= a.merge_max ? 0 : (a.h_u + TR - 1) / TR;
+      if (b >= 0) {
+        B = a.bands[b];
+        g = (b < a.n_levels ? a.level_g : a.band_g) + B.g_off;
+      }
+      tiles = t_user + (b >= 0 ? (B.h + TR - 1) / TR : 0);
+      // This item's first tile; a level's tiles move on by one item per run of chunks.
+      const int shift = nc <= a.merge_max ? (c / kRunChunks) % p.n_groups : 0;
+      tile0 = p.group >= shift ? p.group - shift : p.group - shift + p.n_groups;
+      on = tile0 < tiles;
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, on);
+    if (on) {
+      auto& r = sm.chunk[__popc(mask & ((1u << lane) - 1))];
+      r.first_tile = tile0;
+      r.tiles = tiles;
+      r.t_user = t_user;
+      r.rows4 = (nc + 3) & ~3;
+      r.h = B.h;
+      r.n_q = B.n_q;
+      r.ld = B.ld;
+      r.row = row;
+      r.acc = band_acc;
+      r.ci = ci;
+      r.g = g;
+    }
+    if (lane == 0) {
+      p.chunk0 = c0;
+      p.n_chunks = __popc(mask);
+      p.c = 0;
+    }
+    __syncwarp();
+    if (mask != 0) return true;
+  }
+}
+
+// Moves the producer to its next job (warp 0): the halves of a tile, the tiles of a chunk, the
+// chunks of a work item, the items in the order of the counter. Fills the job's record.
+template <int kMode, class Smem>
+__device__ __forceinline__ bool next_job(const UnitArgs& a, Smem& sm, int job) {
+  constexpr int kHalves = (kMode == 1 || kMode == 3) ? 2 : 1;
+  auto& p = sm.p;
+  const int lane = threadIdx.x & 31;
+  int c = p.c, half = p.half + 1, tile = p.tile;
+  bool found = c < p.n_chunks;
+  if (found && half >= kHalves) {
+    half = 0;
+    tile += p.n_groups;
+    found = tile < sm.chunk[c].tiles;
+  }
+  if (!found) {
+    if (++c >= p.n_chunks) {
+      __syncwarp();
+      if (!next_chunks(a, sm)) return false;
+      c = 0;
+    }
+    half = 0;
+    tile = sm.chunk[c].first_tile;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    const auto& r = sm.chunk[c];
+    const bool user = tile < r.t_user;
+    const int tl = user ? tile : tile - r.t_user;
+    p.c = c;
+    p.half = half;
+    p.tile = tile;
+    p.rows4 = r.rows4;
+    p.k0 = 0;
+    p.g = (user ? a.g_u : r.g) + (int64_t)tl * (user ? a.ld_u : r.ld) * kTableRow;
+    p.x = a.X + (r.row + (int64_t)half * r.rows4) * 128;
+    p.side = a.side + r.ci * a.side_stride;
+    Job& jb = sm.job[job % RING];
+    jb.end = 0;
+    jb.rows4 = r.rows4;
+    jb.r0 = TR * tl;
+    jb.h = user ? a.h_u : r.h;
+    jb.user = user;
+    jb.len = user ? a.n_mu : r.n_q;
+    jb.half = half;
+    jb.out = user ? p.user_acc : r.acc;
+  }
+  __syncwarp();
+  return true;
+}
+
+// Where warp 0 is in producing (the same in its lanes): the next stage and job, the stages of the job
+// still to issue, and whether the end has been issued.
+struct Producer {
+  int stage = 0, job = -1, left = 0;
+  bool done = false;
 };
 
-// The tile C_E = G_E X, C_O = G_O X (32 rows x 128 columns) on the FP64 tensor path: warp w
-// computes rows 8w .. 8w + 7 of all 128 columns as 16 MMA tiles of 8 columns (2 nodes) each for E
-// and O; cE[nt] is D of columns 8 nt ... Every warp does the same work, the MMAs of a group of 4
-// tiles (8 nodes) stopping above the group's largest number of terms (K-a writes zero rows up to
-// the chunk's), so that no warp, and no SM sub-partition, carries the chunk's largest spheres
-// alone.
-// The tile's first stage is already in flight in buffer st0; with nx, the next tile's first stage
-// (same chunk, same coefficient rows) is issued during this tile's last stage, so that the
-// pipeline does not drain between tiles, and st0 returns the buffer it went to.
-__device__ __forceinline__ void gemm_tile_mma(Smem& sm, const TileSrc& src, int nc,
-                                              const double* __restrict__ xc, double cE[16][2],
-                                              double cO[16][2], int& st0, const TileSrc* nx) {
-  const double* __restrict__ ge = src.ge;
-  const double* __restrict__ go = src.go;
-  const int ldr = src.ldr, r0 = src.r0;
-  const int t = threadIdx.x, w = t >> 5, lane = t & 31, q = lane & 3, g = lane >> 2;
-#pragma unroll
-  for (int nt = 0; nt < 16; ++nt) {
-    cE[nt][0] = cE[nt][1] = 0.0;
-    cO[nt][0] = cO[nt][1] = 0.0;
+// Warp 0 issues one stage: up to KB orders of the table's tile and of the chunk's coefficient rows,
+// a bulk copy each, and with a job's first stage its weights. (A copy per row, 24 a stage, was
+// bound by the copies' issue: 168 against 105 ms of the two-barrier cp.async form before, per pass
+// of 64 x 512 units.) Stages run on across jobs, so the pipeline does not drain between tiles or
+// chunks.
+template <int kMode, class Smem>
+__device__ __forceinline__ void issue_stage(const UnitArgs& a, Smem& sm, Producer& pr) {
+  auto& p = sm.p;
+  const int lane = threadIdx.x & 31, slot = pr.stage % NS;
+  bool first = false;
+  if (pr.left == 0) {
+    ++pr.job;
+    first = next_job<kMode>(a, sm, pr.job);
+    if (!first) {
+      if (lane == 0) {
+        sm.job[pr.job % RING].end = 1;
+        mbar_arrive(&sm.full[slot]);
+      }
+      pr.done = true;
+      ++pr.stage;
+      return;
+    }
+    pr.left = (p.rows4 + KB - 1) / KB;
   }
-  int gmax[4] = {0, 0, 0, 0};
+  if (lane == 0) {
+    const int k0 = p.k0, rows = min(KB, p.rows4 - k0);
+    const uint32_t side_bytes = first ? (uint32_t)a.side_stride * 8 : 0;
+    mbar_expect_tx(&sm.full[slot], (uint32_t)rows * (128 + kTableRow) * 8 + side_bytes);
+    bulk_load(sm.xs[slot], p.x + (int64_t)k0 * 128, rows * 1024, &sm.full[slot]);
+    bulk_load(sm.a[slot], p.g + (int64_t)k0 * kTableRow, rows * kTableRow * 8, &sm.full[slot]);
+    if (first) bulk_load(sm.side[pr.job % RING], p.side, side_bytes, &sm.full[slot]);
+    p.k0 = k0 + KB;
+  }
+  --pr.left;
+  ++pr.stage;
+}
+
+// Issues every stage whose buffer is free, up to NS ahead of stage `it`, and waits (bounded) only for
+// the next one that warp 0 itself needs.
+template <int kMode, class Smem>
+__device__ __forceinline__ bool produce(const UnitArgs& a, Smem& sm, Producer& pr, int it) {
+  while (!pr.done && pr.stage < it + NS) {
+    if (pr.stage >= NS) {
+      unsigned long long* e = &sm.empty[pr.stage % NS];
+      const uint32_t parity = ((pr.stage / NS) - 1) & 1;
+      const bool free = __shfl_sync(0xffffffffu, (int)mbar_done(e, parity), 0);
+      if (!free) {
+        if (pr.stage > it) return true;
+        if (!mbar_wait(e, parity, sm, a.wait_err)) return false;
+      }
+    }
+    issue_stage<kMode>(a, sm, pr);
+  }
+  return true;
+}
+
+// The sums over a job's nodes, for the lane's row (g) and column nodes 4 j + q of tile pairs j: the
+// D fragments of tiles 2 j and 2 j + 1 hold (u.re, v.re) and (u.im, v.im) of one node in one
+// thread, so that S1 = E_u +- O_v, S2 = E_v +- O_u (fast.rs:151-204) need no exchange.
+struct Amp {
+  double s1r, s1i, s2r, s2i;
+};
+__device__ __forceinline__ Amp amplitudes(const double (&cE)[16][2], const double (&cO)[16][2],
+                                          int j, double sg) {
+  return Amp{fma(sg, cO[2 * j][1], cE[2 * j][0]), fma(sg, cO[2 * j + 1][1], cE[2 * j + 1][0]),
+             fma(sg, cO[2 * j][0], cE[2 * j][1]), fma(sg, cO[2 * j + 1][0], cE[2 * j + 1][1])};
+}
+// p += f (|S1|^2, |S2|^2, Re S2 S1*, Im S2 S1*) (scatrs/src/mie/phase.rs:54-59).
+__device__ __forceinline__ void add_elements(double p[4], const Amp& s, double f) {
+  const double t1r = f * s.s1r, t1i = f * s.s1i, t2r = f * s.s2r, t2i = f * s.s2i;
+  p[0] = fma(t1r, s.s1r, fma(t1i, s.s1i, p[0]));
+  p[1] = fma(t2r, s.s2r, fma(t2i, s.s2i, p[1]));
+  p[2] = fma(t2r, s.s1r, fma(t2i, s.s1i, p[2]));
+  p[3] = fma(t2i, s.s1r, fma(-t2r, s.s1i, p[3]));
+}
+// The four lanes of a row add up; lane q ends with element q (F11, F12, F33, F34) from the sums of
+// (|S1|^2, |S2|^2) times c and the other two.
+__device__ __forceinline__ double reduce_elements(const double p[4], double c) {
+  const int q = threadIdx.x & 3;
+  const bool hi = q & 2;
+  double a0 = hi ? p[2] : p[0], a1 = hi ? p[3] : p[1];
+  a0 += __shfl_xor_sync(0xffffffffu, hi ? p[0] : p[2], 2);
+  a1 += __shfl_xor_sync(0xffffffffu, hi ? p[1] : p[3], 2);
+  a0 = swap_add(a0, 1);
+  a1 = swap_add(a1, 1);
+  return hi ? (q & 1 ? a1 : a0) : c * (q & 1 ? a1 - a0 : a0 + a1);
+}
+
+// kMode 0: values; 1: with the derivative blocks; 2: adaptive panels (values and the sums of
+// |Kronrod - Gauss| per panel); 3: adaptive panels with the derivative blocks (each block's sums,
+// then its error sums: every 16-node half of a chunk is one panel).
+template <int kMode, int kNw>
+__device__ __forceinline__ void unit_body(const UnitArgs& a) {
+  constexpr bool kDeriv = kMode == 1 || kMode == 3;
+  using Smem = UnitSmem<kNw>;
+  extern __shared__ __align__(16) unsigned char unit_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(unit_raw);
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31, q = lane & 3, g = lane >> 2;
+  if (t == 0) {
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(&sm.full[i], 1);
+      mbar_init(&sm.empty[i], NT / 32);
+    }
+    sm.abort = 0;
+    sm.p.chunk0 = a.cpu;  // no item yet
+    sm.p.n_chunks = sm.p.c = sm.p.half = sm.p.tile = 0;
+    sm.p.next_item = atomicAdd(a.work_counter, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+  bool ok = true;
+  Producer pr;
+  if (w == 0) ok = produce<kMode>(a, sm, pr, 0);
+  int it = 0;
+  for (int job = 0; ok; ++job) {
+    if (!mbar_wait(&sm.full[it % NS], (it / NS) & 1, sm, a.wait_err)) break;
+    const Job jb = sm.job[job % RING];
+    if (jb.end) break;
+    const double* side = sm.side[job % RING];
+    // The rows move round the warps from tile to tile (a row always with the same warp, which owns its
+    // sums); a warp without rows only counts the stages.
+    const int rg = (w + jb.r0 / TR) & 3, row0 = jb.r0 + 8 * rg;
+    const bool active = row0 < jb.h;
+    int gmax[4];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) gmax[i >> 3] = max(gmax[i >> 3], sm.nn[i]);
-  int st = st0;
-  for (int k0 = 0; k0 < nc; k0 += KB, st ^= 1) {
-    cp_wait_all();
-    __syncthreads();
-    if (k0 + KB < nc)
-      load_stage_z(sm, st ^ 1, ge, go, ldr, r0, k0 + KB, nc, xc);
-    else if (nx)
-      load_stage_z(sm, st ^ 1, nx->ge, nx->go, nx->ldr, nx->r0, 0, nc, xc);
-    const int kend = nc - k0 < KB ? nc - k0 : KB;
+    for (int i = 0; i < 4; ++i)
+      gmax[i] = active ? (int)side[a.side_stride - 4 + (kDeriv ? 2 * jb.half + (i & 1) : i)] : 0;
+    double cE[16][2], cO[16][2];
 #pragma unroll
-    for (int k4 = 0; k4 < KB; k4 += 4) {
-      if (k4 < kend) {
+    for (int nt = 0; nt < 16; ++nt) cE[nt][0] = cE[nt][1] = cO[nt][0] = cO[nt][1] = 0.0;
+    for (int k0 = 0; k0 < jb.rows4; k0 += KB, ++it) {
+      if (k0 > 0 && !(ok = mbar_wait(&sm.full[it % NS], (it / NS) & 1, sm, a.wait_err))) break;
+      const int st = it % NS;
+#pragma unroll
+      for (int k4 = 0; k4 < KB; k4 += 4) {
+        if (k0 + k4 >= jb.rows4) break;
         const int kk = k4 + q;
-        const double aE = sm.a[st][0][kk][8 * w + g];
-        const double aO = sm.a[st][1][kk][8 * w + g];
+        const int r = (8 * rg + g) ^ (4 * q);
+        const double aE = sm.a[st][kk][r], aO = sm.a[st][kk][32 + r];
 #pragma unroll
         for (int gr = 0; gr < 4; ++gr) {
           if (k0 + k4 < gmax[gr]) {
-            double b[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = sm.xs[st][kk][32 * gr + 8 * j + g];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              dmma(cE[4 * gr + j][0], cE[4 * gr + j][1], aE, b[j]);
-              dmma(cO[4 * gr + j][0], cO[4 * gr + j][1], aO, b[j]);
+            for (int jj = 0; jj < 2; ++jj) {
+              const int j = 2 * gr + jj;
+              const double2 b = *reinterpret_cast<const double2*>(
+                  &sm.xs[st][kk][16 * j + 4 * ((g >> 1) ^ q) + 2 * (g & 1)]);
+              dmma(cE[2 * j][0], cE[2 * j][1], aE, b.x);
+              dmma(cE[2 * j + 1][0], cE[2 * j + 1][1], aE, b.y);
+              dmma(cO[2 * j][0], cO[2 * j][1], aO, b.x);
+              dmma(cO[2 * j + 1][0], cO[2 * j + 1][1], aO, b.y);
             }
           }
         }
       }
+      warp_arrive(&sm.empty[st]);
+      if (w == 0 && !(ok = produce<kMode>(a, sm, pr, it + 1))) break;
     }
-  }
-  // The next tile's first stage went to buffer st; the next tile's second stage reuses this
-  // tile's last buffer only after the next tile's first barrier, which every warp reaches after
-  // its MMAs here.
-  st0 = st;
-}
-
-// The elements of an MMA tile, scaled, weighted and summed over the chunk's 32 spheres. Lane
-// pairs (q, q ^ 1) hold a node's (u) and (v) columns; after exchanging them the even lane forms
-// the elements at +mu and the odd lane those at -mu of its row (8 w + g) for its node of each
-// tile (2 nt + q / 2); the 16 nodes add in the thread, then node pairs across lanes q, q ^ 2.
-// Thread t ends with v[0], v[1]: row t / 4, side t & 1, elements 2 ((t / 2) & 1) + {0, 1}.
-template <bool kUser>
-__device__ __forceinline__ void chunk_elements_mma(Smem& sm, const double cE[16][2],
-                                                   const double cO[16][2], double v[2]) {
-  const int lane = threadIdx.x & 31, q = lane & 3;
-  const int side = q & 1;
-  const double sg = side ? -1.0 : 1.0;
-  double p[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-  for (int nt = 0; nt < 16; ++nt) {
-    const int node = 2 * nt + (q >> 1);
-    const double wt = sm.w[node], cu = sm.cu[node], ar = sm.area[node], sc = sm.sc[node];
-    const double e0 = cE[nt][0], e1 = cE[nt][1];
-    const double o0 = cO[nt][0], o1 = cO[nt][1];
-    const double pe0 = __shfl_xor_sync(0xffffffffu, e0, 1);
-    const double pe1 = __shfl_xor_sync(0xffffffffu, e1, 1);
-    const double po0 = __shfl_xor_sync(0xffffffffu, o0, 1);
-    const double po1 = __shfl_xor_sync(0xffffffffu, o1, 1);
-    // The even lane of a pair holds u (re, im), the odd one v.
-    const double eur = side ? pe0 : e0, eui = side ? pe1 : e1;
-    const double evr = side ? e0 : pe0, evi = side ? e1 : pe1;
-    const double our = side ? po0 : o0, oui = side ? po1 : o1;
-    const double ovr = side ? o0 : po0, ovi = side ? o1 : po1;
-    double e[4];
-    elements4(eur + sg * ovr, eui + sg * ovi, evr + sg * our, evi + sg * oui, e);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) p[k] += kUser ? wt * ((cu * e[k]) * ar) : wt * (sc * e[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) p[k] += __shfl_xor_sync(0xffffffffu, p[k], 2);
-  const int e2 = 2 * (q >> 1);
-  v[0] = e2 ? p[2] : p[0];
-  v[1] = e2 ? p[3] : p[1];
-}
-// accE/accO[r][c] = sum_k G[r0 + 4 rg + r][k] X[k][4 ng + c (+ 64 for c >= 4)] for k < nc.
-__device__ __forceinline__ void gemm_tile(Smem& sm, const double* __restrict__ ge,
-                                          const double* __restrict__ go, int ldr, int r0, int nc,
-                                          const double* __restrict__ xc, double accE[4][8],
-                                          double accO[4][8]) {
-  const int t = threadIdx.x, rg = t >> 4, ng = t & 15;
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      accE[r][c] = 0.0;
-      accO[r][c] = 0.0;
-    }
-  load_stage(sm, 0, ge, go, ldr, r0, 0, nc, xc);
-  int st = 0;
-  for (int k0 = 0; k0 < nc; k0 += KB, st ^= 1) {
-    cp_wait_all();
-    __syncthreads();
-    if (k0 + KB < nc) load_stage(sm, st ^ 1, ge, go, ldr, r0, k0 + KB, nc, xc);
-    const int kend = nc - k0 < KB ? nc - k0 : KB;
-#pragma unroll 8
-    for (int kk = 0; kk < KB; ++kk) {
-      if (kk < kend) {
-        const double2 e01 = *reinterpret_cast<const double2*>(&sm.a[st][0][kk][rg * 4]);
-        const double2 e23 = *reinterpret_cast<const double2*>(&sm.a[st][0][kk][rg * 4 + 2]);
-        const double2 o01 = *reinterpret_cast<const double2*>(&sm.a[st][1][kk][rg * 4]);
-        const double2 o23 = *reinterpret_cast<const double2*>(&sm.a[st][1][kk][rg * 4 + 2]);
-        const double2 x0 = *reinterpret_cast<const double2*>(&sm.xs[st][kk][ng * 4]);
-        const double2 x1 = *reinterpret_cast<const double2*>(&sm.xs[st][kk][ng * 4 + 2]);
-        const double2 y0 = *reinterpret_cast<const double2*>(&sm.xs[st][kk][(ng + 16) * 4]);
-        const double2 y1 = *reinterpret_cast<const double2*>(&sm.xs[st][kk][(ng + 16) * 4 + 2]);
-        const double ae[4] = {e01.x, e01.y, e23.x, e23.y};
-        const double ao[4] = {o01.x, o01.y, o23.x, o23.y};
-        const double xv[8] = {x0.x, x0.y, x1.x, x1.y, y0.x, y0.y, y1.x, y1.y};
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            accE[r][c] = fma(ae[r], xv[c], accE[r][c]);
-            accO[r][c] = fma(ao[r], xv[c], accO[r][c]);
-          }
-      }
-    }
-  }
-  __syncthreads();  // the stage buffers are free for the next tile
-}
-
-// Sums of p[32] over the 16 threads sharing a row group, scattered: thread ng ends with the
-// sums of entries 2 ng and 2 ng + 1 in v. At offset o a lane keeps the lower half of its values
-// if (ng & o) == 0.
-__device__ __forceinline__ void reduce_scatter16(double p[32], double v[2]) {
-  const int ng = threadIdx.x & 15;
-#pragma unroll
-  for (int lvl = 0, o = 8, h = 16; lvl < 4; ++lvl, o >>= 1, h >>= 1) {
-    const bool lower = (ng & o) == 0;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      if (i < h) {
-        const double mine = lower ? p[i] : p[i + h];
-        const double other = lower ? p[i + h] : p[i];
-        p[i] = mine + __shfl_xor_sync(0xffffffffu, other, o);
-      }
-    }
-  }
-  v[0] = p[0];
-  v[1] = p[1];
-}
-
-// The elements at +mu and -mu of this thread's 4 rows for its 2 spheres, scaled and weighted,
-// summed over the chunk's 32 spheres by a reduce-scatter over the 16 threads sharing the rows:
-// thread ng ends with v[0], v[1] of side ng >> 3 (0: +mu, 1: -mu), row (ng >> 1) & 3 and
-// elements 2 (ng & 1) and 2 (ng & 1) + 1.
-template <bool kUser>
-__device__ __forceinline__ void chunk_elements(const Smem& sm, const double accE[4][8],
-                                               const double accO[4][8], double v[2]) {
-  const int ng = threadIdx.x & 15;
-  double p[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) p[i] = 0.0;
-#pragma unroll
-  for (int nd = 0; nd < 2; ++nd) {
-    const int node = ng + 16 * nd;
-    const double w = sm.w[node], cu = sm.cu[node], ar = sm.area[node], sc = sm.sc[node];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const double eur = accE[r][4 * nd], eui = accE[r][4 * nd + 1];
-      const double evr = accE[r][4 * nd + 2], evi = accE[r][4 * nd + 3];
-      const double our = accO[r][4 * nd], oui = accO[r][4 * nd + 1];
-      const double ovr = accO[r][4 * nd + 2], ovi = accO[r][4 * nd + 3];
-      double ep[4], em[4];
-      elements4(eur + ovr, eui + ovi, evr + our, evi + oui, ep);
-      elements4(eur - ovr, eui - ovi, evr - our, evi - oui, em);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        // Requested cosines: W (4/x^2 F) pi r^2 (phase.rs:204-219, engine.rs:1075); band
-        // tables: W (4/x^2 pi r^2) F (engine.rs:1655-1660).
-        if (kUser) {
-          p[r * 4 + e] += w * ((cu * ep[e]) * ar);
-          p[16 + r * 4 + e] += w * ((cu * em[e]) * ar);
-        } else {
-          p[r * 4 + e] += w * (sc * ep[e]);
-          p[16 + r * 4 + e] += w * (sc * em[e]);
-        }
-      }
-    }
-  }
-  reduce_scatter16(p, v);
-}
-
-// The derivative blocks' elements of this thread's 4 rows for its one sphere (node
-// 16 half + ng; accumulator columns 0-3 its (u, v) sums, 4-7 those of (du/dm, dv/dm)), for
-// block blk: values (weight w), the distribution's parameters (their weights), Re m and Im m
-// (weight w, the element derivatives along dS/dm and i dS/dm; phase.rs:322-335), reduced over
-// the 16 spheres as chunk_elements does.
-// kDiff: with the error weights (w_K - w_G) ... instead.
-template <bool kUser, bool kDiff = false>
-__device__ __forceinline__ void chunk_elements_d(const Smem& sm, const double accE[4][8],
-                                                 const double accO[4][8], int half, int blk,
-                                                 int n_theta, double v[2]) {
-  const int ng = threadIdx.x & 15;
-  const int node = 16 * half + ng;
-  const int kind = blk == 0 ? 0 : (blk <= n_theta ? 0 : blk - n_theta);  // 0 f, 1 Re m, 2 Im m
-  const double wt = kDiff ? ((blk >= 1 && blk <= n_theta) ? sm.wthd[blk - 1][node] : sm.wd[node])
-                          : ((blk >= 1 && blk <= n_theta) ? sm.wth[blk - 1][node] : sm.w[node]);
-  const double cu = sm.cu[node], ar = sm.area[node], sc = sm.sc[node];
-  double p[32];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-#pragma unroll
-    for (int sd = 0; sd < 2; ++sd) {
-      const double sg = sd == 0 ? 1.0 : -1.0;
-      const double s1r = accE[r][0] + sg * accO[r][2], s1i = accE[r][1] + sg * accO[r][3];
-      const double s2r = accE[r][2] + sg * accO[r][0], s2i = accE[r][3] + sg * accO[r][1];
-      double e[4];
-      if (kind == 0) {
-        elements4(s1r, s1i, s2r, s2i, e);
+    if (!ok) break;
+    if (!active) continue;
+    // Where this lane's sums go: row row0 + g at +mu and -mu.
+    const int row = row0 + g;
+    int at[2] = {-1, -1};
+    if (row < jb.h) {
+      if (jb.user) {
+        const int2 mp = a.user_map[row];
+        at[0] = mp.x;
+        at[1] = mp.y;
       } else {
-        double d1r = accE[r][4] + sg * accO[r][6], d1i = accE[r][5] + sg * accO[r][7];
-        double d2r = accE[r][6] + sg * accO[r][4], d2i = accE[r][7] + sg * accO[r][5];
-        if (kind == 2) {
-          const double t1 = d1r, t2 = d2r;
-          d1r = -d1i;
-          d1i = t1;
-          d2r = -d2i;
-          d2i = t2;
-        }
-        element_derivs4(s1r, s1i, s2r, s2i, d1r, d1i, d2r, d2i, e);
+        at[0] = jb.len / 2 + row;
+        at[1] = jb.len - 1 - at[0];
+        if (at[1] == at[0]) at[1] = -1;
       }
+    }
+    double* out = a.acc + jb.out;
+    if constexpr (kMode == 0) {
+      double p[2][4] = {};
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        p[sd * 16 + r * 4 + k] = kUser ? wt * ((cu * e[k]) * ar) : wt * (sc * e[k]);
+      for (int j = 0; j < 8; ++j) {
+        const double f = side[4 * j + q];
+        add_elements(p[0], amplitudes(cE, cO, j, 1.0), f);
+        add_elements(p[1], amplitudes(cE, cO, j, -1.0), f);
+      }
+      // Reductions without a reply: a thread's adds to one sum stay in its program order, and no
+      // other thread adds to it while the kernel runs.
+#pragma unroll
+      for (int sd = 0; sd < 2; ++sd) {
+        const double v = reduce_elements(p[sd], 0.5);
+        if (at[sd] >= 0) atomicAdd(out + (int64_t)q * jb.len + at[sd], v);
+      }
+    } else if constexpr (kMode == 2) {
+#pragma unroll 1
+      for (int sd = 0; sd < 2; ++sd) {
+        const double sg = sd ? -1.0 : 1.0;
+        double p[4] = {}, e[2][4] = {};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const Amp s = amplitudes(cE, cO, j, sg);
+          add_elements(p, s, side[4 * j + q]);
+          add_elements(e[j >> 2], s, side[32 + 4 * j + q]);  // panel A: nodes 0-15, B: 16-31
+        }
+        const double v = reduce_elements(p, 0.5);
+        const double ve = fabs(reduce_elements(e[0], 0.5)) + fabs(reduce_elements(e[1], 0.5));
+        if (at[sd] >= 0) {
+          double* o = out + (int64_t)q * jb.len + at[sd];
+          atomicAdd(o, v);
+          atomicAdd(o + (int64_t)4 * jb.len, ve);
+        }
+      }
+    } else {
+      // The half's 16 nodes: pairs 0-3 their (u, v) sums, pairs 4-7 those of (du/dm, dv/dm).
+      // Blocks: values, the parameters (the elements by their weights), Re m and Im m (the element
+      // derivatives along dS/dm and i dS/dm; phase.rs:62-73, 322-335), by the values' weight.
+      const int n_blk = 3 + a.n_theta;
+#pragma unroll 1
+      for (int pass = 0; pass < (kMode == 3 ? 4 : 2); ++pass) {
+        const int sd = pass & 1, err = pass >> 1;
+        const double sg = sd ? -1.0 : 1.0;
+        const double* wt = side + err * 32 * (1 + a.n_theta) + 16 * jb.half + q;
+        double p[4][4] = {}, d[2][4] = {};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const Amp s = amplitudes(cE, cO, j, sg), ds = amplitudes(cE, cO, j + 4, sg);
+          const double f = wt[4 * j];
+          add_elements(p[0], s, f);
+#pragma unroll
+          for (int b = 1; b < 4; ++b)
+            if (b <= a.n_theta) add_elements(p[b], s, wt[32 * b + 4 * j]);
+          const double t1r = f * s.s1r, t1i = f * s.s1i, t2r = f * s.s2r, t2i = f * s.s2i;
+          d[0][0] = fma(t1r, ds.s1r, fma(t1i, ds.s1i, d[0][0]));
+          d[0][1] = fma(t2r, ds.s2r, fma(t2i, ds.s2i, d[0][1]));
+          d[0][2] = fma(t1r, ds.s2r, fma(t1i, ds.s2i, fma(t2r, ds.s1r, fma(t2i, ds.s1i, d[0][2]))));
+          d[0][3] = fma(t1r, ds.s2i, fma(-t1i, ds.s2r, fma(t2i, ds.s1r, fma(-t2r, ds.s1i, d[0][3]))));
+          // Along i dS: (re, im) -> (-im, re).
+          d[1][0] = fma(-t1r, ds.s1i, fma(t1i, ds.s1r, d[1][0]));
+          d[1][1] = fma(-t2r, ds.s2i, fma(t2i, ds.s2r, d[1][1]));
+          d[1][2] = fma(-t1r, ds.s2i, fma(t1i, ds.s2r, fma(-t2r, ds.s1i, fma(t2i, ds.s1r, d[1][2]))));
+          d[1][3] = fma(t1r, ds.s2r, fma(t1i, ds.s2i, fma(-t2i, ds.s1i, fma(-t2r, ds.s1r, d[1][3]))));
+        }
+        auto emit = [&](int blk, const double (&v)[4], double c) {
+          double x = reduce_elements(v, c);
+          if (err) x = fabs(x);
+          if (at[sd] >= 0)
+            atomicAdd(out + ((int64_t)(err * n_blk + blk) * 4 + q) * jb.len + at[sd], x);
+        };
+        emit(0, p[0], 0.5);
+#pragma unroll
+        for (int b = 1; b < 4; ++b)
+          if (b <= a.n_theta) emit(b, p[b], 0.5);
+        emit(1 + a.n_theta, d[0], 1.0);
+        emit(2 + a.n_theta, d[1], 1.0);
+      }
     }
   }
-  reduce_scatter16(p, v);
+  // A warp that gave up leaves stages in flight: they land before the CTA exits.
+  if (*(volatile int*)&sm.abort && w == 0 && lane == 0)
+    for (int s = pr.stage > NS ? pr.stage - NS : 0; s < pr.stage; ++s)
+      mbar_wait_drain(&sm.full[s % NS], (s / NS) & 1, a.wait_err);
+  __syncthreads();
 }
 
 }  // namespace
 
-// The error block of an adaptive call: |sum over panel A| + |sum over panel B| of the elements
-// weighted by w_K - w_G (sm.wth[0]), the chunk's panels being nodes 0-15 (this thread's node
-// ng) and 16-31 (node ng + 16); each panel reduced over its 16 nodes like chunk_elements.
-template <bool kUser>
-__device__ __forceinline__ void chunk_errors(const Smem& sm, const double accE[4][8],
-                                             const double accO[4][8], double v[2]) {
-  const int ng = threadIdx.x & 15;
-  double out[2] = {0.0, 0.0};
-#pragma unroll 1
-  for (int nd = 0; nd < 2; ++nd) {
-    const int node = ng + 16 * nd;
-    const double w = sm.wth[0][node], cu = sm.cu[node], ar = sm.area[node], sc = sm.sc[node];
-    double p[32];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      double eu_r = nd ? accE[r][4] : accE[r][0], eu_i = nd ? accE[r][5] : accE[r][1];
-      double ev_r = nd ? accE[r][6] : accE[r][2], ev_i = nd ? accE[r][7] : accE[r][3];
-      double ou_r = nd ? accO[r][4] : accO[r][0], ou_i = nd ? accO[r][5] : accO[r][1];
-      double ov_r = nd ? accO[r][6] : accO[r][2], ov_i = nd ? accO[r][7] : accO[r][3];
-      double ep[4], em[4];
-      elements4(eu_r + ov_r, eu_i + ov_i, ev_r + ou_r, ev_i + ou_i, ep);
-      elements4(eu_r - ov_r, eu_i - ov_i, ev_r - ou_r, ev_i - ou_i, em);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        p[r * 4 + e] = kUser ? w * ((cu * ep[e]) * ar) : w * (sc * ep[e]);
-        p[16 + r * 4 + e] = kUser ? w * ((cu * em[e]) * ar) : w * (sc * em[e]);
-      }
-    }
-    double vv[2];
-    reduce_scatter16(p, vv);
-    out[0] += fabs(vv[0]);
-    out[1] += fabs(vv[1]);
-  }
-  v[0] = out[0];
-  v[1] = out[1];
-}
+// K-b and K-c: persistent CTAs work through items (a unit and a share of its row tiles). A tile is 32
+// table rows x the chunk's 128 coefficient columns: C_E = G_E X and C_O = G_O X on the FP64 MMA
+// (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind), each warp 8 rows x all columns, the MMAs of a
+// group of 8 nodes stopping above its largest number of terms. Bulk copies into four stages of 8
+// orders, issued by warp 0 and waited for on mbarriers, run on across tiles and chunks; the warps
+// meet at no barrier, so a warp in its epilogue leaves the FP64 path to the others. Every output sum
+// is owned by one thread of one work item and runs over the chunks in order, so the results do not
+// depend on how a unit's tiles are split into items.
+//
+// Bound by the FP64 tensor path: 30 TFLOP/s executed over a pass of 64 x 512 units of 512 nodes, 0.82
+// of its rate (100 ms; 105 with cp.async stages behind block barriers, which drained at every chunk).
+// The derivative and adaptive forms ran on scalar FMAs with a 16-lane reduce-scatter per block of
+// sums: 1.10 -> 0.69 ms (768 units, 5 blocks) and 10.5 -> 5.9 ms (1024 units).
+__global__ void __launch_bounds__(NT, 3) unit_kernel(UnitArgs a) { unit_body<0, 1>(a); }
 
-// kMode 0: values; 1: with the derivative blocks; 2: adaptive panels (values and errors);
-// 3: adaptive panels with the derivative blocks (each block's sums, then its error sums: every
-// 16-node half of a chunk is one panel).
-template <int kMode>
-__device__ __forceinline__ void unit_body(const UnitArgs& a) {
-  constexpr bool kDeriv = kMode == 1 || kMode == 3;
-  constexpr bool kAdD = kMode == 3;
-  extern __shared__ __align__(16) unsigned char unit_raw[];
-  Smem& sm = *reinterpret_cast<Smem*>(unit_raw);
-  const int t = threadIdx.x, rg = t >> 4, ng = t & 15;
-  // This thread's share of a reduced tile: side (+mu, -mu), row, two elements.
-  const int side = ng >> 3, rr = (ng >> 1) & 3, e0 = 2 * (ng & 1);
-  // Blocks of sums: the values, then (with derivatives) each distribution parameter, Re m and
-  // Im m; halves: a chunk's coefficient rows are one 32-node tile, or two of 16 nodes with
-  // their derivative columns.
-  const int n_blk = kDeriv ? 3 + a.n_theta : (kMode == 2 ? 2 : 1);  // blocks of sums computed
-  constexpr int kHalves = kDeriv ? 2 : 1;
-  for (;;) {
-    if (t == 0) sm.slot = atomicAdd(a.work_counter, 1);
-    __syncthreads();
-    const int slot = sm.slot;
-    __syncthreads();
-    if (slot >= a.n_items) break;
-    const WorkItem it = a.items[slot];
-    const int ul = it.unit;
-    const int64_t unit = a.units[ul];
-    const int64_t d = unit / a.n_wl, i = unit % a.n_wl;
-    const double lam = a.wl[i];
-    double* acc_user = a.acc + a.unit_acc[ul];
-    for (int c = 0; c < a.cpu; ++c) {
-      const int64_t ci = (int64_t)ul * a.cpu + c;
-      const int nc = a.chunk_n[ci];
-      if (nc == 0) continue;
-      if (a.i8_above > 0 && nc > a.i8_above && nc <= kI8MaxTerms) continue;  // the int8 path's
-      const int b = chunk_band(nc, a.merge_max, a.n_levels, a.greek_order);
-      const int t_user = nc <= a.merge_max ? 0 : (a.h_u + TR - 1) / TR;
-      const int t_band = b >= 0 ? (a.bands[b].h + TR - 1) / TR : 0;
-      // This item's first tile; a level's tiles move on by one item per run of chunks.
-      const int shift = nc <= a.merge_max ? (c / kRunChunks) % it.n_groups : 0;
-      const int tile0 = it.group >= shift ? it.group - shift : it.group - shift + it.n_groups;
-      if (tile0 >= t_user + t_band) continue;
-      if (t < 32) {
-        const int j = c * 32 + t;
-        double w = 0.0, cu = 0.0, ar = 0.0, sc = 0.0, wd = 0.0;
-        int nn = 0;
-        double wth[3] = {0.0, 0.0, 0.0}, wthd[3] = {0.0, 0.0, 0.0};
-        const int64_t node = (a.per_unit ? unit : d) * a.n_nodes + j;
-        if (j < a.n_nodes && a.radius[node] > 0.0) {
-          const double r = a.radius[node];
-          const double x = 2.0 * kPi * r / lam;
-          // ceil(x + 6 x^(1/3) + 3), the truncation, plus one for a contraction's rounding.
-          nn = (int)ceil(x + 6.0 * cbrt(x) + 3.0) + 1;
-          w = a.weight[node];  // w_j u(r_j) r_j
-          cu = 4.0 / (x * x);
-          ar = kPi * r * r;
-          sc = 4.0 / (x * x) * (kPi * r * r);
-          if (kDeriv)
-            for (int p = 0; p < a.n_theta; ++p) wth[p] = a.wtheta[node * 3 + p];
-          if (kMode == 2) wth[0] = a.wdiff[node];
-          if (kAdD) {
-            wd = a.wdiff[node];
-            for (int p = 0; p < a.n_theta; ++p) wthd[p] = a.wthdiff[node * 3 + p];
-          }
-        }
-        sm.w[t] = w;
-        sm.cu[t] = cu;
-        sm.area[t] = ar;
-        sm.sc[t] = sc;
-        sm.nn[t] = nn;
-        if (kDeriv || kMode == 2)
-          for (int p = 0; p < 3; ++p) sm.wth[p][t] = wth[p];
-        if (kAdD) {
-          sm.wd[t] = wd;
-          for (int p = 0; p < 3; ++p) sm.wthd[p][t] = wthd[p];
-        }
-      }
-      __syncthreads();
-      for (int half = 0; half < kHalves; ++half) {
-        const double* xc = a.X + (a.chunk_row[ci] + (int64_t)half * nc) * 128;
-        double v[2];
-        // This thread's output of a reduced tile (kMode 0, the MMA tile, owns row t / 4).
-        const int o_row = kMode == 0 ? (t >> 2) : rg * 4 + rr;
-        const int o_side = kMode == 0 ? (t & 1) : side;
-        const int o_e0 = kMode == 0 ? 2 * ((t >> 1) & 1) : e0;
-        // A tile's table rows: the user cosines', then the band's.
-        auto source = [&](int tl) {
-          const bool u = tl < t_user;
-          const BandDesc Bd = u ? BandDesc{} : a.bands[b];
-          const bool lv = b < a.n_levels;
-          return TileSrc{u ? a.ge_u : (lv ? a.level_ge : a.band_ge) + Bd.g_off,
-                         u ? a.go_u : (lv ? a.level_go : a.band_go) + Bd.g_off,
-                         u ? a.h_u_pad : Bd.h_pad, (u ? tl : tl - t_user) * TR};
-        };
-        int st0 = 0;  // the stage buffer of the next MMA tile's first stage (kMode 0)
-        if constexpr (kMode == 0) {
-          const TileSrc s0 = source(tile0);
-          load_stage_z(sm, 0, s0.ge, s0.go, s0.ldr, s0.r0, 0, nc, xc);
-        }
-        for (int tile = tile0; tile < t_user + t_band; tile += it.n_groups) {
-          const bool user = tile < t_user;
-          const BandDesc B = user ? BandDesc{} : a.bands[b];
-          const int r0 = (user ? tile : tile - t_user) * TR;
-          const TileSrc src = source(tile);
-          // The output index of this thread's sums, or -1.
-          const int row = r0 + o_row;
-          int j = -1;
-          if (user) {
-            if (row < a.h_u) {
-              const int2 mp = a.user_map[row];
-              j = o_side ? mp.y : mp.x;
-            }
-          } else if (row < B.h) {
-            const int q = B.n_q, jn = q / 2 + row, mirror = q - 1 - jn;
-            if (o_side == 0 || mirror != jn) j = o_side ? mirror : jn;
-          }
-          const int64_t len = user ? a.n_mu : B.n_q;
-          double* base = user ? acc_user : a.acc + a.chunk_acc[ci];
-          if constexpr (kMode == 0) {
-            double cE[16][2], cO[16][2];
-            const int tn = tile + it.n_groups;
-            const TileSrc nx = source(tn < t_user + t_band ? tn : tile);
-            gemm_tile_mma(sm, src, nc, xc, cE, cO, st0,
-                          tn < t_user + t_band ? &nx : nullptr);
-            if (user)
-              chunk_elements_mma<true>(sm, cE, cO, v);
-            else
-              chunk_elements_mma<false>(sm, cE, cO, v);
-            if (j >= 0) {
-              base[o_e0 * len + j] += v[0];
-              base[(o_e0 + 1) * len + j] += v[1];
-            }
-          } else {
-            double accE[4][8], accO[4][8];
-            gemm_tile(sm, src.ge, src.go, src.ldr, r0, nc, xc, accE, accO);
-            for (int blk = 0; blk < n_blk; ++blk) {
-              if (user) {
-                if (kDeriv)
-                  chunk_elements_d<true>(sm, accE, accO, half, blk, a.n_theta, v);
-                else if (kMode == 2 && blk == 1)
-                  chunk_errors<true>(sm, accE, accO, v);
-                else
-                  chunk_elements<true>(sm, accE, accO, v);
-              } else {
-                if (kDeriv)
-                  chunk_elements_d<false>(sm, accE, accO, half, blk, a.n_theta, v);
-                else if (kMode == 2 && blk == 1)
-                  chunk_errors<false>(sm, accE, accO, v);
-                else
-                  chunk_elements<false>(sm, accE, accO, v);
-              }
-              if (j >= 0) {
-                double* ab = base + (int64_t)blk * 4 * len;
-                ab[o_e0 * len + j] += v[0];
-                ab[(o_e0 + 1) * len + j] += v[1];
-              }
-              if constexpr (kAdD) {
-                // The panel's |Kronrod - Gauss| into the block's error sums.
-                double ve[2];
-                if (user)
-                  chunk_elements_d<true, true>(sm, accE, accO, half, blk, a.n_theta, ve);
-                else
-                  chunk_elements_d<false, true>(sm, accE, accO, half, blk, a.n_theta, ve);
-                if (j >= 0) {
-                  double* ab = base + (int64_t)(n_blk + blk) * 4 * len;
-                  ab[o_e0 * len + j] += fabs(ve[0]);
-                  ab[(o_e0 + 1) * len + j] += fabs(ve[1]);
-                }
-              }
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// K-b and K-c: each work item runs its row tiles of every chunk of its unit and adds the
-// reduced tiles into the unit's accumulators. Every output sum is owned by one thread of one
-// work item and runs over the chunks in order, so the results do not depend on how a unit's
-// tiles are split into work items.
-__global__ void __launch_bounds__(NT, 3) unit_kernel(UnitArgs a) { unit_body<0>(a); }
-
-// The same with the derivative blocks: per chunk, its two 16-node halves in order; per tile,
-// every block's sums (values, distribution parameters, Re m, Im m), each into its own
-// accumulator (4 n_mu or 4 n_q doubles apart).
-__global__ void __launch_bounds__(NT) unit_deriv_kernel(UnitArgs a) { unit_body<1>(a); }
+// With the derivative blocks: per chunk its two 16-node halves, values and derivative columns in
+// one tile.
+__global__ void __launch_bounds__(NT, 2) unit_deriv_kernel(UnitArgs a) { unit_body<1, 4>(a); }
 
 // Adaptive panels: per tile the values' sums and the sums of |Kronrod - Gauss| per panel.
-__global__ void __launch_bounds__(NT) unit_adaptive_kernel(UnitArgs a) { unit_body<2>(a); }
+__global__ void __launch_bounds__(NT, 2) unit_adaptive_kernel(UnitArgs a) { unit_body<2, 2>(a); }
 
 // Adaptive panels with the derivative blocks: per tile every block's sums and error sums.
-__global__ void __launch_bounds__(NT) unit_adaptive_deriv_kernel(UnitArgs a) { unit_body<3>(a); }
+__global__ void __launch_bounds__(NT, 2) unit_adaptive_deriv_kernel(UnitArgs a) {
+  unit_body<3, 8>(a);
+}
 
 // K-d: the Greek coefficients of each band slot, (2l+1)/2 sum_k w_k F(mu_k) d_l(mu_k) with F
 // the slot's averaged tables (fast.rs:238-253): a contraction over the band's n_q nodes shared
@@ -1281,29 +1147,43 @@ static void configure_units() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    for (auto f : {unit_kernel, unit_deriv_kernel, unit_adaptive_kernel, unit_adaptive_deriv_kernel})
-      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
+    const auto set = [](void (*f)(UnitArgs), size_t bytes) {
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    set(unit_kernel, sizeof(UnitSmem<1>));
+    set(unit_deriv_kernel, sizeof(UnitSmem<4>));
+    set(unit_adaptive_kernel, sizeof(UnitSmem<2>));
+    set(unit_adaptive_deriv_kernel, sizeof(UnitSmem<8>));
     configured[dev] = true;
   }
 }
 
-int unit_kernel_blocks_per_sm() {
+int unit_kernel_blocks_per_sm(int mode) {
   configure_units();
   int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, unit_kernel, NT, sizeof(Smem));
+  if (mode == 0)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, unit_kernel, NT, sizeof(UnitSmem<1>));
+  else if (mode == 1)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, unit_deriv_kernel, NT, sizeof(UnitSmem<4>));
+  else if (mode == 2)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, unit_adaptive_kernel, NT,
+                                                  sizeof(UnitSmem<2>));
+  else
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, unit_adaptive_deriv_kernel, NT,
+                                                  sizeof(UnitSmem<8>));
   return n > 0 ? n : 1;
 }
 
 void launch_units(const UnitArgs& a, int grid, cudaStream_t s) {
   configure_units();
-  if (a.deriv && a.wdiff)
-    unit_adaptive_deriv_kernel<<<grid, NT, sizeof(Smem), s>>>(a);
+  if (a.deriv && a.adaptive)
+    unit_adaptive_deriv_kernel<<<grid, NT, sizeof(UnitSmem<8>), s>>>(a);
   else if (a.deriv)
-    unit_deriv_kernel<<<grid, NT, sizeof(Smem), s>>>(a);
-  else if (a.wdiff)
-    unit_adaptive_kernel<<<grid, NT, sizeof(Smem), s>>>(a);
+    unit_deriv_kernel<<<grid, NT, sizeof(UnitSmem<4>), s>>>(a);
+  else if (a.adaptive)
+    unit_adaptive_kernel<<<grid, NT, sizeof(UnitSmem<2>), s>>>(a);
   else
-    unit_kernel<<<grid, NT, sizeof(Smem), s>>>(a);
+    unit_kernel<<<grid, NT, sizeof(UnitSmem<1>), s>>>(a);
 }
 
 void launch_proj(const ProjArgs& a, cudaStream_t s) {
