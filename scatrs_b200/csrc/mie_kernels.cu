@@ -7,6 +7,7 @@
 // n (scatrs/src/ensemble/fast.rs:95-137), zero above the node's own N.
 #include "kernels.h"
 #include "layered_deriv.cuh"
+#include "layered_fixed.cuh"
 #include "mie_device.cuh"
 
 namespace sb {
@@ -61,7 +62,8 @@ __device__ __forceinline__ void put_side(const MieFixedArgs& a, int chunk, int l
   if ((lane & 7) == 0) o[a.side_stride - 4 + (lane >> 3)] = (double)top;
 }
 
-template <bool kLayered, bool kAdaptive>
+// kL: 1 homogeneous, 2 to 4 layers with the state sized at compile time, 0 any number of layers.
+template <int kL, bool kAdaptive>
 __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
   int wslot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
@@ -76,6 +78,7 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
   // This lane's place in the coefficient row of order index k (kernels.h).
   auto Xk = [&](int64_t k) { return a.X + (row0 + k) * 128 + ((lane ^ (int)(k & 3)) << 2); };
   // Scratch: 2L - 1 complex ratio arrays (one for a sphere) of nc + 2 rows, and u_k(x).
+  constexpr bool kLayered = kL != 1;
   const int n_arr = kLayered ? 2 * a.n_layers - 1 : 1;
   Scratch s;
   s.uz = a.uz + (row0 + 2 * (int64_t)chunk) * n_arr * 32 + lane;
@@ -114,10 +117,11 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
       }
     } else {
       // A layered sphere: x_l = f_l x, the outer surface's x last (ensemble/particle.rs:186-195).
-      const int L = a.n_layers;
-      double xs[kMaxLayers];
-      cplx ms[kMaxLayers];
+      const int L = kL > 1 ? kL : a.n_layers;
+      double xs[kL > 1 ? kL : kMaxLayers];
+      cplx ms[kL > 1 ? kL : kMaxLayers];
       bool lossless = true;
+#pragma unroll
       for (int l = 0; l < L; ++l) {
         xs[l] = l < L - 1 ? a.fractions[d * (L - 1) + l] * x : x;
         const double2 mv = a.m_layers[(d * L + l) * a.n_wl + i];
@@ -127,15 +131,21 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
       st = check_layered(xs, ms, L, n, a.allow_unvalidated != 0);
       if (st == 0 && n <= nc) {
         mie_prepare(x, ms[L - 1], n, s);
-        Layered lay;
-        lay.layers = L;
-        lay.x = xs;
-        lay.m = ms;
-        lay.arr.base = s.uz;
-        lay.arr.astride = (int64_t)(nc + 2) * 32;
-        lay.arr.stride = 32;
-        lay.prepare(n);
-        asum = mie_finish(x, ms[L - 1], n, s, vs, emit, lay);
+        const LayerArrays arr{s.uz, (int64_t)(nc + 2) * 32, 32};
+        if constexpr (kL > 1) {
+          lfix::LayeredT<kL, -1> lay;
+          lay.arr.arr = arr;
+          lay.prepare(n, xs, ms);
+          asum = mie_finish(x, ms[L - 1], n, s, vs, emit, lay);
+        } else {
+          Layered lay;
+          lay.layers = L;
+          lay.x = xs;
+          lay.m = ms;
+          lay.arr = arr;
+          lay.prepare(n);
+          asum = mie_finish(x, ms[L - 1], n, s, vs, emit, lay);
+        }
         // A lossless particle absorbs nothing (layered/kernel.rs:455-464).
         if (lossless) asum = 0.0;
       }
@@ -314,14 +324,14 @@ __device__ __forceinline__ void mie_chunk_deriv(const MieFixedArgs& a) {
 // warps per SM hide more of it than 12 (160 registers, no spills) did: 54.4 -> 49.7 ms per step
 // of the batched workload (5 CTAs, 96 registers: 60.5 ms).
 __global__ void __launch_bounds__(128, 4) mie_fixed_kernel(MieFixedArgs a) {
-  mie_chunk<false, false>(a);
+  mie_chunk<1, false>(a);
 }
 
 // Homogeneous spheres on adaptive panels (with the chunk's |Kronrod - Gauss| sums). 4 CTAs per
 // SM as mie_fixed_kernel (178 -> 128 registers): 7.8 -> 5.1 ms on a batch of 16 lognormals x 256
 // wavelengths (3 CTAs: 6.0 ms).
 __global__ void __launch_bounds__(128, 4) mie_adaptive_kernel(MieFixedArgs a) {
-  mie_chunk<false, true>(a);
+  mie_chunk<1, true>(a);
 }
 
 // Homogeneous spheres with derivatives.
@@ -332,7 +342,8 @@ __global__ void __launch_bounds__(128) mie_deriv_kernel(MieFixedArgs a) { mie_ch
 // row layout and chunk sums as mie_chunk_deriv, the blocks "Re" and "Im" being the derivative
 // along the direction and along i times it (meaningful for the index directions only).
 // Scratch per chunk: 2 (2L - 1) arrays (the ratios and their derivatives) of nc + 2 rows.
-template <int kCap>
+// kL: 2 or 3 layers and the direction kDir known at compile time (layered_fixed.cuh); 0: any.
+template <int kCap, int kL = 0, int kDir = 0>
 __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
   int wslot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
@@ -349,7 +360,7 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
     return a.X + (row0 + (int64_t)(lane >> 4) * nc4 + k) * 128 +
            (((lane & 15) ^ (int)(k & 3)) << 2);
   };
-  const int L = a.n_layers, n_arr = 2 * L - 1;
+  const int L = kL > 0 ? kL : a.n_layers, n_arr = 2 * L - 1;
   Scratch s;
   s.uz = a.uz + (row0 + 2 * (int64_t)chunk) * (2 * n_arr) * 32 + lane;
   s.ux = a.ux + (row0 + 2 * (int64_t)chunk) * 32 + lane;
@@ -374,7 +385,8 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
     lder::DR xd[kCap];
     lder::DC md[kCap];
     bool lossless = true;
-    const int dir = a.deriv_dir;
+    const int dir = kL > 0 ? kDir : a.deriv_dir;
+#pragma unroll
     for (int l = 0; l < L; ++l) {
       xs[l] = l < L - 1 ? a.fractions[d * (L - 1) + l] * x : x;
       const double2 mv = a.m_layers[(d * L + l) * a.n_wl + i];
@@ -389,15 +401,7 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
     DerivSums ds;
     if (st == 0 && n <= nc) {
       mie_prepare(x, ms[L - 1], n, s);  // u_k(x); array 0 is redone with its derivatives
-      lder::LayeredD<kCap> lay;
-      lay.layers = L;
-      lay.x = xd;
-      lay.m = md;
-      lay.arr.arr.base = s.uz;
-      lay.arr.arr.astride = (int64_t)(nc + 2) * 32;
-      lay.arr.arr.stride = 32;
-      lay.arr.n_val = n_arr;
-      lay.prepare(n, lder::DR{x, 0.0});
+      const LayerArrays arr{s.uz, (int64_t)(nc + 2) * 32, 32};
       auto emit = [&](int64_t k, cplx an, cplx bn, cplx dan, cplx dbn) {
         const bool odd = (k & 1) != 0;
         const cplx u = odd ? an : bn, v = odd ? bn : an;
@@ -408,7 +412,21 @@ __device__ __forceinline__ void layered_deriv_chunk(const MieFixedArgs& a) {
             make_double4(du.re, du.im, dv.re, dv.im);
         ds.add(k, an, bn, dan, dbn);
       };
-      asum = lder::layered_finish_d(x, md[L - 1], n, s, vs, emit, lay, abs_d);
+      if constexpr (kL > 0) {
+        lfix::LayeredT<kL, kDir> lay;
+        lay.arr.arr = arr;
+        lay.prepare(n, xs, ms);
+        asum = lfix::finish(x, ms[kL - 1], n, s, vs, emit, lay, abs_d);
+      } else {
+        lder::LayeredD<kCap> lay;
+        lay.layers = L;
+        lay.x = xd;
+        lay.m = md;
+        lay.arr.arr = arr;
+        lay.arr.n_val = n_arr;
+        lay.prepare(n, lder::DR{x, 0.0});
+        asum = lder::layered_finish_d(x, md[L - 1], n, s, vs, emit, lay, abs_d);
+      }
       ds.close(n);
       // A lossless particle absorbs nothing (layered/kernel.rs:455-464); its derivatives stand.
       if (lossless) asum = 0.0;
@@ -479,14 +497,16 @@ __global__ void __launch_bounds__(128) mie_layered_deriv16_kernel(MieFixedArgs a
   layered_deriv_chunk<kMaxLayers>(a);
 }
 
-// Layered spheres (their per-layer state lives in local memory).
-__global__ void __launch_bounds__(128) mie_layered_kernel(MieFixedArgs a) {
-  mie_chunk<true, false>(a);
+// 2 or 3 layers along one direction known at compile time.
+template <int kL, int kDir>
+__global__ void __launch_bounds__(128) mie_layered_deriv_fixed_kernel(MieFixedArgs a) {
+  layered_deriv_chunk<kL, kL, kDir>(a);
 }
 
-// Layered spheres on adaptive panels.
-__global__ void __launch_bounds__(128) mie_layered_adaptive_kernel(MieFixedArgs a) {
-  mie_chunk<true, true>(a);
+// Layered spheres: 2 to 4 layers with their state in registers, more in local memory.
+template <int kL, bool kAdaptive>
+__global__ void __launch_bounds__(128) mie_layered_kernel(MieFixedArgs a) {
+  mie_chunk<kL, kAdaptive>(a);
 }
 
 // Independent spheres, one per thread (the batched Mie::compute): coefficients a_1..a_N then
@@ -726,17 +746,34 @@ void launch_plan_chunks(const PlanArgs& a, cudaStream_t s) {
 void launch_mie_fixed(const MieFixedArgs& a, cudaStream_t s) {
   int threads = 128;
   int blocks = (a.n_chunks * 32 + threads - 1) / threads;
-  if (a.deriv && a.n_layers > 4)
-    mie_layered_deriv16_kernel<<<blocks, threads, 0, s>>>(a);
-  else if (a.deriv && a.n_layers > 1)
-    mie_layered_deriv_kernel<<<blocks, threads, 0, s>>>(a);
-  else if (a.deriv)
-    mie_deriv_kernel<<<blocks, threads, 0, s>>>(a);
-  else if (a.n_layers > 1 && a.wdiff)
-    mie_layered_adaptive_kernel<<<blocks, threads, 0, s>>>(a);
-  else if (a.n_layers > 1)
-    mie_layered_kernel<<<blocks, threads, 0, s>>>(a);
-  else if (a.wdiff)
+  const auto run = [&](void (*f)(MieFixedArgs)) { f<<<blocks, threads, 0, s>>>(a); };
+  if (a.deriv && a.n_layers > 4) {
+    run(mie_layered_deriv16_kernel);
+  } else if (a.deriv && a.n_layers == 2) {
+    run(a.deriv_dir == 0   ? mie_layered_deriv_fixed_kernel<2, 0>
+        : a.deriv_dir == 1 ? mie_layered_deriv_fixed_kernel<2, 1>
+                           : mie_layered_deriv_fixed_kernel<2, 2>);
+  } else if (a.deriv && a.n_layers == 3) {
+    run(a.deriv_dir == 0   ? mie_layered_deriv_fixed_kernel<3, 0>
+        : a.deriv_dir == 1 ? mie_layered_deriv_fixed_kernel<3, 1>
+        : a.deriv_dir == 2 ? mie_layered_deriv_fixed_kernel<3, 2>
+        : a.deriv_dir == 3 ? mie_layered_deriv_fixed_kernel<3, 3>
+                           : mie_layered_deriv_fixed_kernel<3, 4>);
+  } else if (a.deriv && a.n_layers > 1) {
+    run(mie_layered_deriv_kernel);
+  } else if (a.deriv) {
+    run(mie_deriv_kernel);
+  } else if (a.n_layers > 1) {
+    const bool ad = a.wdiff != nullptr;
+    if (a.n_layers == 2)
+      run(ad ? mie_layered_kernel<2, true> : mie_layered_kernel<2, false>);
+    else if (a.n_layers == 3)
+      run(ad ? mie_layered_kernel<3, true> : mie_layered_kernel<3, false>);
+    else if (a.n_layers == 4)
+      run(ad ? mie_layered_kernel<4, true> : mie_layered_kernel<4, false>);
+    else
+      run(ad ? mie_layered_kernel<0, true> : mie_layered_kernel<0, false>);
+  } else if (a.wdiff)
     mie_adaptive_kernel<<<blocks, threads, 0, s>>>(a);
   else
     mie_fixed_kernel<<<blocks, threads, 0, s>>>(a);
