@@ -89,7 +89,7 @@ __device__ __forceinline__ void ratios_d(DC m, DR x, int64_t n, const ArraysD& A
     for (int64_t k = start; k >= 1; --k) {
       const DC c = dscl(inv_z, (double)(2 * k + 1));
       DC den = c - u;
-      if (den.v.re == 0.0 && den.v.im == 0.0) den = dc(rl(kEps * (cabs_(c.v) + cabs_(u.v))));
+      if (den.v.re == 0.0 && den.v.im == 0.0) den = dc(rl(step_eps(c.v, u.v)));
       u = dinv(den);
       if (k <= top) A.put(a, k, u);
     }

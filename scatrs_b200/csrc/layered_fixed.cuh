@@ -199,7 +199,7 @@ LF_FN void ratios(V<Dm> m, R<Dx> x, int64_t n, const Arrays<kVal>& A, int a) {
       const V<D> c = vscl(inv_z, (double)(2 * k + 1));
       V<D> den = c - u;
       if (den.v.re == 0.0 && den.v.im == 0.0)
-        den = vv<D>(rl(kEps * (cabs_(c.v) + cabs_(u.v))));
+        den = vv<D>(rl(step_eps(c.v, u.v)));
       u = vinv(den);
       if (k <= top) A.put(a, k, u);
     }

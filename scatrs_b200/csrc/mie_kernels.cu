@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(128) mie_layered_deriv_fixed_kernel(MieFixedAr
 
 // Layered spheres: 2 to 4 layers with their state in registers, more in local memory.
 template <int kL, bool kAdaptive>
-__global__ void __launch_bounds__(128) mie_layered_kernel(MieFixedArgs a) {
+__global__ void __launch_bounds__(128, 3) mie_layered_kernel(MieFixedArgs a) {
   mie_chunk<kL, kAdaptive>(a);
 }
 
