@@ -83,10 +83,12 @@ template <bool A>
 LF_FN V<A> operator+(V<A> a, cplx b) { return a + V<false>{b}; }
 template <bool A>
 LF_FN V<A> operator-(V<A> a, cplx b) { return a - V<false>{b}; }
+// One copy of the reciprocal for the tens of them in an order.
+static __device__ __noinline__ cplx cinv_call(cplx z) { return cinv(z); }
 template <bool A>
 LF_FN V<A> vinv(V<A> a) {
   V<A> r;
-  r.v = cinv(a.v);
+  r.v = cinv_call(a.v);
   if constexpr (A) r.d = -(a.d * r.v * r.v);
   return r;
 }
