@@ -232,7 +232,7 @@ struct Context {
     std::vector<I8Table> user, band;
     DevBuf dig, scale, user_d, band_d;
   } i8;
-  DevBuf xdig, xside, colmax, chunk_xoff, chunk_xidx, i8_list, side;
+  DevBuf xdig, xside, colmax, chunk_xoff, chunk_xidx, i8_list, side, split, split_rows;
   // Spheroid T-matrices.
   DevBuf tm_geoms, tm_jobs, tm_rules, tm_node, tm_rad, tm_ang, tm_ser, tm_J, tm_work, tm_list, tm_T,
       tm_sums, tm_err;
@@ -948,7 +948,9 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   const int t_user = (c.user.h + 31) / 32;
   const int tile_slots = ad.on ? 32 : kSlotGroup;  // slots per projection item
   const int64_t acc_head = 4 * n_mu * n_blk;
-  std::vector<int64_t> urows(n_units), uacc(n_units), ui8(n_units, 0), ui8n(n_units, 0);
+  std::vector<int64_t> urows(n_units), uacc(n_units), ui8(n_units, 0), ui8n(n_units, 0),
+      uorders(n_units, 0);
+  const bool may_split = L_layers == 1 && !dv.on;  // homogeneous values
   std::vector<int> uslots(n_units), utiles(n_units);
   std::vector<double> ucost(n_units);
   int64_t total_rows = 0;
@@ -961,6 +963,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     for (int k = 0; k < cpu; ++k) {
       const int nc = cu[k];
       rows += (int64_t)rows_per_term * round_up(nc, 4);
+      uorders[u] += nc;
       if (on_i8(nc)) {
         ui8[u] += 2 * (int64_t)((nc + kI8KB - 1) / kI8KB) * kI8HalfBytes;
         ui8n[u] += 1;
@@ -1038,6 +1041,9 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     int64_t acc_len = 0;
     int64_t n_proj = 0;
     int64_t i8_bytes = 0, i8_chunks = 0;  // the mixed form's chunk digits
+    int64_t orders = 0;                   // the chunks' terms together
+    // K-a with a block per chunk: every chunk of the slab, or none.
+    int64_t split0 = 0, n_split = 0, split_rows = 0;
   };
   std::vector<Slab> slabs(n_slabs);
   std::vector<int> members(n_units);
@@ -1051,6 +1057,29 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       S.acc_len += uacc[u];
       S.i8_bytes += ui8[u];
       S.i8_chunks += ui8n[u];
+      S.orders += uorders[u];
+    }
+    // A chunk's recurrences take about 2000 cycles an order on one warp; the slab's, at 16 warps per
+    // SM, about 250 per chunk and order. Where most of a slab's orders are in chunks that would each
+    // take more than half of the slab's time, every chunk gets a block (mie_split_kernel).
+    if (may_split) {
+      int64_t s0 = 0;
+      std::vector<int64_t> long_orders(n_slabs, 0);
+      for (int64_t u = 0; u < n_units; ++u) {
+        const Slab& S = slabs[slab_of[u]];
+        const double half = 0.5 * 250.0 / 2000.0 * (double)S.orders / c.sms;
+        for (int k = 0; k < cpu; ++k)
+          if (cn[u * cpu + k] > half) long_orders[slab_of[u]] += cn[u * cpu + k];
+      }
+      for (int64_t sl = 0; sl < n_slabs; ++sl)
+        if (2 * long_orders[sl] > slabs[sl].orders) slabs[sl].n_split = count[sl] * cpu;
+      for (int64_t u = 0; u < n_units; ++u)
+        if (slabs[slab_of[u]].n_split > 0)
+          for (int k = 0; k < cpu; ++k) slabs[slab_of[u]].split_rows += cn[u * cpu + k] + 2;
+      for (Slab& S : slabs) {
+        S.split0 = s0;
+        s0 += S.n_split;
+      }
     }
     int64_t u0 = 0, sl0 = 0, pi0 = 0, it0 = 0;
     for (int64_t sl = 0; sl < n_slabs; ++sl) {
@@ -1075,13 +1104,14 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     }
   }
   int64_t acc_max = 1, slots_max = 1, stage_max = 0, n_slots_all = 0, n_proj_all = 0,
-          n_items_all = 0, i8_bytes_max = 16, i8_chunks_max = 1;
+          n_items_all = 0, i8_bytes_max = 16, i8_chunks_max = 1, n_split_all = 0, split_rows_max = 0;
   auto stage_bytes = [&](const Slab& S) {
     return S.nu * (int64_t)(sizeof(int) + 8 + sizeof(int2)) +
            S.nu * cpu * (int64_t)(sizeof(int) + 16) +
            S.n_slots * (int64_t)(sizeof(BandSlot) + sizeof(int)) +
            S.pi_cap * (int64_t)sizeof(ProjItem) + S.n_items * (int64_t)sizeof(WorkItem) +
-           (i8_above > 0 ? S.nu * cpu * (int64_t)(8 + 2 * sizeof(int)) + 64 : 0) + 256;
+           (i8_above > 0 ? S.nu * cpu * (int64_t)(8 + 2 * sizeof(int)) + 64 : 0) +
+           S.n_split * (int64_t)sizeof(MieSplit) + 256;
   };
   for (const Slab& S : slabs) {
     acc_max = std::max(acc_max, S.acc_len);
@@ -1092,6 +1122,8 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     n_items_all += S.n_items;
     i8_bytes_max = std::max(i8_bytes_max, S.i8_bytes);
     i8_chunks_max = std::max(i8_chunks_max, S.i8_chunks);
+    n_split_all += S.n_split;
+    split_rows_max = std::max(split_rows_max, S.split_rows);
   }
   // Device buffers: the plan's flat arrays (every slab its own segment), arena, scratch, sums.
   int* units_d = c.plan_units.as<int>(n_units);
@@ -1104,6 +1136,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   int* slot_index_d = c.slot_index.as<int>(std::max<int64_t>(n_slots_all, 1));
   ProjItem* proj_d = c.proj_items.as<ProjItem>(std::max<int64_t>(n_proj_all, 1));
   WorkItem* items_d = c.items.as<WorkItem>(std::max<int64_t>(n_items_all, 1));
+  MieSplit* split_d = c.split.as<MieSplit>(std::max<int64_t>(n_split_all, 1));
   double* X = c.X.as<double>((size_t)arena * 128);
   const int n_arr = L_layers > 1 ? 2 * L_layers - 1 : 1;
   // Layered derivatives keep each ratio array's derivative beside it.
@@ -1156,6 +1189,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   const int side_stride = 32 * (dv.on ? 1 + dv.n_theta : 1) * (ad.on ? 2 : 1) + 4;
   double* side = c.side.as<double>((size_t)kMaxSlabChunks * side_stride);
   ka.side = side;
+  if (may_split) ka.split_rows = c.split_rows.as<double4>((size_t)split_rows_max * 64);
   ka.side_stride = side_stride;
   ka.colmax = colmax;  // the mixed form's digit scales; null otherwise
   ka.uz = uz;
@@ -1274,6 +1308,8 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     int64_t* P_xoff = i8_above > 0 ? (int64_t*)take(nch * 8) : nullptr;
     int* P_xidx = i8_above > 0 ? (int*)take(nch * sizeof(int)) : nullptr;
     int* P_list = i8_above > 0 ? (int*)take(nch * sizeof(int)) : nullptr;
+    MieSplit* P_split = (MieSplit*)take(S.n_split * sizeof(MieSplit));
+    int64_t n_split = 0;
     int64_t xoff = 0;
     int n_i8 = 0;
     const size_t used = (size_t)(base - c.staging_half(sl & 1));
@@ -1291,6 +1327,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
         const int nc = cn[(int64_t)u * cpu + k];
         P_cn[ci] = nc;
         P_row[ci] = row;
+        if (S.n_split > 0) P_split[n_split++] = MieSplit{(int)ci, nc, 0};
         if (P_xoff) {
           P_xoff[ci] = -1;
           P_xidx[ci] = 0;
@@ -1347,6 +1384,14 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
                      [](const std::pair<double, int64_t>& x, const std::pair<double, int64_t>& y) {
                        return x.first < y.first;
                      });
+    // The split chunks, the longest first.
+    std::sort(P_split, P_split + n_split, [](const MieSplit& x, const MieSplit& y) {
+      return x.n != y.n ? x.n > y.n : x.chunk < y.chunk;
+    });
+    for (int64_t k = 0, at = 0; k < n_split; ++k) {
+      P_split[k].row = at;
+      at += P_split[k].n + 2;
+    }
     for (size_t k = 0; k < order.size(); ++k) {
       const int64_t lu = order[k].second / 65536;
       P_items[k].unit = (int)lu;
@@ -1404,6 +1449,9 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
                               cudaMemcpyHostToDevice, s));
     SB_CUDA(cudaMemcpyAsync(items_d + S.it0, P_items, S.n_items * sizeof(WorkItem),
                             cudaMemcpyHostToDevice, s));
+    if (n_split > 0)
+      SB_CUDA(cudaMemcpyAsync(split_d + S.split0, P_split, n_split * sizeof(MieSplit),
+                              cudaMemcpyHostToDevice, s));
     if (i8_above > 0) {
       SB_CUDA(cudaMemcpyAsync(chunk_xoff_d + ch0, P_xoff, nch * 8, cudaMemcpyHostToDevice, s));
       SB_CUDA(cudaMemcpyAsync(chunk_xidx_d + ch0, P_xidx, nch * sizeof(int),
@@ -1418,7 +1466,16 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     ka.n_chunks = (int)nch;
     ka.chunk_n = chunk_n_d + ch0;
     ka.chunk_row = chunk_row_d + ch0;
-    timed_launch(K_MIE, s, [&] { launch_mie_fixed(ka, s); });
+    if (may_split) {
+      ka.split_list = split_d + S.split0;
+      ka.n_split = (int)S.n_split;
+    }
+    timed_launch(K_MIE, s, [&] {
+      if (S.n_split > 0)
+        launch_mie_split(ka, s);
+      else
+        launch_mie_fixed(ka, s);
+    });
     SB_CUDA(cudaGetLastError());
     SB_CUDA(cudaMemsetAsync(acc, 0, (size_t)S.acc_len * 8, s));
     SB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), s));
@@ -6737,7 +6794,7 @@ void scatrs_release(void) {
                       &c.X, &c.uz, &c.ux, &c.chunk_sums, &c.err, &c.acc,
                       &c.counter, &c.values, &c.phase, &c.greek, &c.user.g,
                       &c.user.map, &c.user.rows_d, &c.tc_a_hi, &c.tc_a_lo, &c.tc_prod, &c.tc_err, &c.xdig,
-                      &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.side,
+                      &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.side, &c.split, &c.split_rows,
                       &c.i8.dig, &c.i8.scale, &c.i8.user_d, &c.i8.band_d, &c.ro_cgr, &c.ro_cgw})
       b->release();
     for (auto& kv : c.projectors)

@@ -17,6 +17,12 @@ struct PlanArgs {
   int per_unit;  // nodes per unit ([n_units][n_nodes]) rather than per distribution
 };
 
+// A chunk that K-a gives a block of its own, and its first scratch row.
+struct MieSplit {
+  int chunk, n;  // n: its orders
+  int64_t row;
+};
+
 // K-a over one slab: its units (global indices), each with cpu chunks of 32 nodes.
 struct MieFixedArgs {
   const double* radius;  // [n_dist][n_nodes]
@@ -42,6 +48,10 @@ struct MieFixedArgs {
   double* chunk_sums;       // [n_chunks][8] weighted per-particle quantities
   unsigned long long* err;
   int allow_unvalidated;
+  // mie_split_kernel's chunks and their scratch (64 (n + 2) from each one's row).
+  const MieSplit* split_list;
+  int n_split;
+  double4* split_rows;
   // Derivatives (homogeneous spheres): chunk rows of two 16-node halves, chunk_sums
   // [n_chunks][3 + n_theta][8], and the parameter weights w_j (du/dtheta_p)(r_j) r_j.
   int deriv;
@@ -465,6 +475,7 @@ struct Pass1Args {
 void launch_pass1_layered_deriv(const Pass1Args& a, cudaStream_t s);
 void launch_plan_chunks(const PlanArgs& a, cudaStream_t s);
 void launch_mie_fixed(const MieFixedArgs& a, cudaStream_t s);
+void launch_mie_split(const MieFixedArgs& a, cudaStream_t s);
 void launch_mie_nodes(const MieNodesArgs& a, cudaStream_t s);
 int unit_kernel_blocks_per_sm(int mode);  // 0 values, 1 derivatives, 2 adaptive, 3 both
 void launch_units(const UnitArgs& a, int grid, cudaStream_t s);

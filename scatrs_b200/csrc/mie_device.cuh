@@ -143,7 +143,7 @@ struct Scratch {
 
 // State::prepare (kernel.rs:249-313): u_k(mx) for k = 1..n+1 and u_k(x) for the orders above
 // the upward recurrences. The two recurrences are independent; they run one after the other.
-__device__ __forceinline__ void mie_prepare(double x, cplx m, int64_t n, const Scratch& s) {
+__device__ __forceinline__ void mie_prepare_x(double x, int64_t n, const Scratch& s) {
   int64_t n_s = upward_orders(x, n);
   int64_t top = n + 1;
   if (n_s < n) {
@@ -156,6 +156,9 @@ __device__ __forceinline__ void mie_prepare(double x, cplx m, int64_t n, const S
       if (k <= top) s.put_x(k, ux);
     }
   }
+}
+__device__ __forceinline__ void mie_prepare_z(double x, cplx m, int64_t n, const Scratch& s) {
+  int64_t top = n + 1;
   cplx z = scl(m, x);
   if (m.im == 0.0) {
     double inv_rho = 1.0 / z.re;
@@ -174,6 +177,10 @@ __device__ __forceinline__ void mie_prepare(double x, cplx m, int64_t n, const S
       if (k <= top) s.put_z(k, u);
     }
   }
+}
+__device__ __forceinline__ void mie_prepare(double x, cplx m, int64_t n, const Scratch& s) {
+  mie_prepare_x(x, n, s);
+  mie_prepare_z(x, m, n, s);
 }
 
 // Running sums of value_sums (scatrs/src/mie/efficiencies.rs:64-84), fed one order at a time

@@ -62,13 +62,32 @@ __device__ __forceinline__ void put_side(const MieFixedArgs& a, int chunk, int l
   if ((lane & 7) == 0) o[a.side_stride - 4 + (lane >> 3)] = (double)top;
 }
 
+// The chunk's weighted sums of the 8 per-particle quantities, in a fixed tree order; on adaptive
+// panels (qe weighted by w_K - w_G) then |Kronrod - Gauss| of each of the chunk's two panels (lanes
+// 0-15, 16-31), added.
+template <bool kAdaptive>
+__device__ __forceinline__ void put_sums(const MieFixedArgs& a, int chunk, int lane,
+                                         const double* q, const double* qe) {
+  const int stride = kAdaptive ? 16 : 8;
+  for (int k = 0; k < 8; ++k) {
+    double v = q[k];
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) a.chunk_sums[(int64_t)chunk * stride + k] = v;
+  }
+  if constexpr (kAdaptive) {
+    for (int k = 0; k < 8; ++k) {
+      double v = qe[k];
+      for (int off = 8; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+      const double other = __shfl_sync(0xffffffffu, v, 16);
+      if (lane == 0) a.chunk_sums[(int64_t)chunk * 16 + 8 + k] = fabs(v) + fabs(other);
+    }
+  }
+}
+
 // kL: 1 homogeneous, 2 to 4 layers with the state sized at compile time, 0 any number of layers.
 template <int kL, bool kAdaptive>
-__device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
-  int wslot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void mie_chunk(const MieFixedArgs& a, int chunk) {
   int lane = threadIdx.x & 31;
-  if (wslot >= a.n_chunks) return;
-  int chunk = wslot;
   int64_t unit = a.units[chunk / a.cpu];
   int c = chunk % a.cpu;
   int64_t d = unit / a.n_wl, i = unit % a.n_wl;
@@ -176,22 +195,220 @@ __device__ __forceinline__ void mie_chunk(const MieFixedArgs& a) {
   if (a.colmax != nullptr)
     *reinterpret_cast<double4*>(a.colmax + (int64_t)chunk * 128 + lane * 4) =
         make_double4(cm[0], cm[1], cm[2], cm[3]);
-  // The chunk's weighted sums, in a fixed tree order.
-  const int stride = kAdaptive ? 16 : 8;
-  for (int k = 0; k < 8; ++k) {
-    double v = q[k];
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) a.chunk_sums[(int64_t)chunk * stride + k] = v;
-  }
-  if constexpr (kAdaptive) {
-    // |Kronrod - Gauss| of each of the chunk's two panels (lanes 0-15, 16-31), then added.
-    for (int k = 0; k < 8; ++k) {
-      double v = qe[k];
-      for (int off = 8; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      const double other = __shfl_sync(0xffffffffu, v, 16);
-      if (lane == 0) a.chunk_sums[(int64_t)chunk * 16 + 8 + k] = fabs(v) + fabs(other);
+  put_sums<kAdaptive>(a, chunk, lane, q, qe);
+}
+
+// One chunk of homogeneous spheres by the kSplitWarps warps of a block. The serial recurrences run side
+// by side: warp 0 the downward u_k(mx), warp 1 the downward u_k(x) and the upward psi, chi (to order
+// floor(x)) and xi ratios beyond, which leave each order's factors in its coefficient row (4 doubles a
+// node) and a scratch row (1/xi). The orders are then independent: each warp takes a run of them and
+// overwrites the rows with the coefficients, in the operations of mie_finish, and leaves each order's
+// terms of the sums. Last, warp 0 adds the terms up over the orders, in the order of ValueSums and
+// mie_finish, so that every result has the bits of a warp on its own (mie_chunk).
+//
+// Bound by the recurrences' latency (a complex reciprocal per order): on its own a warp takes about
+// 2000 cycles per order, this block about 550.
+constexpr int kSplitWarps = 8;
+template <bool kAdaptive>
+__device__ __forceinline__ void mie_split_chunk(const MieFixedArgs& a, int chunk, int64_t scratch) {
+  constexpr int kW = kSplitWarps;
+  __shared__ double part[4][kW][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t unit = a.units[chunk / a.cpu];
+  const int c = chunk % a.cpu;
+  const int64_t d = unit / a.n_wl, i = unit % a.n_wl;
+  const int j = c * 32 + lane;
+  const int nc = a.chunk_n[chunk], nc4 = (nc + 3) & ~3;
+  const int64_t row0 = a.chunk_row[chunk];
+  auto Xk = [&](int64_t k) { return a.X + (row0 + k) * 128 + ((lane ^ (int)(k & 3)) << 2); };
+  // Scratch rows: u_k(mx) and u_k(x); 1/xi_k, later an order's terms of the sums (absorption, own and
+  // pair terms of g, sca; back).
+  Scratch s;
+  s.uz = a.uz + (row0 + 2 * (int64_t)chunk) * 32 + lane;
+  s.ux = a.ux + (row0 + 2 * (int64_t)chunk) * 32 + lane;
+  s.stride = 32;
+  double4* terms = a.split_rows + scratch * 64 + lane;
+  const int64_t node = (a.per_unit ? unit : d) * a.n_nodes + j;
+  const double r = j < a.n_nodes ? a.radius[node] : 0.0;
+  const double2 mv = a.m[unit];
+  const cplx m = mk(mv.x, mv.y);
+  double x = 0.0;
+  int64_t n = 0, n_s = 0;
+  if (r > 0.0) {
+    x = 2.0 * kPi * r / a.wl[i];
+    n = default_n_max(x);
+    int st = check_node(x, m, n, a.allow_unvalidated != 0);
+    if (st == 0 && n > nc) st = 1;
+    if (st != 0) {
+      if (warp == 0) record_error(a.err, i, d, j, a.n_dist, a.n_nodes, st);
+      n = 0;
+    } else {
+      n_s = upward_orders(x, n);
     }
   }
+  const double inv_x = 1.0 / x;
+  if (n > 0 && warp == 0) {
+    mie_prepare_z(x, m, n, s);
+  } else if (n > 0 && warp == 1) {
+    mie_prepare_x(x, n, s);
+    double sin_x, cos_x;
+    sincos(x, &sin_x, &cos_x);
+    double psi_prev = cos_x, psi = sin_x;
+    double chi_prev = -sin_x, chi = cos_x;
+    cplx t = rl(0.0), inv_xi = rl(0.0), rr = rl(0.0);
+    if (n_s == 0) {
+      cplx xi0 = mk(sin_x, -cos_x);
+      t = rl(sin_x) * cinv(xi0);
+      inv_xi = mk(sin_x, cos_x);
+      rr = mk(0.0, 1.0);
+    }
+    for (int64_t k = 1; k <= n_s; ++k) {
+      const double cc = (double)(2 * k - 1) * inv_x;
+      const double psi_next = cc * psi - psi_prev;
+      psi_prev = psi;
+      psi = psi_next;
+      const double chi_next = cc * chi - chi_prev;
+      chi_prev = chi;
+      chi = chi_next;
+      *reinterpret_cast<double4*>(Xk(k - 1)) = make_double4(psi, chi, psi_prev, chi_prev);
+    }
+    if (n_s > 0) {
+      const cplx xi = mk(psi, -chi);
+      inv_xi = cinv(xi);
+      t = rl(psi) * inv_xi;
+      rr = mk(psi_prev, -chi_prev) * inv_xi;
+    }
+    for (int64_t k = n_s + 1; k <= n; ++k) {
+      rr = cinv(rl((double)(2 * k - 1) * inv_x) - rr);
+      t = scl(t * rr, s.get_x(k));
+      inv_xi = inv_xi * rr;
+      *reinterpret_cast<double4*>(Xk(k - 1)) = make_double4(rr.re, rr.im, t.re, t.im);
+      terms[k * 64] = make_double4(inv_xi.re, inv_xi.im, 0.0, 0.0);
+    }
+  }
+  __syncthreads();
+  const int run = (nc + kW - 1) / kW;
+  const int64_t k_lo = 1 + (int64_t)warp * run, k_hi = min((int64_t)(warp + 1) * run, (int64_t)nc);
+  double cm[4] = {0.0, 0.0, 0.0, 0.0};
+  cplx a_prev = rl(0.0), b_prev = rl(0.0);
+  if (n > 0) {
+    const cplx inv_z = cinv(scl(m, x)), inv_m = cinv(m), inv_m2 = inv_m * inv_m;
+    const cplx c_a = -((m - rl(1.0)) * (m + rl(1.0)) * inv_m2);
+    const int64_t last = min(k_hi, n);
+    for (int64_t k = k_lo; k <= last; ++k) {
+      const double4 f = *reinterpret_cast<const double4*>(Xk(k - 1));
+      const double k_x = (double)k * inv_x;
+      const cplx u_z1 = s.get_z(k + 1);
+      const cplx dl = scl(inv_z, (double)(k + 1)) - u_z1;
+      const cplx d_m = dl * inv_m, md = dl * m;
+      const cplx big_a = d_m + rl(k_x), big_b = md + rl(k_x);
+      cplx an, bn, inv_da, inv_db;
+      if (k <= n_s) {
+        const double psi = f.x, psi_prev = f.z;
+        const cplx xi = mk(psi, -f.y), xi_prev = mk(psi_prev, -f.w);
+        inv_da = cinv(big_a * xi - xi_prev);
+        inv_db = cinv(big_b * xi - xi_prev);
+        an = (scl(big_a, psi) - rl(psi_prev)) * inv_da;
+        bn = (scl(big_b, psi) - rl(psi_prev)) * inv_db;
+      } else {
+        const cplx rr = mk(f.x, f.y), t = mk(f.z, f.w);
+        const double4 iv = terms[k * 64];
+        const cplx inv_xi = mk(iv.x, iv.y);
+        const cplx u_x1 = rl(s.get_x(k + 1));
+        const cplx num_a = scl(c_a, (double)(k + 1) * inv_x) + u_x1 - u_z1 * inv_m;
+        const cplx num_b = u_x1 - m * u_z1;
+        const cplx ia = cinv(big_a - rr), ib = cinv(big_b - rr);
+        an = t * num_a * ia;
+        bn = t * num_b * ib;
+        inv_da = inv_xi * ia;
+        inv_db = inv_xi * ib;
+      }
+      const bool odd = (k & 1) != 0;
+      const cplx u = odd ? an : bn, v = odd ? bn : an;
+      *reinterpret_cast<double4*>(Xk(k - 1)) = make_double4(u.re, u.im, v.re, v.im);
+      cm[0] = fmax(cm[0], fabs(u.re));
+      cm[1] = fmax(cm[1], fabs(u.im));
+      cm[2] = fmax(cm[2], fabs(v.re));
+      cm[3] = fmax(cm[3], fabs(v.im));
+      const double kf = (double)k, w = (double)(2 * k + 1);
+      // The terms of ValueSums::add, the pair term of orders k - 1 and k at order k (that of a run's
+      // first order follows below).
+      const double kp = kf - 1.0;
+      const double pair = k > k_lo ? kp * (kp + 2.0) / (kp + 1.0) * (re_mul_conj(a_prev, an) +
+                                                                     re_mul_conj(b_prev, bn))
+                                   : 0.0;
+      const cplx tb = scl(an - bn, w);
+      terms[k * 64] = make_double4(w * (-(d_m.im * nsq(inv_da)) - md.im * nsq(inv_db)),
+                                   w / (kf * (kf + 1.0)) * re_mul_conj(an, bn), pair,
+                                   w * (nsq(an) + nsq(bn)));
+      terms[k * 64 + 32] = odd ? make_double4(-tb.re, -tb.im, 0.0, 0.0)
+                               : make_double4(tb.re, tb.im, 0.0, 0.0);
+      a_prev = an;
+      b_prev = bn;
+    }
+  }
+  // Orders above the node's own N are zero up to the chunk's, rounded up to the GEMM's 4.
+  const int64_t z_hi = warp == kW - 1 ? (int64_t)nc4 : k_hi;
+  for (int64_t k = max(n + 1, min(k_lo, (int64_t)nc + 1)); k <= z_hi; ++k)
+    *reinterpret_cast<double4*>(Xk(k - 1)) = make_double4(0.0, 0.0, 0.0, 0.0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) part[k][warp][lane] = cm[k];
+  __syncthreads();
+  if (warp != 0) return;
+  // The pair terms at the runs' first orders.
+  for (int w = 1; w < kW; ++w) {
+    const int64_t k = 1 + (int64_t)w * run;
+    if (k > n) break;
+    const double4 p = *reinterpret_cast<const double4*>(Xk(k - 2));
+    const double4 q = *reinterpret_cast<const double4*>(Xk(k - 1));
+    // The rows hold (a, b) at odd and (b, a) at even orders.
+    const cplx p0 = mk(p.x, p.y), p1 = mk(p.z, p.w), q0 = mk(q.x, q.y), q1 = mk(q.z, q.w);
+    const bool odd = (k & 1) != 0;
+    const double kp = (double)(k - 1);
+    terms[k * 64].z = kp * (kp + 2.0) / (kp + 1.0) *
+                      (re_mul_conj(odd ? p1 : p0, odd ? q0 : q1) +
+                       re_mul_conj(odd ? p0 : p1, odd ? q1 : q0));
+  }
+  ValueSums vs;
+  double asum = 0.0, own = 0.0;
+#pragma unroll 4
+  for (int64_t k = 1; k <= n; ++k) {
+    const double4 p = terms[k * 64], q = terms[k * 64 + 32];
+    if (k > 1) {
+      vs.g += p.z;
+      vs.g += own;
+    }
+    own = p.y;
+    asum += p.x;
+    vs.sca += p.w;
+    vs.back = vs.back + mk(q.x, q.y);
+  }
+  if (n > 0) vs.g += own;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    cm[k] = part[k][0][lane];
+    for (int w = 1; w < kW; ++w) cm[k] = fmax(cm[k], part[k][w][lane]);
+  }
+  double q[8] = {0, 0, 0, 0, 0, 0, 0, 0}, qe[kAdaptive ? 8 : 1] = {};
+  double sc = 0.0, wv = 0.0, wd = 0.0;
+  if (n > 0) {
+    const Eff e = efficiencies_from(x, asum, vs);
+    const double area = kPi * r * r;
+    const double qv[8] = {1.0,           area * e.q_ext, area * e.q_sca, area * e.q_sca * e.g,
+                          area * e.q_abs, area * e.q_back, r * r,         r * r * r};
+    wv = a.weight[node];
+    sc = 4.0 / (x * x) * area;
+    for (int k = 0; k < 8; ++k) q[k] = wv * qv[k];
+    if constexpr (kAdaptive) {
+      wd = a.wdiff[node];
+      for (int k = 0; k < 8; ++k) qe[k] = wd * qv[k];
+    }
+  }
+  put_side(a, chunk, lane, sc, &wv, kAdaptive ? &wd : nullptr, 0, n);
+  if (a.colmax != nullptr)
+    *reinterpret_cast<double4*>(a.colmax + (int64_t)chunk * 128 + lane * 4) =
+        make_double4(cm[0], cm[1], cm[2], cm[3]);
+  put_sums<kAdaptive>(a, chunk, lane, q, qe);
 }
 
 // Homogeneous spheres with the derivatives along the distribution's parameters and m. The
@@ -319,19 +536,25 @@ __device__ __forceinline__ void mie_chunk_deriv(const MieFixedArgs& a) {
   }
 }
 
-// Homogeneous spheres.
-// 4 CTAs per SM (128 registers, 216 bytes spilled): the recurrences are latency-bound, and 16
-// warps per SM hide more of it than 12 (160 registers, no spills) did: 54.4 -> 49.7 ms per step
-// of the batched workload (5 CTAs, 96 registers: 60.5 ms).
+// Homogeneous spheres, a chunk per warp. 16 warps per SM (128 registers): the recurrences are
+// latency-bound, and they hide more of it than 12 (160 registers) did: 54.4 -> 49.7 ms per step of the
+// batched workload (20 warps, 96 registers: 60.5 ms); adaptive panels 7.8 -> 5.1 ms on 16 lognormals x
+// 256 wavelengths.
+template <bool kAdaptive>
 __global__ void __launch_bounds__(128, 4) mie_fixed_kernel(MieFixedArgs a) {
-  mie_chunk<1, false>(a);
+  const int chunk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (chunk < a.n_chunks) mie_chunk<1, kAdaptive>(a, chunk);
 }
 
-// Homogeneous spheres on adaptive panels (with the chunk's |Kronrod - Gauss| sums). 4 CTAs per
-// SM as mie_fixed_kernel (178 -> 128 registers): 7.8 -> 5.1 ms on a batch of 16 lognormals x 256
-// wavelengths (3 CTAs: 6.0 ms).
-__global__ void __launch_bounds__(128, 4) mie_adaptive_kernel(MieFixedArgs a) {
-  mie_chunk<1, true>(a);
+// A chunk per block, the longest first, where a slab has too few chunks for their latency to hide
+// (run_fixed): a warp's chunk of 750 orders takes 1.6 ms on its own. 96 units of droplets to 1800
+// orders 1.93 -> 0.98 ms, 165 units to 170 orders 251 -> 126 us, 3 units 49 -> 21 us. Full slabs lose:
+// the chunks take twice the SMs' time (64 x 512 units 24 -> 48 ms), and splitting only the longest
+// beside the others gained nothing on 2048 units to 750 orders.
+template <bool kAdaptive>
+__global__ void __launch_bounds__(32 * kSplitWarps, 2) mie_split_kernel(MieFixedArgs a) {
+  const MieSplit b = a.split_list[blockIdx.x];
+  mie_split_chunk<kAdaptive>(a, b.chunk, b.row);
 }
 
 // Homogeneous spheres with derivatives.
@@ -506,7 +729,8 @@ __global__ void __launch_bounds__(128) mie_layered_deriv_fixed_kernel(MieFixedAr
 // Layered spheres: 2 to 4 layers with their state in registers, more in local memory.
 template <int kL, bool kAdaptive>
 __global__ void __launch_bounds__(128, 3) mie_layered_kernel(MieFixedArgs a) {
-  mie_chunk<kL, kAdaptive>(a);
+  const int chunk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (chunk < a.n_chunks) mie_chunk<kL, kAdaptive>(a, chunk);
 }
 
 // Independent spheres, one per thread (the batched Mie::compute): coefficients a_1..a_N then
@@ -773,10 +997,15 @@ void launch_mie_fixed(const MieFixedArgs& a, cudaStream_t s) {
       run(ad ? mie_layered_kernel<4, true> : mie_layered_kernel<4, false>);
     else
       run(ad ? mie_layered_kernel<0, true> : mie_layered_kernel<0, false>);
-  } else if (a.wdiff)
-    mie_adaptive_kernel<<<blocks, threads, 0, s>>>(a);
-  else
-    mie_fixed_kernel<<<blocks, threads, 0, s>>>(a);
+  } else {
+    run(a.wdiff ? mie_fixed_kernel<true> : mie_fixed_kernel<false>);
+  }
+}
+
+void launch_mie_split(const MieFixedArgs& a, cudaStream_t s) {
+  if (a.n_split <= 0) return;
+  auto f = a.wdiff ? mie_split_kernel<true> : mie_split_kernel<false>;
+  f<<<a.n_split, 32 * kSplitWarps, 0, s>>>(a);
 }
 
 void launch_mie_nodes(const MieNodesArgs& a, cudaStream_t s) {
