@@ -255,27 +255,19 @@ std::vector<std::pair<double, double>> initial_panels(double t_lo, double t_hi, 
 // parameter), |Kronrod - Gauss| of the same, the Kronrod sums of |du/dtheta| r |q| and of
 // u r |q| (the scales of the parameter blocks and of the derivatives along m), and the
 // integrands per unit ln r at the first and last nodes.
-// One panel's pass-1 sums for one part, in one buffer (a panel of a job of many parts holds one
-// per part): the Kronrod sums k[nb] and their |Kronrod - Gauss| errors err[nb], the parameter
-// blocks' absolute integrals abs[nt nr], the absolute value integrals absv[nr], and the
+// One panel's pass-1 sums for one part, in the panel's buffer (Panel::buf, one allocation for all
+// of its job's parts): the Kronrod sums k[nb] and their |Kronrod - Gauss| errors err[nb], the
+// parameter blocks' absolute integrals abs[nt nr], the absolute value integrals absv[nr], and the
 // integrands at the panel's two ends edge(0)[nb], edge(1)[nb].
 struct Sums1 {
-  std::vector<double> buf;
+  double* buf = nullptr;
   int nb = 0, nab = 0, nr = 0;
-  void init(int nb_, int nab_, int nr_) {
-    nb = nb_, nab = nab_, nr = nr_;
-    buf.assign((size_t)4 * nb + nab + nr, 0.0);
-  }
-  double* k() { return buf.data(); }
-  double* err() { return buf.data() + nb; }
-  double* abs() { return buf.data() + 2 * nb; }
-  double* absv() { return buf.data() + 2 * nb + nab; }
-  double* edge(int e) { return buf.data() + 2 * nb + nab + nr + e * nb; }
-  const double* k() const { return buf.data(); }
-  const double* err() const { return buf.data() + nb; }
-  const double* abs() const { return buf.data() + 2 * nb; }
-  const double* absv() const { return buf.data() + 2 * nb + nab; }
-  const double* edge(int e) const { return buf.data() + 2 * nb + nab + nr + e * nb; }
+  static size_t length(int nb, int nab, int nr) { return (size_t)4 * nb + nab + nr; }
+  double* k() const { return buf; }
+  double* err() const { return buf + nb; }
+  double* abs() const { return buf + 2 * nb; }
+  double* absv() const { return buf + 2 * nb + nab; }
+  double* edge(int e) const { return buf + 2 * nb + nab + nr + e * nb; }
 };
 
 // The targets, errors and ends of a part (engine.rs:620-720, no Greek refinement).
@@ -290,16 +282,15 @@ Status status_of(const Part& part, const std::vector<const Sums1*>& s, const Opt
   const int n_greek = kPass1;
   Status st;
   st.target.assign(nb, 0.0);
-  auto total = [&](int j) {
-    double t = 0.0;
-    for (auto* x : s) t += x->k()[j];
-    return t;
-  };
-  auto abs_of = [&](int k) {
-    double t = 0.0;
-    for (auto* x : s) t += x->abs()[k];
-    return t;
-  };
+  // Every sum over the panels in one pass over their buffers, each in panel order.
+  std::vector<double> sums((size_t)2 * nb + nt * nr + nr, 0.0);
+  for (auto* x : s) {
+    const double* b = x->k();  // k, err, abs and absv lie one after the other
+    for (size_t j = 0; j < sums.size(); ++j) sums[j] += b[j];
+  }
+  const double *err = sums.data() + nb, *absv = sums.data() + 2 * nb + nt * nr;
+  auto total = [&](int j) { return sums[j]; };
+  auto abs_of = [&](int k) { return sums[2 * nb + k]; };
   // C_abs and each direction's derivative of it are refined to rtol of C_ext's.
   auto scale_of = [&](int j) {
     if (j == ABS) return EXT;
@@ -315,8 +306,7 @@ Status status_of(const Part& part, const std::vector<const Sums1*>& s, const Opt
       scale = std::max(std::fabs(total(BACK)), c_sca);
     } else if (j >= n_greek) {
       // The derivatives along m can cancel: their absolute integrands.
-      scale = 0.0;
-      for (auto* x : s) scale += x->absv()[scale_of(j)];
+      scale = absv[scale_of(j)];
     } else {
       scale = std::fabs(total(scale_of(j)));
     }
@@ -335,10 +325,8 @@ Status status_of(const Part& part, const std::vector<const Sums1*>& s, const Opt
   st.errors.assign(nb, 0.0);
   st.met = true;
   for (int j = 0; j < nb; ++j) {
-    double e = 0.0;
-    for (auto* x : s) e += x->err()[j];
-    st.errors[j] = e;
-    st.met = st.met && e <= st.target[j];
+    st.errors[j] = err[j];
+    st.met = st.met && st.errors[j] <= st.target[j];
   }
   // The ends: a tenth of the target per ext/STEP units of ln r; the parameter blocks against
   // their own size, floored at 1e-3 of the absolute integral.
@@ -365,7 +353,8 @@ struct Panel {
   double a, b;
   bool done = false;
   int64_t n_terms = 0;
-  std::vector<Sums1> sums;  // per part of the job
+  std::vector<Sums1> sums;  // per part of the job, in buf
+  std::vector<double> buf;
 };
 
 struct State {
@@ -590,7 +579,6 @@ void pass1(std::vector<Job>& jobs, const std::vector<Part>& parts, const double*
       pn.done = true;
       pn.n_terms = 0;
       for (int i = 0; i < 15; ++i) pn.n_terms = std::max(pn.n_terms, res[15 * k + i].n);
-      pn.sums.assign(jobs[ji].parts.size(), Sums1{});
       // The quantities of the group's first part's directions (engine.rs:491-506).
       const Part& first = parts[jobs[ji].parts[0]];
       const int nr = first.n_refined();
@@ -602,15 +590,30 @@ void pass1(std::vector<Job>& jobs, const std::vector<Part>& parts, const double*
           if (first.dirs[dir])
             for (int j = 0; j < kGroup; ++j) qi[at++] = kPass1 + kGroup * dir + j;
       }
+      pn.sums.resize(jobs[ji].parts.size());
+      size_t len = 0;
+      int nb_max = 0;
+      for (size_t p = 0; p < pn.sums.size(); ++p) {
+        const int nt = (int)parts[jobs[ji].parts[p]].grads.size(), nb = (1 + nt) * nr;
+        pn.sums[p].nb = nb, pn.sums[p].nab = nt * nr, pn.sums[p].nr = nr;
+        len += Sums1::length(nb, nt * nr, nr);
+        nb_max = std::max(nb_max, nb);
+      }
+      pn.buf.assign(len, 0.0);
+      double* at = pn.buf.data();
+      for (Sums1& s : pn.sums) {
+        s.buf = at;
+        at += Sums1::length(s.nb, s.nab, s.nr);
+      }
+      std::vector<double> g(nb_max);
       double grad[3];
       for (size_t p = 0; p < jobs[ji].parts.size(); ++p) {
         const Part& part = parts[jobs[ji].parts[p]];
         const int nt = (int)part.grads.size(), nb = (1 + nt) * nr;
-        Sums1& s = pn.sums[p];
-        s.init(nb, nt * nr, nr);
+        const Sums1& s = pn.sums[p];
         double *sk = s.k(), *serr = s.err(), *sabs = s.abs(), *sabsv = s.absv();
         double *e0 = s.edge(0), *e1 = s.edge(1);
-        std::vector<double> g(nb, 0.0);
+        std::fill(g.begin(), g.end(), 0.0);
         for (int i = 0; i < 15; ++i) {
           const double r = qs[15 * k + i].r;
           const double base = (nt > 0 ? part.u(r, grad) : part.u(r)) * r;

@@ -95,9 +95,11 @@ struct Query {
   int wl;
 };
 struct NodeResult {
-  double q[kNodeQ];  // the kPass1 quantities, then kGroup derivatives along each direction
+  // The kPass1 quantities, then, where a part asks for them, kGroup derivatives along each
+  // direction; owned by the evaluator until its next call.
+  const double* q = nullptr;
   // If set, the kGroup derivatives of every direction of the particle, in order, in place of
-  // q's (a layered sphere's, more than kMaxDirs); owned by the evaluator until its next call.
+  // q's (a layered sphere's, more than kMaxDirs); owned likewise.
   const double* dq = nullptr;
   int64_t n;
   int status;

@@ -215,6 +215,7 @@ struct Context {
       chunk_sums, err, acc, counter, values, phase, greek;
   // Pass 1 of the adaptive ensemble.
   DevBuf p1_radius, p1_wl, p1_wlu, p1_scratch, p1_uz, p1_ux, p1_q, p1_n, p1_status;
+  DevBuf node_rec;  // the node tables' records, a block at a time
   DevBuf avg, mix_first, mix_part, mix_frac;
   // The Greek projection of tables at Gauss cosines: per (n_q, L) the matrices (FP64 and their
   // TF32 heads and tails), and the workspaces of the tensor-core form.
@@ -722,6 +723,54 @@ void check_options(const scatrs_fixed_options* o, int64_t n_units, int64_t n_mu,
                   "the ensemble outputs would exceed 2 * MAX_MIE_VALUES = 268435456 real values"};
 }
 
+bool pinned_host(const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeHost;
+}
+
+// A call's outputs to the caller, all of them there when it returns. Large ones to pageable memory
+// go through the pinned staging halves, a block's copy from the device beside the host threads'
+// copy of the block before: the driver's own path is one thread, which also takes the page faults
+// of an array written for the first time (1.8 MB in all: the call 1.07 -> 0.87 ms; 4 MB: 6.6 -> 5.9).
+struct OutCopy {
+  void* dst;
+  const void* src;
+  int64_t bytes;
+};
+void copy_out(Context& c, const std::vector<OutCopy>& outs, cudaMemcpyKind kind, cudaStream_t s) {
+  constexpr int64_t kBlock = int64_t(2) << 20, kPiece = int64_t(64) << 10, kLeast = int64_t(256) << 10;
+  std::vector<OutCopy> blocks;
+  for (const OutCopy& o : outs) {
+    if (kind != cudaMemcpyDeviceToHost || o.bytes < kLeast || !o.dst || pinned_host(o.dst)) {
+      SB_CUDA(cudaMemcpyAsync(o.dst, o.src, (size_t)o.bytes, kind, s));
+      continue;
+    }
+    for (int64_t at = 0; at < o.bytes; at += kBlock)
+      blocks.push_back({(char*)o.dst + at, (const char*)o.src + at, std::min(kBlock, o.bytes - at)});
+  }
+  if (!blocks.empty()) c.ensure_staging((size_t)kBlock);
+  for (size_t i = 0; i <= blocks.size() && !blocks.empty(); ++i) {
+    if (i < blocks.size()) {
+      unsigned char* half = c.staging_half(i & 1);
+      SB_CUDA(cudaMemcpyAsync(half, blocks[i].src, (size_t)blocks[i].bytes, kind, s));
+      c.staging_uploaded(i & 1, s);
+    }
+    if (i == 0) continue;
+    const OutCopy& b = blocks[i - 1];
+    const unsigned char* half = c.staging_half((i - 1) & 1);  // waits for its copy
+    const int64_t pieces = (b.bytes + kPiece - 1) / kPiece;
+#pragma omp parallel for schedule(static)
+    for (int64_t p = 0; p < pieces; ++p)
+      memcpy((char*)b.dst + p * kPiece, half + p * kPiece,
+             (size_t)std::min(kPiece, b.bytes - p * kPiece));
+  }
+  SB_CUDA(cudaStreamSynchronize(s));
+}
+
 std::string node_message(int status, double lambda, double r) {
   char buf[256];
   snprintf(buf, sizeof buf, "at wavelength %e, radius %e: %s", lambda, r,
@@ -734,7 +783,7 @@ std::string node_message(int status, double lambda, double r) {
 
 struct FixedCall {
   // Host copies needed for error messages.
-  std::vector<double> radius;  // [n_dist][n_nodes], or [n_units][n_nodes] with per_unit
+  std::vector<double> radius;  // [n_dist][n_nodes]; with per_unit on the device (Context::radius)
   std::vector<double> wl_host;
   int64_t n_dist = 0, n_wl = 0, n_nodes = 0;
   bool per_unit = false;
@@ -775,17 +824,12 @@ struct DerivOutput {
 // per-unit normalization (8 doubles, see FinalArgs) and the device error outputs.
 struct AdaptiveInput {
   bool on = false;
-  const double* radius = nullptr;
-  const double* weight = nullptr;
-  const double* wdiff = nullptr;
   const double* unit_norm = nullptr;
   double* avg = nullptr;  // the units' averages, mixed and assembled by mix_assemble_kernel
   // With derivatives (and DerivOutput::on with n_theta parameters): per unit and node the
   // parameters' Kronrod weights w_K (du/dtheta) r and error weights (w_K - w_G) (du/dtheta) r
   // ([n_units][n_nodes][3]); unit_norm then holds kNormStrideD doubles per unit and avg the
   // per-block averages of final_adaptive_d_kernel.
-  const double* wtheta = nullptr;
-  const double* wthdiff = nullptr;
 };
 
 void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, const double* wl_dev,
@@ -862,20 +906,9 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
                             n_dist * (L_layers - 1) * 8, cudaMemcpyHostToDevice, s));
   }
   if (ad.on) {
-    // Nodes per unit.
-    const size_t cnt = (size_t)n_units * n_nodes;
-    SB_CUDA(cudaMemcpyAsync(c.radius.get(cnt * 8), ad.radius, cnt * 8, cudaMemcpyHostToDevice, s));
-    SB_CUDA(cudaMemcpyAsync(c.weight.get(cnt * 8), ad.weight, cnt * 8, cudaMemcpyHostToDevice, s));
-    SB_CUDA(cudaMemcpyAsync(c.wdiff.get(cnt * 8), ad.wdiff, cnt * 8, cudaMemcpyHostToDevice, s));
     const size_t norm_bytes = (size_t)n_units * (dv.on ? kNormStrideD : 8) * 8;
     SB_CUDA(cudaMemcpyAsync(c.unit_norm.get(norm_bytes), ad.unit_norm, norm_bytes,
                             cudaMemcpyHostToDevice, s));
-    if (dv.on) {
-      SB_CUDA(cudaMemcpyAsync(c.wtheta.get(cnt * 24), ad.wtheta, cnt * 24,
-                              cudaMemcpyHostToDevice, s));
-      SB_CUDA(cudaMemcpyAsync(c.wthdiff.get(cnt * 24), ad.wthdiff, cnt * 24,
-                              cudaMemcpyHostToDevice, s));
-    }
   } else {
     SB_CUDA(cudaMemcpyAsync(c.radius.get(radius.size() * 8), radius.data(), radius.size() * 8,
                             cudaMemcpyHostToDevice, s));
@@ -1638,7 +1671,14 @@ void check_device_errors(Context& c, cudaStream_t s, const FixedCall* call) {
       double lam = i < (int64_t)call->wl_host.size() ? call->wl_host[i] : NAN;
       const int64_t row = call->per_unit ? d * call->n_wl + i : d;
       const size_t at = (size_t)(row * call->n_nodes + j);
-      msg = node_message(status, lam, at < call->radius.size() ? call->radius[at] : NAN);
+      double r = NAN;
+      if (!call->per_unit) {
+        if (at < call->radius.size()) r = call->radius[at];
+      } else if (i < call->n_wl) {
+        SB_CUDA(cudaMemcpyAsync(&r, c.radius.as<double>(0) + at, 8, cudaMemcpyDeviceToHost, s));
+        SB_CUDA(cudaStreamSynchronize(s));
+      }
+      msg = node_message(status, lam, r);
     }
     throw Failure{status, msg};
   }
@@ -2099,42 +2139,54 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
   // 3 L - 1), filled by one pass per requested group, read by pass 1 through NodeResult::dq.
   const bool layered_dirs = L > 1 && any_dirs;
   std::vector<double> dq_store;
+  // The evaluations' host arrays, kept across pass 1's rounds (their memory touched once).
+  std::vector<double> q_store, r;
+  std::vector<int64_t> cap, off, nt;
+  std::vector<int> wi, st;
   const int64_t row_cap =
       layered_dirs ? std::max<int64_t>(int64_t(1) << 20, kRows / (2 * (2 * L - 1))) : kRows;
   auto eval = [&](const std::vector<adaptive::Query>& qs, std::vector<adaptive::NodeResult>& out) {
     size_t k0 = 0;
-    std::vector<double> r;
-    std::vector<int> wi;
-    std::vector<int64_t> off;
+    // A sphere's directions come with its values; a layered sphere's in the group passes.
+    const bool sphere_dirs = any_dirs && L == 1;
+    const int nq = sphere_dirs ? adaptive::kSphereQ : adaptive::kPass1;
+    const size_t n_qs = qs.size();
+    if (q_store.size() < n_qs * nq) q_store.resize(n_qs * nq);
+    if (r.size() < n_qs) {
+      r.resize(n_qs);
+      wi.resize(n_qs);
+      cap.resize(n_qs);
+      nt.resize(n_qs);
+      st.resize(n_qs);
+      off.resize(n_qs + 1);
+    }
+#pragma omp parallel for schedule(static)
+    for (int64_t k = 0; k < (int64_t)n_qs; ++k) {
+      const double x = 2.0 * 3.14159265358979323846 * qs[k].r / wavelengths[qs[k].wl % n_wl];
+      cap[k] = (std::isfinite(x) && x > 0.0 && x <= 1e6)
+                   ? (int64_t)std::ceil(x + 6.0 * std::cbrt(x) + 3.0) + 4
+                   : 0;
+      r[k] = qs[k].r;
+      wi[k] = qs[k].wl;
+    }
     const int64_t dstride = (int64_t)n_dirs_all * adaptive::kGroup;
     if (layered_dirs) dq_store.assign(qs.size() * (size_t)dstride, 0.0);
     while (k0 < qs.size()) {
-      r.clear();
-      wi.clear();
-      off.assign(1, 0);
       size_t k1 = k0;
-      while (k1 < qs.size()) {
-        const double x =
-            2.0 * 3.14159265358979323846 * qs[k1].r / wavelengths[qs[k1].wl % n_wl];
-        const int64_t cap = (std::isfinite(x) && x > 0.0 && x <= 1e6)
-                                ? (int64_t)std::ceil(x + 6.0 * std::cbrt(x) + 3.0) + 4
-                                : 0;
-        if (k1 > k0 && off.back() + cap > row_cap) break;
-        r.push_back(qs[k1].r);
-        wi.push_back(qs[k1].wl);
-        off.push_back(off.back() + cap);
+      off[0] = 0;
+      while (k1 < n_qs) {
+        const int64_t top = off[k1 - k0];
+        if (k1 > k0 && top + cap[k1] > row_cap) break;
+        off[k1 - k0 + 1] = top + cap[k1];
         ++k1;
       }
-      const int64_t n = (int64_t)r.size(), rows = std::max<int64_t>(off.back(), 1);
+      const int64_t n = (int64_t)(k1 - k0), rows = std::max<int64_t>(off[n], 1);
       Pass1Args a{};
       a.radius = c.p1_radius.as<double>(n);
       a.wl_index = c.p1_wl.as<int>(n);
       a.scratch = c.p1_scratch.as<int64_t>(n + 1);
       a.uz = c.p1_uz.as<double2>((size_t)rows * (2 * L - 1));
       a.ux = c.p1_ux.as<double>(rows);
-      // A sphere's directions come with its values; a layered sphere's in the group passes.
-      const bool sphere_dirs = any_dirs && L == 1;
-      const int nq = sphere_dirs ? adaptive::kSphereQ : adaptive::kPass1;
       a.deriv = sphere_dirs ? 1 : 0;
       a.q = c.p1_q.as<double>(nq * n);
       a.n_terms = c.p1_n.as<int64_t>(n);
@@ -2147,22 +2199,20 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
       a.n_wl = (int)n_wl;
       a.fractions = fr_d;
       a.m_layers = reinterpret_cast<const double2*>(ml_d);
-      SB_CUDA(cudaMemcpyAsync((void*)a.radius, r.data(), n * 8, cudaMemcpyHostToDevice, s));
-      SB_CUDA(cudaMemcpyAsync((void*)a.wl_index, wi.data(), n * 4, cudaMemcpyHostToDevice, s));
+      SB_CUDA(cudaMemcpyAsync((void*)a.radius, r.data() + k0, n * 8, cudaMemcpyHostToDevice, s));
+      SB_CUDA(cudaMemcpyAsync((void*)a.wl_index, wi.data() + k0, n * 4, cudaMemcpyHostToDevice, s));
       SB_CUDA(cudaMemcpyAsync((void*)a.scratch, off.data(), (n + 1) * 8, cudaMemcpyHostToDevice,
                               s));
       timed_launch(K_NODES, s, [&] { launch_pass1(a, s); });
       SB_CUDA(cudaGetLastError());
-      std::vector<double> q(nq * n);
-      std::vector<int64_t> nt(n);
-      std::vector<int> st(n);
-      SB_CUDA(cudaMemcpyAsync(q.data(), a.q, nq * n * 8, cudaMemcpyDeviceToHost, s));
+      double* q = q_store.data() + k0 * nq;
+      SB_CUDA(cudaMemcpyAsync(q, a.q, nq * n * 8, cudaMemcpyDeviceToHost, s));
       SB_CUDA(cudaMemcpyAsync(nt.data(), a.n_terms, n * 8, cudaMemcpyDeviceToHost, s));
       SB_CUDA(cudaMemcpyAsync(st.data(), a.status, n * 4, cudaMemcpyDeviceToHost, s));
       SB_CUDA(cudaStreamSynchronize(s));
       for (int64_t k = 0; k < n; ++k) {
         adaptive::NodeResult& x = out[k0 + k];
-        for (int j = 0; j < adaptive::kNodeQ; ++j) x.q[j] = j < nq ? q[nq * k + j] : 0.0;
+        x.q = q + nq * k;
         x.n = nt[k];
         x.status = st[k];
         x.dq = layered_dirs ? dq_store.data() + (k0 + k) * dstride : nullptr;
@@ -2295,48 +2345,92 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
   if ((double)n_units * (double)n_nodes > 4e9)
     throw Failure{SCATRS_INVALID_INPUT, "too many (unit, node) pairs for one call"};
   const int ns = deriv ? kNormStrideD : 8;  // unit_norm doubles per unit
-  std::vector<double> radius((size_t)n_units * n_nodes, 0.0), weight(radius.size(), 0.0),
-      wdiff(radius.size(), 0.0), norm((size_t)n_units * ns, 0.0);
-  std::vector<double> wth(deriv ? 3 * radius.size() : 0, 0.0), wthd(wth.size(), 0.0);
+  std::vector<double> norm((size_t)n_units * ns, 0.0);
   std::vector<char> unit_converged(n_units, 1);
   std::vector<int64_t> unit_panels(n_units, 0);
-  // Every unit's nodes and weights on its own (the host's threads; each unit writes its rows).
-#pragma omp parallel for schedule(dynamic, 4)
+  // The units' node tables, on the device: per (unit, panel) a record of what the host's densities
+  // give, written by the host's threads into pinned staging block by block (at most kBlock bytes a
+  // half) and spread over the padded tables by node_table_kernel. (Padded tables cleared, filled
+  // and copied by the host took 34 ms for 1,024 units of up to 174 panels; this takes 3.1 ms.)
+  std::vector<int64_t> first_rec(n_units + 1, 0);
+  for (int64_t u = 0; u < n_units; ++u)
+    first_rec[u + 1] =
+        first_rec[u] + (job_of[u] < 0 ? 1 : (int64_t)jobs[job_of[u]].panels.size());
+  {
+    constexpr int64_t kBlock = int64_t(8) << 20;
+    const int64_t n_rec = first_rec[n_units], rec = node_record(deriv ? n_theta : 0);
+    const int64_t per_block = std::min(n_rec, std::max<int64_t>(1, kBlock / (rec * 8)));
+    const size_t cnt = (size_t)n_units * n_nodes;
+    NodeTableArgs a{};
+    a.n_theta = deriv ? n_theta : 0;
+    a.radius = c.radius.as<double>(cnt);
+    a.weight = c.weight.as<double>(cnt);
+    a.wdiff = c.wdiff.as<double>(cnt);
+    SB_CUDA(cudaMemsetAsync(a.radius, 0, cnt * 8, s));
+    SB_CUDA(cudaMemsetAsync(a.weight, 0, cnt * 8, s));
+    SB_CUDA(cudaMemsetAsync(a.wdiff, 0, cnt * 8, s));
+    if (deriv) {
+      a.wtheta = c.wtheta.as<double>(3 * cnt);
+      a.wthdiff = c.wthdiff.as<double>(3 * cnt);
+      SB_CUDA(cudaMemsetAsync(a.wtheta, 0, cnt * 24, s));
+      SB_CUDA(cudaMemsetAsync(a.wthdiff, 0, cnt * 24, s));
+    }
+    adaptive::Node unit_panel[15];
+    adaptive::gk15(-1.0, 1.0, unit_panel);  // half width 1
+    for (int k = 0; k < 15; ++k) a.wk[k] = unit_panel[k].wk, a.wg[k] = unit_panel[k].wg;
+    double* rec_d = c.node_rec.as<double>(per_block * rec);
+    a.rec = rec_d;
+    c.ensure_staging((size_t)(per_block * rec * 8));
+    int half = 0;
+    for (int64_t r0 = 0; r0 < n_rec; r0 += per_block, half ^= 1) {
+      double* out = reinterpret_cast<double*>(c.staging_half(half));
+      a.n_rec = std::min(per_block, n_rec - r0);
+#pragma omp parallel for schedule(static)
+      for (int64_t i = 0; i < a.n_rec; ++i) {
+        const int64_t u =
+            std::upper_bound(first_rec.begin(), first_rec.end(), r0 + i) - first_rec.begin() - 1;
+        const size_t pi = (size_t)(r0 + i - first_rec[u]);
+        const adaptive::Part& part = parts[u / n_wl];
+        double* o = out + i * rec;
+        int64_t at = u * n_nodes;
+        if (job_of[u] < 0) {
+          std::fill(o, o + rec, 0.0);
+          o[1] = -1.0;
+          o[2] = part.lo;
+        } else {
+          const auto& panel = jobs[job_of[u]].panels[pi];
+          at += slot_of[job_of[u]][pi];
+          o[1] = 0.5 * (panel.second - panel.first);
+          adaptive::Node g[15];
+          adaptive::gk15(panel.first, panel.second, g);
+          for (int k = 0; k < 15; ++k) {
+            const double r = std::exp(g[k].t);
+            double grad[3];
+            o[2 + k] = r;
+            o[17 + k] = (part.grads.empty() ? part.u(r) : part.u(r, grad)) * r;
+            // Each requested parameter's (du/dtheta) r (engine.rs:1637-1644).
+            for (int b = 0; b < a.n_theta; ++b)
+              o[32 + 15 * b + k] =
+                  b < (int)part.grads.size() ? grad[part.grads[b]] * r : 0.0;
+          }
+        }
+        memcpy(o, &at, 8);
+      }
+      SB_CUDA(cudaMemcpyAsync(rec_d, out, (size_t)(a.n_rec * rec * 8), cudaMemcpyHostToDevice, s));
+      c.staging_uploaded(half, s);
+      timed_launch(K_PLAN, s, [&] { launch_node_table(a, s); });
+      SB_CUDA(cudaGetLastError());
+    }
+  }
   for (int64_t u = 0; u < n_units; ++u) {
-    const int64_t p = u / n_wl;
-    const adaptive::Part& part = parts[p];
-    double* nr = &radius[(size_t)u * n_nodes];
-    double* nw = &weight[(size_t)u * n_nodes];
-    double* nd = &wdiff[(size_t)u * n_nodes];
+    const adaptive::Part& part = parts[u / n_wl];
     double* un = &norm[(size_t)u * ns];
     if (part.support == adaptive::POINT) {
-      nr[0] = part.lo;
-      nw[0] = 1.0;
       un[0] = 1.0;
       un[3] = 1.0;
       continue;
     }
     const adaptive::Job& jb = jobs[job_of[u]];
-    for (size_t pi = 0; pi < jb.panels.size(); ++pi) {
-      adaptive::Node g[15];
-      adaptive::gk15(jb.panels[pi].first, jb.panels[pi].second, g);
-      const size_t base = (size_t)slot_of[job_of[u]][pi];
-      for (int k = 0; k < 15; ++k) {
-        const double r = std::exp(g[k].t);
-        double grad[3];
-        const double ur = (part.grads.empty() ? part.u(r) : part.u(r, grad)) * r;
-        nr[base + k] = r;
-        nw[base + k] = g[k].wk * ur;
-        nd[base + k] = g[k].wk * ur - g[k].wg * ur;
-        // Each requested parameter's weights w (du/dtheta) r (engine.rs:1637-1644).
-        for (size_t b = 0; b < part.grads.size(); ++b) {
-          const double dw = grad[part.grads[b]] * r;
-          const size_t at = ((size_t)u * n_nodes + base + k) * 3 + b;
-          wth[at] = g[k].wk * dw;
-          wthd[at] = g[k].wk * dw - g[k].wg * dw;
-        }
-      }
-    }
     un[0] = part.mom.z;
     un[1] = part.mom.ez;
     un[2] = part.support == adaptive::UNBOUNDED ? 0.2 * o.rtol : 0.0;
@@ -2365,15 +2459,10 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
   double* avg = c.avg.as<double>((size_t)n_units * stride);
   AdaptiveInput ad;
   ad.on = true;
-  ad.radius = radius.data();
-  ad.weight = weight.data();
-  ad.wdiff = wdiff.data();
   ad.unit_norm = norm.data();
   ad.avg = avg;
   DerivOutput dvo;
   if (deriv) {
-    ad.wtheta = wth.data();
-    ad.wthdiff = wthd.data();
     dvo.on = true;
     dvo.n_theta = n_theta;
   }
@@ -2399,7 +2488,6 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
     const int n_all = 1 + n_theta + n_dirs_all;
     const int64_t cstride = 2 * (int64_t)n_all * row;
     std::vector<double> hav((size_t)n_units * cstride, 0.0), one((size_t)n_units * stride);
-    call.radius = radius;
     for (size_t pi = 0; pi < passes.size(); ++pi) {
       const int g = passes[pi];
       DerivOutput dvg = dvo;
@@ -2495,7 +2583,6 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
   run_fixed(c, dummy.data(), n_parts, wl_d, n_wl, m_d, mu, n_mu, &fo, nullptr, nullptr, nullptr,
             s, &call, li, dvo, ad);
   if (deriv) {
-    call.radius = std::move(radius);
     check_device_errors(c, s, &call);
     std::vector<double> hav((size_t)n_units * stride), hav_x;
     SB_CUDA(cudaMemcpyAsync(hav.data(), avg, hav.size() * 8, cudaMemcpyDeviceToHost, s));
@@ -2527,7 +2614,6 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
     return;
   }
   if (rows_out) {
-    call.radius = std::move(radius);
     check_device_errors(c, s, &call);
     rows_out->stride = stride;
     rows_out->rows.resize((size_t)n_units * stride);
@@ -2580,19 +2666,14 @@ void adaptive_call_order(const std::vector<AdPart>& in, int n_out, bool batch,
   mx.err = c.err.as<unsigned long long>(3);
   timed_launch(K_FINAL, s, [&] { launch_mix(mx, s); });
   SB_CUDA(cudaGetLastError());
-  call.radius = std::move(radius);
   check_device_errors(c, s, &call);
-  SB_CUDA(cudaMemcpyAsync(res.values, v_d, vl * 8, cudaMemcpyDeviceToHost, s));
-  if (res.errors) SB_CUDA(cudaMemcpyAsync(res.errors, v_d + vl, vl * 8, cudaMemcpyDeviceToHost, s));
-  if (pl > 0 && res.phase)
-    SB_CUDA(cudaMemcpyAsync(res.phase, p_d, pl * 8, cudaMemcpyDeviceToHost, s));
-  if (pl > 0 && res.phase_err)
-    SB_CUDA(cudaMemcpyAsync(res.phase_err, p_d + pl, pl * 8, cudaMemcpyDeviceToHost, s));
-  if (gl > 0 && res.greek)
-    SB_CUDA(cudaMemcpyAsync(res.greek, g_d, gl * 8, cudaMemcpyDeviceToHost, s));
-  if (gl > 0 && res.greek_err)
-    SB_CUDA(cudaMemcpyAsync(res.greek_err, g_d + gl, gl * 8, cudaMemcpyDeviceToHost, s));
-  SB_CUDA(cudaStreamSynchronize(s));
+  std::vector<OutCopy> outs{{res.values, v_d, vl * 8}};
+  if (res.errors) outs.push_back({res.errors, v_d + vl, vl * 8});
+  if (pl > 0 && res.phase) outs.push_back({res.phase, p_d, pl * 8});
+  if (pl > 0 && res.phase_err) outs.push_back({res.phase_err, p_d + pl, pl * 8});
+  if (gl > 0 && res.greek) outs.push_back({res.greek, g_d, gl * 8});
+  if (gl > 0 && res.greek_err) outs.push_back({res.greek_err, g_d + gl, gl * 8});
+  copy_out(c, outs, cudaMemcpyDeviceToHost, s);
   adaptive_flags(in, jobs, job_of, unit_converged, unit_panels, n_out, n_wl, res);
 }
 
@@ -3540,7 +3621,9 @@ void spheroid_call(const std::vector<SphParticle>& ps, bool batch, const double*
     memcpy(&b, &r, 8);
     return std::make_tuple(q, i, b);
   };
+  std::vector<double> q_store;
   auto eval = [&](const std::vector<adaptive::Query>& qs, std::vector<adaptive::NodeResult>& out) {
+    q_store.resize(qs.size() * adaptive::kPass1);
     std::vector<double> xs, es, ms;
     std::vector<size_t> which;
     for (size_t k = 0; k < qs.size(); ++k) {
@@ -3571,7 +3654,9 @@ void spheroid_call(const std::vector<SphParticle>& ps, bool batch, const double*
       adaptive::NodeResult& x = out[k];
       const double q[6] = {1.0, area * v.q_ext, area * v.q_sca, area * v.q_sca * v.g,
                            area * v.q_back, area * v.q_abs};
-      for (int j = 0; j < 6; ++j) x.q[j] = q[j];
+      double* to = q_store.data() + k * adaptive::kPass1;
+      for (int j = 0; j < 6; ++j) to[j] = q[j];
+      x.q = to;
       x.n = v.n;
       x.status = 0;
     }
@@ -3971,8 +4056,10 @@ void spheroid_call_d(const std::vector<SphParticle>& ps, const std::vector<SphDe
   };
   // The pass-1 quantities (quantities1, engine.rs:379-417): the values, then per direction
   // d C_ext, d C_sca, d(C_sca g), d C_back, d C_abs.
+  std::vector<double> q_store;
   auto eval = [&](const std::vector<adaptive::Query>& qs, std::vector<adaptive::NodeResult>& out) {
     solve(qs);
+    q_store.assign(qs.size() * adaptive::kNodeQ, 0.0);
     for (size_t k = 0; k < qs.size(); ++k) {
       const Node& nd = cache.at(key_u(qs[k].wl, qs[k].r));
       const SpheroidResult& v = nd.v;
@@ -3980,11 +4067,12 @@ void spheroid_call_d(const std::vector<SphParticle>& ps, const std::vector<SphDe
       adaptive::NodeResult& x = out[k];
       const double q[6] = {1.0, area * v.q_ext, area * v.q_sca, area * v.q_sca * v.g,
                            area * v.q_back, area * v.q_abs};
-      for (int j = 0; j < adaptive::kNodeQ; ++j) x.q[j] = 0.0;
-      for (int j = 0; j < 6; ++j) x.q[j] = q[j];
+      double* to = q_store.data() + k * adaptive::kNodeQ;
+      for (int j = 0; j < 6; ++j) to[j] = q[j];
+      x.q = to;
       for (int dir = 0; dir < 3 && any_dir; ++dir) {
         const std::vector<double>& dq = nd.d[dir];
-        double* o5 = x.q + adaptive::kPass1 + adaptive::kGroup * dir;
+        double* o5 = to + adaptive::kPass1 + adaptive::kGroup * dir;
         o5[0] = area * dq[0];
         o5[1] = area * dq[1];
         o5[2] = area * (dq[1] * v.g + v.q_sca * dq[4]);
@@ -5329,16 +5417,8 @@ int fixed_host(const scatrs_distribution* dists, int64_t n_dist, const double* w
     call.wl_host.assign(wavelengths, wavelengths + n_wl);
     set_mixed(call, mixed);
     // Pinned outputs are copied slab by slab beside the computation; others at the end.
-    auto pinned = [](const void* p) {
-      cudaPointerAttributes at{};
-      if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-      }
-      return at.type == cudaMemoryTypeHost;
-    };
-    const bool overlap = pinned(values) && (pl == 0 || !phase || pinned(phase)) &&
-                         (gl == 0 || !greek || pinned(greek));
+    const bool overlap = pinned_host(values) && (pl == 0 || !phase || pinned_host(phase)) &&
+                         (gl == 0 || !greek || pinned_host(greek));
     // Waits for the slab copies into the caller's pinned arrays on every exit, the error
     // exits included, so that no copy outlives the call.
     struct CopyWait {
@@ -5363,10 +5443,10 @@ int fixed_host(const scatrs_distribution* dists, int64_t n_dist, const double* w
       return;
     }
     check_device_errors(c, s, &call);
-    SB_CUDA(cudaMemcpyAsync(values, v_d, vl * 8, cudaMemcpyDeviceToHost, s));
-    if (pl > 0 && phase) SB_CUDA(cudaMemcpyAsync(phase, p_d, pl * 8, cudaMemcpyDeviceToHost, s));
-    if (gl > 0 && greek) SB_CUDA(cudaMemcpyAsync(greek, g_d, gl * 8, cudaMemcpyDeviceToHost, s));
-    SB_CUDA(cudaStreamSynchronize(s));
+    std::vector<OutCopy> outs{{values, v_d, vl * 8}};
+    if (pl > 0 && phase) outs.push_back({phase, p_d, pl * 8});
+    if (gl > 0 && greek) outs.push_back({greek, g_d, gl * 8});
+    copy_out(c, outs, cudaMemcpyDeviceToHost, s);
   });
 }
 
@@ -5488,13 +5568,13 @@ void fixed_d_impl(const scatrs_distribution* dists, int64_t n_dist, const double
   run_fixed(c, dists, n_dist, wl_d, n_wl, m_d, mu, n_mu, options, v_d, p_d, g_d, s, &call,
             LayerInput(), dv);
   check_device_errors(c, s, &call);
-  SB_CUDA(cudaMemcpyAsync(values, v_d, vl * 8, out, s));
-  if (d_values) SB_CUDA(cudaMemcpyAsync(d_values, dv.d_values, P * vl * 8, out, s));
-  if (pl > 0 && phase) SB_CUDA(cudaMemcpyAsync(phase, p_d, pl * 8, out, s));
-  if (pl > 0 && d_phase) SB_CUDA(cudaMemcpyAsync(d_phase, dv.d_phase, P * pl * 8, out, s));
-  if (gl > 0 && greek) SB_CUDA(cudaMemcpyAsync(greek, g_d, gl * 8, out, s));
-  if (gl > 0 && d_greek) SB_CUDA(cudaMemcpyAsync(d_greek, dv.d_greek, P * gl * 8, out, s));
-  SB_CUDA(cudaStreamSynchronize(s));
+  std::vector<OutCopy> outs{{values, v_d, vl * 8}};
+  if (d_values) outs.push_back({d_values, dv.d_values, P * vl * 8});
+  if (pl > 0 && phase) outs.push_back({phase, p_d, pl * 8});
+  if (pl > 0 && d_phase) outs.push_back({d_phase, dv.d_phase, P * pl * 8});
+  if (gl > 0 && greek) outs.push_back({greek, g_d, gl * 8});
+  if (gl > 0 && d_greek) outs.push_back({d_greek, dv.d_greek, P * gl * 8});
+  copy_out(c, outs, out, s);
 }
 }  // namespace
 }  // namespace sb
@@ -6439,10 +6519,10 @@ int scatrs_ensemble_fixed_layered(const scatrs_distribution* dists, int64_t n_di
     call.wl_host.assign(wavelengths, wavelengths + n_wl);
     run_fixed(c, dists, n_dist, wl_d, n_wl, m_d, mu, n_mu, options, v_d, p_d, g_d, s, &call, li);
     check_device_errors(c, s, &call);
-    SB_CUDA(cudaMemcpyAsync(values, v_d, vl * 8, cudaMemcpyDeviceToHost, s));
-    if (pl > 0 && phase) SB_CUDA(cudaMemcpyAsync(phase, p_d, pl * 8, cudaMemcpyDeviceToHost, s));
-    if (gl > 0 && greek) SB_CUDA(cudaMemcpyAsync(greek, g_d, gl * 8, cudaMemcpyDeviceToHost, s));
-    SB_CUDA(cudaStreamSynchronize(s));
+    std::vector<OutCopy> outs{{values, v_d, vl * 8}};
+    if (pl > 0 && phase) outs.push_back({phase, p_d, pl * 8});
+    if (gl > 0 && greek) outs.push_back({greek, g_d, gl * 8});
+    copy_out(c, outs, cudaMemcpyDeviceToHost, s);
   });
 }
 
@@ -6509,24 +6589,17 @@ void fixed_layered_d_impl(const scatrs_distribution* dists, int64_t n_dist,
       run_fixed(c, dists, n_dist, wl_d, n_wl, m_d, mu, n_mu, options, v_d, p_d, g_d, s, &call, li,
                 dv);
       check_device_errors(c, s, &call);
+      std::vector<OutCopy> outs;
       auto take = [&](int from, int to) {
-        if (d_values)
-          SB_CUDA(cudaMemcpyAsync(d_values + to * vl, dv.d_values + from * vl, vl * 8,
-                                  out, s));
-        if (pl > 0 && d_phase)
-          SB_CUDA(cudaMemcpyAsync(d_phase + to * pl, dv.d_phase + from * pl, pl * 8,
-                                  out, s));
-        if (gl > 0 && d_greek)
-          SB_CUDA(cudaMemcpyAsync(d_greek + to * gl, dv.d_greek + from * gl, gl * 8,
-                                  out, s));
+        if (d_values) outs.push_back({d_values + to * vl, dv.d_values + from * vl, vl * 8});
+        if (pl > 0 && d_phase) outs.push_back({d_phase + to * pl, dv.d_phase + from * pl, pl * 8});
+        if (gl > 0 && d_greek) outs.push_back({d_greek + to * gl, dv.d_greek + from * gl, gl * 8});
       };
       if (g == 0) {
         for (int p = 0; p < P_th; ++p) take(p, p);
-        SB_CUDA(cudaMemcpyAsync(values, v_d, vl * 8, out, s));
-        if (pl > 0 && phase)
-          SB_CUDA(cudaMemcpyAsync(phase, p_d, pl * 8, out, s));
-        if (gl > 0 && greek)
-          SB_CUDA(cudaMemcpyAsync(greek, g_d, gl * 8, out, s));
+        outs.push_back({values, v_d, vl * 8});
+        if (pl > 0 && phase) outs.push_back({phase, p_d, pl * 8});
+        if (gl > 0 && greek) outs.push_back({greek, g_d, gl * 8});
       }
       if (g < L) {
         take(P_th, P_th + 2 * g);
@@ -6534,6 +6607,7 @@ void fixed_layered_d_impl(const scatrs_distribution* dists, int64_t n_dist,
       } else {
         take(P_th, P_th + 2 * L + (g - L));
       }
+      copy_out(c, outs, out, s);
       SB_CUDA(cudaStreamSynchronize(s));
     }
   }
@@ -6794,7 +6868,7 @@ void scatrs_release(void) {
                       &c.X, &c.uz, &c.ux, &c.chunk_sums, &c.err, &c.acc,
                       &c.counter, &c.values, &c.phase, &c.greek, &c.user.g,
                       &c.user.map, &c.user.rows_d, &c.tc_a_hi, &c.tc_a_lo, &c.tc_prod, &c.tc_err, &c.xdig,
-                      &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.side, &c.split, &c.split_rows,
+                      &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.side, &c.split, &c.split_rows, &c.node_rec,
                       &c.i8.dig, &c.i8.scale, &c.i8.user_d, &c.i8.band_d, &c.ro_cgr, &c.ro_cgw})
       b->release();
     for (auto& kv : c.projectors)

@@ -17,6 +17,23 @@ struct PlanArgs {
   int per_unit;  // nodes per unit ([n_units][n_nodes]) rather than per distribution
 };
 
+// Adaptive panels: each record's 15 nodes and weights to its half chunk of 16 nodes (the 16th
+// stays 0). A record: the half chunk's first node (an int64's bits), the panel's half width h (< 0:
+// a single radius, weight 1), the radii r[15], u r at them [15], then per parameter (du/dtheta) r
+// [15]. Kronrod weights h wk, Gauss weights h wg.
+struct NodeTableArgs {
+  const double* rec;
+  int64_t n_rec;
+  int n_theta;
+  double* radius;
+  double* weight;   // h wk u r
+  double* wdiff;    // h wk u r - h wg u r
+  double* wtheta;   // [node][3], with n_theta > 0
+  double* wthdiff;
+  double wk[15], wg[15];
+};
+constexpr int node_record(int n_theta) { return 32 + 15 * n_theta; }
+
 // A chunk that K-a gives a block of its own, and its first scratch row.
 struct MieSplit {
   int chunk, n;  // n: its orders
@@ -474,6 +491,7 @@ struct Pass1Args {
 
 void launch_pass1_layered_deriv(const Pass1Args& a, cudaStream_t s);
 void launch_plan_chunks(const PlanArgs& a, cudaStream_t s);
+void launch_node_table(const NodeTableArgs& a, cudaStream_t s);
 void launch_mie_fixed(const MieFixedArgs& a, cudaStream_t s);
 void launch_mie_split(const MieFixedArgs& a, cudaStream_t s);
 void launch_mie_nodes(const MieNodesArgs& a, cudaStream_t s);
