@@ -2996,7 +2996,7 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
     std::map<int64_t, int64_t> rule_at;
     std::vector<double> rules;
     int64_t nodes = 0, rad = 0, ang_nodes = 0, ang = 0, pairs = 0, J = 0, W = 0, T = 0;
-    int64_t ser = 0, ser_threads = 0, forms_threads = 0;
+    int64_t ser = 0, ser_threads = 0, n_forms = 0;
     double bytes = 0.0;
     size_t j1 = j0;
     for (; j1 < specs.size(); ++j1) {
@@ -3040,12 +3040,12 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
         g.rad0 = rad;
         g.ser0 = ser;
         g.sth0 = ser_threads;
-        g.fth0 = forms_threads;
+        g.fth0 = n_forms;
         nodes += nq;
         rad += (int64_t)nq * (t.N + 1) * 20;
         ser += (int64_t)t.n_theta * (t.N + 1) * tm_series_slot(t.N);
         ser_threads += (int64_t)t.n_theta * t.N;
-        forms_threads += (int64_t)t.n_theta * t.N * t.N;
+        n_forms += (int64_t)4 * t.n_theta * forms_threads(t.N);
         geoms.push_back(g);
       }
       TmJob jb{};
@@ -3081,7 +3081,7 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
     a.ang = c.tm_ang.as<double>((size_t)ang);
     a.ser = c.tm_ser.as<double>((size_t)ser);
     a.n_ser_total = ser_threads;
-    a.n_forms_total = forms_threads;
+    a.n_forms_total = n_forms;
     a.form = tm_form_override();
     a.J = c.tm_J.as<double>(4 * (size_t)J);
     a.work = c.tm_work.as<double>((size_t)W);

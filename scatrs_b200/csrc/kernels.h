@@ -501,6 +501,14 @@ void launch_proj(const ProjArgs& a, cudaStream_t s);
 void launch_final(const FinalArgs& a, cudaStream_t s);
 void launch_pass1(const Pass1Args& a, cudaStream_t s);
 
+// The forms kernel's threads per (node, product): the pairs n > k in bands of kFormsBand diagonals
+// (N - 1, N - 1 - kFormsBand, ... columns, the rows above N idle) and the pairs n < k.
+constexpr int kFormsBand = 4;
+constexpr int forms_threads(int N) {
+  const int b = (N - 1 + kFormsBand - 1) / kFormsBand;
+  return kFormsBand * (b * (N - 1) - kFormsBand * (b * (b - 1) / 2)) + N * (N - 1) / 2;
+}
+
 // The Greek projection of tables at Gauss cosines (greek_tc.cu): the 3xTF32 tensor-core GEMM's
 // arguments (products [6][n_units][len] in FP32, an error word for its bounded waits).
 struct TcArgs {

@@ -428,6 +428,7 @@ __device__ __forceinline__ void reg_forms(const YTab& yt, int Ly, const JSlot& s
   l_end[0] = min(min(i0 + 1, Ly), G - 1);
   l_end[1] = min(min(max(i0, 0), Ly), G - 1);
   double neg_abs[2] = {0.0, 0.0}, pos_abs[2] = {0.0, 0.0};
+#pragma unroll 4
   for (int l = 0; l < l_end[0]; ++l) {
     const double ya = fabs(yt.hi(l, n) * xe.hi);
 #pragma unroll
@@ -469,81 +470,85 @@ __device__ __forceinline__ void reg_forms(const YTab& yt, int Ly, const JSlot& s
   }
 }
 
-// The series' view at one node for a row order n and a column order k.
-struct SerView {
-  YTab yt[3];  // y-table of the node per kind
-  JSlot sk;    // j-slot of (node, k)
-  int Ly, Lj;
-};
-
 // The radial products of an (n, k) pair's nonzero elements, by the parity of n + k, as (y kind,
 // j kind, e): even (MN, NM): R_1, R_4, R_6, R_2; odd (MM, NN): R_0, R_3, R_5, R_7.
 __device__ __forceinline__ void product_kind(bool even, int ts, int* yk, int* jk, int* e) {
-  constexpr int kEven[4][3] = {{0, 1, 2}, {0, 2, 4}, {2, 0, 4}, {1, 0, 2}};
-  constexpr int kOdd[4][3] = {{0, 0, 2}, {1, 1, 2}, {1, 2, 4}, {2, 1, 4}};
-  const int* v = even ? kEven[ts] : kOdd[ts];
-  *yk = v[0];
-  *jk = v[1];
-  *e = v[2];
+  *yk = (even ? 0x60 : 0x94) >> (2 * ts) & 3;
+  *jk = (even ? 0x09 : 0x64) >> (2 * ts) & 3;
+  *e = *yk == 2 || *jk == 2 ? 4 : 2;
 }
 
 }  // namespace
 
 // The regularized forms of the radial products of the y-part, which do not depend on the
-// azimuthal mode: one thread per (spheroid, node of the half surface, column order k, row order
-// n != k), rows fastest (the reference computes them once per node before its mode loop,
-// kernel.rs:327-342). Per product of the pair's nonzero elements the forms without the powers
-// <= 0 and (|n - k| >= 3) without those < 0, with their magnitude sums, into the forms table.
+// azimuthal mode: one thread per (spheroid, node of the half surface, product of the pair's nonzero
+// elements, row order n != column order k) (the reference computes them once per node before its
+// mode loop, kernel.rs:327-342): the form without the powers <= 0 and (|n - k| >= 3) the one
+// without those < 0, with their magnitude sums, into the forms table.
+//
+// Bound by the latency of the sums' loads (a third of the issue slots). The sums run over
+// (n - k) / 2 terms, none below the diagonal: with a column's rows side by side and a thread's four
+// products one after the other, a warp waited for its longest row with a third of its lanes at work
+// and 2.6 warps a scheduler. By bands of diagonals the lanes of a warp run alike, and 4 rows of a
+// column keep loads and stores in whole sectors (bands of 1, 2, 4, 8, 16: 80.4, 80.3, 78.6, 84.0,
+// 95.3 ms); a product per thread halves the registers; four of the magnitudes' terms are loaded at
+// once (78.6 -> 72.5). In all 134 -> 72.5 ms per pass of 288 spheroids to x = 21.
 __global__ void __launch_bounds__(128) tm_forms_kernel(TmArgs a) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n_forms_total) return;
   const int gi = owner(a.n_geoms, t, [&](int i) { return a.geoms[i].fth0; });
   const TmGeom g = a.geoms[gi];
   const int N = g.N, G = N / 2 + 2, nh = g.n_theta;
-  const int64_t local = t - g.fth0, NN = (int64_t)N * N;
-  const int h = (int)(local / NN), rem = (int)(local % NN);
-  const int k = 1 + rem / N, n = 1 + rem % N;
-  if (n == k) return;
+  // Node, product and pair: the pairs n > k by bands of kFormsBand diagonals, a column's rows of the
+  // band side by side; then those with n < k, column by column.
+  const int64_t local = t - g.fth0;
+  const int per = forms_threads(N), upper = per - N * (N - 1) / 2;
+  const int hs = (int)(local / per), h = hs >> 2, ts = hs & 3;
+  int p = (int)(local % per), n, k;
+  if (p < upper) {
+    int band = 0, len = kFormsBand * (N - 1);
+    for (; p >= len; len -= kFormsBand * kFormsBand, ++band) p -= len;
+    k = 1 + p / kFormsBand;
+    n = k + kFormsBand * band + 1 + p % kFormsBand;
+    if (n > N) return;
+  } else {
+    p -= upper;
+    int line = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
+    while (line * (line + 1) / 2 > p) --line;
+    while ((line + 1) * (line + 2) / 2 <= p) ++line;
+    k = line + 2;
+    n = 1 + p - line * (line + 1) / 2;
+  }
   const int q = nh + h;
   const double* ser = a.ser + g.ser0;
   const int64_t JS = j_slot_size(G);
-  SerView sv;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) sv.yt[c] = YTab{y_table(ser, nh, N, G, h, c), N + 1};
-  sv.sk = JSlot{ser + ((int64_t)h * (N + 1) + k) * JS, G};
-  sv.Ly = (int)ser[(int64_t)n * JS];
-  sv.Lj = (int)ser[(int64_t)k * JS + 1];
+  const JSlot sk{ser + ((int64_t)h * (N + 1) + k) * JS, G};
+  const int Ly = (int)ser[(int64_t)n * JS], Lj = (int)ser[(int64_t)k * JS + 1];
   const double* ns = a.node + (g.node0 + q) * kNodeD;
-  const dd r = ld(ns), ir = ld(ns + 2), r2 = r * r, r4 = r2 * r2;
   const double* ri = a.rad + g.rad0 + ((int64_t)q * (N + 1) + n) * kRadD;
   const double* rk = a.rad + g.rad0 + ((int64_t)q * (N + 1) + k) * kRadD;
-  const dd yr = ld(ri + 4), ydr = ld(ri + 6), yo = yr * ir;
-  const cdd w = ldc(rk + 8), wd = ldc(rk + 12), u = ldc(rk + 16);
-  const bool even = ((n + k) & 1) == 0;
   const int n1 = N + 1;
+  int yk, jk, e;
+  product_kind(((n + k) & 1) == 0, ts, &yk, &jk, &e);
+  const dd r = ld(ns), r2 = r * r, xe = e == 2 ? r2 : r2 * r2;
+  dd yv = ld(ri + (yk == 1 ? 6 : 4));
+  if (yk == 2) yv = yv * ld(ns + 2);
+  const cdd full = ldc(rk + 8 + 4 * jk) * (yv * xe);
+  double* fs = forms_slot(ser, nh, N, G, h, k, ts) + n;
+  const bool below = abs(n - k) >= 3;
+  const YTab yt{y_table(ser, nh, N, G, h, yk), N + 1};
+  cdd v[2];
+  double va[2];
+  reg_forms(yt, Ly, sk, Lj, yk, jk, e, n, k, below, xe, full, v, va);
 #pragma unroll
-  for (int ts = 0; ts < 4; ++ts) {
-    int yk, jk, e;
-    product_kind(even, ts, &yk, &jk, &e);
-    const dd yv = yk == 0 ? yr : (yk == 1 ? ydr : yo);
-    const cdd jv = jk == 0 ? w : (jk == 1 ? wd : u);
-    const dd xe = e == 2 ? r2 : r4;
-    const cdd full = jv * (yv * xe);
-    double* fs = forms_slot(ser, nh, N, G, h, k, ts) + n;
-    const bool below = abs(n - k) >= 3;
-    cdd v[2];
-    double va[2];
-    reg_forms(sv.yt[yk], sv.Ly, sv.sk, sv.Lj, yk, jk, e, n, k, below, xe, full, v, va);
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      if (c == 1 && !below) continue;
-      double* f = fs + (int64_t)5 * c * n1;
-      f[0] = v[c].re.hi;
-      f[n1] = v[c].re.lo;
-      f[2 * n1] = v[c].im.hi;
-      f[3 * n1] = v[c].im.lo;
-      f[4 * n1] = va[c];
-    }
+  for (int c = 0; c < 2; ++c) {
+    if (c == 1 && !below) continue;
+    double* f = fs + (int64_t)5 * c * n1;
+    f[0] = v[c].re.hi;
+    f[n1] = v[c].re.lo;
+    f[2 * n1] = v[c].im.hi;
+    f[3 * n1] = v[c].im.lo;
+    f[4 * n1] = va[c];
   }
 }
 
