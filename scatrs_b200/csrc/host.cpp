@@ -3060,7 +3060,7 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       jb.T0 = T;
       ang_nodes += nq;
       ang += (int64_t)nq * (t.N + 1) * 6;
-      pairs += (int64_t)K * K;
+      pairs += (int64_t)2 * ((K + 1) / 2) * K;
       J += 8 * (int64_t)K * K;
       W += 28 * (int64_t)K * K;
       T += (int64_t)n2 * n2;

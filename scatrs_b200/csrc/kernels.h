@@ -556,7 +556,7 @@ struct TmJob {
   int geom, m, K, pad;
   int64_t ang_node0;  // first (job, node) index of the angular table
   int64_t ang0;       // angular table [node][order 0..N][6]
-  int64_t pair0;      // first (i, k) pair
+  int64_t pair0;      // first (i, k) pair: 2 ceil(K / 2) K threads, some of odd K idle
   int64_t J0;         // surface integrals: 8 K^2 complex double-doubles (4 doubles each)
   int64_t W0;         // workspace: 28 K^2 doubles
   int64_t T0;         // T: (2K)^2 complex doubles (2 each), if kept

@@ -576,7 +576,9 @@ __global__ void __launch_bounds__(128) tm_forms_kernel(TmArgs a) {
 //
 // One form instead of three (and no state for the others) halves the
 // operations and leaves the reads of the forms table (3 TB/s) as its bound: 196 -> 128 ms per pass
-// of 288 spheroids to x = 21 (3 blocks per SM without spills: the same).
+// of 288 spheroids to x = 21 (3 blocks per SM without spills: the same). Rows of both parities of
+// i + k in a warp ran the two parities' code one after the other; one parity at a time: 128 -> 98 ms
+// (the table's rows ordered by parity too: no faster, and its writer slower).
 namespace {
 
 // One (mode, i, k): its rows of the tables and the half surface's sums.
@@ -729,9 +731,12 @@ __global__ void __launch_bounds__(128, 4) tm_surface_kernel(TmArgs a) {
   const TmJob jb = a.jobs[ji];
   const TmGeom g = a.geoms[jb.geom];
   const int N = g.N, m = jb.m, n0 = m > 1 ? m : 1, K = jb.K;
-  // Rows fastest: a warp's threads share the column order k and read the forms table's
-  // consecutive orders.
-  const int pr = (int)(t - jb.pair0), i = n0 + pr % K, k = n0 + pr / K;
+  // The pairs of even i + k, then those of odd, rows fastest: a warp's threads run one parity's
+  // code, mostly share the column order k and read the forms table's consecutive rows.
+  const int half = (K + 1) >> 1, pr = (int)(t - jb.pair0), cls = pr >= half * K;
+  const int col = pr / half - cls * K, row = 2 * (pr % half) + ((col + cls) & 1);
+  if (row >= K) return;
+  const int i = n0 + row, k = n0 + col;
   const int G = N / 2 + 2, nh = g.n_theta;
   SurfacePair P;
   P.node = a.node + (g.node0 + nh) * kNodeD;
