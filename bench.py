@@ -325,8 +325,41 @@ class Clocks:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
+def _bucket(n):
+    """The projector band (orders 1, 2, 3, 4, 5, 7, ...) of each n."""
+    u = np.ones_like(n)
+    while np.any(u < n):
+        u = np.where(u < n, np.ceil(u * 1.25), u)
+    return u
+
+
+def _band_rows(u, order: int):
+    """The table rows of a projector band of u orders: half its Gauss nodes."""
+    nq = u + np.floor((np.minimum(order, 2 * u) + 2) / 2)
+    return nq - np.floor(nq / 2)
+
+
+def level_tiles(user_rows: int, order: int):
+    """The tiles (32 table rows) of the phase levels in use: a level of t tiles serves the chunks
+    of at most 32 t - 1 orders while it is cheaper than the requested cosines' tiles and the
+    projector band's (level_limit)."""
+    out, t, size = [], 1, 0.0
+    while user_rows > 0 and len(out) < 48:
+        upper = 32 * t - 1
+        direct = -(-user_rows // 32)
+        if order >= 0:
+            direct += -(-int(_band_rows(_bucket(np.array([float(upper)])), order)[0]) // 32)
+        size += 16.0 * 32 * t * (-(-user_rows // 32) * 32)
+        if not t + user_rows / 512 < direct or size > 1 << 30:
+            break
+        out.append(t)
+        t += 1 if t < 8 else t // 8
+    return out
+
+
 def chunk_shape(w, user_rows: int):
-    """Per wavelength: each node's N, each chunk's N_c and its band's table rows h_b."""
+    """Per wavelength: each node's N, each chunk's N_c and the table rows it runs: its phase
+    level's, or the requested cosines' and its band's beyond the levels."""
     from scatrs_b200 import _native
 
     r = np.empty((w.dists.size, w.n_nodes))
@@ -337,31 +370,29 @@ def chunk_shape(w, user_rows: int):
     L = w.greek_order
     cpu = (w.n_nodes + 31) // 32
     pad = cpu * 32 - w.n_nodes
+    levels = level_tiles(user_rows, L)
     for lam in w.wavelengths:
         x = 2.0 * np.pi * r / lam
         n = np.ceil(x + 6.0 * np.cbrt(x) + 3.0)
         npad = np.pad(n, ((0, 0), (0, pad)))
         nc = npad.reshape(w.dists.size, cpu, 32).max(axis=2)
-        hb = np.zeros_like(nc)
+        rows = np.full_like(nc, float(user_rows))
         if L >= 0:
-            u = np.ones_like(nc)
-            while np.any(u < nc):
-                u = np.where(u < nc, np.ceil(u * 1.25), u)
-            order = np.minimum(L, 2 * u)
-            nq = u + np.floor((order + 2) / 2)
-            hb = nq - np.floor(nq / 2)
-        yield n, nc, hb
+            rows += _band_rows(_bucket(nc), L)
+        for t in reversed(levels):
+            rows = np.where(nc <= 32 * t - 1, 32.0 * t, rows)
+        yield n, nc, rows
 
 
 def algorithmic_i8_ops(w, user_rows: int, above: int, levels: int = 5):
     """The mixed form's int8 work per step: per chunk with above < N_c <= 4096, the digit
-    products (15 for 5 levels, 19 for 6) of its two GEMMs [2 (h_u + h_b) rows x N_c orders] x
-    [N_c x 128 columns], 2 ops per multiply-add, at the real (unpadded) sizes."""
+    products (15 for 5 levels, 19 for 6) of its two GEMMs [2 h rows x N_c orders] x
+    [N_c x 128 columns], h the chunk's table rows (chunk_shape), 2 ops per multiply-add, at the real (unpadded) sizes."""
     prods = 19 if levels == 6 else 15
     total = 0.0
-    for _, nc, hb in chunk_shape(w, user_rows):
+    for _, nc, rows in chunk_shape(w, user_rows):
         sel = (nc > above) & (nc <= 4096)
-        total += float(np.sum(np.where(sel, prods * 2.0 * 2 * (user_rows + hb) * 128 * nc,
+        total += float(np.sum(np.where(sel, prods * 2.0 * 2 * rows * 128 * nc,
                                        0.0)))
     return total
 
@@ -389,44 +420,15 @@ def int8_peak_tops(torch):
 
 
 def algorithmic_flops(w, user_rows: int, at_most: int | None = None):
-    """FP64 flops of K-b per step: 16 N_j (h_u + h_b) for node j (2 GEMMs x 4 real columns x 2
-    flops per order and table row; h_u the requested cosines' table rows, h_b the rows of the
-    band of the node's chunk) -- the per-node figure of the angle sums. at_most: only the nodes
-    of chunks with N_c <= at_most (or above 4096), those the mixed form leaves in FP64."""
-    if at_most is not None:
-        total = 0.0
-        for n, nc, hb in chunk_shape(w, user_rows):
-            keep = (nc <= at_most) | (nc > 4096)
-            nrow = np.repeat(np.where(keep, 1.0, 0.0), 32, axis=1)[:, : w.n_nodes]
-            hrow = np.repeat(hb, 32, axis=1)[:, : w.n_nodes]
-            total += float(np.sum(nrow * 16.0 * n * (user_rows + hrow)))
-        return total
-    r = np.empty((w.dists.size, w.n_nodes))
-    from scatrs_b200 import _native
-
-    xi, om = _native.gauss_legendre(w.n_nodes)
-    for d in range(w.dists.size):
-        a, b = np.log(w.dists["r_lo"][d]), np.log(w.dists["r_hi"][d])
-        r[d] = np.exp(0.5 * (a + b) + 0.5 * (b - a) * xi)
+    """FP64 flops of K-b per step: 16 N_j h for node j (2 GEMMs x 4 real columns x 2 flops per
+    order and table row; h the table rows of the node's chunk) -- the per-node figure of the angle
+    sums. at_most: only the nodes of chunks with N_c <= at_most (or above 4096), those the mixed
+    form leaves in FP64."""
     total = 0.0
-    L = w.greek_order
-    cpu = (w.n_nodes + 31) // 32
-    pad = cpu * 32 - w.n_nodes
-    for i, lam in enumerate(w.wavelengths):
-        x = 2.0 * np.pi * r / lam
-        n = np.ceil(x + 6.0 * np.cbrt(x) + 3.0)
-        npad = np.pad(n, ((0, 0), (0, pad)))
-        nc = npad.reshape(w.dists.size, cpu, 32).max(axis=2)
-        hb = np.zeros_like(nc)
-        if L >= 0:
-            u = np.ones_like(nc)
-            while np.any(u < nc):
-                u = np.where(u < nc, np.ceil(u * 1.25), u)
-            order = np.minimum(L, 2 * u)
-            nq = u + np.floor((order + 2) / 2)
-            hb = nq - np.floor(nq / 2)
-        hrow = np.repeat(hb, 32, axis=1)[:, : w.n_nodes]
-        total += float(np.sum(16.0 * n * (user_rows + hrow)))
+    for n, nc, rows in chunk_shape(w, user_rows):
+        if at_most is not None:
+            rows = np.where((nc <= at_most) | (nc > 4096), rows, 0.0)
+        total += float(np.sum(16.0 * n * np.repeat(rows, 32, axis=1)[:, : w.n_nodes]))
     return total
 
 

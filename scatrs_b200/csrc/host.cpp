@@ -1,12 +1,15 @@
 // The C ABI of include/scatrs_b200.h: input checks, the cached tables, slab planning and the
-// launches of K-a (mie_kernels.cu) and K-b/c/d (unit_kernel.cu).
+// launches of K-a (mie_kernels.cu), K-b/c (unit_kernel.cu) and K-d (phase_levels.cu, unit_kernel.cu).
 //
 // A call of the fixed-grid ensemble runs, per device and in one stream:
 //   1. the node table (radii and weights w_j u(r_j) r_j per distribution) on the host;
 //   2. plan_chunks: each chunk's largest number of terms N_c, copied back to the host, which
-//      picks the projector bands, grows the tables if needed, and cuts the units into slabs
-//      whose coefficient rows fit the arena;
-//   3. per slab, K-a (one warp per chunk) then the unit kernel (one persistent CTA per SM slot).
+//      picks the phase levels and projector bands, grows the tables if needed, and cuts the
+//      units into slabs whose coefficient rows fit the arena;
+//   3. per slab, K-a (one warp per chunk; a block where the chunks are few), the unit kernel (one
+//      persistent CTA per SM slot), the slots' interpolation and projection (phase_levels.cu), and
+//      the final kernel.
+// An adaptive call refines its panels first (adaptive.cpp) and fills the node tables on the device.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
