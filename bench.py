@@ -33,9 +33,9 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# DRAM bytes per node of the unit kernel: (805.47 MB read + 27.56 MB written) / 313,344 nodes in
+# DRAM bytes per node of the unit kernel: (874.36 MB read + 40.12 MB written) / 313,344 nodes in
 # one ncu capture of the 0.1-scale batched workload (the traffic grows with the nodes).
-UNIT_DRAM_BYTES_PER_NODE = (720.229632e6 + 27.529984e6) / 313344
+UNIT_DRAM_BYTES_PER_NODE = (874.359552e6 + 40.118272e6) / 313344
 
 METRIC = "Mie ensemble nodes/s on 1 B200, batched vs plain FP64, at 1e-10 rel err vs FP64"
 UNIT = "nodes/s"
