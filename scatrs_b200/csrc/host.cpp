@@ -143,10 +143,14 @@ int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 std::atomic<int64_t> g_fail_allocation{0};
 std::atomic<unsigned long long> g_forced_node_error{~0ull};
 
-// A grow-only device buffer.
+// A grow-only device buffer, freed with its owner (on the device that is then current).
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  ~DevBuf() { release(); }
   void* get(size_t bytes) {
     if (bytes > cap) {
       // Regrown with room to spare (half, at most 64 MiB), so that calls of slightly varying
@@ -199,10 +203,6 @@ struct BandTables {
   std::vector<double> mu;         // the cosines me_d and mo_d interpolate onto
   DevBuf g_d, lg_d, d_d, desc_d, half0_d, x0_d, node_d, me_d, mo_d;
   int merge_max() const { return n_levels > 0 ? desc[n_levels - 1].upper : 0; }
-  void release() {
-    for (DevBuf* b : {&g_d, &lg_d, &d_d, &desc_d, &half0_d, &x0_d, &node_d, &me_d, &mo_d})
-      b->release();
-  }
 };
 
 struct Context {
@@ -288,10 +288,22 @@ struct Context {
     SB_CUDA(cudaEventRecord(staged[h], s));
     staged_pending[h] = true;
   }
+  ~Context() {
+    for (int h = 0; h < 2; ++h)
+      if (staged[h]) {
+        cudaEventSynchronize(staged[h]);
+        cudaEventDestroy(staged[h]);
+      }
+    if (copies) cudaStreamDestroy(copies);
+    if (slab_done) cudaEventDestroy(slab_done);
+    if (staging) cudaFreeHost(staging);
+    if (pinned_chunk_n) cudaFreeHost(pinned_chunk_n);
+  }
 };
 
 std::mutex g_ctx_mtx;
-std::vector<std::unique_ptr<Context>> g_ctx;
+// Never destroyed: at process exit the runtime may be gone before a static's destructor runs.
+std::vector<std::unique_ptr<Context>>& g_ctx = *new std::vector<std::unique_ptr<Context>>;
 
 Context& context() {
   int dev = 0;
@@ -434,12 +446,10 @@ BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream
     for (auto& kv : c.bands) sets += kv.first.second > 0;
     if (sets >= kMaxLevelSets)
       for (auto it = c.bands.begin(); it != c.bands.end();) {
-        if (it->first.second > 0) {
-          it->second.release();
+        if (it->first.second > 0)
           it = c.bands.erase(it);
-        } else {
+        else
           ++it;
-        }
       }
   }
   BandTables& bt = c.bands[{L, limit}];
@@ -6676,12 +6686,6 @@ int scatrs_mie(const double* x, const double* m, int64_t n, int32_t allow_unvali
     std::lock_guard<std::mutex> lk(c.mtx);
     cudaStream_t s = 0;
     DevBuf xb, mb, nb, ob, cb, eb, uzb, uxb;
-    struct Free {
-      DevBuf* b[8];
-      ~Free() {
-        for (auto* p : b) p->release();
-      }
-    } guard{{&xb, &mb, &nb, &ob, &cb, &eb, &uzb, &uxb}};
     double* xd = xb.as<double>(n);
     double2* md = mb.as<double2>(n);
     int64_t* nd = nb.as<int64_t>(n);
@@ -6863,29 +6867,7 @@ void scatrs_release(void) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
   std::lock_guard<std::mutex> lk(g_ctx_mtx);
-  if (dev < (int)g_ctx.size() && g_ctx[dev]) {
-    Context& c = *g_ctx[dev];
-    for (DevBuf* b : {&c.radius, &c.weight, &c.wtheta, &c.wthdiff, &c.wdiff, &c.unit_norm, &c.wl, &c.m, &c.fractions, &c.chunk_n, &c.chunk_n_slab,
-                      &c.chunk_row, &c.chunk_acc, &c.plan_units, &c.unit_acc, &c.unit_slots,
-                      &c.slots, &c.items, &c.proj_items, &c.slot_index, &c.slot_greek, &c.slot_phase,
-                      &c.X, &c.uz, &c.ux, &c.chunk_sums, &c.err, &c.acc,
-                      &c.counter, &c.values, &c.phase, &c.greek, &c.user.g,
-                      &c.user.map, &c.user.rows_d, &c.tc_a_hi, &c.tc_a_lo, &c.tc_prod, &c.tc_err, &c.xdig,
-                      &c.xside, &c.colmax, &c.chunk_xoff, &c.chunk_xidx, &c.i8_list, &c.side, &c.split, &c.split_rows, &c.node_rec,
-                      &c.i8.dig, &c.i8.scale, &c.i8.user_d, &c.i8.band_d, &c.ro_cgr, &c.ro_cgw})
-      b->release();
-    for (auto& kv : c.projectors)
-      for (DevBuf* b : {&kv.second.d, &kv.second.d_hi, &kv.second.d_lo}) b->release();
-    for (auto& kv : c.bands) kv.second.release();
-    if (c.pinned_chunk_n) cudaFreeHost(c.pinned_chunk_n);
-    for (int h = 0; h < 2; ++h)
-      if (c.staged[h]) {
-        cudaEventSynchronize(c.staged[h]);
-        cudaEventDestroy(c.staged[h]);
-      }
-    if (c.staging) cudaFreeHost(c.staging);
-    g_ctx[dev].reset();
-  }
+  if (dev < (int)g_ctx.size()) g_ctx[dev].reset();
 }
 
 }  // extern "C"

@@ -1,0 +1,48 @@
+"""Device memory the library holds: given back by scatrs_release, and sized by the call."""
+
+import numpy as np
+import pytest
+
+from scatrs_b200 import _scatrs
+from scatrs_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+def _free():
+    import torch
+
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _used(lib, call):
+    """What a call leaves on the device, from a released library to the next release."""
+    lib.scatrs_release()
+    before = _free()
+    call()
+    return before - _free()
+
+
+def test_release_gives_every_buffer_back(gpu):
+    lib = gpu.load()
+    mu, wl = W.gauss_legendre(32), np.array([0.5, 0.8])
+    m = np.full(2, 1.5 + 1e-2j)
+
+    def calls():
+        d = W.lognormals([0.3], [1.5], 3)
+        gpu.ensemble_fixed(d, wl, m[None], mu, 64, 16)
+        _scatrs.ensemble_compute([(("lognormal", 0.2, 1.5), ("sphere", m), 1.0)], wl, False, 16,
+                                 False, mu, True, [], 1e-6, 4096, False, False)
+        gpu.spheroid_compute(np.full(4, 12.0), 2.0, 1.5 + 1e-2j, n_terms=24, n_theta=60)
+
+    calls()  # the modules are loaded with their first launches
+    lib.scatrs_release()
+    before = _free()
+    calls()
+    held = before - _free()
+    lib.scatrs_release()
+    assert held > 64 * MIB
+    assert before - _free() <= 4 * MIB
