@@ -225,7 +225,7 @@ struct Context {
   struct Projector {
     DevBuf d, d_hi, d_lo;
   };
-  std::map<std::pair<int64_t, int>, Projector> projectors;
+  std::map<std::pair<int64_t, int>, std::unique_ptr<Projector>> projectors;
   DevBuf tc_a_hi, tc_a_lo, tc_prod, tc_err;
   // The mixed form: digit tables (I8Tables) and the slabs' chunk digits.
   struct I8Tables {
@@ -2893,8 +2893,7 @@ CUtensorMap tensor_map_2d(float* base, int64_t n_q_pad, int64_t rows, int box_ro
 Context::Projector& projector(Context& c, int64_t n_q, int L, cudaStream_t s) {
   auto key = std::make_pair(n_q, L);
   auto it = c.projectors.find(key);
-  if (it != c.projectors.end()) return it->second;
-  Context::Projector& p = c.projectors[key];
+  if (it != c.projectors.end()) return *it->second;
   const auto& r = rule(c, n_q);
   const int64_t len = L + 1;
   std::vector<double> d(4 * (size_t)n_q * len), buf(len);
@@ -2905,15 +2904,17 @@ Context::Projector& projector(Context& c, int64_t n_q, int L, cudaStream_t s) {
       for (int64_t l = 0; l < len; ++l)
         d[((size_t)f * n_q + k) * len + l] = (double)(2 * l + 1) * 0.5 * r.second[k] * buf[l];
     }
-  double* dd = p.d.as<double>(d.size());
+  // Kept only once it is whole: a call that fails here leaves no entry.
+  auto p = std::make_unique<Context::Projector>();
+  double* dd = p->d.as<double>(d.size());
   SB_CUDA(cudaMemcpyAsync(dd, d.data(), d.size() * 8, cudaMemcpyHostToDevice, s));
   const int64_t n_q_pad = round_up(n_q, 4);
-  float* hi = p.d_hi.as<float>(4 * (size_t)len * n_q_pad);
-  float* lo = p.d_lo.as<float>(4 * (size_t)len * n_q_pad);
+  float* hi = p->d_hi.as<float>(4 * (size_t)len * n_q_pad);
+  float* lo = p->d_lo.as<float>(4 * (size_t)len * n_q_pad);
   launch_greek_split_d(dd, (int)n_q, (int)n_q_pad, (int)len, hi, lo, s);
   SB_CUDA(cudaGetLastError());
   SB_CUDA(cudaStreamSynchronize(s));
-  return p;
+  return *c.projectors.emplace(key, std::move(p)).first->second;
 }
 
 // ---------------------------------------------------------------------------------------

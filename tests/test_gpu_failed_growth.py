@@ -1,0 +1,63 @@
+"""Every device allocation of a call failing in turn, as an out-of-memory cudaMalloc would: the
+failed call raises, and the next ones give what an undisturbed library gives."""
+
+import numpy as np
+import pytest
+
+from scatrs_b200.errors import DeviceError
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(got, want):
+    if isinstance(want, dict):
+        return set(got) == set(want) and all(_same(got[k], want[k]) for k in want)
+    if isinstance(want, (list, tuple)):
+        return len(got) == len(want) and all(_same(a, b) for a, b in zip(got, want))
+    if want is None or got is None:
+        return got is want
+    return np.array_equal(got, want)
+
+
+def _each_growth(lib, small, large):
+    """`large` with its k-th growth failing, k = 1, 2, ..., in a fresh library and after `small`
+    grew it halfway; then `large` and `small` again. Returns the number of growths that failed."""
+    want_small, want_large = small(), large()
+    failed = 0
+    for first in (None, small):
+        k = 0
+        while True:
+            k += 1
+            lib.scatrs_release()
+            if first is not None:
+                first()
+            lib.scatrs_testing_fail_allocation(k)
+            try:
+                large()
+                break
+            except DeviceError as e:
+                assert "out of memory" in str(e)
+            finally:
+                lib.scatrs_testing_fail_allocation(0)
+            failed += 1
+            assert _same(large(), want_large), (k, first is not None)
+            assert _same(small(), want_small), (k, first is not None)
+    return failed
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_projection(gpu, precision):
+    import torch
+
+    def call(n_q, order):
+        f = torch.linspace(0.5, 1.5, 6 * 3 * n_q, dtype=torch.float64, device="cuda")
+        out = torch.zeros(6, 3, order + 1, dtype=torch.float64, device="cuda")
+
+        def run():
+            out.zero_()
+            gpu.project_greek_device(f.data_ptr(), 3, n_q, order, precision, out.data_ptr())
+            return out.cpu().numpy()
+
+        return run
+
+    assert _each_growth(gpu.load(), call(96, 20), call(128, 40)) >= 6
