@@ -3180,13 +3180,17 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       }
       r.sph = c.ro_sph.as<RoSph>(sph.size());
       r.n_sph = (int)sph.size();
-      // The coefficient tables, for the largest order met so far (they depend on nothing else).
+      // The coefficient tables, for the largest order met so far (they depend on nothing else). The
+      // reach is 0 until both are there and filled: a call that fails here leaves none.
       if (c.ro_cg.n < r.max_n) {
-        c.ro_cg.n = std::min(kRoMaxN, (r.max_n + 7) / 8 * 8);
-        launch_cg(c.ro_cg, c.ro_cgr.as<double>((size_t)c.ro_cg.r_size()),
-                  c.ro_cgw.as<double>((size_t)c.ro_cg.w_size()), s);
+        const RoCg cg{std::min(kRoMaxN, (r.max_n + 7) / 8 * 8)};
+        c.ro_cg.n = 0;
+        double* cg_r = c.ro_cgr.as<double>((size_t)cg.r_size());
+        double* cg_w = c.ro_cgw.as<double>((size_t)cg.w_size());
+        launch_cg(cg, cg_r, cg_w, s);
         SB_CUDA(cudaGetLastError());
         g_launches++;
+        c.ro_cg = cg;
       }
       r.cg = c.ro_cg;
       r.cg_r = c.ro_cgr.as<double>(0);

@@ -61,3 +61,13 @@ def test_projection(gpu, precision):
         return run
 
     assert _each_growth(gpu.load(), call(96, 20), call(128, 40)) >= 6
+
+
+def test_orientation_average(gpu):
+    def call(n):
+        return lambda: gpu.spheroid_compute(np.array([1.5, 2.0]), [1.5, 0.6], 1.4 + 1e-2j,
+                                            n_terms=n, n_theta=2 * n, greek_order=8)
+
+    # A fresh library: 13 buffers of the T-matrices, 3 of the projection, 10 of the average, the two
+    # Clebsch-Gordan tables among them.
+    assert _each_growth(gpu.load(), call(6), call(20)) >= 26
