@@ -336,8 +336,10 @@ void ensure_user(Context& c, const double* mu, int64_t n_mu, int64_t n_orders, c
   bool same = (int64_t)u.mu.size() == n_mu && u.n_orders >= n_orders &&
               (n_mu == 0 || memcmp(u.mu.data(), mu, n_mu * sizeof(double)) == 0);
   if (same) return;
+  const int64_t reach =
+      std::max<int64_t>(round_up(std::max<int64_t>(n_orders, 1), 16), u.n_orders);
+  u.n_orders = 0;  // until the tables are on the device: a call that fails here leaves none
   u.mu.assign(mu, mu + n_mu);
-  u.n_orders = std::max<int64_t>(round_up(std::max<int64_t>(n_orders, 1), 16), u.n_orders);
   // Pair each cosine with its exact negative where the list has one.
   std::unordered_multimap<uint64_t, int> by_bits;
   for (int j = 0; j < n_mu; ++j) {
@@ -376,11 +378,11 @@ void ensure_user(Context& c, const double* mu, int64_t n_mu, int64_t n_orders, c
   u.h = (int)cosines.size();
   u.rows = cosines;
   u.h_pad = (int)round_up(std::max(u.h, 1), 32);
-  u.ld = (int)u.n_orders;
+  u.ld = (int)reach;
   std::vector<double> tab(2 * (size_t)u.h_pad * u.ld, 0.0);
   std::vector<double> re(u.ld), ro(u.ld);
   for (int r = 0; r < u.h; ++r) {
-    pi_tau_row(cosines[r], u.n_orders, re.data(), ro.data());
+    pi_tau_row(cosines[r], reach, re.data(), ro.data());
     for (int k = 0; k < u.ld; ++k) {
       tab[table_at(r, k, u.ld)] = re[k];
       tab[table_at(r, k, u.ld) + 32] = ro[k];
@@ -395,6 +397,7 @@ void ensure_user(Context& c, const double* mu, int64_t n_mu, int64_t n_orders, c
     SB_CUDA(cudaMemcpyAsync(u.rows_d.get(cosines.size() * 8), cosines.data(), cosines.size() * 8,
                             cudaMemcpyHostToDevice, s));
   SB_CUDA(cudaStreamSynchronize(s));
+  u.n_orders = reach;
 }
 
 // The level limit of the fixed grid for h_u requested rows and Greek order L: a level of t tiles
@@ -437,29 +440,15 @@ void append_projection(const std::pair<std::vector<double>, std::vector<double>>
     }
 }
 
-// The tables for chunks of up to n_max terms and Greek order L (engine.rs:2034-2072): phase
-// levels up to `limit` tiles (0: none), projector bands for the chunks beyond them.
-BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream_t s) {
-  constexpr size_t kMaxLevelSets = 8;  // (Greek order, limit) pairs with levels kept
-  if (limit > 0 && !c.bands.count({L, limit})) {
-    size_t sets = 0;
-    for (auto& kv : c.bands) sets += kv.first.second > 0;
-    if (sets >= kMaxLevelSets)
-      for (auto it = c.bands.begin(); it != c.bands.end();) {
-        if (it->first.second > 0)
-          it = c.bands.erase(it);
-        else
-          ++it;
-      }
-  }
-  BandTables& bt = c.bands[{L, limit}];
+// Grows `bt` to chunks of up to n_max terms (ensure_bands); after a failure it is not usable.
+void grow_bands(Context& c, BandTables& bt, int L, int limit, int64_t n_max, cudaStream_t s) {
   bt.order = L;
   int need_levels = 0;
   int64_t reach = 0;
   for (int t = 1; t <= limit && reach < n_max; t = next_level_tiles(t), ++need_levels)
     reach = 32 * (int64_t)t - 1;
   int need_bands = L >= 0 && n_max > reach ? band_index(n_max) + 1 : 0;
-  if (bt.n_levels >= need_levels && bt.n_bands >= need_bands) return bt;
+  if (bt.n_levels >= need_levels && bt.n_bands >= need_bands) return;
   // Built for half as many terms again (levels), a quarter (bands), so that slightly larger
   // inputs find them ready.
   if (need_bands > 0) need_bands += 1;
@@ -561,6 +550,31 @@ BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream
   bt.n_levels = n_levels;
   bt.n_bands = (int)bt.bands.size();
   SB_CUDA(cudaStreamSynchronize(s));
+}
+
+// The tables for chunks of up to n_max terms and Greek order L (engine.rs:2034-2072): phase
+// levels up to `limit` tiles (0: none), projector bands for the chunks beyond them.
+BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream_t s) {
+  constexpr size_t kMaxLevelSets = 8;  // (Greek order, limit) pairs with levels kept
+  if (limit > 0 && !c.bands.count({L, limit})) {
+    size_t sets = 0;
+    for (auto& kv : c.bands) sets += kv.first.second > 0;
+    if (sets >= kMaxLevelSets)
+      for (auto it = c.bands.begin(); it != c.bands.end();) {
+        if (it->first.second > 0)
+          it = c.bands.erase(it);
+        else
+          ++it;
+      }
+  }
+  BandTables& bt = c.bands[{L, limit}];
+  try {
+    grow_bands(c, bt, L, limit, n_max, s);
+  } catch (...) {
+    // Half-grown tables would be taken for whole ones: the next call starts from none.
+    c.bands.erase({L, limit});
+    throw;
+  }
   return bt;
 }
 
@@ -569,6 +583,7 @@ void ensure_interp(Context& c, BandTables& bt, cudaStream_t s) {
   if (bt.n_levels == 0 || bt.mu == c.user.mu) return;
   const BandDesc& last = bt.desc[bt.n_levels - 1];
   const size_t n_half = (size_t)bt.half0.back() + last.h;
+  bt.mu.clear();  // until the matrices are made (with levels there are cosines)
   double* node = bt.node_d.as<double>(0);
   LevelMatrixArgs la{};
   la.n_levels = bt.n_levels;
@@ -659,6 +674,7 @@ void ensure_i8(Context& c, int64_t n_max, const BandTables* bt, cudaStream_t s) 
   if (T.mu == c.user.mu && T.user_orders >= ((int64_t)kI8KB << (n_ver - 1)) && T.order == L &&
       T.n_bands == nb && T.n_levels == n_levels)
     return;
+  T.order = -2;  // until the digits are on the device: matches no call
   std::vector<unsigned char> dig;
   std::vector<double> scale;
   T.user.clear();

@@ -4,6 +4,7 @@ failed call raises, and the next ones give what an undisturbed library gives."""
 import numpy as np
 import pytest
 
+from scatrs_b200 import workloads as W
 from scatrs_b200.errors import DeviceError
 
 pytestmark = pytest.mark.gpu
@@ -19,10 +20,12 @@ def _same(got, want):
     return np.array_equal(got, want)
 
 
-def _each_growth(lib, small, large):
+def _each_growth(lib, small, large, larger=None):
     """`large` with its k-th growth failing, k = 1, 2, ..., in a fresh library and after `small`
-    grew it halfway; then `large` and `small` again. Returns the number of growths that failed."""
+    grew it halfway; then `large`, `small` and `larger` again. Returns the number of growths that
+    failed."""
     want_small, want_large = small(), large()
+    want_larger = larger() if larger else None
     failed = 0
     for first in (None, small):
         k = 0
@@ -42,7 +45,42 @@ def _each_growth(lib, small, large):
             failed += 1
             assert _same(large(), want_large), (k, first is not None)
             assert _same(small(), want_small), (k, first is not None)
+            if larger:
+                assert _same(larger(), want_larger), (k, first is not None)
     return failed
+
+
+@pytest.fixture
+def small_arena(gpu):
+    """Slabs of 64 MiB, so that a fresh library grows quickly."""
+    gpu.set_tuning(arena_rows=1 << 16)
+    yield gpu
+    gpu.set_tuning()
+
+
+WL = np.array([0.5, 0.7])
+M = np.array([[1.5 + 1e-2j, 1.4 + 1e-3j]])
+FORMS = {
+    # Projector bands alone, on no cosines; phase levels with and without bands beyond them.
+    "bands": lambda gpu, d: gpu.ensemble_fixed(d, WL, M, None, 64, 12),
+    "levels": lambda gpu, d: gpu.ensemble_fixed(d, WL, M, W.gauss_legendre(90), 64, 12),
+    "beyond": lambda gpu, d: gpu.ensemble_fixed(d, WL, M, W.gauss_legendre(4), 64, 12),
+    "mixed": lambda gpu, d: gpu.ensemble_fixed(d, WL, M, W.gauss_legendre(60), 64, 12,
+                                               i8_above=16),
+    "derivatives": lambda gpu, d: gpu.ensemble_fixed_d(d, WL, M, W.gauss_legendre(60), 64, 12),
+    "adaptive": lambda gpu, d: gpu.ensemble_adaptive(d, WL, M[0], W.gauss_legendre(20), 12,
+                                                     rtol=1e-4),
+}
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_tables(small_arena, form):
+    gpu = small_arena
+
+    def call(median):
+        return lambda: FORMS[form](gpu, W.lognormals([median], [1.3], 2))
+
+    assert _each_growth(gpu.load(), call(0.1), call(0.8), call(3.0)) >= 10
 
 
 @pytest.mark.parametrize("precision", [0, 1])
