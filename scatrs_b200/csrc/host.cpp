@@ -1212,8 +1212,11 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       L >= 0 ? c.slot_greek.as<double>((size_t)slots_max * 6 * (L + 1)) : nullptr;
   double* slot_phase =
       n_levels > 0 ? c.slot_phase.as<double>((size_t)slots_max * 4 * n_mu) : nullptr;
-  // The row tiles of a slot's projections at most (slot_project_kernel).
-  const int slot_tiles = (n_levels > 0 ? t_user : 0) + (L >= 0 ? 2 * (L / 32 + 1) : 0);
+  // The row tiles of a slot's projections at most (slot_project_kernel): the tables reach
+  // min(L, 2 N) orders, however large L is.
+  int reach = -1;
+  for (int k = 0; k < nb; ++k) reach = std::max(reach, bt->desc[k].order);
+  const int slot_tiles = (n_levels > 0 ? t_user : 0) + (L >= 0 ? 2 * (reach / 32 + 1) : 0);
   int* counter = c.counter.as<int>(64);
   int64_t* chunk_xoff_d = nullptr;
   int* chunk_xidx_d = nullptr;

@@ -298,8 +298,7 @@ __global__ void __launch_bounds__(128, 4) slot_project_kernel(SlotArgs a) {
   const BandDesc B = a.bands[it.band];
   const bool level = it.band < a.n_levels;
   const int tu = level ? (a.h_u + 31) / 32 : 0, tg = a.greek_order >= 0 ? B.order / 32 + 1 : 0;
-  int tile = blockIdx.y;
-  if (tile >= tu + 2 * tg) return;
+  if ((int)blockIdx.y >= tu + 2 * tg) return;
   if (threadIdx.x < it.count) {
     const int k = a.slot_index[it.first + threadIdx.x];
     const BandSlot s = a.slots[k];
@@ -307,13 +306,15 @@ __global__ void __launch_bounds__(128, 4) slot_project_kernel(SlotArgs a) {
     sm.off[threadIdx.x] = s.off;
     sm.reps[threadIdx.x] = s.reps;
   }
-  __syncthreads();
-  if (tile < tu) {
-    slot_tile<0>(a, sm, B, it.band, it.count, 32 * tile);
-  } else if ((tile -= tu) < tg) {
-    slot_tile<1>(a, sm, B, it.band, it.count, 32 * tile);
-  } else {
-    slot_tile<2>(a, sm, B, it.band, it.count, 32 * (tile - tg));
+  // A block per tile; beyond the grid's 65,535 rows (2^21 cosines) a block takes several.
+  for (int tile = blockIdx.y; tile < tu + 2 * tg; tile += gridDim.y) {
+    __syncthreads();
+    if (tile < tu)
+      slot_tile<0>(a, sm, B, it.band, it.count, 32 * tile);
+    else if (tile < tu + tg)
+      slot_tile<1>(a, sm, B, it.band, it.count, 32 * (tile - tu));
+    else
+      slot_tile<2>(a, sm, B, it.band, it.count, 32 * (tile - tu - tg));
   }
 }
 
@@ -331,8 +332,8 @@ cudaError_t launch_slot_project(const SlotArgs& a, int max_tiles, cudaStream_t s
   cudaError_t e = cudaFuncSetAttribute(
       slot_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SlotSmem));
   if (e != cudaSuccess) return e;
-  slot_project_kernel<<<dim3((unsigned)a.n_items, (unsigned)max_tiles), 128, sizeof(SlotSmem),
-                        s>>>(a);
+  slot_project_kernel<<<dim3((unsigned)a.n_items, (unsigned)(max_tiles < 65535 ? max_tiles : 65535)),
+                        128, sizeof(SlotSmem), s>>>(a);
   return cudaGetLastError();
 }
 
