@@ -3017,6 +3017,7 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
   if (t_out) t_out->assign(specs.size(), {});
   if (greek_out) greek_out->clear();
   constexpr double kBudget = 8.0e9;  // bytes of device workspace per batch
+  constexpr size_t kMaxRows = 65535;  // gridDim.y
   const bool ro = greek_out != nullptr;
   auto same_geom = [](const TmSpec& p, const TmSpec& q) {
     return p.x == q.x && p.eps == q.eps && p.s_re == q.s_re && p.s_im == q.s_im && p.N == q.N &&
@@ -3052,8 +3053,10 @@ void run_tmatrices(Context& c, const std::vector<TmSpec>& specs, std::vector<dou
       }
       if (ro && !new_geom && t.m != specs[j1 - 1].m + 1)
         throw Failure{SCATRS_INVALID_INPUT, "the orientation average needs the modes 0..N in order"};
-      // Batches break between spheroids when their modes must stay together.
+      // Batches break between spheroids when their modes must stay together; the orientation
+      // average has a spheroid per row of its grid.
       if (j1 > j0 && bytes + b > kBudget && (!ro || new_geom)) break;
+      if (ro && new_geom && geoms.size() == kMaxRows) break;
       bytes += b;
       if (new_geom) {
         if (!rule_at.count(nq)) {

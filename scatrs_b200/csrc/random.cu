@@ -536,15 +536,20 @@ cudaError_t launch_random(const RoArgs& a, cudaStream_t s) {
   if (a.n_sph <= 0) return cudaSuccess;
   auto grid = [](int64_t n) { return (unsigned)((n + 127) / 128); };
   ro_rank_kernel<<<dim3(a.max_n * (a.max_n + 1) / 2, (a.n_sph + 1) / 2), 128, 0, s>>>(a);
+  // Each launch's own status: a later launch that succeeds can hide an earlier one's refusal.
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
   const int q_tiles = (2 * a.max_n + 3 + 7) / 8;
   ro_w_kernel<<<dim3(2 * a.max_n * q_tiles, a.n_sph, (2 * a.max_n + 1 + 127) / 128), 128, 0, s>>>(a);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   // Shared memory: the angular parts of the four helicity keys at a tile of 32 cosines for the
   // batch's largest N.
   const size_t pt_bytes = (size_t)4 * ((a.max_n + 3) & ~3) * kPhiStride * sizeof(double);
-  const cudaError_t e = cudaFuncSetAttribute(
-      ro_phi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pt_bytes);
+  e = cudaFuncSetAttribute(ro_phi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)pt_bytes);
   if (e != cudaSuccess) return e;
   ro_phi_kernel<<<(unsigned)a.n_phi, 256, pt_bytes, s>>>(a);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   ro_f_kernel<<<grid(a.n_f), 128, 0, s>>>(a);
   ro_greek_kernel<<<grid(a.n_g), 128, 0, s>>>(a);
   return cudaGetLastError();

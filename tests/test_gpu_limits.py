@@ -32,3 +32,16 @@ def test_cosines_beyond_the_grids_rows(gpu):
     _, ph, _ = gpu.ensemble_fixed(d, WL, M, mu, 32)
     _, want, _ = gpu.ensemble_fixed(d, WL, M, mu[at], 32)
     assert np.max(np.abs(ph[..., at] - want)) <= 1e-12 * want[0].max()
+
+
+def test_more_spheroids_than_grid_rows(gpu):
+    # 70,000 spheroids of one truncation in a call: every one as on its own.
+    n = 70_000
+    x = np.full(n, 0.3)
+    x[::7], x[-1] = 0.2, 0.25
+    got = gpu.spheroid_compute(x, 1.5, 1.5 + 1e-2j, n_terms=2, n_theta=4, greek_order=2)
+    for v in (0.2, 0.25, 0.3):
+        want = gpu.spheroid_compute(np.array([v]), 1.5, 1.5 + 1e-2j, n_terms=2, n_theta=4,
+                                    greek_order=2)
+        assert (got["efficiencies"][x == v] == want["efficiencies"][0]).all()
+        assert (got["greek"][x == v] == want["greek"][0]).all()
