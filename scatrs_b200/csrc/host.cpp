@@ -200,8 +200,8 @@ struct BandTables {
   std::vector<BandDesc> bands;
   std::vector<double> g, d;       // host copies, appended band by band
   std::vector<int> half0;         // each level's first half node
-  std::vector<double> mu;         // the cosines me_d and mo_d interpolate onto
-  DevBuf g_d, lg_d, d_d, desc_d, half0_d, x0_d, node_d, me_d, mo_d;
+  std::vector<double> mu;         // the cosines lp_d and lm_d interpolate onto
+  DevBuf g_d, lg_d, d_d, desc_d, half0_d, x0_d, node_d, lp_d, lm_d;
   int merge_max() const { return n_levels > 0 ? desc[n_levels - 1].upper : 0; }
 };
 
@@ -402,9 +402,9 @@ void ensure_user(Context& c, const double* mu, int64_t n_mu, int64_t n_orders, c
 
 // The level limit of the fixed grid for h_u requested rows and Greek order L: a level of t tiles
 // is used while it runs fewer tiles than the requested rows and its largest chunk's projector
-// band. A unit's interpolation from the level costs about h_u / 1024 of the tiles it replaces per
-// chunk (2 h_u h multiply-adds per element against 8 x 32 x 32 per tile row and order), counted
-// twice as it runs at a lower rate. The levels' interpolation matrices stay below 1 GiB. Returns
+// band. A unit's interpolation from the level costs about h_u / 512 of the tiles it replaces per
+// chunk (4 h_u h multiply-adds per element against 8 x 32 x 32 per tile row and order). The levels'
+// interpolation matrices stay below 1 GiB. Returns
 // the tiles of the last level, 0 for none.
 int level_limit(int h_u, int L) {
   const int t_user = (h_u + 31) / 32;
@@ -595,8 +595,8 @@ void ensure_interp(Context& c, BandTables& bt, cudaStream_t s) {
   la.x_lo = node + n_half;
   la.bary = node + 2 * n_half;
   la.rows = c.user.rows_d.as<double>(0);
-  la.me = bt.me_d.as<double>(n_half * c.user.h_pad);
-  la.mo = bt.mo_d.as<double>(n_half * c.user.h_pad);
+  la.lp = bt.lp_d.as<double>(n_half * c.user.h_pad);
+  la.lm = bt.lm_d.as<double>(n_half * c.user.h_pad);
   launch_level_matrices(la, s);
   SB_CUDA(cudaGetLastError());
   g_launches++;
@@ -1628,8 +1628,8 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
       sa.h_pad = c.user.h_pad;
       if (n_levels > 0) {
         sa.half0 = bt->half0_d.as<int>(0);
-        sa.me = bt->me_d.as<double>(0);
-        sa.mo = bt->mo_d.as<double>(0);
+        sa.lp = bt->lp_d.as<double>(0);
+        sa.lm = bt->lm_d.as<double>(0);
       }
       sa.user_map = ua.user_map;
       sa.slot_phase = slot_phase;

@@ -172,7 +172,7 @@ struct LevelTableArgs {
   double* bary;
   double* g;
 };
-// The interpolation onto the requested rows: per half node h_pad even and h_pad odd weights.
+// The interpolation onto the requested rows: per half node h_pad weights of it and h_pad of its mirror.
 struct LevelMatrixArgs {
   int n_levels, h_u, h_pad;
   const BandDesc* bands;
@@ -181,8 +181,8 @@ struct LevelMatrixArgs {
   const double* x_lo;
   const double* bary;
   const double* rows;  // the requested rows' cosines
-  double* me;
-  double* mo;
+  double* lp;
+  double* lm;
 };
 void launch_level_tables(const LevelTableArgs& a, cudaStream_t s);
 void launch_level_matrices(const LevelMatrixArgs& a, cudaStream_t s);
@@ -234,8 +234,8 @@ struct SlotArgs {
   // The requested cosines.
   int n_mu, h_u, h_pad;
   const int* half0;
-  const double* me;
-  const double* mo;
+  const double* lp;
+  const double* lm;
   const int2* user_map;
   double* slot_phase;
   // The Greek coefficients.

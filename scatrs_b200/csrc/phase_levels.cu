@@ -12,10 +12,13 @@
 //
 // Accuracy: the nodes are held in double-double (one Newton step from the double rule), the
 // tables at them are rounded once from a double-double recurrence, and the interpolation is the
-// barycentric form with the weights 1 / P_n'(x_k) of the same step. Against extended precision
-// the interpolated elements are within a small factor of the direct sums pointwise (the
-// Lagrange functions of Gauss nodes fall off away from a node, so the forward peak's rounding
-// does not reach the backward directions). Compiled with -fmad=false (double-double).
+// barycentric form with the weights 1 / P_n'(x_k) of the same step. The Lagrange functions of
+// Gauss nodes fall off away from a node, so the forward peak's rounding does not reach the backward
+// directions: relative to its own value F11 there is 5e-15 off extended precision at x = 30, 3e-14
+// at x = 300 (direct sums on tables from double recurrences: 6e-14, 3e-13). That needs the values at
+// +mu and -mu kept apart: folded into even and odd parts, which halves the products, a backward
+// element is the difference of two sums of the forward peak's size (5e-13, 7e-12). Compiled with
+// -fmad=false (double-double).
 #include "dd.cuh"
 #include "kernels.h"
 
@@ -75,8 +78,9 @@ __global__ void __launch_bounds__(128) level_table_kernel(LevelTableArgs a) {
   o[0] = o[32] = 0.0;
 }
 
-// One thread per (level, requested row): the row's interpolation weights onto the level's half
-// nodes, even part l_k + l_{-k} and odd part l_k - l_{-k} (the middle node alone, even).
+// One thread per (level, requested row): the row's interpolation weights l_k of the level's half
+// nodes and l_{-k} of their mirrors (the middle node once). The row -c has the two exchanged, the
+// middle node's weight being even in c.
 __global__ void __launch_bounds__(128) level_matrix_kernel(LevelMatrixArgs a) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x, lv = blockIdx.y;
   if (r >= a.h_pad) return;
@@ -84,10 +88,10 @@ __global__ void __launch_bounds__(128) level_matrix_kernel(LevelMatrixArgs a) {
   const double* xh = a.x_hi + k0;
   const double* xl = a.x_lo + k0;
   const double* v = a.bary + k0;
-  double* me = a.me + (int64_t)k0 * a.h_pad + r;
-  double* mo = a.mo + (int64_t)k0 * a.h_pad + r;
+  double* lp = a.lp + (int64_t)k0 * a.h_pad + r;
+  double* lm = a.lm + (int64_t)k0 * a.h_pad + r;
   if (r >= a.h_u) {
-    for (int k = 0; k < h; ++k) me[(int64_t)k * a.h_pad] = mo[(int64_t)k * a.h_pad] = 0.0;
+    for (int k = 0; k < h; ++k) lp[(int64_t)k * a.h_pad] = lm[(int64_t)k * a.h_pad] = 0.0;
     return;
   }
   const double c = a.rows[r];
@@ -105,25 +109,24 @@ __global__ void __launch_bounds__(128) level_matrix_kernel(LevelMatrixArgs a) {
   }
   const double is = hit < 0 ? 1.0 / sum : 0.0;
   for (int k = 0; k < h; ++k) {
-    double e, o;
+    double p, m;
     if (hit >= 0) {
-      e = k == hit ? 1.0 : 0.0;
-      o = (k == hit && k > 0) ? (double)hit_sign : 0.0;
+      p = k == hit && hit_sign > 0 ? 1.0 : 0.0;
+      m = k == hit && hit_sign < 0 ? 1.0 : 0.0;
     } else {
       const double dm = (c - xh[k]) - xl[k], dp = (c + xh[k]) + xl[k];
-      const double lp = (v[k] / dm) * is, lm = k == 0 ? 0.0 : (v[k] / dp) * is;
-      e = lp + lm;
-      o = k == 0 ? 0.0 : lp - lm;
+      p = (v[k] / dm) * is;
+      m = k == 0 ? 0.0 : (v[k] / dp) * is;
     }
-    me[(int64_t)k * a.h_pad] = e;
-    mo[(int64_t)k * a.h_pad] = o;
+    lp[(int64_t)k * a.h_pad] = p;
+    lm[(int64_t)k * a.h_pad] = m;
   }
 }
 
 // The slots' sums (the fixed grid) onto the requested cosines and the Greek coefficients: two FP64
 // GEMMs side by side per tile of 32 output rows and up to 16 slots of one table,
-//   the requested cosines (levels): M_E F_E and M_O F_O over the half nodes, F_E, F_O the even and
-//     odd parts of the 4 elements; their sum and difference are the elements at +c and -c;
+//   the requested cosines (levels): of the 4 elements at the half nodes (F+) and their mirrors (F-),
+//     L+ F+ + L- F- at +c and L- F+ + L+ F- at -c;
 //   alpha1, alpha4 and beta1, beta2: d00 [F11, F33] and d02 [F12, F34] over the n_q nodes;
 //   alpha2, alpha3: d22 (F11 + F33) and d2-2 (F11 - F33); half their sum and difference.
 // blockIdx.y runs over the row tiles in that order. Each output is one slot's (final_kernel adds a
@@ -163,8 +166,8 @@ __device__ __forceinline__ void slot_tile(const SlotArgs& a, SlotSmem& sm, const
   const double* ma;
   const double* mb;
   if (kType == 0) {
-    ma = a.me + (int64_t)a.half0[level] * ld;
-    mb = a.mo + (int64_t)a.half0[level] * ld;
+    ma = a.lp + (int64_t)a.half0[level] * ld;
+    mb = a.lm + (int64_t)a.half0[level] * ld;
   } else {
     const double* D = a.band_d + B.d_off;  // d00, d22, d2-2, d02
     ma = D + (int64_t)(kType == 1 ? 0 : 1) * nq * ld;
@@ -219,14 +222,8 @@ __device__ __forceinline__ void slot_tile(const SlotArgs& a, SlotSmem& sm, const
   auto store_f = [&](int st) {
 #pragma unroll
     for (int j = 0; j < kN; ++j) {
-      if (kType == 1) {
-        sm.b[st][0][kh + j][col] = f0[j];
-        sm.b[st][1][kh + j][col] = f1[j];
-      } else {
-        const double s = kType == 0 ? 0.5 : 1.0;
-        sm.b[st][0][kh + j][col] = s * (f0[j] + f1[j]);
-        sm.b[st][1][kh + j][col] = s * (f0[j] - f1[j]);
-      }
+      sm.b[st][0][kh + j][col] = kType == 2 ? f0[j] + f1[j] : f0[j];
+      sm.b[st][1][kh + j][col] = kType == 2 ? f0[j] - f1[j] : f1[j];
     }
   };
   load_a(0, 0);
@@ -247,8 +244,13 @@ __device__ __forceinline__ void slot_tile(const SlotArgs& a, SlotSmem& sm, const
 #pragma unroll
       for (int nt = 0; nt < kNt; ++nt)
         if (nt < n_nt) {
-          dmma(cA[nt][0], cA[nt][1], va, sm.b[st][0][k4 + q][8 * nt + g]);
-          dmma(cB[nt][0], cB[nt][1], vb, sm.b[st][1][k4 + q][8 * nt + g]);
+          const double b0 = sm.b[st][0][k4 + q][8 * nt + g], b1 = sm.b[st][1][k4 + q][8 * nt + g];
+          dmma(cA[nt][0], cA[nt][1], va, b0);
+          dmma(cB[nt][0], cB[nt][1], vb, kType == 0 ? b0 : b1);
+          if (kType == 0) {
+            dmma(cA[nt][0], cA[nt][1], vb, b1);
+            dmma(cB[nt][0], cB[nt][1], va, b1);
+          }
         }
     }
     if (more) store_f(st ^ 1);
@@ -264,8 +266,8 @@ __device__ __forceinline__ void slot_tile(const SlotArgs& a, SlotSmem& sm, const
       double* out = a.slot_phase + (int64_t)sm.slot[s] * 4 * a.n_mu;
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        out[(int64_t)(e + j) * a.n_mu + mp.x] = cA[nt][j] + cB[nt][j];
-        if (mp.y >= 0) out[(int64_t)(e + j) * a.n_mu + mp.y] = cA[nt][j] - cB[nt][j];
+        out[(int64_t)(e + j) * a.n_mu + mp.x] = cA[nt][j];
+        if (mp.y >= 0) out[(int64_t)(e + j) * a.n_mu + mp.y] = cB[nt][j];
       }
     }
   } else {
