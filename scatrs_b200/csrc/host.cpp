@@ -861,6 +861,13 @@ struct AdaptiveInput {
   // per-block averages of final_adaptive_d_kernel.
 };
 
+// The device's error words, cleared: invalid nodes, undefined ratios, a bounded wait that gave up.
+unsigned long long* clear_errors(Context& c, cudaStream_t s) {
+  unsigned long long* err = c.err.as<unsigned long long>(3);
+  SB_CUDA(cudaMemsetAsync(err, 0xff, 3 * sizeof(unsigned long long), s));
+  return err;
+}
+
 void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, const double* wl_dev,
                int64_t n_wl, const double* m_dev, const double* mu, int64_t n_mu,
                const scatrs_fixed_options* opt, double* values, double* phase, double* greek,
@@ -952,9 +959,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   // Adaptive calls add the error sums of every block (a second set of n_blk / 2).
   const int n_blk = (dv.on ? 3 + dv.n_theta : 1) * (ad.on ? 2 : 1);
   const int rows_per_term = dv.on ? 2 : 1;
-  // Error words: invalid nodes, undefined ratios, a bounded wait that gave up.
-  unsigned long long* err = c.err.as<unsigned long long>(3);
-  SB_CUDA(cudaMemsetAsync(err, 0xff, 3 * sizeof(unsigned long long), s));
+  unsigned long long* err = clear_errors(c, s);
   unsigned* wait_err = reinterpret_cast<unsigned*>(err + 2);
   // 2. Plan: every chunk's largest number of terms.
   PlanArgs pa{};
@@ -1684,6 +1689,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
 
 // Reads the error words of the last call (synchronizes the stream).
 void check_device_errors(Context& c, cudaStream_t s, const FixedCall* call) {
+  if (!c.err.p) clear_errors(c, s);  // no call yet
   unsigned long long h[3];
   SB_CUDA(cudaMemcpyAsync(h, c.err.as<unsigned long long>(3), sizeof h, cudaMemcpyDeviceToHost, s));
   SB_CUDA(cudaStreamSynchronize(s));
@@ -6725,8 +6731,7 @@ int scatrs_mie(const double* x, const double* m, int64_t n, int32_t allow_unvali
     int64_t* nd = nb.as<int64_t>(n);
     SB_CUDA(cudaMemcpyAsync(xd, x, n * 8, cudaMemcpyHostToDevice, s));
     SB_CUDA(cudaMemcpyAsync(md, m, n * 16, cudaMemcpyHostToDevice, s));
-    unsigned long long* errw = c.err.as<unsigned long long>(2);
-    SB_CUDA(cudaMemsetAsync(errw, 0xff, 16, s));
+    unsigned long long* errw = clear_errors(c, s);
     MieNodesArgs a{};
     a.x = xd;
     a.m = md;

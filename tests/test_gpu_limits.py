@@ -45,3 +45,12 @@ def test_more_spheroids_than_grid_rows(gpu):
                                     greek_order=2)
         assert (got["efficiencies"][x == v] == want["efficiencies"][0]).all()
         assert (got["greek"][x == v] == want["greek"][0]).all()
+
+
+def test_no_errors_before_the_first_ensemble_call(gpu):
+    lib = gpu.load()
+    lib.scatrs_release()
+    gpu.check_errors()
+    lib.scatrs_release()
+    gpu.mie(np.array([1.0]), np.array([1.5 + 0j]))
+    gpu.check_errors()
