@@ -355,6 +355,12 @@ struct Panel {
   int64_t n_terms = 0;
   std::vector<Sums1> sums;  // per part of the job, in buf
   std::vector<double> buf;
+  // Moved only: a copy's sums would point into the original's buf.
+  Panel(double a_, double b_) : a(a_), b(b_) {}
+  Panel(const Panel&) = delete;
+  Panel& operator=(const Panel&) = delete;
+  Panel(Panel&&) = default;
+  Panel& operator=(Panel&&) = default;
 };
 
 struct State {
