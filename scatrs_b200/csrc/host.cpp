@@ -1171,7 +1171,8 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     }
   }
   int64_t acc_max = 1, slots_max = 1, stage_max = 0, n_slots_all = 0, n_proj_all = 0,
-          n_items_all = 0, i8_bytes_max = 16, i8_chunks_max = 1, n_split_all = 0, split_rows_max = 0;
+          n_items_all = 0, i8_bytes_max = 16, i8_chunks_max = 1, n_split_all = 0, split_rows_max = 0,
+          chunks_max = 1;
   auto stage_bytes = [&](const Slab& S) {
     return S.nu * (int64_t)(sizeof(int) + 8 + sizeof(int2)) +
            S.nu * cpu * (int64_t)(sizeof(int) + 16) +
@@ -1183,6 +1184,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   for (const Slab& S : slabs) {
     acc_max = std::max(acc_max, S.acc_len);
     slots_max = std::max(slots_max, S.n_slots);
+    chunks_max = std::max(chunks_max, S.nu * cpu);
     stage_max = std::max(stage_max, stage_bytes(S));
     n_slots_all += S.n_slots;
     n_proj_all += S.pi_cap;
@@ -1257,7 +1259,7 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   ka.X = X;
   // Weights per node: values, each parameter's, and the same with the error weights.
   const int side_stride = 32 * (dv.on ? 1 + dv.n_theta : 1) * (ad.on ? 2 : 1) + 4;
-  double* side = c.side.as<double>((size_t)kMaxSlabChunks * side_stride);
+  double* side = c.side.as<double>((size_t)chunks_max * side_stride);
   ka.side = side;
   if (may_split) ka.split_rows = c.split_rows.as<double4>((size_t)split_rows_max * 64);
   ka.side_stride = side_stride;

@@ -46,3 +46,29 @@ def test_release_gives_every_buffer_back(gpu):
     lib.scatrs_release()
     assert held > 64 * MIB
     assert before - _free() <= 4 * MIB
+
+
+@pytest.fixture
+def small_arena(gpu):
+    """Coefficient arenas of 64 MiB."""
+    gpu.set_tuning(arena_rows=1 << 16)
+    yield gpu
+    gpu.set_tuning()
+
+
+# The buffers of a call whatever its size, in MiB, at that arena: the coefficient rows, u_k(mx) and
+# u_k(x) of the rows and of two more per chunk of the largest slab, and 64 KiB for each of the rest.
+FIXED = 64 + (64 + 512) / 2 + (64 + 512) / 4 + 16
+
+
+def test_a_small_call_holds_little(small_arena):
+    gpu = small_arena
+    wl, m = np.array([0.5, 0.8]), np.full((1, 2), 1.5 + 1e-2j)
+    d = W.lognormals([0.1], [1.4], 3)
+
+    def call():
+        gpu.ensemble_fixed_d(d, wl, m, W.gauss_legendre(32), 64, 16)
+
+    call()
+    # And the sums of the largest slab's chunks, 5 blocks of 8.
+    assert _used(gpu.load(), call) <= (FIXED + 80 + 16) * MIB
