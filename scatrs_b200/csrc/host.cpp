@@ -163,7 +163,12 @@ struct DevBuf {
       if (g_fail_allocation.load() > 0 && g_fail_allocation.fetch_sub(1) == 1)
         throw Failure{SCATRS_CUDA, std::string("cudaMalloc(&p, want): ") +
                                        cudaGetErrorString(cudaErrorMemoryAllocation)};
-      SB_CUDA(cudaMalloc(&p, want));
+      if (cudaMalloc(&p, want) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+        want = bytes;  // without the room to spare it may still fit
+        SB_CUDA(cudaMalloc(&p, want));
+      }
       cap = want;
     }
     return p;

@@ -72,3 +72,24 @@ def test_a_small_call_holds_little(small_arena):
     call()
     # And the sums of the largest slab's chunks, 5 blocks of 8.
     assert _used(gpu.load(), call) <= (FIXED + 80 + 16) * MIB
+
+
+def test_a_growth_that_fits_only_exactly(gpu):
+    # Regrown buffers take room to spare where there is some: 200 and 200 and 30 MiB, with the room
+    # 264, 264 and 45, in 520 MiB.
+    import torch
+
+    n_q, n, order = 64, 200 * MIB // (24 * 64), 8
+    phase = torch.ones(6, n, n_q, dtype=torch.float64, device="cuda")
+    out = torch.empty(6, n, order + 1, dtype=torch.float64, device="cuda")
+    gpu.project_greek_device(phase.data_ptr(), 4, n_q, order, 1, out.data_ptr())
+    torch.cuda.empty_cache()
+    fill = torch.empty(_free() - 520 * MIB, dtype=torch.uint8, device="cuda")
+    try:
+        gpu.project_greek_device(phase.data_ptr(), n, n_q, order, 1, out.data_ptr())
+        torch.cuda.synchronize()
+        assert abs(float(out[0, -1, 0]) - 1.0) < 1e-5
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+        gpu.load().scatrs_release()
