@@ -1133,21 +1133,28 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
     }
     // A chunk's recurrences take about 2000 cycles an order on one warp; the slab's, at 16 warps per
     // SM, about 250 per chunk and order. Where most of a slab's orders are in chunks that would each
-    // take more than half of the slab's time, every chunk gets a block (mie_split_kernel).
+    // take more than half of the slab's time, every chunk gets a block (mie_split_kernel). Its scratch
+    // is 2 KiB per order, twice the coefficients', and stays within half of the arena's bytes (2 GiB;
+    // without the bound up to 8.6): slabs of more rows than a quarter of the arena keep the one warp
+    // (K-a of droplets to x = 1,000 in 256 nodes: 150 units 3.2 -> 3.7 ms beside 9.9 of unit kernel; of
+    // 300 units the blocks are the slower, 5.4 against 4.7).
     if (may_split) {
       int64_t s0 = 0;
-      std::vector<int64_t> long_orders(n_slabs, 0);
+      std::vector<int64_t> long_orders(n_slabs, 0), rows(n_slabs, 0);
       for (int64_t u = 0; u < n_units; ++u) {
         const Slab& S = slabs[slab_of[u]];
         const double half = 0.5 * 250.0 / 2000.0 * (double)S.orders / c.sms;
-        for (int k = 0; k < cpu; ++k)
-          if (cn[u * cpu + k] > half) long_orders[slab_of[u]] += cn[u * cpu + k];
+        for (int k = 0; k < cpu; ++k) {
+          const int nc = cn[u * cpu + k];
+          if (nc > half) long_orders[slab_of[u]] += nc;
+          rows[slab_of[u]] += nc + 2;
+        }
       }
       for (int64_t sl = 0; sl < n_slabs; ++sl)
-        if (2 * long_orders[sl] > slabs[sl].orders) slabs[sl].n_split = count[sl] * cpu;
-      for (int64_t u = 0; u < n_units; ++u)
-        if (slabs[slab_of[u]].n_split > 0)
-          for (int k = 0; k < cpu; ++k) slabs[slab_of[u]].split_rows += cn[u * cpu + k] + 2;
+        if (2 * long_orders[sl] > slabs[sl].orders && 4 * rows[sl] <= arena) {
+          slabs[sl].n_split = count[sl] * cpu;
+          slabs[sl].split_rows = rows[sl];
+        }
       for (Slab& S : slabs) {
         S.split0 = s0;
         s0 += S.n_split;

@@ -93,3 +93,27 @@ def test_a_growth_that_fits_only_exactly(gpu):
         del fill
         torch.cuda.empty_cache()
         gpu.load().scatrs_release()
+
+
+def test_split_chunks_scratch_is_bounded(gpu):
+    # 200 chunks of 1,600 orders, few enough for a block each: their scratch is 2 KiB per order, at
+    # most half of the arena's bytes. The results have the same bits with and without.
+    wl = np.linspace(0.5, 0.501, 200)
+    d = W.lognormals([1500 * 0.5 / (2 * np.pi)], [1.01], 1)
+    m = np.full((1, 200), 1.33 + 1e-4j)
+
+    def call():
+        return gpu.ensemble_fixed(d, wl, m, np.array([-0.5, 0.9]), 32)
+
+    try:
+        gpu.set_tuning(arena_rows=1 << 22)
+        want = call()
+        gpu.set_tuning(arena_rows=1 << 20)
+        # The coefficient rows, u_k(mx) and u_k(x) with two rows for each of 2^18 chunks, the sums.
+        fixed = 1024 + (1024 + 512) / 2 + (1024 + 512) / 4 + 16
+        assert _used(gpu.load(), call) <= (fixed + 64) * MIB
+        for a, b in zip(call()[:2], want[:2]):
+            assert np.array_equal(a, b)
+    finally:
+        gpu.set_tuning()
+        gpu.load().scatrs_release()
