@@ -1074,25 +1074,29 @@ void run_fixed(Context& c, const scatrs_distribution* dists, int64_t n_dist, con
   });
   // Cut the units, in order, into slabs of consecutive units (so that a slab's outputs are a few
   // contiguous ranges, copied out while the next slabs run) of about equal work, each within the
-  // arena and the chunk limit.
+  // arena and the chunk limit, the slots' elements at the requested cosines (slot_phase) within a
+  // quarter of the arena's bytes.
+  const int64_t slot_cap =
+      n_levels > 0 ? std::max<int64_t>(1, arena * 1024 / 4 / (4 * n_mu * 8)) : INT64_MAX;
   int64_t n_slabs = std::max<int64_t>(1, (total_rows + arena - 1) / arena);
   n_slabs = std::max<int64_t>(n_slabs, (n_chunks + kMaxSlabChunks - 1) / kMaxSlabChunks);
   std::vector<int> slab_of(n_units);
   std::vector<int64_t> slab_lo;  // the first unit of each slab
   {
     const double target = total_cost / (double)n_slabs;
-    int64_t rows = 0, chunks = 0;
+    int64_t rows = 0, chunks = 0, slots = 0;
     double cost = 0.0;
     for (int64_t u = 0; u < n_units; ++u) {
       if (u == 0 || rows + urows[u] > arena || chunks + cpu > kMaxSlabChunks ||
-          cost >= target) {
+          slots + uslots[u] > slot_cap || cost >= target) {
         slab_lo.push_back(u);
-        rows = chunks = 0;
+        rows = chunks = slots = 0;
         cost = 0.0;
       }
       slab_of[u] = (int)slab_lo.size() - 1;
       rows += urows[u];
       chunks += cpu;
+      slots += uslots[u];
       cost += ucost[u];
     }
     n_slabs = (int64_t)slab_lo.size();

@@ -117,3 +117,24 @@ def test_split_chunks_scratch_is_bounded(gpu):
     finally:
         gpu.set_tuning()
         gpu.load().scatrs_release()
+
+
+def test_slot_elements_are_bounded(small_arena):
+    # 4,000 units of one phase level each at 2,048 cosines: 64 KiB of interpolated elements a unit, a
+    # quarter of the arena's bytes at a time.
+    gpu = small_arena
+    wl = np.linspace(0.5, 0.6, 4000)
+    d = W.lognormals([0.1], [1.3], 2)
+    m = np.full((1, 4000), 1.5 + 1e-2j)
+    mu = W.gauss_legendre(2048)
+
+    def call(sel=slice(None)):
+        return gpu.ensemble_fixed(d, wl[sel], m[:, sel], mu, 32)
+
+    phase = 6 * 4000 * 2048 * 8 / MIB
+    assert _used(gpu.load(), call) <= (FIXED + phase + 96) * MIB
+    got = call()
+    for u in (0, 255, 256, 3999):
+        one = call(slice(u, u + 1))
+        for a, b in zip(got[:2], one[:2]):
+            assert np.array_equal(a[:, u], b[:, 0])
