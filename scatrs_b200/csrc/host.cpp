@@ -208,6 +208,12 @@ struct BandTables {
   std::vector<double> mu;         // the cosines lp_d and lm_d interpolate onto
   DevBuf g_d, lg_d, d_d, desc_d, half0_d, x0_d, node_d, lp_d, lm_d;
   int merge_max() const { return n_levels > 0 ? desc[n_levels - 1].upper : 0; }
+  size_t bytes() const {
+    size_t sum = 0;
+    for (const DevBuf* b : {&g_d, &lg_d, &d_d, &desc_d, &half0_d, &x0_d, &node_d, &lp_d, &lm_d})
+      sum += b->cap;
+    return sum;
+  }
 };
 
 struct Context {
@@ -560,11 +566,13 @@ void grow_bands(Context& c, BandTables& bt, int L, int limit, int64_t n_max, cud
 // The tables for chunks of up to n_max terms and Greek order L (engine.rs:2034-2072): phase
 // levels up to `limit` tiles (0: none), projector bands for the chunks beyond them.
 BandTables& ensure_bands(Context& c, int L, int limit, int64_t n_max, cudaStream_t s) {
-  constexpr size_t kMaxLevelSets = 8;  // (Greek order, limit) pairs with levels kept
+  // (Greek order, limit) pairs with levels kept: 8, and 1 GiB together before another is added.
+  constexpr size_t kMaxLevelSets = 8, kLevelSetBytes = size_t(1) << 30;
   if (limit > 0 && !c.bands.count({L, limit})) {
-    size_t sets = 0;
-    for (auto& kv : c.bands) sets += kv.first.second > 0;
-    if (sets >= kMaxLevelSets)
+    size_t sets = 0, bytes = 0;
+    for (auto& kv : c.bands)
+      if (kv.first.second > 0) sets += 1, bytes += kv.second.bytes();
+    if (sets >= kMaxLevelSets || bytes > kLevelSetBytes)
       for (auto it = c.bands.begin(); it != c.bands.end();) {
         if (it->first.second > 0)
           it = c.bands.erase(it);

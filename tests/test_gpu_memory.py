@@ -138,3 +138,28 @@ def test_slot_elements_are_bounded(small_arena):
         one = call(slice(u, u + 1))
         for a, b in zip(got[:2], one[:2]):
             assert np.array_equal(a[:, u], b[:, 0])
+
+
+def test_kept_level_sets_are_bounded(small_arena):
+    # Greek orders in turn, each with its own phase levels (about 500 MiB at these cosines and sizes).
+    gpu = small_arena
+    lib = gpu.load()
+    wl, m = np.array([0.5]), np.array([[1.33 + 1e-4j]])
+    d = W.lognormals([900 * 0.5 / (2 * np.pi)], [1.02], 1)
+    mu = W.gauss_legendre(4096)
+
+    def call(order):
+        return gpu.ensemble_fixed(d, wl, m, mu, 32, order)
+
+    one = _used(lib, lambda: call(4))
+    assert one > 256 * MIB
+    want = call(6)
+
+    def several():
+        for order in range(4, 11):
+            call(order)
+
+    # Sets up to 1 GiB together, and the one that is added then.
+    assert _used(lib, several) <= one + (1024 + 64) * MIB + one
+    for a, b in zip(call(6), want):
+        assert np.array_equal(a, b)
