@@ -458,12 +458,13 @@ void grow_bands(Context& c, BandTables& bt, int L, int limit, int64_t n_max, cud
   int64_t reach = 0;
   for (int t = 1; t <= limit && reach < n_max; t = next_level_tiles(t), ++need_levels)
     reach = 32 * (int64_t)t - 1;
-  int need_bands = L >= 0 && n_max > reach ? band_index(n_max) + 1 : 0;
+  const int need_bands = L >= 0 && n_max > reach ? band_index(n_max) + 1 : 0;
   if (bt.n_levels >= need_levels && bt.n_bands >= need_bands) return;
-  // Built for half as many terms again (levels), a quarter (bands), so that slightly larger
-  // inputs find them ready.
-  if (need_bands > 0) need_bands += 1;
-  for (int64_t at = reach; reach < limit * 32 - 1 && reach < at + at / 2; ++need_levels) {
+  // Levels are built for half as many terms again, so that slightly larger inputs find them ready;
+  // to kSpareReach, as their host tables (a Gauss rule, the projection) grow with its square.
+  constexpr int64_t kSpareReach = 512;
+  for (int64_t at = reach;
+       reach < limit * 32 - 1 && reach < std::min(at + at / 2, kSpareReach); ++need_levels) {
     int t = 1;
     for (int l = 0; l < need_levels; ++l) t = next_level_tiles(t);
     reach = 32 * (int64_t)t - 1;

@@ -163,3 +163,25 @@ def test_kept_level_sets_are_bounded(small_arena):
     assert _used(lib, several) <= one + (1024 + 64) * MIB + one
     for a, b in zip(call(6), want):
         assert np.array_equal(a, b)
+
+
+def test_bands_are_built_for_the_call_alone(small_arena):
+    # No cosines, so projector bands alone: 4 n_q (L + 1) and 2 h ld doubles for each up to the
+    # largest chunk's (bands of 1.25 times the last one's terms).
+    gpu = small_arena
+    wl, m, order = np.array([0.5]), np.array([[1.33 + 1e-4j]]), 2000
+    x, n = 800.0, []
+    d = W.lognormals([x * wl[0] / (2 * np.pi)], [1.001], 1)
+    top = x * 1.001 + 6 * x ** (1 / 3) + 4
+    tables, u = 0, 1
+    while not n or n[-1] < top:
+        k = min(order, 2 * u)
+        n_q = u + (k + 2) // 2
+        tables += 4 * n_q * (k + 32) * 8 + (n_q + 64) * (u + 16) * 8
+        n.append(u)
+        u = -(-5 * u // 4)
+
+    def call():
+        return gpu.ensemble_fixed(d, wl, m, None, 32, order)
+
+    assert _used(gpu.load(), call) <= (FIXED + 64) * MIB + tables
