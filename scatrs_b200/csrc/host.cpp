@@ -337,7 +337,9 @@ const std::pair<std::vector<double>, std::vector<double>>& rule(Context& c, int6
   auto it = c.rules.find(n);
   if (it != c.rules.end()) return it->second;
   std::vector<double> x(n), w(n);
-  gauss_legendre(n, x.data(), w.data());
+  // On the host's threads: a new call's phase levels alone take up to tens of rules.
+#pragma omp parallel for schedule(dynamic, 8) if (n > 64)
+  for (int64_t i = 0; i < (n + 1) / 2; ++i) gauss_legendre_node(n, i, x.data(), w.data());
   return c.rules.emplace(n, std::make_pair(std::move(x), std::move(w))).first->second;
 }
 
@@ -441,14 +443,14 @@ void append_projection(const std::pair<std::vector<double>, std::vector<double>>
   const size_t off = d.size();
   const int64_t ld = round_up(len, 32);
   d.resize(off + 4 * (size_t)n_q * ld, 0.0);
-  std::vector<double> buf(len);
   const int mn[4][2] = {{0, 0}, {2, 2}, {2, -2}, {0, 2}};
-  for (int f = 0; f < 4; ++f)
-    for (int64_t k = 0; k < n_q; ++k) {
-      wigner_d(mn[f][0], mn[f][1], r.first[k], buf.data(), len);
-      double* dst = &d[off + ((size_t)f * n_q + k) * ld];
-      for (int64_t l = 0; l < len; ++l) dst[l] = (double)(2 * l + 1) * 0.5 * r.second[k] * buf[l];
-    }
+#pragma omp parallel for schedule(static) if (n_q * len > 4096)
+  for (int64_t i = 0; i < 4 * n_q; ++i) {
+    const int64_t f = i / n_q, k = i % n_q;
+    double* dst = &d[off + (size_t)i * ld];
+    wigner_d(mn[f][0], mn[f][1], r.first[k], dst, len);
+    for (int64_t l = 0; l < len; ++l) dst[l] = (double)(2 * l + 1) * 0.5 * r.second[k] * dst[l];
+  }
 }
 
 // Grows `bt` to chunks of up to n_max terms (ensure_bands); after a failure it is not usable.

@@ -9,7 +9,7 @@
 
 namespace sb {
 
-void gauss_legendre(int64_t n, double* nodes, double* weights) {
+void gauss_legendre_node(int64_t n, int64_t i, double* nodes, double* weights) {
   typedef long double ld;
   const double pi = 3.14159265358979323846264338327950288;
   // P_n and P_{n-1} at x by the three-term recurrence.
@@ -23,37 +23,39 @@ void gauss_legendre(int64_t n, double* nodes, double* weights) {
     *p = b;
     *pm = a;
   };
-  for (int64_t i = 0; i < (n + 1) / 2; ++i) {
-    ld x, s2, p, pm;
-    if (2 * i + 1 == n) {
-      x = 0.0L;
-      s2 = 1.0L;
-      legendre(x, &p, &pm);
-    } else {
-      // Tricomi's approximation of the (i+1)-th largest root (gauss_legendre.rs:128-137),
-      // then Newton on theta: theta += P_n(cos theta) / (sin theta P_n'(cos theta)).
-      double nf = (double)n, k = (double)(i + 1);
-      double th0 = pi * (4.0 * k - 1.0) / (4.0 * nf + 2.0);
-      ld th = acosl((ld)((1.0 - (nf - 1.0) / (8.0 * nf * nf * nf)) * std::cos(th0)));
-      for (int it = 0, small = 0; it < 100 && small < 2; ++it) {
-        ld c = cosl(th), s = sinl(th);
-        legendre(c, &p, &pm);
-        ld step = p * s / ((ld)n * (pm - c * p));
-        th += step;
-        if (std::fabs((double)step) <= 1e-17) ++small;
-      }
-      x = cosl(th);
-      ld s = sinl(th);
-      s2 = s * s;
-      legendre(x, &p, &pm);
+  ld x, s2, p, pm;
+  if (2 * i + 1 == n) {
+    x = 0.0L;
+    s2 = 1.0L;
+    legendre(x, &p, &pm);
+  } else {
+    // Tricomi's approximation of the (i+1)-th largest root (gauss_legendre.rs:128-137),
+    // then Newton on theta: theta += P_n(cos theta) / (sin theta P_n'(cos theta)).
+    double nf = (double)n, k = (double)(i + 1);
+    double th0 = pi * (4.0 * k - 1.0) / (4.0 * nf + 2.0);
+    ld th = acosl((ld)((1.0 - (nf - 1.0) / (8.0 * nf * nf * nf)) * std::cos(th0)));
+    for (int it = 0, small = 0; it < 100 && small < 2; ++it) {
+      ld c = cosl(th), s = sinl(th);
+      legendre(c, &p, &pm);
+      ld step = p * s / ((ld)n * (pm - c * p));
+      th += step;
+      if (std::fabs((double)step) <= 1e-17) ++small;
     }
-    ld dp = (ld)n * (pm - x * p) / s2;
-    ld w = 2.0L / (s2 * dp * dp);
-    nodes[n - 1 - i] = (double)x;
-    nodes[i] = 2 * i + 1 == n ? 0.0 : -(double)x;
-    weights[n - 1 - i] = (double)w;
-    weights[i] = (double)w;
+    x = cosl(th);
+    ld s = sinl(th);
+    s2 = s * s;
+    legendre(x, &p, &pm);
   }
+  ld dp = (ld)n * (pm - x * p) / s2;
+  ld w = 2.0L / (s2 * dp * dp);
+  nodes[n - 1 - i] = (double)x;
+  nodes[i] = 2 * i + 1 == n ? 0.0 : -(double)x;
+  weights[n - 1 - i] = (double)w;
+  weights[i] = (double)w;
+}
+
+void gauss_legendre(int64_t n, double* nodes, double* weights) {
+  for (int64_t i = 0; i < (n + 1) / 2; ++i) gauss_legendre_node(n, i, nodes, weights);
 }
 
 namespace {

@@ -13,6 +13,8 @@ namespace sb {
 // n-point Gauss-Legendre rule on [-1, 1], nodes ascending, exactly symmetric
 // (scatrs/src/special/gauss_legendre.rs:188-260).
 void gauss_legendre(int64_t n, double* nodes, double* weights);
+// Its (i + 1)-th largest node and that node's mirror, i < (n + 1) / 2.
+void gauss_legendre_node(int64_t n, int64_t i, double* nodes, double* weights);
 
 // d^l_{mn}(x) for l = 0..len-1 and |m|, |n| <= 2 (scatrs/src/special/wigner.rs:152-184).
 void wigner_d(int m, int n, double x, double* out, int64_t len);
