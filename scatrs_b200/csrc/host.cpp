@@ -768,14 +768,15 @@ void check_options(const scatrs_fixed_options* o, int64_t n_units, int64_t n_mu,
                   "the ensemble outputs would exceed 2 * MAX_MIE_VALUES = 268435456 real values"};
 }
 
-bool pinned_host(const void* p) {
+cudaMemoryType memory_type(const void* p) {
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return cudaMemoryTypeUnregistered;
   }
-  return at.type == cudaMemoryTypeHost;
+  return at.type;
 }
+bool pinned_host(const void* p) { return memory_type(p) == cudaMemoryTypeHost; }
 
 // A call's outputs to the caller, all of them there when it returns. Large ones to pageable memory
 // go through the pinned staging halves, a block's copy from the device beside the host threads'
@@ -790,7 +791,9 @@ void copy_out(Context& c, const std::vector<OutCopy>& outs, cudaMemcpyKind kind,
   constexpr int64_t kBlock = int64_t(2) << 20, kPiece = int64_t(64) << 10, kLeast = int64_t(256) << 10;
   std::vector<OutCopy> blocks;
   for (const OutCopy& o : outs) {
-    if (kind != cudaMemcpyDeviceToHost || o.bytes < kLeast || !o.dst || pinned_host(o.dst)) {
+    // Memory the runtime knows (pinned, managed, a device pointer passed by mistake) is its to copy.
+    if (kind != cudaMemcpyDeviceToHost || o.bytes < kLeast || !o.dst ||
+        memory_type(o.dst) != cudaMemoryTypeUnregistered) {
       SB_CUDA(cudaMemcpyAsync(o.dst, o.src, (size_t)o.bytes, kind, s));
       continue;
     }

@@ -42,3 +42,36 @@ def test_node_records_of_several_blocks(gpu):
     sub = {key: v[..., unit, :] if v.ndim == 3 else v[..., unit] for key, v in got.items()}
     few = _dists(*[specs[k] for k in part])
     _compare(sub, O.ensemble_adaptive(_odist(few), wl, m, mu=MU, greek_order=8))
+
+
+def test_managed_outputs(gpu):
+    # Memory that the runtime manages is left to its own copy, whatever the size.
+    import ctypes
+
+    from scatrs_b200._native import FixedOptions, _p
+
+    import torch
+
+    n, n_mu = 400, 64  # 1.2 MB of phase matrix
+    d, wl = W.lognormals(np.full(n, 0.1), 1.4, 2), np.array([0.6])
+    m, mu = np.full((n, 1), 1.4 + 0.01j), W.gauss_legendre(n_mu)
+    want = _native.ensemble_fixed(d, wl, m, mu, 8)[:2]
+    cudart = ctypes.CDLL(None if hasattr(ctypes.CDLL(None), "cudaMallocManaged") else
+                         next(p.split()[-1] for p in open("/proc/self/maps")
+                              if "libcudart" in p))
+    torch.cuda.init()
+    got = []
+    for a in want:
+        p = ctypes.c_void_p()
+        assert cudart.cudaMallocManaged(ctypes.byref(p), ctypes.c_size_t(a.nbytes), 1) == 0
+        got.append((p, np.ctypeslib.as_array((ctypes.c_double * a.size).from_address(p.value))))
+    err = ctypes.create_string_buffer(512)
+    opts = FixedOptions(8, -1, 1, 0)
+    st = gpu.load().scatrs_ensemble_fixed(
+        d.ctypes.data, n, _p(wl), 1, _p(m.view(np.float64).reshape(-1)), _p(mu), n_mu,
+        ctypes.byref(opts), ctypes.cast(got[0][0], ctypes.POINTER(ctypes.c_double)),
+        ctypes.cast(got[1][0], ctypes.POINTER(ctypes.c_double)), None, err, 512)
+    assert st == 0, err.value
+    for (p, a), b in zip(got, want):
+        assert np.array_equal(a, b.reshape(-1))
+        cudart.cudaFree(p)
