@@ -133,10 +133,11 @@ __global__ void __launch_bounds__(128) level_matrix_kernel(LevelMatrixArgs a) {
 // unit's slots in order), so the results do not depend on which slots share a tile.
 //
 // Bound by latency for a few units (a table's 4 to 100 stages of 8 nodes) and by the FP64 tensor
-// path for many. One tile per table, not one per unit over all its tables, keeps the stages few and
-// the tiles many: 96 units x 4096 cosines 2.54 -> 0.64 ms, 165 units x 181 cosines with
-// L = 50 299 -> 53 us (against one launch for the cosines over all of a unit's tables and
-// one for the coefficients of 32 slots with a lane per slot).
+// path for many (57 % at 96 units x 4096 cosines). One tile per table, not one per unit over all its
+// tables, keeps the stages few and the tiles many: 96 units x 4096 cosines 2.54 -> 0.94 ms, 165 units
+// x 181 cosines with L = 50 299 -> 55 us (against one launch for the cosines over all of a unit's
+// tables and one for the coefficients of 32 slots with a lane per slot); 0.64 ms and 53 us of them
+// with the values at +mu and -mu folded, which is not accurate (above).
 namespace {
 constexpr int IK = 8;    // nodes per stage
 constexpr int IG = kSlotGroup;

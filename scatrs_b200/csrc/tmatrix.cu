@@ -574,11 +574,11 @@ __global__ void __launch_bounds__(128) tm_forms_kernel(TmArgs a) {
 // magnitude sum is the smallest is kept: the magnitudes are summed first, in FP64, and only the
 // chosen form runs in double-double.
 //
-// One form instead of three (and no state for the others) halves the
-// operations and leaves the reads of the forms table (3 TB/s) as its bound: 196 -> 128 ms per pass
-// of 288 spheroids to x = 21 (3 blocks per SM without spills: the same). Rows of both parities of
-// i + k in a warp ran the two parities' code one after the other; one parity at a time: 128 -> 98 ms
-// (the table's rows ordered by parity too: no faster, and its writer slower).
+// Bound by the latency of its loads, the forms table's above all (9 of 13 cycles per issue; L1 43 %,
+// FP64 16 % busy). One form instead of three (and no state for the others) halves the operations:
+// 196 -> 128 ms per pass of 288 spheroids to x = 21 (3 blocks per SM without spills: the same). Rows of both
+// parities of i + k in a warp ran the two parities' code one after the other; one parity at a time:
+// 128 -> 98 ms (the table's rows ordered by parity too: no faster, and its writer slower).
 namespace {
 
 // One (mode, i, k): its rows of the tables and the half surface's sums.

@@ -472,8 +472,8 @@ __device__ __forceinline__ void unit_body(const UnitArgs& a) {
 // is owned by one thread of one work item and runs over the chunks in order, so the results do not
 // depend on how a unit's tiles are split into items.
 //
-// Bound by the FP64 tensor path: 30 TFLOP/s executed over a pass of 64 x 512 units of 512 nodes, 0.82
-// of its rate (100 ms; 105 with cp.async stages behind block barriers, which drained at every chunk).
+// Bound by the FP64 tensor path (71 to 76 % busy): the algorithmic operations of a pass of 64 x 512
+// units of 512 nodes at 29 TFLOP/s, 0.82 of the DGEMM rate (100 ms; 105 with cp.async stages behind block barriers, which drained at every chunk).
 // The derivative and adaptive forms ran on scalar FMAs with a 16-lane reduce-scatter per block of
 // sums: 1.10 -> 0.69 ms (768 units, 5 blocks) and 10.5 -> 5.9 ms (1024 units).
 __global__ void __launch_bounds__(NT, 3) unit_kernel(UnitArgs a) { unit_body<0, 1>(a); }
